@@ -35,6 +35,7 @@
 #include "../../include/cuflye.h"
 #include "kernels.h"
 #include "r2g.h"
+#include "runs.h"
 
 namespace cuflye {
 
@@ -79,8 +80,11 @@ struct cuflye_ctx {
   // logf exception table
   LogfTable logt{};
   size_t queries_per_pass = 0;
-  // timing
-  cudaEvent_t ev[8]{};
+  // stage clock: the events of the pass, each closing an interval of its stage
+  std::vector<cudaEvent_t> clock;
+  std::vector<int> clock_stage;
+  size_t marks = 0;
+  void* back = nullptr;  // page-locked host words for read backs
   // the segmented sort's side streams and its fork / rounds-done / join events
   cudaStream_t side = nullptr, side2 = nullptr;
   cudaEvent_t side_ev[4]{};
@@ -97,7 +101,10 @@ struct cuflye_ctx {
   int servers = 0;           // open serving loops and shared contexts borrowing this index
   cuflye_ctx* lender = nullptr;  // the context whose index this one borrows (cuflye_open_shared)
   int sorted_emission = 1;  // see cuflye_set_sorted_emission
-  double other_per_hit = 0;  // a pass body's buffers beyond the per-hit ones, per hit
+  // a pass body's buffers beyond the per-hit ones, per hit ([1]: beyond the
+  // per-run ones, per run, on the run path)
+  double other_per_hit[2] = {0, 0};
+  uint64_t runs_chained = 0, hits_in_runs = 0;  // of the last call, on the run path
   std::map<std::string, uint64_t> pass_need;  // bytes each buffer was asked for in this pass
   uint64_t pass_retries = 0;   // passes of the last call run again on half their queries
   uint64_t pass_hit_cap = 0;   // hits a pass may take after a retry in this call (0: no cap)
@@ -169,16 +176,55 @@ void sync(cuflye_ctx* c) { CUFLYE_CHECK(cudaStreamSynchronize(c->stream)); }
 
 template <typename T>
 T read_scalar(cuflye_ctx* c, const T* dev) {
-  T v;
-  CUFLYE_CHECK(cudaMemcpyAsync(&v, dev, sizeof(T), cudaMemcpyDeviceToHost, c->stream));
+  CUFLYE_CHECK(cudaMemcpyAsync(c->back, dev, sizeof(T), cudaMemcpyDeviceToHost, c->stream));
   sync(c);
-  return v;
+  return *static_cast<T*>(c->back);
 }
 
+// Several small read backs with one wait: queued into the context's
+// page-locked words, then (after read_all) at the returned places.
+constexpr size_t kBackBytes = 4096;
+struct ReadBack {
+  cuflye_ctx* c;
+  size_t used = 0;
+  template <typename T>
+  const T* add(const T* dev, size_t n = 1) {
+    used = (used + 15) / 16 * 16;
+    if (used + n * sizeof(T) > kBackBytes) throw Error(CUFLYE_ERR_CUDA, "read back too large");
+    void* h = static_cast<char*>(c->back) + used;
+    used += n * sizeof(T);
+    CUFLYE_CHECK(cudaMemcpyAsync(h, dev, n * sizeof(T), cudaMemcpyDeviceToHost, c->stream));
+    return static_cast<const T*>(h);
+  }
+  void read_all() { sync(c); }
+};
+
+// Stage clock: clock_start opens a pass, mark closes the interval since the
+// last event for `stage` (see cuflye_last_timing).
+void clock_event(cuflye_ctx* c, int stage) {
+  if (c->marks == c->clock.size()) {
+    cudaEvent_t e = nullptr;
+    CUFLYE_CHECK(cudaEventCreate(&e));
+    c->clock.push_back(e);
+    c->clock_stage.push_back(0);
+  }
+  c->clock_stage[c->marks] = stage;
+  CUFLYE_CHECK(cudaEventRecord(c->clock[c->marks], c->stream));
+  ++c->marks;
+}
+void clock_start(cuflye_ctx* c) {
+  c->marks = 0;
+  clock_event(c, 0);
+}
+void mark(cuflye_ctx* c, int stage) { clock_event(c, stage); }
+
+void raise_device_status(cuflye_ctx* c, const DeviceStatus& st);
+
 void check_device_status(cuflye_ctx* c) {
-  DeviceStatus st;
-  CUFLYE_CHECK(cudaMemcpyAsync(&st, c->status, sizeof(st), cudaMemcpyDeviceToHost, c->stream));
-  sync(c);
+  raise_device_status(c, read_scalar(c, c->status));
+}
+
+void raise_device_status(cuflye_ctx* c, const DeviceStatus& st) {
   if (st.code == kDevOk) return;
   CUFLYE_CHECK(cudaMemsetAsync(c->status, 0, sizeof(DeviceStatus), c->stream));
   switch (st.code) {
@@ -536,9 +582,46 @@ BuiltIndex build_key_ranges(cuflye_ctx* c, const WindowSet& w, const std::vector
   return bi;
 }
 
+// The run path's part of the index: the bases around every entry's k-mer, and
+// the packed targets it reads run lengths from.
+void drop_run_tables(cuflye_ctx* c) {
+  for (const char* t : {"ix_nbr", "ix_words", "ix_base"}) release(c, t);
+  c->idx.nbr = nullptr;
+  c->idx.twords = nullptr;
+  c->idx.tbase = nullptr;
+}
+
+// Kept for an odd k (an even k has k-mers that equal their reverse
+// complement) and while they take at most a quarter of the memory the index
+// leaves (1 byte an entry, 1/4 byte a base: beside the 8 bytes of an entry
+// and its share of the table they shorten a pass by a few per cent at most).
+void keep_run_tables(cuflye_ctx* c, const BuiltIndex& bi, int k, const int32_t* d_len) {
+  const uint64_t limit = effective_budget(c);
+  const uint64_t left = limit > c->in_use ? limit - c->in_use : 0;
+  if (k % 2 == 0 || bi.npos + 16 > left / 4) return;
+  try {
+    uint8_t* nbr = buf<uint8_t>(c, "ix_nbr", bi.npos + 32);
+    auto keep = [&](const char* from, const char* to) {
+      // the scratch buffer becomes part of the index
+      release(c, to);
+      c->bufs[to] = c->bufs[from];
+      c->bufs.erase(from);
+      return c->bufs[to].p;
+    };
+    c->idx.twords = static_cast<uint64_t*>(keep("ib_words", "ix_words"));
+    c->idx.tbase = static_cast<uint64_t*>(keep("ib_base", "ix_base"));
+    CUFLYE_CHECK(index_neighbours(bi.pos, bi.npos, c->idx.twords, c->idx.tbase, d_len, k, nbr,
+                                  c->stream));
+    c->idx.nbr = nbr;
+  } catch (const Error& e) {
+    if (e.code != CUFLYE_ERR_BUDGET) throw;
+    drop_run_tables(c);
+  }
+}
+
 void build_index(cuflye_ctx* c, int k, size_t n, const int64_t* ids, const int64_t* offsets,
                  const char* bases, uint32_t min_freq, uint32_t max_freq) {
-  c->other_per_hit = 0;  // a new workload: learned again
+  c->other_per_hit[0] = c->other_per_hit[1] = 0;  // a new workload: learned again
   if (k < 1 || k > 31) throw Error(CUFLYE_ERR_UNSUPPORTED, "k must be in [1, 31]");
   if (n == 0) throw Error(CUFLYE_ERR_INVALID, "index needs at least one target");
   if (max_freq >= (1u << kCountBits) - 1)
@@ -581,6 +664,7 @@ void build_index(cuflye_ctx* c, int k, size_t n, const int64_t* ids, const int64
   release(c, "ix_table");
   release(c, "ix_selfat");
   release(c, "ix_winoff");
+  drop_run_tables(c);
   c->idx.self_at = nullptr;
   c->idx.win_off = nullptr;
   // bases packed in chunks of 256 MiB (a multiple of 32 bases: chunks start on
@@ -636,6 +720,7 @@ void build_index(cuflye_ctx* c, int k, size_t n, const int64_t* ids, const int64
   }
   if (ranges) bi = build_key_ranges(c, ws, digits, min_freq, max_freq);
   release_build_scratch(c);
+  keep_run_tables(c, bi, k, d_len);
   for (const char* t : {"ib_words", "ib_base", "ib_win", "ib_bins"}) release(c, t);
   c->idx.k = k;
   c->idx.transform = true;
@@ -736,6 +821,7 @@ void build_index_entries(cuflye_ctx* c, int k, size_t n, const int64_t* tids, co
   c->idx.transform = false;
   release(c, "ix_selfat");
   release(c, "ix_winoff");
+  drop_run_tables(c);
   c->idx.self_at = nullptr;
   c->idx.win_off = nullptr;
   c->idx.table = table;
@@ -779,7 +865,17 @@ struct PassState {
   const uint64_t* wmeta = nullptr;
   const uint8_t* wflags = nullptr;
   const uint32_t* wself = nullptr;
-  uint64_t fit_hits = 0;  // the hits the memory left could hold when the pass was cut
+  // hits (runs on the run path) of the pass, and how many of them the memory
+  // left could hold when it was cut
+  uint64_t units = 0, fit_units = 0;
+  // run path: the pass's runs instead of hits; nhits counts those of its hits
+  // that the hit path chains
+  bool runs = false;
+  uint64_t run_hits = 0;
+  const uint32_t* cbits = nullptr;  // per 32 windows: the solid ones
+  std::vector<uint64_t> base_off_h, win_off_h;  // nq + 1
+  std::vector<int32_t> qdi_h;
+  std::vector<QueryInfo> qinfo_h;
 };
 
 // Buffers sized by the hit count of a pass (reused by the next pass).
@@ -789,6 +885,11 @@ const char* const kPerHitBuffers[] = {"h_keys",  "h_vals",   "h_kmers", "s_l",  
                                       "g_toff"};
 
 
+// Buffers sized by the run count of a pass on the run path.
+const char* const kPerRunBuffers[] = {"n_keys", "n_vals", "n_akeys", "n_avals", "n_rlen", "n_pa",
+                                      "n_pb",   "n_pl",   "n_ps",    "n_pk",    "n_po",   "n_pd",
+                                      "n_pm",   "m_tiles", "m_counts", "n_tcount", "n_toffg"};
+
 // The pass's hits in Flye's generation order (and the filtered positions).
 void emit_generation_order(cuflye_ctx* c, PassState& ps) {
   CUFLYE_CHECK(hits_emit(c->idx, ps.qb, ps.hit_off, ps.filt_off, ps.wmeta, ps.wflags, ps.keys,
@@ -796,9 +897,6 @@ void emit_generation_order(cuflye_ctx* c, PassState& ps) {
   ps.emitted = true;
 }
 
-// Upload a run of queries starting at q0 and produce the hits of the longest
-// prefix of them that fits in device memory (ps.nq queries), in Flye's
-// generation order.
 // Device bytes per query window of a pass's run: bases (1), packed words
 // (0.25), hit and filter counts (8), window metadata (8) and flags (1), the
 // two offset arrays (16), rounded up.
@@ -807,21 +905,31 @@ constexpr uint64_t kRunBytesPerWindow = 40;
 const char* const kPerWindowBuffers[] = {"q_ascii", "q_words",  "w_cnt",     "w_filt", "w_meta",
                                          "w_flags", "w_hitoff", "w_filtoff", "w_scan", "w_self"};
 
+// Bytes of the buffers that a pass of this kind reuses from the last one.
+uint64_t reusable_bytes(const cuflye_ctx* c, bool runs, bool windows) {
+  uint64_t bytes = 0;
+  auto held = [&](const char* name) {
+    auto it = c->bufs.find(name);
+    if (it != c->bufs.end()) bytes += it->second.cap;
+  };
+  if (windows)
+    for (const char* nm : kPerWindowBuffers) held(nm);
+  if (runs)
+    for (const char* nm : kPerRunBuffers) held(nm);
+  else
+    for (const char* nm : kPerHitBuffers) held(nm);
+  return bytes;
+}
+
 // The end of the run of queries from q0 (at most q1) whose windows' buffers
 // take at most a quarter of the memory the budget leaves; the rest is for
 // the run's hits.  With the hits per window of the call's previous pass
 // (hpw > 0), the run also stops about where its hits stop fitting, so that
 // few of its queries are counted again by the next pass.  At least one query.
 size_t run_end(cuflye_ctx* c, const Queries& Q, size_t q0, size_t q1, uint64_t bytes_per_hit,
-               double hpw) {
+               double hpw, bool runs) {
   const uint64_t limit = effective_budget(c);
-  uint64_t reusable = 0;
-  auto held = [&](const char* name) {
-    auto it = c->bufs.find(name);
-    if (it != c->bufs.end()) reusable += it->second.cap;
-  };
-  for (const char* nm : kPerWindowBuffers) held(nm);
-  for (const char* nm : kPerHitBuffers) held(nm);
+  const uint64_t reusable = reusable_bytes(c, runs, true);
   const uint64_t used = c->in_use > reusable ? c->in_use - reusable : 0;
   const uint64_t avail = limit > used ? limit - used : 0;
   uint64_t cap = avail / 4 / kRunBytesPerWindow;
@@ -843,6 +951,29 @@ size_t run_end(cuflye_ctx* c, const Queries& Q, size_t q0, size_t q1, uint64_t b
   return q;
 }
 
+// ps's queries (host vectors) as a device batch in one copy; ps.qb (but its
+// words) and ps.qinfo point into it.
+void upload_batch(cuflye_ctx* c, const char* name, PassState& ps) {
+  const size_t nq = ps.nq;
+  const size_t o_win = (nq + 1) * 8, o_info = o_win + (nq + 1) * 8,
+               o_qdi = o_info + nq * sizeof(QueryInfo), bytes = o_qdi + nq * 4;
+  std::vector<unsigned char> h(bytes);
+  std::memcpy(h.data(), ps.base_off_h.data(), (nq + 1) * 8);
+  std::memcpy(h.data() + o_win, ps.win_off_h.data(), (nq + 1) * 8);
+  if (nq) {
+    std::memcpy(h.data() + o_info, ps.qinfo_h.data(), nq * sizeof(QueryInfo));
+    std::memcpy(h.data() + o_qdi, ps.qdi_h.data(), nq * 4);
+  }
+  unsigned char* d = buf<unsigned char>(c, name, bytes);
+  CUFLYE_CHECK(cudaMemcpyAsync(d, h.data(), bytes, cudaMemcpyHostToDevice, c->stream));
+  ps.qb.base_off = reinterpret_cast<const uint64_t*>(d);
+  ps.qb.win_off = reinterpret_cast<const uint64_t*>(d + o_win);
+  ps.qb.qdi = reinterpret_cast<const int32_t*>(d + o_qdi);
+  ps.qb.nq = ps.nq;
+  ps.qb.nwin = ps.nwin;
+  ps.qinfo = reinterpret_cast<QueryInfo*>(d + o_info);
+}
+
 // Hits per window below which a pass takes the emit + sort path.
 constexpr uint64_t kSortedEmissionMinHitsPerWindow = 6;
 
@@ -853,16 +984,18 @@ bool sorted_emission(const cuflye_ctx* c, bool want_kmers) {
   return !want_kmers && c->idx.transform && c->sorted_emission != 0;
 }
 
-bool run_hits(cuflye_ctx* c, const Queries& Q, size_t q0, size_t q1, bool want_kmers,
-              uint64_t bytes_per_hit, PassState& ps) {
+// Uploads the queries [q0, q1): their bases packed, their offsets, ids and
+// lengths (one copy), also kept on the host in ps.
+void upload_queries(cuflye_ctx* c, const Queries& Q, size_t q0, size_t q1, PassState& ps) {
   const int k = c->idx.k;
   const uint32_t nq = static_cast<uint32_t>(q1 - q0);
   ps.nq = nq;
-  std::vector<uint64_t> base_off(nq + 1), win_off(nq + 1);
-  std::vector<int32_t> qdi(nq);
-  std::vector<QueryInfo> qinfo(nq);
-  base_off[0] = 0;
-  win_off[0] = 0;
+  std::vector<uint64_t>& base_off = ps.base_off_h;
+  std::vector<uint64_t>& win_off = ps.win_off_h;
+  base_off.assign(nq + 1, 0);
+  win_off.assign(nq + 1, 0);
+  ps.qdi_h.resize(nq);
+  ps.qinfo_h.resize(nq);
   for (uint32_t i = 0; i < nq; ++i) {
     const int64_t id = Q.ids[q0 + i];
     if (id == 0) throw Error(CUFLYE_ERR_INVALID, "query id must not be zero");
@@ -873,44 +1006,42 @@ bool run_hits(cuflye_ctx* c, const Queries& Q, size_t q0, size_t q1, bool want_k
     win_off[i + 1] = win_off[i] + (len >= k ? static_cast<uint64_t>(len - k + 1) : 0);
     const int64_t a = id < 0 ? -id : id;
     auto it = c->slot_of.find(a);
-    qdi[i] = it == c->slot_of.end() ? -1 : static_cast<int32_t>(2u * it->second + (id < 0 ? 1u : 0u));
-    qinfo[i] = QueryInfo{id, static_cast<int32_t>(len), 0};
+    ps.qdi_h[i] =
+        it == c->slot_of.end() ? -1 : static_cast<int32_t>(2u * it->second + (id < 0 ? 1u : 0u));
+    ps.qinfo_h[i] = QueryInfo{id, static_cast<int32_t>(len), 0};
   }
   const uint64_t nbases = base_off[nq];
-  const uint64_t nwin = win_off[nq];
-  ps.nwin = nwin;
+  ps.nwin = win_off[nq];
   cudaStream_t st = c->stream;
   uint8_t* d_ascii = buf<uint8_t>(c, "q_ascii", nbases + 16);
   if (nbases)
     CUFLYE_CHECK(cudaMemcpyAsync(d_ascii, Q.bases + Q.offsets[q0], nbases, cudaMemcpyHostToDevice,
                                  st));
   uint64_t* words = buf<uint64_t>(c, "q_words", (nbases + 31) / 32 + 2);
-  uint64_t* d_base = buf<uint64_t>(c, "q_base", nq + 1);
-  uint64_t* d_win = buf<uint64_t>(c, "q_win", nq + 1);
-  int32_t* d_qdi = buf<int32_t>(c, "q_qdi", nq);
-  ps.qinfo = buf<QueryInfo>(c, "q_info", nq);
-  CUFLYE_CHECK(cudaMemcpyAsync(d_base, base_off.data(), (nq + 1) * 8ull, cudaMemcpyHostToDevice, st));
-  CUFLYE_CHECK(cudaMemcpyAsync(d_win, win_off.data(), (nq + 1) * 8ull, cudaMemcpyHostToDevice, st));
-  CUFLYE_CHECK(cudaMemcpyAsync(d_qdi, qdi.data(), nq * 4ull, cudaMemcpyHostToDevice, st));
-  CUFLYE_CHECK(cudaMemcpyAsync(ps.qinfo, qinfo.data(), nq * sizeof(QueryInfo),
-                               cudaMemcpyHostToDevice, st));
+  upload_batch(c, "q_batch", ps);
+  ps.qb.words = words;
   // inputs are on the device from here on
-  CUFLYE_CHECK(cudaEventRecord(c->ev[5], st));
+  mark(c, 6);
   CUFLYE_CHECK(pack_bases(d_ascii, nbases, words, st));
-  QueryBatch qb;
-  qb.words = words;
-  qb.base_off = d_base;
-  qb.win_off = d_win;
-  qb.qdi = d_qdi;
-  qb.nq = nq;
-  qb.nwin = nwin;
+}
+
+// Counts and writes the hits of ps's queries (uploaded; ps.*_h and ps.qb hold
+// them) on the hit path: the longest prefix of them whose hits fit in device
+// memory stays in ps.  generation: in generation order whatever the pass.
+void run_hits(cuflye_ctx* c, PassState& ps, bool want_kmers, uint64_t bytes_per_hit,
+              bool generation = false) {
+  const uint32_t nq = ps.nq;
+  const uint64_t nwin = ps.nwin;
+  const std::vector<uint64_t>& win_off = ps.win_off_h;
+  cudaStream_t st = c->stream;
+  QueryBatch qb = ps.qb;
   uint32_t* cnt = buf<uint32_t>(c, "w_cnt", nwin);
   uint32_t* filt = buf<uint32_t>(c, "w_filt", nwin);
   uint64_t* wmeta = buf<uint64_t>(c, "w_meta", nwin);
   uint8_t* wflags = buf<uint8_t>(c, "w_flags", nwin);
   ps.q_tie = buf<uint32_t>(c, "q_tie", nq);
   CUFLYE_CHECK(cudaMemsetAsync(ps.q_tie, 0, std::max<uint64_t>(nq, 1) * 4ull, st));
-  const bool fused = sorted_emission(c, want_kmers);
+  const bool fused = !generation && sorted_emission(c, want_kmers);
   uint32_t* wself = fused ? buf<uint32_t>(c, "w_self", nwin) : nullptr;
   CUFLYE_CHECK(hits_count(c->idx, qb, cnt, filt, wmeta, wflags, ps.q_tie, wself, st));
   uint64_t* hit_off = buf<uint64_t>(c, "w_hitoff", nwin + 1);
@@ -919,17 +1050,12 @@ bool run_hits(cuflye_ctx* c, const Queries& Q, size_t q0, size_t q1, bool want_k
   ps.nfilt = scan_u32(c, filt, filt_off, nwin, "w_scan");
   ps.q_off = buf<uint64_t>(c, "q_hitoff", nq + 1);
   ps.f_off = buf<uint64_t>(c, "q_filtoff", nq + 1);
-  CUFLYE_CHECK(gather_query_offsets(d_win, hit_off, nq, ps.q_off, st));
-  CUFLYE_CHECK(gather_query_offsets(d_win, filt_off, nq, ps.f_off, st));
+  CUFLYE_CHECK(gather_query_offsets(qb.win_off, hit_off, nq, ps.q_off, st));
+  CUFLYE_CHECK(gather_query_offsets(qb.win_off, filt_off, nq, ps.f_off, st));
   // Keep the longest prefix of queries whose hits fit the memory left; the
   // per-hit buffers of an earlier pass are reused, so they count as free.
   const uint64_t limit = effective_budget(c);
-  uint64_t reusable = 0;
-  for (const char* nm : kPerHitBuffers) {
-    auto it = c->bufs.find(nm);
-    if (it != c->bufs.end()) reusable += it->second.cap;
-  }
-  const uint64_t used = c->in_use - reusable;
+  const uint64_t used = c->in_use - reusable_bytes(c, false, false);
   // under a caller's budget an eighth stays free for the pass body's other
   // buffers (row pool, rows, per-group tables); without one, the device's
   // own margin covers them
@@ -937,9 +1063,9 @@ bool run_hits(cuflye_ctx* c, const Queries& Q, size_t q0, size_t q1, bool want_k
   const uint64_t avail = c->budget ? free_b - free_b / 8 : free_b;
   // the pass body's other buffers, per hit, as earlier passes needed them
   const uint64_t fits = static_cast<uint64_t>(
-      static_cast<double>(avail) / (static_cast<double>(bytes_per_hit) + c->other_per_hit));
+      static_cast<double>(avail) / (static_cast<double>(bytes_per_hit) + c->other_per_hit[0]));
   uint64_t hit_limit = fits;
-  ps.fit_hits = fits;
+  ps.fit_units = fits;
   if (c->pass_hit_cap) hit_limit = std::min(hit_limit, c->pass_hit_cap);
   // Under a caller's budget a pass keeps to the per-hit buffers an earlier
   // pass grew when they hold at least 90 % of what fits: growing them frees
@@ -959,7 +1085,8 @@ bool run_hits(cuflye_ctx* c, const Queries& Q, size_t q0, size_t q1, bool want_k
     if (m == 0 && qoff[1] <= fits) m = 1;  // a first query beyond the held buffers
     if (m == 0)
       throw Error(CUFLYE_ERR_BUDGET,
-                  "device memory budget exceeded: query " + std::to_string(Q.ids[q0]) + " has " +
+                  "device memory budget exceeded: query " +
+                      std::to_string(ps.qinfo_h[0].signed_id) + " has " +
                       std::to_string(qoff[1]) + " hits needing " +
                       std::to_string(qoff[1] * bytes_per_hit) + " bytes; " +
                       std::to_string(avail) + " available");
@@ -968,11 +1095,9 @@ bool run_hits(cuflye_ctx* c, const Queries& Q, size_t q0, size_t q1, bool want_k
     ps.nwin = win_off[m];
     qb.nq = m;
     qb.nwin = win_off[m];
-    uint64_t fo = 0;
-    CUFLYE_CHECK(cudaMemcpyAsync(&fo, ps.f_off + m, 8, cudaMemcpyDeviceToHost, st));
-    sync(c);
-    ps.nfilt = fo;
+    ps.nfilt = read_scalar(c, ps.f_off + m);
   }
+  ps.units = ps.nhits;
   ps.keys = buf<uint64_t>(c, "h_keys", ps.nhits);
   ps.vals = buf<uint32_t>(c, "h_vals", ps.nhits);
   ps.kmers = want_kmers ? buf<uint64_t>(c, "h_kmers", ps.nhits) : nullptr;
@@ -994,7 +1119,96 @@ bool run_hits(cuflye_ctx* c, const Queries& Q, size_t q0, size_t q1, bool want_k
                             ps.nq >= 2ull * static_cast<uint64_t>(c->num_sms) &&
                             c->emission_fallbacks < 2)));
   if (ps.emitted) emit_generation_order(c, ps);
-  return true;
+}
+
+// Whether calls with these parameters take the run path (runs.cu): the index
+// holds its tables, and a hit one base after another in both positions always
+// follows it in Flye's DP.  cuflye_set_sorted_emission modes 0 and 2 ask for a
+// hit path.
+bool run_path(const cuflye_ctx* c, const ChainParams& cp) {
+  return c->idx.nbr && c->sorted_emission == 1 && cp.k >= 2 && cp.max_jump >= 2 &&
+         cp.max_gap >= 0;
+}
+
+// Device bytes per run: sorted pairs and their second buffer (24), length
+// (4), pieces with score, link and walk state (40 and half as much for cut
+// ones), and about as much for the per-group tables.
+constexpr uint64_t kRunBytes = 128;
+
+// Counts ps's run starts (queries uploaded): the longest prefix of the queries
+// whose runs fit in device memory stays in ps, sorted out but not written.
+void run_runs(cuflye_ctx* c, PassState& ps) {
+  const uint32_t nq = ps.nq;
+  const uint64_t nwin = ps.nwin, nt = (nwin + 31) / 32;
+  cudaStream_t st = c->stream;
+  ps.runs = true;
+  uint64_t* wmeta = buf<uint64_t>(c, "w_meta", nwin);
+  uint8_t* wflags = buf<uint8_t>(c, "w_flags", nwin);
+  uint32_t* wself = buf<uint32_t>(c, "w_self", nwin);
+  uint32_t* nstart = buf<uint32_t>(c, "w_cnt", nwin);
+  uint32_t* cbits = buf<uint32_t>(c, "n_cbits", nt + 2);
+  uint32_t* fbits = buf<uint32_t>(c, "n_fbits", nt);
+  uint32_t* tfilt = buf<uint32_t>(c, "n_tfilt", nt);
+  uint32_t* tstart = buf<uint32_t>(c, "n_tstart", nt);
+  uint64_t* tile_off = buf<uint64_t>(c, "n_toff", nt + 1);
+  uint64_t* ftile_off = buf<uint64_t>(c, "n_ftoff", nt + 1);
+  unsigned long long* total = buf<unsigned long long>(c, "n_total", 64);
+  CUFLYE_CHECK(cudaMemsetAsync(total, 0, 64 * sizeof(unsigned long long), st));
+  CUFLYE_CHECK(runs_probe(c->idx, ps.qb, wmeta, wflags, wself, cbits, fbits, tfilt, total, st));
+  CUFLYE_CHECK(runs_count(c->idx, ps.qb, wmeta, wflags, wself, nstart, tstart, st));
+  scan_u32_async(c, tstart, tile_off, nt, "n_scan");
+  scan_u32_async(c, tfilt, ftile_off, nt, "n_scan2");
+  ps.q_off = buf<uint64_t>(c, "n_qoff", nq + 1);
+  ps.f_off = buf<uint64_t>(c, "n_foff", nq + 1);
+  CUFLYE_CHECK(runs_query_offsets(ps.qb, nstart, tile_off, fbits, ftile_off, ps.q_off, ps.f_off,
+                                  st));
+  ReadBack rb{c};
+  const uint64_t* nr = rb.add(tile_off + nt);
+  const uint64_t* nf = rb.add(ftile_off + nt);
+  const unsigned long long* nh = rb.add(total, 64);
+  rb.read_all();
+  uint64_t hits = 0;
+  for (int i = 0; i < 64; ++i) hits += nh[i];
+  ps.units = *nr;
+  ps.nfilt = *nf;
+  const uint64_t limit = effective_budget(c);
+  const uint64_t used = c->in_use - reusable_bytes(c, true, false);
+  const uint64_t free_b = limit > used ? limit - used : 0;
+  const uint64_t avail = c->budget ? free_b - free_b / 8 : free_b;
+  uint64_t fits = static_cast<uint64_t>(
+      static_cast<double>(avail) / (static_cast<double>(kRunBytes) + c->other_per_hit[1]));
+  fits = std::min<uint64_t>(fits, 0xf0000000ull);  // group numbers are 32 bits
+  ps.fit_units = fits;
+  uint64_t run_limit = fits;
+  if (c->pass_hit_cap) run_limit = std::min(run_limit, c->pass_hit_cap);
+  if (ps.units > run_limit) {
+    std::vector<uint64_t> qoff(nq + 1);
+    CUFLYE_CHECK(cudaMemcpyAsync(qoff.data(), ps.q_off, (nq + 1) * 8ull, cudaMemcpyDeviceToHost,
+                                 st));
+    sync(c);
+    uint32_t m = 0;
+    while (m < nq && qoff[m + 1] <= run_limit) ++m;
+    if (m == 0 && qoff[1] <= fits) m = 1;
+    if (m == 0) {
+      ps.nq = 1;
+      throw Error(CUFLYE_ERR_BUDGET, "device memory budget exceeded: a query's runs");
+    }
+    hits = static_cast<uint64_t>(static_cast<double>(hits) * static_cast<double>(qoff[m]) /
+                                 static_cast<double>(ps.units));
+    ps.nq = m;
+    ps.units = qoff[m];
+    ps.nwin = ps.win_off_h[m];
+    ps.qb.nq = m;
+    ps.qb.nwin = ps.nwin;
+    ps.nfilt = read_scalar(c, ps.f_off + m);
+  }
+  ps.run_hits = hits;
+  ps.keys = buf<uint64_t>(c, "n_keys", ps.units);
+  ps.vals = buf<uint32_t>(c, "n_vals", ps.units);
+  ps.fpos = buf<int32_t>(c, "n_fpos", ps.nfilt);
+  CUFLYE_CHECK(runs_emit(c->idx, ps.qb, wmeta, wflags, wself, nstart, tile_off, fbits, ftile_off,
+                         ps.keys, ps.vals, ps.fpos, st));
+  ps.cbits = cbits;
 }
 
 ChainParams to_chain_params(const cuflye_overlap_params* p) {
@@ -1157,10 +1371,33 @@ void flagged_sort(cuflye_ctx* c, PassState& ps, const MatchEmitLists& L, uint64_
                                   st));
 }
 
-// Sort + chaining of the pass's hits; returns the number of overlap rows left
-// on the device in "o_rows" (OverlapRow, query order, Flye emission order).
-uint64_t run_chain(cuflye_ctx* c, PassState& ps, const ChainParams& cp,
-                   uint64_t* rows_per_query = nullptr) {
+// Overlap rows on the device, in query order and Flye's emission order, and
+// each query's first row (nq + 1).
+struct ChainRows {
+  uint64_t n = 0;
+  OverlapRow* rows = nullptr;
+  const uint64_t* q_row = nullptr;
+};
+
+// Rows of chained groups before their compaction: pool rows, and rows per group.
+struct GroupRows {
+  OverlapRow* pool = nullptr;
+  uint32_t* pool_count = nullptr;
+  uint64_t pool_cap = 0;
+  uint32_t* rows = nullptr;
+};
+
+// Chains groups of hits: the surviving groups in dp_list (counts[1]), those
+// of them sorted by ext pos in ext_list (counts[0]), the hits of group g at
+// groups[g].start in KmerMatch order.
+GroupRows chain_groups(cuflye_ctx* c, uint64_t* keys, uint32_t* vals, uint64_t H,
+                       GroupInfo* groups, uint64_t G, const uint32_t* ext_list,
+                       const uint32_t* dp_list, const uint32_t* gcounts, const ChainParams& cp,
+                       const QueryInfo* qinfo, const uint64_t* f_off, const int32_t* fpos,
+                       uint64_t* sstats, bool tally_pending);
+
+// Sort + chaining of the pass's hits.
+ChainRows chain_hits(cuflye_ctx* c, PassState& ps, const ChainParams& cp) {
   cudaStream_t st = c->stream;
   const uint64_t H = ps.nhits;
   const uint32_t nq = ps.nq;
@@ -1170,7 +1407,6 @@ uint64_t run_chain(cuflye_ctx* c, PassState& ps, const ChainParams& cp,
   uint32_t* scounts = buf<uint32_t>(c, "s_counts", 16);
   uint32_t* ecount = buf<uint32_t>(c, "s_ecount", 1);
   uint64_t* sstats = buf<uint64_t>(c, "x_sortstats", kSortStats);
-  CUFLYE_CHECK(cudaMemsetAsync(sstats, 0, kSortStats * 8, st));
   uint64_t* qb = buf<uint64_t>(c, "s_qb", nq);
   uint64_t* qe = buf<uint64_t>(c, "s_qe", nq);
   // second buffer of the radix passes (or the sorted emission's dictionary);
@@ -1238,11 +1474,11 @@ uint64_t run_chain(cuflye_ctx* c, PassState& ps, const ChainParams& cp,
       CUFLYE_CHECK(cudaMemsetAsync(L.tie_count, 0, sizeof(uint32_t), st));
       CUFLYE_CHECK(match_emit(a, alt_keys, q_ng, q_dbase, q_goff, ps.q_tie, ps.qinfo, cp, ps.keys,
                               ps.vals, groups, L, mwords + 1, c->num_sms, st));
-      CUFLYE_CHECK(cudaEventRecord(c->ev[1], st));
+      mark(c, 0);
       // 1. the flagged queries' KmerMatch sort in libstdc++ order
       CUFLYE_CHECK(sort_stats_add(sstats, 0, 1, nullptr, nq, ecount, st));
       flagged_sort(c, ps, L, qb, qe, ecount, alt_keys, alt_vals, lscr, rscr, lists, scounts);
-      CUFLYE_CHECK(cudaEventRecord(c->ev[2], st));
+      mark(c, 1);
       // 2. the prefilter of the groups the emission left open
       CUFLYE_CHECK(groups_prefilter_list(ps.keys, ps.vals, groups, pf_list, ps.qinfo, slot_len, cp,
                                          ext_list, dp_list, gcounts, static_cast<uint32_t>(G),
@@ -1262,7 +1498,7 @@ uint64_t run_chain(cuflye_ctx* c, PassState& ps, const ChainParams& cp,
     uint64_t* tile_off = buf<uint64_t>(c, "m_tileoff", nq + 1);
     int id_bits = 0;
     while (id_bits < 32 && ((2ull * c->idx.nslots - 1) >> id_bits) != 0) ++id_bits;
-    CUFLYE_CHECK(cudaEventRecord(c->ev[1], st));
+    mark(c, 0);
     CUFLYE_CHECK(match_plan(ps.q_off, ps.q_tie, nq, ntiles, qb, qe, ecount, st));
     CUFLYE_CHECK(sort_stats_add(sstats, 0, 1, nullptr, nq, ecount, st));
     const uint64_t NT = scan_u32(c, ntiles, tile_off, nq, "m_scan");
@@ -1274,7 +1510,7 @@ uint64_t run_chain(cuflye_ctx* c, PassState& ps, const ChainParams& cp,
                              mcounts, c->num_sms, c->shape.scatter_blocks_per_sm, st));
     CUFLYE_CHECK(segmented_std_sort(ps.keys, ps.vals, lscr, rscr, qb, qe, nq, ecount, lists,
                                     scounts, c->num_sms, st, sort_tasks(c, "s", H, nq)));
-    CUFLYE_CHECK(cudaEventRecord(c->ev[2], st));
+    mark(c, 1);
     // 2. groups: runs of one ext id within a query
     const uint64_t gtiles = (H + kGroupTile - 1) / kGroupTile;
     uint32_t* gtcount = buf<uint32_t>(c, "g_tcount", gtiles);
@@ -1290,6 +1526,48 @@ uint64_t run_chain(cuflye_ctx* c, PassState& ps, const ChainParams& cp,
                                     ext_list, dp_list, gcounts, st));
     c->hits_emit_sort += H;
   }
+  const GroupRows gr = chain_groups(c, ps.keys, ps.vals, H, groups, G, ext_list, dp_list, gcounts,
+                                    cp, ps.qinfo, ps.f_off, ps.fpos, sstats, tally_pending);
+  check_device_status(c);
+  // 7. max_overlaps + compaction in group order
+  uint64_t* qg = buf<uint64_t>(c, "o_qg", nq + 1);
+  CUFLYE_CHECK(query_group_offsets(groups, G, nq, qg, st));
+  uint32_t* kept = gr.rows;
+  if (cp.max_overlaps > 0) {
+    kept = buf<uint32_t>(c, "o_kept", G);
+    CUFLYE_CHECK(rows_limit(gr.rows, qg, nq, cp.max_overlaps, kept, st));
+  }
+  uint64_t* kept_off = buf<uint64_t>(c, "o_keptoff", G + 1);
+  scan_u32_async(c, kept, kept_off, G, "o_scan");
+  ReadBack rb{c};
+  const uint64_t* R = rb.add(kept_off + G);
+  const uint32_t* npool = rb.add(gr.pool_count);
+  rb.read_all();
+  ChainRows out;
+  out.n = *R;
+  const uint32_t np = *npool;
+  out.rows = buf<OverlapRow>(c, "o_rows", out.n);
+  CUFLYE_CHECK(rows_scatter(gr.pool, np, kept, kept_off, out.rows, st));
+  // each query's first row (rows are in query order)
+  uint64_t* q_row = buf<uint64_t>(c, "o_qrowoff", nq + 1);
+  CUFLYE_CHECK(gather_query_offsets(qg, kept_off, nq, q_row, st));
+  out.q_row = q_row;
+  mark(c, 4);
+  return out;
+}
+
+GroupRows chain_groups(cuflye_ctx* c, uint64_t* keys, uint32_t* vals, uint64_t H,
+                       GroupInfo* groups, uint64_t G, const uint32_t* ext_list,
+                       const uint32_t* dp_list, const uint32_t* gcounts, const ChainParams& cp,
+                       const QueryInfo* qinfo, const uint64_t* f_off, const int32_t* fpos,
+                       uint64_t* sstats, bool tally_pending) {
+  cudaStream_t st = c->stream;
+  uint32_t* lscr = buf<uint32_t>(c, "s_l", H + 1);
+  uint32_t* rscr = buf<uint32_t>(c, "s_r", H + 1);
+  uint32_t* scounts = buf<uint32_t>(c, "s_counts", 16);
+  uint32_t* ecount = buf<uint32_t>(c, "s_ecount", 1);
+  uint64_t* alt_keys = buf<uint64_t>(c, "c_akeys", H + 1);
+  uint32_t* alt_vals = buf<uint32_t>(c, "c_avals", H + 1);
   uint64_t* sb = buf<uint64_t>(c, "g_sb", G);
   uint64_t* se = buf<uint64_t>(c, "g_se", G);
   uint32_t* glists = buf<uint32_t>(c, "g_lists", 4 * std::max<uint64_t>(G, 1));
@@ -1300,12 +1578,12 @@ uint64_t run_chain(cuflye_ctx* c, PassState& ps, const ChainParams& cp,
   uint32_t* work = buf<uint32_t>(c, "c_work", 1);
   uint32_t* resort = buf<uint32_t>(c, "g_resort", G);
   uint32_t* resort_count = buf<uint32_t>(c, "g_resortcount", 1);
-  CUFLYE_CHECK(groups_ext_presorted(ps.vals, groups, ext_list, gcounts, resort, resort_count, st));
-  CUFLYE_CHECK(group_ext_sort(ps.keys, ps.vals, groups, resort, resort_count, G32, sb, se, ecount,
+  CUFLYE_CHECK(groups_ext_presorted(vals, groups, ext_list, gcounts, resort, resort_count, st));
+  CUFLYE_CHECK(group_ext_sort(keys, vals, groups, resort, resort_count, G32, sb, se, ecount,
                               lscr, rscr, reinterpret_cast<uint32_t*>(alt_keys), H, work,
                               c->num_sms, st));
   CUFLYE_CHECK(sort_stats_add(sstats, 2, 3, gcounts + 0, 0, ecount, st));
-  CUFLYE_CHECK(segmented_std_sort(ps.keys, ps.vals, lscr, rscr, sb, se, G32, ecount, glists,
+  CUFLYE_CHECK(segmented_std_sort(keys, vals, lscr, rscr, sb, se, G32, ecount, glists,
                                   scounts, c->num_sms, st, sort_tasks(c, "s", H, G32)));
   // 4. DP over the sorted pairs
   int32_t* score = buf<int32_t>(c, "c_score", H);
@@ -1316,11 +1594,11 @@ uint64_t run_chain(cuflye_ctx* c, PassState& ps, const ChainParams& cp,
   uint32_t* blist = buf<uint32_t>(c, "g_lenlist", G);
   CUFLYE_CHECK(groups_length_order(groups, dp_list, gcounts + 1, G32,
                                    buf<uint32_t>(c, "g_lenscr", 10), blist, st));
-  CUFLYE_CHECK(cudaEventRecord(c->ev[6], st));
+  mark(c, 2);
   int32_t* pmc = buf<int32_t>(c, "c_pmc", chain_dp_pmc_words(H, G));
-  CUFLYE_CHECK(chain_dp(ps.keys, ps.vals, score, bt, groups, blist, gcounts, cp, top, pmc, work,
+  CUFLYE_CHECK(chain_dp(keys, vals, score, bt, groups, blist, gcounts, cp, top, pmc, work,
                         c->num_sms, c->shape.dp_blocks_per_sm, st));
-  CUFLYE_CHECK(cudaEventRecord(c->ev[7], st));
+  mark(c, 3);
   // 5. the backtrack picks its chain starts by score itself; groups where
   // Flye's order among equal scores could matter get that order (libstdc++
   // order of indices by score descending) and run again.  The (key, index)
@@ -1346,8 +1624,8 @@ uint64_t run_chain(cuflye_ctx* c, PassState& ps, const ChainParams& cp,
   uint32_t* redo_count = buf<uint32_t>(c, "o_redocount", 1);
   CUFLYE_CHECK(cudaMemsetAsync(redo_count, 0, 4, st));
   const int64_t* slot_signed = c->idx.slot_signed;
-  CUFLYE_CHECK(chain_backtrack(ps.keys, ps.vals, score, bt, order, groups, blist, gcounts + 1, top,
-                               redo, redo_count, ps.qinfo, ps.f_off, ps.fpos, slot_signed, c->logt,
+  CUFLYE_CHECK(chain_backtrack(keys, vals, score, bt, order, groups, blist, gcounts + 1, top,
+                               redo, redo_count, qinfo, f_off, fpos, slot_signed, c->logt,
                                cp, pool, pool_cap, pool_count, group_rows, c->status, G32, gmaps,
                                gmap_words, work, c->shape.backtrack_blocks_per_sm, st));
   CUFLYE_CHECK(sort_stats_add(sstats, 4, 6, gcounts + 1, 0, redo_count, st));
@@ -1356,35 +1634,357 @@ uint64_t run_chain(cuflye_ctx* c, PassState& ps, const ChainParams& cp,
   CUFLYE_CHECK(chain_prepare_order(score, okeys, order, groups, redo, redo_count, sb, se, st));
   CUFLYE_CHECK(segmented_std_sort(okeys, order, lscr, rscr, sb, se, G32, redo_count, glists,
                                   scounts, c->num_sms, st, sort_tasks(c, "s", H, G32)));
-  CUFLYE_CHECK(chain_backtrack(ps.keys, ps.vals, score, bt, order, groups, redo, redo_count, nullptr,
-                               nullptr, nullptr, ps.qinfo, ps.f_off, ps.fpos, slot_signed, c->logt,
+  CUFLYE_CHECK(chain_backtrack(keys, vals, score, bt, order, groups, redo, redo_count, nullptr,
+                               nullptr, nullptr, qinfo, f_off, fpos, slot_signed, c->logt,
                                cp, pool, pool_cap, pool_count, group_rows, c->status, G32, gmaps,
                                gmap_words, work, c->shape.backtrack_blocks_per_sm, st));
-  check_device_status(c);
-  // 7. max_overlaps + compaction in group order
-  uint64_t* qg = buf<uint64_t>(c, "o_qg", nq + 1);
-  CUFLYE_CHECK(query_group_offsets(groups, G, nq, qg, st));
-  uint32_t* kept = buf<uint32_t>(c, "o_kept", G);
-  if (cp.max_overlaps > 0) {
-    CUFLYE_CHECK(rows_limit(group_rows, qg, nq, cp.max_overlaps, kept, st));
-  } else {
-    kept = group_rows;
+  return GroupRows{pool, pool_count, pool_cap, group_rows};
+}
+
+uint64_t* upload(cuflye_ctx* c, const char* name, const std::vector<uint64_t>& v) {
+  uint64_t* d = buf<uint64_t>(c, name, v.size());
+  CUFLYE_CHECK(cudaMemcpyAsync(d, v.data(), v.size() * 8ull, cudaMemcpyHostToDevice, c->stream));
+  return d;
+}
+
+// Device bytes per hit of one pass: keys, values, the two rank maps, the
+// radix sort's second key / value buffer, score and backtrack, plus about 2
+// bytes for the per-group tables, tiles, bitmaps and the sort's task list.
+constexpr uint64_t kChainBytesPerHit = 8 + 4 + 4 + 4 + 8 + 4 + 4 + 4 + 2;
+
+// Hits of sp (generation order, sp.keys / sp.vals) in KmerMatch order, exact
+// among the equal keys listed as (query of sp, key): a stable radix sort by ext
+// id, and libstdc++'s introsort emulated on a copy over the ranges that may
+// hold listed keys, which replace the radix sort's (see flagged_sort).  Hits
+// with other equal keys may come out wrong: nothing reads them.
+void sort_listed_ties(cuflye_ctx* c, PassState& sp, std::vector<std::pair<uint32_t, uint64_t>> ties) {
+  cudaStream_t st = c->stream;
+  const uint64_t H = sp.nhits;
+  const uint32_t nq = sp.nq;
+  uint32_t* lscr = buf<uint32_t>(c, "s_l", H + 1);
+  uint32_t* rscr = buf<uint32_t>(c, "s_r", H + 1);
+  uint32_t* lists = buf<uint32_t>(c, "s_lists", 4ull * std::max<uint64_t>(nq, 1));
+  uint32_t* scounts = buf<uint32_t>(c, "s_counts", 16);
+  const uint64_t* qb = sp.q_off;
+  if (ties.size() * 64u > H) {
+    // equal keys everywhere: the pruning would keep most ranges
+    CUFLYE_CHECK(segmented_std_sort(sp.keys, sp.vals, lscr, rscr, qb, qb + 1, nq, nullptr, lists,
+                                    scounts, c->num_sms, st, sort_tasks(c, "s", H, nq)));
+    return;
   }
-  uint64_t* kept_off = buf<uint64_t>(c, "o_keptoff", G + 1);
-  const uint64_t R = scan_u32(c, kept, kept_off, G, "o_scan");
-  const uint32_t npool = read_scalar(c, pool_count);
-  OverlapRow* rows = buf<OverlapRow>(c, "o_rows", R);
-  CUFLYE_CHECK(rows_scatter(pool, npool, kept, kept_off, rows, st));
-  // each query's first row (rows are in query order)
-  CUFLYE_CHECK(gather_query_offsets(qg, kept_off, nq, buf<uint64_t>(c, "o_qrowoff", nq + 1), st));
-  if (rows_per_query) {
-    uint64_t* qrows = buf<uint64_t>(c, "o_qrows", nq);
-    CUFLYE_CHECK(query_row_counts(qg, kept_off, nq, qrows, st));
-    CUFLYE_CHECK(cudaMemcpyAsync(rows_per_query, qrows, nq * sizeof(uint64_t),
-                                 cudaMemcpyDeviceToHost, st));
+  std::sort(ties.begin(), ties.end());
+  ties.erase(std::unique(ties.begin(), ties.end()), ties.end());
+  std::vector<uint32_t> poff(nq + 1, 0);
+  std::vector<uint64_t> pkeys;
+  for (const auto& t : ties) {
+    ++poff[t.first + 1];
+    pkeys.push_back(t.second);
   }
-  CUFLYE_CHECK(cudaEventRecord(c->ev[3], st));
-  return R;
+  for (uint32_t i = 0; i < nq; ++i) poff[i + 1] += poff[i];
+  uint32_t* dpoff = buf<uint32_t>(c, "f_poff", nq + 1);
+  CUFLYE_CHECK(cudaMemcpyAsync(dpoff, poff.data(), poff.size() * 4ull, cudaMemcpyHostToDevice, st));
+  uint64_t* dpkeys = upload(c, "f_pkeys", pkeys);
+  uint64_t* gk = buf<uint64_t>(c, "f_gk", H);
+  uint32_t* gv = buf<uint32_t>(c, "f_gv", H);
+  uint64_t* alt_keys = buf<uint64_t>(c, "c_akeys", H + 1);
+  uint32_t* alt_vals = buf<uint32_t>(c, "c_avals", H + 1);
+  uint32_t* ntiles = buf<uint32_t>(c, "m_ntiles", nq);
+  uint64_t* tile_off = buf<uint64_t>(c, "m_tileoff", nq + 1);
+  int id_bits = 0;
+  while (id_bits < 32 && ((2ull * c->idx.nslots - 1) >> id_bits) != 0) ++id_bits;
+  CUFLYE_CHECK(match_plan(qb, nullptr, nq, ntiles, nullptr, nullptr, nullptr, st, true));
+  const uint64_t NT = scan_u32(c, ntiles, tile_off, nq, "m_scan");
+  MatchTile* tiles = buf<MatchTile>(c, "m_tiles", NT);
+  uint32_t* mcounts = buf<uint32_t>(c, "m_counts", 256 * NT);
+  CUFLYE_CHECK(match_tiles(qb, ntiles, tile_off, nq, tiles, st));
+  SortTasks t = sort_tasks(c, "f", H, nq);
+  t.prune_keys = dpkeys;
+  t.prune_off = dpoff;
+  CUFLYE_CHECK(cudaMemcpyAsync(gk, sp.keys, H * 8, cudaMemcpyDeviceToDevice, st));
+  CUFLYE_CHECK(cudaMemcpyAsync(gv, sp.vals, H * 4, cudaMemcpyDeviceToDevice, st));
+  // the radix sort on the side stream beside the emulation, every buffer
+  // allocated before the fork (see flagged_sort)
+  CUFLYE_CHECK(cudaEventRecord(c->side_ev[0], st));
+  CUFLYE_CHECK(cudaStreamWaitEvent(c->side, c->side_ev[0], 0));
+  CUFLYE_CHECK(match_radix(sp.keys, sp.vals, alt_keys, alt_vals, tiles, static_cast<uint32_t>(NT),
+                           qb, ntiles, tile_off, nq, id_bits, mcounts, c->num_sms,
+                           c->shape.scatter_blocks_per_sm, c->side));
+  CUFLYE_CHECK(segmented_std_sort(gk, gv, lscr, rscr, qb, qb + 1, nq, nullptr, lists, scounts,
+                                  c->num_sms, st, t));
+  CUFLYE_CHECK(copy_sorted_ranges(gk, gv, qb, qb + 1, qb, nq, scounts, t, sp.keys, sp.vals,
+                                  c->num_sms, st));
+}
+
+// The open groups through the hit path's chaining; their rows join the pool.
+// Groups that repeat a cur position take their hits from their query's sorted
+// hits, as many such queries at a time as fit.  Returns those queries.
+uint64_t chain_open_groups(cuflye_ctx* c, PassState& ps, const RunTables& t, uint32_t nopen,
+                           const ChainParams& cp, uint64_t* sstats, OverlapRow* pool,
+                           uint64_t pool_cap, uint32_t* group_rows) {
+  cudaStream_t st = c->stream;
+  OpenInfo* d_info = buf<OpenInfo>(c, "n_oinfo", nopen);
+  CUFLYE_CHECK(runs_open_info(t, nopen, d_info, st));
+  std::vector<OpenInfo> info(nopen);
+  CUFLYE_CHECK(cudaMemcpyAsync(info.data(), d_info, nopen * sizeof(OpenInfo),
+                               cudaMemcpyDeviceToHost, st));
+  sync(c);
+  // groups without equal cur positions first, then the others by query
+  auto key = [](const OpenInfo& o) {
+    const uint64_t q = (o.flags & kRunCurTies) ? o.query + 1ull : 0ull;
+    return std::make_pair(q, o.group);
+  };
+  std::sort(info.begin(), info.end(),
+            [&](const OpenInfo& a, const OpenInfo& b) { return key(a) < key(b); });
+  uint64_t exact = 0;
+  for (size_t i = 0; i < info.size();) {
+    size_t j = i;
+    OpenBatch o;
+    std::vector<uint32_t> list, src;
+    std::vector<uint64_t> off;
+    uint64_t X = 0;
+    auto take = [&](uint32_t q) {
+      list.push_back(info[j].group);
+      src.push_back(q);
+      off.push_back(X);
+      X += info[j].nhits;
+      ++j;
+    };
+    PassState sp;
+    if (!(info[i].flags & kRunCurTies)) {
+      while (j < info.size() && !(info[j].flags & kRunCurTies)) take(kNoLink);
+    } else {
+      sp.win_off_h.push_back(0);
+      for (size_t a = i; a < info.size(); ++a) {
+        const uint32_t q = info[a].query;
+        if (a > i && info[a - 1].query == q) continue;
+        sp.base_off_h.push_back(ps.base_off_h[q]);
+        sp.win_off_h.push_back(sp.win_off_h.back() + (ps.win_off_h[q + 1] - ps.win_off_h[q]));
+        sp.qdi_h.push_back(ps.qdi_h[q]);
+        sp.qinfo_h.push_back(ps.qinfo_h[q]);
+      }
+      sp.base_off_h.push_back(0);  // queries are not adjacent: only their starts are read
+      sp.nq = static_cast<uint32_t>(sp.qdi_h.size());
+      sp.nwin = sp.win_off_h.back();
+      upload_batch(c, "x_batch", sp);
+      sp.qb.words = ps.qb.words;
+      run_hits(c, sp, false, kChainBytesPerHit, true);  // a prefix of them, as many as fit
+      uint32_t sq = 0;
+      for (;;) {
+        take(sq);
+        if (j == info.size()) break;
+        if (info[j].query != info[j - 1].query && ++sq == sp.nq) break;
+      }
+      exact += sp.nq;
+    }
+    o.n = static_cast<uint32_t>(list.size());
+    uint32_t* d_list = buf<uint32_t>(c, "n_olist", o.n);
+    uint32_t* d_src = buf<uint32_t>(c, "n_osrc", o.n);
+    CUFLYE_CHECK(cudaMemcpyAsync(d_list, list.data(), o.n * 4ull, cudaMemcpyHostToDevice, st));
+    CUFLYE_CHECK(cudaMemcpyAsync(d_src, src.data(), o.n * 4ull, cudaMemcpyHostToDevice, st));
+    o.list = d_list;
+    o.src_q = d_src;
+    o.off = upload(c, "n_ooff", off);
+    uint64_t* keys;
+    uint32_t* vals;
+    if (sp.nq) {
+      const uint32_t cap = static_cast<uint32_t>(std::min<uint64_t>(sp.nhits / 16 + 1024, 1u << 22));
+      uint64_t* tq = buf<uint64_t>(c, "f_tieh0", cap);
+      uint64_t* tk = buf<uint64_t>(c, "f_tiekey", cap);
+      uint32_t* count = buf<uint32_t>(c, "s_ecount", 1);
+      CUFLYE_CHECK(cudaMemsetAsync(count, 0, 4, st));
+      CUFLYE_CHECK(runs_tie_keys(t, o, tq, tk, count, cap, st));
+      const uint32_t T = read_scalar(c, count);
+      std::vector<std::pair<uint32_t, uint64_t>> ties(T);
+      if (T <= cap) {
+        std::vector<uint64_t> hq(T), hk(T);
+        CUFLYE_CHECK(cudaMemcpyAsync(hq.data(), tq, T * 8ull, cudaMemcpyDeviceToHost, st));
+        CUFLYE_CHECK(cudaMemcpyAsync(hk.data(), tk, T * 8ull, cudaMemcpyDeviceToHost, st));
+        sync(c);
+        for (uint32_t a = 0; a < T; ++a) ties[a] = {static_cast<uint32_t>(hq[a]), hk[a]};
+      }  // else: more than one tie per 64 hits
+      sort_listed_ties(c, sp, std::move(ties));
+      o.sorted_off = sp.q_off;
+      o.sorted_keys = sp.keys;
+      o.sorted_vals = sp.vals;
+      keys = buf<uint64_t>(c, "x_keys", X);
+      vals = buf<uint32_t>(c, "x_vals", X);
+    } else {
+      keys = buf<uint64_t>(c, "h_keys", X);
+      vals = buf<uint32_t>(c, "h_vals", X);
+    }
+    mark(c, 1);
+    GroupInfo* groups = buf<GroupInfo>(c, "g_info", o.n);
+    uint32_t* ext_list = buf<uint32_t>(c, "g_extlist", o.n);
+    uint32_t* dp_list = buf<uint32_t>(c, "g_dplist", o.n);
+    uint32_t* gcounts = buf<uint32_t>(c, "g_counts", 4);
+    CUFLYE_CHECK(cudaMemsetAsync(gcounts, 0, 4 * sizeof(uint32_t), st));
+    CUFLYE_CHECK(runs_expand(t, o, keys, vals, groups, ext_list, dp_list, gcounts, c->num_sms, st));
+    const GroupRows open = chain_groups(c, keys, vals, X, groups, o.n, ext_list, dp_list, gcounts,
+                                        cp, ps.qinfo, ps.f_off, ps.fpos, sstats, false);
+    CUFLYE_CHECK(runs_fold_rows(o.list, o.n, open.rows, group_rows, st));
+    CUFLYE_CHECK(runs_append_rows(open.pool, open.pool_count, o.list, pool, pool_cap,
+                                  t.counts + kRcPool, c->status, c->num_sms, st));
+    mark(c, 4);
+    ps.nhits += X;
+    i = j;
+  }
+  return exact;
+}
+
+// Chaining of the pass's runs (run_runs): sort, groups, pieces, DP and
+// backtrack over runs.  Groups left open take the hit path with their own hits,
+// queries left to it run through it whole.
+ChainRows chain_runs(cuflye_ctx* c, PassState& ps, const ChainParams& cp) {
+  cudaStream_t st = c->stream;
+  const uint64_t NR = ps.units;
+  const uint32_t nq = ps.nq;
+  uint64_t* sstats = buf<uint64_t>(c, "x_sortstats", kSortStats);
+  mark(c, 0);
+  // 1. the runs in (ext id, cur pos) order: a stable radix sort by ext id of
+  // each query's runs (generated in cur-pos order).  Tiles of kMatchTile runs
+  // within a query: at most this many, the unused ones empty
+  uint32_t* ntiles = buf<uint32_t>(c, "m_ntiles", nq);
+  uint64_t* mtile_off = buf<uint64_t>(c, "m_tileoff", nq + 1);
+  const uint64_t NT = NR / kMatchTile + nq;
+  int id_bits = 0;
+  while (id_bits < 32 && ((2ull * c->idx.nslots - 1) >> id_bits) != 0) ++id_bits;
+  MatchTile* tiles = buf<MatchTile>(c, "m_tiles", NT);
+  uint32_t* mcounts = buf<uint32_t>(c, "m_counts", 256 * NT);
+  uint64_t* akeys = buf<uint64_t>(c, "n_akeys", NR);
+  uint32_t* avals = buf<uint32_t>(c, "n_avals", NR);
+  CUFLYE_CHECK(cudaMemsetAsync(tiles, 0, NT * sizeof(MatchTile), st));
+  CUFLYE_CHECK(match_plan(ps.q_off, nullptr, nq, ntiles, nullptr, nullptr, nullptr, st, true));
+  scan_u32_async(c, ntiles, mtile_off, nq, "m_scan");
+  CUFLYE_CHECK(match_tiles(ps.q_off, ntiles, mtile_off, nq, tiles, st));
+  CUFLYE_CHECK(match_radix(ps.keys, ps.vals, akeys, avals, tiles, static_cast<uint32_t>(NT),
+                           ps.q_off, ntiles, mtile_off, nq, id_bits, mcounts, c->num_sms,
+                           c->shape.scatter_blocks_per_sm, st));
+  mark(c, 1);
+  // 2. groups.  Small passes size everything by their runs (a group has at
+  // least one) and read nothing back before the rows; large ones read the
+  // number of groups, then of survivors
+  const uint64_t gtiles = (NR + kGroupTile - 1) / kGroupTile;
+  uint32_t* gtcount = buf<uint32_t>(c, "n_tcount", gtiles);
+  uint64_t* gtoff = buf<uint64_t>(c, "n_toffg", gtiles + 1);
+  CUFLYE_CHECK(groups_count(ps.keys, ps.q_off, nq, NR, gtcount, st));
+  scan_u32_async(c, gtcount, gtoff, gtiles, "n_scan");
+  constexpr uint64_t kSmallPass = 1u << 15;
+  const bool small = NR <= kSmallPass;
+  RunTables t;
+  t.max_groups = small ? NR : read_scalar(c, gtoff + gtiles);
+  const uint64_t G = t.max_groups;
+  GroupInfo* bounds = buf<GroupInfo>(c, "n_bounds", G);
+  CUFLYE_CHECK(groups_write(ps.keys, ps.q_off, nq, NR, gtoff, bounds, st));
+  t.idx = c->idx;
+  t.qb = ps.qb;
+  t.qinfo = ps.qinfo;
+  t.cbits = ps.cbits;
+  t.keys = ps.keys;
+  t.vals = ps.vals;
+  t.nruns = NR;
+  t.bounds = bounds;
+  t.ngroups = gtoff + gtiles;
+  t.rlen = buf<uint32_t>(c, "n_rlen", NR);
+  t.groups = buf<RunGroup>(c, "n_groups", G);
+  t.spare0 = NR + G;
+  t.spare_cap = NR / 2 + 8192;
+  const uint64_t P = t.spare0 + t.spare_cap;
+  t.pa = buf<int32_t>(c, "n_pa", P);
+  t.pb = buf<int32_t>(c, "n_pb", P);
+  t.pl = buf<int32_t>(c, "n_pl", P);
+  t.ps = buf<int32_t>(c, "n_ps", P);
+  t.pk = buf<uint32_t>(c, "n_pk", P);
+  t.po = buf<int32_t>(c, "n_po", P);
+  t.pd = buf<int32_t>(c, "n_pd", P);
+  t.pm = buf<uint32_t>(c, "n_pm", 3 * P);
+  t.lists = buf<uint32_t>(c, "n_lists", kRunClasses * G);
+  t.sort_lists = buf<uint32_t>(c, "n_slists", 2 * G);
+  t.open_list = buf<uint32_t>(c, "n_open", G);
+  uint32_t* group_rows = buf<uint32_t>(c, "n_grows", G);
+  // counters and the spare slots' cursor: zeroed at once
+  uint32_t* words = buf<uint32_t>(c, "n_words", kRcWords + 2);
+  static_assert(kRcWords % 2 == 0, "the cursor after the counters is 8-byte aligned");
+  t.counts = words;
+  t.spare_cursor = reinterpret_cast<unsigned long long*>(words + kRcWords);
+  CUFLYE_CHECK(cudaMemsetAsync(words, 0, (kRcWords + 2) * 4, st));
+  CUFLYE_CHECK(cudaMemsetAsync(group_rows, 0, std::max<uint64_t>(G, 1) * 4, st));
+  CUFLYE_CHECK(runs_groups(t, cp, c->num_sms, st));
+  CUFLYE_CHECK(runs_order(t, c->num_sms, st));
+  mark(c, 2);
+  // 3. DP, backtrack
+  uint64_t survivors = G;
+  if (!small) {
+    ReadBack rb{c};
+    const uint32_t* n = rb.add(t.counts, kRunClasses);
+    rb.read_all();
+    survivors = 0;
+    for (int i = 0; i < kRunClasses; ++i) survivors += n[i];
+  }
+  CUFLYE_CHECK(runs_dp(t, cp, c->num_sms, c->shape.dp_blocks_per_sm, st));
+  mark(c, 3);
+  const uint64_t pool_cap = 8ull * survivors + 1024;
+  OverlapRow* pool = buf<OverlapRow>(c, "n_pool", pool_cap);
+  CUFLYE_CHECK(runs_backtrack(t, cp, ps.f_off, ps.fpos, c->logt, pool, pool_cap, group_rows,
+                              c->status, c->num_sms, c->shape.backtrack_blocks_per_sm, st));
+  // 4. max_overlaps + compaction in group order
+  uint64_t* qg = buf<uint64_t>(c, "n_qg", nq + 1);
+  uint64_t* kept_off = buf<uint64_t>(c, "n_keptoff", G + 1);
+  uint32_t* kept = group_rows;
+  CUFLYE_CHECK(runs_query_groups(t, qg, st));
+  auto compact = [&]() {
+    if (cp.max_overlaps > 0) {
+      kept = buf<uint32_t>(c, "n_kept", G);
+      CUFLYE_CHECK(cudaMemsetAsync(kept, 0, std::max<uint64_t>(G, 1) * 4, st));
+      CUFLYE_CHECK(rows_limit(group_rows, qg, nq, cp.max_overlaps, kept, st));
+    }
+    scan_u32_async(c, kept, kept_off, G, "n_scan");
+  };
+  compact();
+  ReadBack rb{c};
+  const uint32_t* counts = rb.add(t.counts, kRcWords);
+  const DeviceStatus* status = rb.add(c->status);
+  const uint64_t* nrows = rb.add(kept_off + G);
+  rb.read_all();
+  raise_device_status(c, *status);
+  const uint32_t nopen = counts[kRcOpen];
+  uint64_t chained = 0;  // groups the run DP took
+  for (int i = 0; i < kRunClasses; ++i) chained += counts[i];
+  const uint64_t ext = counts[kRcExt];
+  ChainRows out;
+  out.n = *nrows;
+  mark(c, 4);
+  uint64_t exact = 0;
+  if (nopen) {
+    exact = chain_open_groups(c, ps, t, nopen, cp, sstats, pool, pool_cap, group_rows);
+    compact();
+    ReadBack rb2{c};
+    const DeviceStatus* status2 = rb2.add(c->status);
+    const uint64_t* n2 = rb2.add(kept_off + G);
+    rb2.read_all();
+    raise_device_status(c, *status2);
+    out.n = *n2;
+  }
+  out.rows = buf<OverlapRow>(c, "n_rows", out.n);
+  CUFLYE_CHECK(runs_scatter_rows(pool, t.counts + kRcPool, std::min<uint64_t>(pool_cap, 1u << 20),
+                                 kept, kept_off, out.rows, st));
+  uint64_t* q_row = buf<uint64_t>(c, "n_qrow", nq + 1);
+  CUFLYE_CHECK(gather_query_offsets(qg, kept_off, nq, q_row, st));
+  out.q_row = q_row;
+  mark(c, 4);
+  c->sort_stats[0] += nq - exact;
+  c->sort_stats[1] += exact;
+  c->sort_stats[2] += ext;
+  c->sort_stats[4] += chained;
+  c->hits_in_runs += ps.run_hits;
+  c->runs_chained += NR;
+  return out;
+}
+
+// Sort + chaining of the pass.
+ChainRows run_chain(cuflye_ctx* c, PassState& ps, const ChainParams& cp) {
+  uint64_t* sstats = buf<uint64_t>(c, "x_sortstats", kSortStats);
+  CUFLYE_CHECK(cudaMemsetAsync(sstats, 0, kSortStats * 8, c->stream));
+  return ps.runs ? chain_runs(c, ps, cp) : chain_hits(c, ps, cp);
 }
 
 float elapsed(cudaEvent_t a, cudaEvent_t b) {
@@ -1401,6 +2001,7 @@ void reset_timing(cuflye_ctx* c) {
   c->pass_retries = 0;
   c->pass_hit_cap = 0;
   c->alloc_ms = 0;
+  c->runs_chained = c->hits_in_runs = 0;
   c->emission_fallbacks = 0;
   c->sort_stats[7] = 0;
   c->hits_sorted_emission = c->hits_flagged = c->hits_prefiltered = c->hits_emit_sort = 0;
@@ -1414,39 +2015,37 @@ void reset_timing(cuflye_ctx* c) {
 // Stages (see cuflye_last_timing): 0 hits, 1 match sort, 2 groups, 3 DP,
 // 4 backtrack + rows, 5 output + D2H, 6 H2D.
 void accumulate_timing(cuflye_ctx* c, bool chained) {
+  if (chained)
+    CUFLYE_CHECK(cudaMemcpyAsync(c->back, buf<uint64_t>(c, "x_sortstats", kSortStats),
+                                 kSortStats * 8, cudaMemcpyDeviceToHost, c->stream));
   sync(c);
   if (chained) {
-    uint64_t st[kSortStats];
-    CUFLYE_CHECK(cudaMemcpy(st, buf<uint64_t>(c, "x_sortstats", kSortStats), sizeof(st),
-                            cudaMemcpyDeviceToHost));
+    const uint64_t* st = static_cast<const uint64_t*>(c->back);
     for (int i = 0; i < kSortStats; ++i) c->sort_stats[i] += st[i];
     c->sort_stats[7] = c->emission_fallbacks;
   }
-  c->stage_ms[6] += elapsed(c->ev[0], c->ev[5]);
-  c->stage_ms[0] += elapsed(c->ev[5], c->ev[1]);
-  if (chained) {
-    c->stage_ms[1] += elapsed(c->ev[1], c->ev[2]);
-    c->stage_ms[2] += elapsed(c->ev[2], c->ev[6]);
-    c->stage_ms[3] += elapsed(c->ev[6], c->ev[7]);
-    c->stage_ms[4] += elapsed(c->ev[7], c->ev[3]);
-    c->stage_ms[5] += elapsed(c->ev[3], c->ev[4]);
-  }
+  for (size_t i = 1; i < c->marks; ++i)
+    c->stage_ms[c->clock_stage[i]] += elapsed(c->clock[i - 1], c->clock[i]);
 }
 
-// Compulsory traffic per stage: the bases and one probe sector per window,
+// Compulsory traffic per stage, for the hits the hit path took: the bases and one probe sector per window,
 // bucket entries read (8 B) and hit records written (12 B); a read and a
 // write of every 12-byte record the KmerMatch sort moves (all hits on the
 // emit + sort path, the flagged queries' hits on the sorted emission); the
 // group stage reads the records of the groups it prefilters (12 B each, and
 // on the emit + sort path another 8 B for the group bounds and ext
 // positions); the DP reads (cur, ext) and writes (score, backtrack); the
-// backtrack reads its table once.
+// backtrack reads its table once.  On the run path a hit costs the byte of
+// its bucket entry's neighbours; a run its entry (8) and record (12), the sort's
+// 24, its record read and its piece written (24), the piece read and its score
+// and link written (24), and the link table read (12).
 void set_stage_bytes(cuflye_ctx* c, uint64_t bases, uint64_t windows, uint64_t hits) {
-  c->stage_bytes[0] = bases / 4 + windows * 32 + hits * 20;
-  c->stage_bytes[1] = (c->hits_emit_sort + c->hits_flagged) * 24;
-  c->stage_bytes[2] = c->hits_emit_sort * 20 + c->hits_prefiltered * 12;
-  c->stage_bytes[3] = hits * 16;
-  c->stage_bytes[4] = hits * 4;
+  const uint64_t r = c->runs_chained;
+  c->stage_bytes[0] = bases / 4 + windows * 32 + hits * 20 + c->hits_in_runs + r * 20;
+  c->stage_bytes[1] = (c->hits_emit_sort + c->hits_flagged + r) * 24;
+  c->stage_bytes[2] = c->hits_emit_sort * 20 + c->hits_prefiltered * 12 + r * 24;
+  c->stage_bytes[3] = hits * 16 + r * 24;
+  c->stage_bytes[4] = hits * 4 + r * 12;
 }
 
 size_t pass_size(cuflye_ctx* c, size_t n) {
@@ -1462,6 +2061,8 @@ bool kept_buffer(const std::string& name) {
     if (name.compare(0, std::strlen(p), p) == 0) return true;
   if (name == "status") return true;
   for (const char* nm : kPerHitBuffers)
+    if (name == nm) return true;
+  for (const char* nm : kPerRunBuffers)
     if (name == nm) return true;
   for (const char* nm : kPerWindowBuffers)
     if (name == nm) return true;
@@ -1481,60 +2082,71 @@ void release_pass_buffers(cuflye_ctx* c) {
 // runs again on the first half of the pass's queries; bodies make their
 // results visible only after their last allocation, so the retry repeats no
 // output.
+//
+// runs: passes take the run path.  A single query whose run path does not fit
+// takes the hit path.
 template <typename Body>
-void for_each_pass(cuflye_ctx* c, const Queries& Q, bool kmers, uint64_t bytes_per_hit,
+void for_each_pass(cuflye_ctx* c, const Queries& Q, bool kmers, uint64_t bytes_per_hit, bool runs,
                    Body body) {
   size_t q0 = 0;
   const size_t full = std::max<size_t>(pass_size(c, Q.n), 1);
   size_t step = full;
-  double hpw = 0;  // hits per window of the previous pass
+  double upw = 0;  // units (hits or runs) per window of the previous pass
+  bool hit_path = !runs;
   while (q0 < Q.n) {
-    size_t q1 = run_end(c, Q, q0, std::min(Q.n, q0 + step), bytes_per_hit, hpw);
+    const bool by_runs = !hit_path;
+    size_t q1 = run_end(c, Q, q0, std::min(Q.n, q0 + step), by_runs ? kRunBytes : bytes_per_hit,
+                        upw, by_runs);
     PassState ps;
     c->pass_need.clear();
-    CUFLYE_CHECK(cudaEventRecord(c->ev[0], c->stream));
-    run_hits(c, Q, q0, q1, kmers, bytes_per_hit, ps);
-    q1 = q0 + ps.nq;
-    CUFLYE_CHECK(cudaEventRecord(c->ev[1], c->stream));
+    clock_start(c);
+    upload_queries(c, Q, q0, q1, ps);
+    if (!by_runs) run_hits(c, ps, kmers, bytes_per_hit);
     try {
+      if (by_runs) run_runs(c, ps);
+      q1 = q0 + ps.nq;
       body(q0, q1, ps);
     } catch (const Error& e) {
-      if (e.code != CUFLYE_ERR_BUDGET || ps.nq <= 1) throw;
+      if (e.code != CUFLYE_ERR_BUDGET || (ps.nq <= 1 && !by_runs)) throw;
       // the failed body's buffers go, so that half the queries find room
       sync(c);
       release_pass_buffers(c);
       ++c->pass_retries;
+      if (ps.nq <= 1) {
+        hit_path = true;
+        for (const char* nm : kPerRunBuffers) release(c, nm);
+        step = 1;
+        upw = 0;
+        continue;
+      }
       // later passes of the call stay at the size that is tried next
-      c->pass_hit_cap = std::max<uint64_t>(1, ps.nhits / 2);
+      c->pass_hit_cap = std::max<uint64_t>(1, ps.units / 2);
       step = std::max<size_t>(ps.nq / 2, 1);
       continue;
     }
-    // Learn the body's other buffers per hit from the ones this pass used
+    // Learn the body's other buffers per unit from the ones this pass used
     // (at the size they are held), and only from passes of at least a 64th
     // of what the memory left could hold: a small pass's tables (held at the
     // size an earlier, larger pass grew them to), divided by its few hits,
     // would make every later pass of the context tiny.
-    if (c->budget && ps.nhits && ps.nhits * 64 >= ps.fit_hits) {
+    if (c->budget && ps.units && ps.units * 64 >= ps.fit_units) {
       uint64_t other = 0;
       for (const auto& kv : c->pass_need) {
         if (kept_buffer(kv.first)) continue;
         auto it = c->bufs.find(kv.first);
         if (it != c->bufs.end()) other += it->second.cap;
       }
-      c->other_per_hit =
-          std::max(c->other_per_hit, static_cast<double>(other) / static_cast<double>(ps.nhits));
+      double& learned = c->other_per_hit[by_runs ? 1 : 0];
+      learned = std::max(learned, static_cast<double>(other) / static_cast<double>(ps.units));
     }
     ++c->passes;
     q0 = q1;
     step = std::min(full, step * 2);  // a halved step grows back after a pass that fits
-    if (ps.nwin) hpw = static_cast<double>(ps.nhits) / static_cast<double>(ps.nwin);
+    upw = by_runs == runs && ps.nwin ? static_cast<double>(ps.units) /
+                                           static_cast<double>(ps.nwin) : 0;
+    hit_path = !runs;
   }
 }
-
-// Device bytes per hit of one pass: keys, values, the two rank maps, the
-// radix sort's second key / value buffer, score and backtrack, plus about 2
-// bytes for the per-group tables, tiles, bitmaps and the sort's task list.
-constexpr uint64_t kChainBytesPerHit = 8 + 4 + 4 + 4 + 8 + 4 + 4 + 4 + 2;
 
 void require_index(cuflye_ctx* c) {
   if (!c->has_index) throw Error(CUFLYE_ERR_NO_INDEX, "no k-mer index: call cuflye_index_build");
@@ -1629,7 +2241,7 @@ cuflye_status cuflye_open(int device, uint64_t memory_budget_bytes, cuflye_ctx**
     CUFLYE_CHECK(cudaSetDevice(device));
     CUFLYE_CHECK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
     CUFLYE_CHECK(cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device));
-    for (auto& e : c->ev) CUFLYE_CHECK(cudaEventCreate(&e));
+    CUFLYE_CHECK(cudaMallocHost(&c->back, kBackBytes));
     CUFLYE_CHECK(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
     CUFLYE_CHECK(cudaStreamCreateWithFlags(&c->side2, cudaStreamNonBlocking));
     for (auto& e : c->side_ev) CUFLYE_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -1723,8 +2335,8 @@ void cuflye_close(cuflye_ctx* c) {
     if (kv.second.p) cudaFree(kv.second.p);
   if (c->side) cudaStreamSynchronize(c->side);
   if (c->side2) cudaStreamSynchronize(c->side2);
-  for (auto& e : c->ev)
-    if (e) cudaEventDestroy(e);
+  for (auto& e : c->clock) cudaEventDestroy(e);
+  if (c->back) cudaFreeHost(c->back);
   for (auto& e : c->side_ev)
     if (e) cudaEventDestroy(e);
   if (c->side) cudaStreamDestroy(c->side);
@@ -1820,9 +2432,10 @@ namespace {
 // device.
 double overlaps_device_ms(cuflye_ctx* c, const Queries& Q, const ChainParams& cp) {
   reset_timing(c);
-  for_each_pass(c, Q, false, kChainBytesPerHit, [&](size_t, size_t, PassState& ps) {
+  for_each_pass(c, Q, false, kChainBytesPerHit, run_path(c, cp),
+                [&](size_t, size_t, PassState& ps) {
     run_chain(c, ps, cp);
-    CUFLYE_CHECK(cudaEventRecord(c->ev[4], c->stream));
+    mark(c, 5);
     accumulate_timing(c, true);
   });
   double ms = 0;
@@ -1895,7 +2508,8 @@ cuflye_status cuflye_candidates(cuflye_ctx* c, size_t n, const int64_t* ids,
   Queries Q{n, ids, offsets, bases};
   size_t total = 0, ftotal = 0;
   bool overflow = false;
-  for_each_pass(c, Q, true, 8 + 4 + 8 + 32, [&](size_t, size_t, PassState& ps) {
+  for_each_pass(c, Q, true, 8 + 4 + 8 + 32, false, [&](size_t, size_t, PassState& ps) {
+    mark(c, 0);
     if (!overflow && total + ps.nhits <= out_cap && ftotal + ps.nfilt <= filtered_cap) {
       cuflye_candidate* d_out = buf<cuflye_candidate>(c, "a_cand", ps.nhits);
       cuflye_filtered_pos* d_f = buf<cuflye_filtered_pos>(c, "a_filt", ps.nfilt);
@@ -1940,12 +2554,13 @@ cuflye_status cuflye_overlaps(cuflye_ctx* c, size_t n, const int64_t* ids, const
   size_t total = 0;
   bool overflow = false;
   uint64_t hits_total = 0, windows_total = 0, bases_total = 0;
-  for_each_pass(c, Q, false, kChainBytesPerHit, [&](size_t q0, size_t q1, PassState& ps) {
-    const uint64_t R = run_chain(c, ps, cp);
+  for_each_pass(c, Q, false, kChainBytesPerHit, run_path(c, cp),
+                [&](size_t q0, size_t q1, PassState& ps) {
+    const ChainRows rows = run_chain(c, ps, cp);
+    const uint64_t R = rows.n;
     if (!overflow && total + R <= out_cap) {
       cuflye_overlap_range* d_out = buf<cuflye_overlap_range>(c, "a_ovl", R);
-      CUFLYE_CHECK(rows_to_abi(buf<OverlapRow>(c, "o_rows", R), R, ps.qinfo,
-                               c->idx.slot_signed, d_out, c->stream));
+      CUFLYE_CHECK(rows_to_abi(rows.rows, R, ps.qinfo, c->idx.slot_signed, d_out, c->stream));
       if (R)
         CUFLYE_CHECK(cudaMemcpyAsync(out + total, d_out, R * sizeof(cuflye_overlap_range),
                                      cudaMemcpyDeviceToHost, c->stream));
@@ -1955,7 +2570,7 @@ cuflye_status cuflye_overlaps(cuflye_ctx* c, size_t n, const int64_t* ids, const
     hits_total += ps.nhits;
     windows_total += ps.nwin;
     bases_total += static_cast<uint64_t>(offsets[q1] - offsets[q0]);
-    CUFLYE_CHECK(cudaEventRecord(c->ev[4], c->stream));
+    mark(c, 5);
     total += R;
     accumulate_timing(c, true);
   });
@@ -2047,13 +2662,14 @@ void r2g_alloc(cuflye_ctx* c, R2GPass& rp2, uint64_t A, uint32_t nq) {
 R2GPass r2g_candidates(cuflye_ctx* c, PassState& ps, const ChainParams& cp, const R2GParams& rp,
                        const int64_t* ids) {
   cudaStream_t st = c->stream;
-  const uint64_t R = run_chain(c, ps, cp);
+  const ChainRows cr = run_chain(c, ps, cp);
+  const uint64_t R = cr.n;
   const uint32_t nq = ps.nq;
   const uint32_t ns = c->idx.nslots;
   R2GGraph g{buf<int64_t>(c, "gr_edge", ns), buf<int32_t>(c, "gr_left", ns),
              buf<int32_t>(c, "gr_right", ns), c->idx.slot_signed};
-  OverlapRow* rows = buf<OverlapRow>(c, "o_rows", R);
-  const uint64_t* row_off = buf<uint64_t>(c, "o_qrowoff", nq + 1);
+  OverlapRow* rows = cr.rows;
+  const uint64_t* row_off = cr.q_row;
   uint32_t* keep = buf<uint32_t>(c, "r_keep", R);
   uint64_t* kpos = buf<uint64_t>(c, "r_kpos", R + 1);
   CUFLYE_CHECK(r2g_filter(rows, R, rp, keep, st));
@@ -2097,12 +2713,6 @@ std::vector<uint64_t> host_offsets(cuflye_ctx* c, const uint32_t* counts, uint32
   off[0] = base;
   for (uint32_t i = 0; i < n; ++i) off[i + 1] = off[i] + h[i];
   return off;
-}
-
-uint64_t* upload(cuflye_ctx* c, const char* name, const std::vector<uint64_t>& v) {
-  uint64_t* d = buf<uint64_t>(c, name, v.size());
-  CUFLYE_CHECK(cudaMemcpyAsync(d, v.data(), v.size() * 8ull, cudaMemcpyHostToDevice, c->stream));
-  return d;
 }
 
 // Divergence + accept of the pass's candidate chains, then the kept chains
@@ -2174,7 +2784,8 @@ cuflye_status cuflye_read_to_graph(cuflye_ctx* c, size_t n, const int64_t* ids,
   size_t total = 0;
   uint64_t chain_base = 0;
   bool overflow = false;
-  for_each_pass(c, Q, false, kChainBytesPerHit, [&](size_t q0, size_t, PassState& ps) {
+  for_each_pass(c, Q, false, kChainBytesPerHit, run_path(c, cp),
+                [&](size_t q0, size_t, PassState& ps) {
     R2GPass r = r2g_candidates(c, ps, cp, rp, ids + q0);
     const uint64_t nrows =
         r2g_good_rows(c, r, rp, nullptr, nullptr, nullptr, nullptr, chain_base);
@@ -2186,7 +2797,7 @@ cuflye_status cuflye_read_to_graph(cuflye_ctx* c, size_t n, const int64_t* ids,
     } else {
       overflow = true;
     }
-    CUFLYE_CHECK(cudaEventRecord(c->ev[4], c->stream));
+    mark(c, 5);
     total += nrows;
     accumulate_timing(c, true);
   });
@@ -2215,7 +2826,8 @@ cuflye_status cuflye_read_to_graph_chains(cuflye_ctx* c, size_t n, const int64_t
   Queries Q{n, ids, offsets, bases};
   size_t total = 0;
   bool overflow = false;
-  for_each_pass(c, Q, false, kChainBytesPerHit, [&](size_t q0, size_t, PassState& ps) {
+  for_each_pass(c, Q, false, kChainBytesPerHit, run_path(c, cp),
+                [&](size_t q0, size_t, PassState& ps) {
     R2GPass r = r2g_candidates(c, ps, cp, rp, ids + q0);
     const uint64_t nrec = r2g_chain_records(c, r, rp, r.read_ids);
     if (!overflow && total + nrec <= out_cap) {
@@ -2233,7 +2845,7 @@ cuflye_status cuflye_read_to_graph_chains(cuflye_ctx* c, size_t n, const int64_t
       sync(c);
       for (uint32_t q = 0; q < r.nq; ++q) inputs_per_read[q0 + q] = a[q + 1] - a[q];
     }
-    CUFLYE_CHECK(cudaEventRecord(c->ev[4], c->stream));
+    mark(c, 5);
     total += nrec;
     accumulate_timing(c, true);
   });
@@ -2524,18 +3136,23 @@ void overlaps_collect(cuflye_ctx* c, const Queries& Q, const ChainParams& cp,
   rows.clear();
   per_query.assign(Q.n, 0);
   reset_timing(c);
-  for_each_pass(c, Q, false, kChainBytesPerHit, [&](size_t q0, size_t, PassState& ps) {
-    const uint64_t R = run_chain(c, ps, cp, per_query.data() + q0);
+  for_each_pass(c, Q, false, kChainBytesPerHit, run_path(c, cp),
+                [&](size_t q0, size_t, PassState& ps) {
+    const ChainRows cr = run_chain(c, ps, cp);
+    const uint64_t R = cr.n;
+    std::vector<uint64_t> first(ps.nq + 1ull);
+    CUFLYE_CHECK(cudaMemcpyAsync(first.data(), cr.q_row, first.size() * 8, cudaMemcpyDeviceToHost,
+                                 c->stream));
     cuflye_overlap_range* d_out = buf<cuflye_overlap_range>(c, "a_ovl", R);
     const size_t base = rows.size();
     rows.resize(base + R);
-    CUFLYE_CHECK(rows_to_abi(buf<OverlapRow>(c, "o_rows", R), R, ps.qinfo, c->idx.slot_signed, d_out,
-                             c->stream));
+    CUFLYE_CHECK(rows_to_abi(cr.rows, R, ps.qinfo, c->idx.slot_signed, d_out, c->stream));
     if (R)
       CUFLYE_CHECK(cudaMemcpyAsync(rows.data() + base, d_out, R * sizeof(cuflye_overlap_range),
                                    cudaMemcpyDeviceToHost, c->stream));
-    CUFLYE_CHECK(cudaEventRecord(c->ev[4], c->stream));
+    mark(c, 5);
     accumulate_timing(c, true);  // synchronises the pass
+    for (uint32_t q = 0; q < ps.nq; ++q) per_query[q0 + q] = first[q + 1] - first[q];
   });
 }
 

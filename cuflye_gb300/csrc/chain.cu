@@ -18,8 +18,8 @@
 #include <cstdint>
 
 #include "common.cuh"
-#include "introsort.cuh"
 #include "kernels.h"
+#include "proposals.cuh"
 
 namespace cuflye {
 namespace {
@@ -551,47 +551,6 @@ __global__ void prepare_order_kernel(const int32_t* __restrict__ score, uint64_t
 
 // ---------------------------------------------------------------- backtrack
 
-constexpr int kMaxProposals = 64;
-
-struct Prop {
-  int32_t cb, ce, eb, ee, score, clen;
-  float div;
-};
-
-__device__ __forceinline__ bool overlap_test(const Prop& o, int64_t cur_id, int64_t ext_id,
-                                             int32_t cur_len, int32_t ext_len,
-                                             const ChainParams& p) {
-  const int32_t cr = o.ce - o.cb, er = o.ee - o.eb;
-  if (cr < p.min_overlap || er < p.min_overlap) return false;
-  const int32_t diff = abs(cr - er);
-  if (static_cast<float>(diff) > fmul(0.5f, static_cast<float>(min(cr, er)))) return false;
-  if (cur_id == ext_id) {
-    const int32_t inter = min(o.ce, o.ee) - max(o.cb, o.eb);
-    if (static_cast<float>(inter) > fdiv(static_cast<float>(cr), 2.0f)) return false;
-  }
-  if (cur_id == -ext_id) {
-    const int32_t inter = min(o.ce, ext_len - o.eb) - max(o.cb, ext_len - o.ee);
-    if (static_cast<float>(inter) > fdiv(static_cast<float>(cr), 2.0f)) return false;
-  }
-  if (!p.force_local && p.check_overhang) {
-    const int32_t lr = max(min(o.cb, o.eb), min(cur_len - o.ce, ext_len - o.ee));
-    if (lr > p.max_overhang) return false;
-  }
-  return true;
-}
-
-__device__ __forceinline__ uint32_t lower_bound_i32(const int32_t* a, uint32_t n, int32_t x) {
-  uint32_t lo = 0, hi = n;
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (a[mid] < x)
-      lo = mid + 1;
-    else
-      hi = mid;
-  }
-  return lo;
-}
-
 // Flye walks chains in score order: from each start whose backtrack entry is
 // still set it follows the links, clearing every entry it visits, and the
 // chain ends at the first node whose entry is -1 (never linked, or cleared
@@ -688,8 +647,8 @@ __device__ __forceinline__ void add_proposal(
     const QueryInfo& qi, int64_t ext_signed, const GroupInfo& g, const int32_t* fq, uint32_t nf,
     const LogfTable& logt, const ChainParams& p, DeviceStatus* st, uint32_t gidx, Prop* props,
     int& np, bool& overflow) {
-  const int32_t k = p.k;
   const bool swapped = g.ext_sorted == 1;
+  const int32_t k = p.k;
   int32_t c0, e0, c1, e1;
   load_match(keys, vals, swapped, b + first, c0, e0);
   load_match(keys, vals, swapped, b + s0, c1, e1);
@@ -700,28 +659,7 @@ __device__ __forceinline__ void add_proposal(
   o.ee = e1 + k - 1;
   o.score = score[b + s0] - score[b + first] + k - 1;
   o.clen = clen;
-  bool keep = overlap_test(o, qi.signed_id, ext_signed, qi.len, g.ext_len, p);
-  if (keep) {
-    const uint32_t lo = lower_bound_i32(fq, nf, o.cb);
-    const uint32_t hi = lower_bound_i32(fq, nf, o.ce + 1);
-    const int32_t norm = max(o.ce - o.cb, o.ee - o.eb) - static_cast<int32_t>(hi - lo);
-    keep = norm > 0;
-    if (keep) {
-      float rate = fdiv(fmul(static_cast<float>(clen), p.sample_rate), static_cast<float>(norm));
-      rate = rate < 1.0f ? rate : 1.0f;
-      const float x = fdiv(1.0f, rate);
-      if (!(x < 16777216.0f)) raise_status(st, kDevLogDomain, 0, static_cast<int64_t>(gidx));
-      o.div = fdiv(flye_logf(x, logt), static_cast<float>(k));
-    }
-  }
-  if (keep) {
-    if (np == kMaxProposals) {
-      raise_status(st, kDevProposalOverflow, 0, static_cast<int64_t>(gidx));
-      overflow = true;
-    } else {
-      props[np++] = o;
-    }
-  }
+  keep_proposal(o, qi, ext_signed, g.ext_len, fq, nf, logt, p, st, gidx, props, np, overflow);
 }
 
 __global__ void __launch_bounds__(kBtWarps * 32, 4) backtrack_kernel(
@@ -744,7 +682,6 @@ __global__ void __launch_bounds__(kBtWarps * 32, 4) backtrack_kernel(
   const uint32_t gidx = dp_list[li];
   const GroupInfo g = groups[gidx];
   const uint64_t b = g.start;
-  const int32_t k = p.k;
   const QueryInfo qi = qinfo[g.query];
   const int64_t ext_signed = (g.ext_di & 1u) ? -slot_signed[g.ext_di >> 1]
                                              : slot_signed[g.ext_di >> 1];
@@ -927,60 +864,8 @@ __global__ void __launch_bounds__(kBtWarps * 32, 4) backtrack_kernel(
     group_rows[gidx] = 0;
     continue;
   }
-  // proposals by score descending, libstdc++ order
-  uint64_t K[kMaxProposals];
-  uint32_t V[kMaxProposals];
-  for (int i = 0; i < np; ++i) {
-    K[i] = static_cast<uint64_t>(static_cast<uint32_t>(INT_MAX - props[i].score));
-    V[i] = static_cast<uint32_t>(i);
-  }
-  isort::serial_introsort(K, V, 0, static_cast<uint32_t>(np),
-                          isort::depth_limit(static_cast<uint32_t>(np)));
-  int prim[kMaxProposals];
-  int nprim = 0;
-  if (p.only_max_ext) {
-    if (np > 0) prim[nprim++] = static_cast<int>(V[0]);
-  } else {
-    for (int s = 0; s < np; ++s) {
-      const Prop& o = props[V[s]];
-      bool contained = false;
-      for (int t = 0; t < nprim && !contained; ++t) {
-        const Prop& pr = props[prim[t]];
-        contained = pr.cb <= o.cb && o.ce <= pr.ce && pr.eb <= o.eb && o.ee <= pr.ee &&
-                    pr.score > o.score;
-      }
-      if (!contained) prim[nprim++] = static_cast<int>(V[s]);
-    }
-  }
-  int keep[kMaxProposals];
-  int nk = 0;
-  for (int t = 0; t < nprim; ++t)
-    if (props[prim[t]].div < p.max_divergence) keep[nk++] = prim[t];
-  group_rows[gidx] = static_cast<uint32_t>(nk);
-  if (nk == 0) continue;
-  const uint32_t base = atomicAdd(pool_count, static_cast<uint32_t>(nk));
-  if (base + nk > pool_cap) {
-    raise_status(st, kDevProposalOverflow, 1, static_cast<int64_t>(gidx));
-    continue;
-  }
-  for (int t = 0; t < nk; ++t) {
-    const Prop& o = props[keep[t]];
-    OverlapRow r;
-    r.query = g.query;
-    r.ext_di = g.ext_di;
-    r.cur_begin = o.cb;
-    r.cur_end = o.ce;
-    r.cur_len = qi.len;
-    r.ext_begin = o.eb;
-    r.ext_end = o.ee;
-    r.ext_len = g.ext_len;
-    r.score = o.score;
-    r.chain_len = o.clen;
-    r.div = o.div;
-    r.group = gidx;
-    r.rank = static_cast<uint32_t>(t);
-    pool[base + t] = r;
-  }
+  finish_group(props, np, qi, g.query, g.ext_di, g.ext_len, gidx, p, pool, pool_cap, pool_count,
+               group_rows, st);
   }
 }
 
@@ -1163,23 +1048,6 @@ cudaError_t chain_dp(const uint64_t* keys, const uint32_t* vals, int32_t* score,
   count_launch();
   dp_kernel<<<num_sms * blocks, kDpWarps * 32, 0, s>>>(keys, vals, score, bt, groups, dp_list,
                                                        counts, p, top, pmc, work);
-  return cudaGetLastError();
-}
-
-namespace {
-__global__ void query_rows_kernel(const uint64_t* __restrict__ q_group_off,
-                                  const uint64_t* __restrict__ kept_off, uint32_t nq,
-                                  uint64_t* __restrict__ out) {
-  const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q < nq) out[q] = kept_off[q_group_off[q + 1]] - kept_off[q_group_off[q]];
-}
-}  // namespace
-
-cudaError_t query_row_counts(const uint64_t* q_group_off, const uint64_t* kept_off, uint32_t nq,
-                             uint64_t* out, cudaStream_t s) {
-  if (nq == 0) return cudaSuccess;
-  count_launch();
-  query_rows_kernel<<<grid(nq, 256), 256, 0, s>>>(q_group_off, kept_off, nq, out);
   return cudaGetLastError();
 }
 

@@ -68,8 +68,8 @@ __global__ void match_plan_kernel(const uint64_t* __restrict__ q_off,
     const uint64_t b = q_off[q], e = q_off[q + 1];
     uint32_t t = 0;
     if (tile_flagged) {
-      // the flagged queries only, all by radix tiles
-      if (e - b > 1 && q_tie[q]) t = static_cast<uint32_t>((e - b + kMatchTile - 1) / kMatchTile);
+      // the flagged queries (all of them without flags), all by radix tiles
+      if (e - b > 1 && (!q_tie || q_tie[q])) t = static_cast<uint32_t>((e - b + kMatchTile - 1) / kMatchTile);
     } else if (e - b > 1) {
       if (q_tie[q]) {
         const uint32_t s = atomicAdd(emu_count, 1u);

@@ -13,40 +13,11 @@
 #include <cstdint>
 
 #include "common.cuh"
+#include "hits.cuh"
 #include "kernels.h"
 
 namespace cuflye {
 namespace {
-
-
-__device__ __forceinline__ uint32_t query_of(const uint64_t* __restrict__ win_off, uint32_t nq,
-                                             uint64_t w) {
-  uint32_t lo = 0, hi = nq - 1;
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi + 1) >> 1;
-    if (__ldg(win_off + mid) <= w)
-      lo = mid;
-    else
-      hi = mid - 1;
-  }
-  return lo;
-}
-
-struct WindowKmer {
-  uint64_t x;    // forward k-mer (Kmer::numRepr)
-  uint64_t key;  // standard form
-  bool rev;      // x is not in standard form
-};
-
-__device__ __forceinline__ WindowKmer window_kmer(const QueryBatch& q, uint32_t qi, uint64_t p,
-                                                  int k) {
-  WindowKmer w;
-  w.x = kmer_at(q.words, q.base_off[qi] + p, k);
-  const uint64_t rc = revcomp(w.x, k);
-  w.rev = rc < w.x;
-  w.key = w.rev ? rc : w.x;
-  return w;
-}
 
 __global__ void count_kernel(DeviceIndex idx, QueryBatch q, uint32_t* __restrict__ cnt,
                              uint32_t* __restrict__ filt, uint64_t* __restrict__ wmeta,
@@ -56,77 +27,12 @@ __global__ void count_kernel(DeviceIndex idx, QueryBatch q, uint32_t* __restrict
   if (w >= q.nwin) return;
   const uint32_t qi = query_of(q.win_off, q.nq, w);
   const uint64_t p = w - q.win_off[qi];
-  const WindowKmer km = window_kmer(q, qi, p, idx.k);
-  bool found;
-  const uint64_t meta = table_probe(idx.table, idx.cap, km.key, &found);
-  uint32_t c = 0;
-  uint8_t fl = km.rev ? kWinRev : 0;
-  if (found && (meta & kRepetitiveBit)) {
-    fl |= kWinFiltered;
-  } else if (found) {
-    c = static_cast<uint32_t>((meta >> 40) & ((1ULL << kCountBits) - 1));
-    if ((meta & kDupIdsBit) && q_tie[qi] == 0) atomicOr(q_tie + qi, 1u);
-    const int32_t qdi = q.qdi[qi];
-    if (c > 0 && qdi >= 0) {
-      // Is the query's own window among the bucket entries?  Stored form of
-      // the self hit: (qdi, p), or flipped when the lookup flips.
-      uint64_t want;
-      if (idx.transform && km.rev) {
-        const uint32_t sid = static_cast<uint32_t>(qdi) ^ 1u;
-        const int32_t slen = idx.slot_len[sid >> 1];
-        const int64_t sp = static_cast<int64_t>(slen) - static_cast<int64_t>(p) - idx.k;
-        want = sp >= 0 ? ((static_cast<uint64_t>(sid) << 32) | static_cast<uint32_t>(sp)) : ~0ULL;
-      } else {
-        want = (static_cast<uint64_t>(qdi) << 32) | static_cast<uint32_t>(p);
-      }
-      const uint64_t off = meta & kOffsetMask;
-      uint32_t self_hits = 0;
-      if (idx.transform) {
-        // built buckets are sorted by (stored id, stored position), entries
-        // unique.  A query that is an indexed target finds its own entry
-        // where the index recorded it (checked: a query sequence that
-        // differs from the indexed one searches as any other)
-        bool known = false;
-        uint32_t at = 0;
-        if (idx.self_at && !(qdi & 1)) {
-          const uint32_t slot = static_cast<uint32_t>(qdi) >> 1;
-          const uint64_t w0 = idx.win_off[slot];
-          if (w0 + p < idx.win_off[slot + 1]) {
-            const uint32_t g = idx.self_at[w0 + p];
-            if (g < c && __ldg(idx.pos + off + g) == want) {
-              known = true;
-              at = g;
-            }
-          }
-        }
-        if (!known) {
-          uint32_t lo = 0, hi = c;
-          while (lo < hi) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (__ldg(idx.pos + off + mid) < want)
-              lo = mid + 1;
-            else
-              hi = mid;
-          }
-          known = lo < c && __ldg(idx.pos + off + lo) == want;
-          at = lo;
-        }
-        self_hits = known ? 1u : 0u;
-        if (self_hits && wself) wself[w] = at;
-      } else {
-        // explicit entries keep input order and may repeat
-        for (uint32_t e = 0; e < c; ++e) self_hits += __ldg(idx.pos + off + e) == want;
-      }
-      if (self_hits) {
-        c -= self_hits;
-        fl |= kWinTrivial;
-      }
-    }
-  }
-  cnt[w] = c;
-  filt[w] = (fl & kWinFiltered) ? 1u : 0u;
-  wmeta[w] = meta;
-  wflags[w] = fl;
+  const WindowProbe x = probe_window(idx, q, qi, p, q_tie);
+  if (wself && (x.flags & kWinTrivial)) wself[w] = x.self;
+  cnt[w] = x.hits;
+  filt[w] = (x.flags & kWinFiltered) ? 1u : 0u;
+  wmeta[w] = x.meta;
+  wflags[w] = x.flags;
 }
 
 // A warp owns 32 consecutive windows (lane L <-> window w0 + L) and writes

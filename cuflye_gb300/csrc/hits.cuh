@@ -1,0 +1,124 @@
+// hits.cuh — one query window's table probe, shared by hit counting (hits.cu)
+// and run counting (runs.cu).
+#pragma once
+
+#include <cstdint>
+
+#include "common.cuh"
+#include "kernels.h"
+
+namespace cuflye {
+
+__device__ __forceinline__ uint32_t query_of(const uint64_t* __restrict__ win_off, uint32_t nq,
+                                             uint64_t w) {
+  uint32_t lo = 0, hi = nq - 1;
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi + 1) >> 1;
+    if (__ldg(win_off + mid) <= w)
+      lo = mid;
+    else
+      hi = mid - 1;
+  }
+  return lo;
+}
+
+struct WindowKmer {
+  uint64_t x;    // forward k-mer (Kmer::numRepr)
+  uint64_t key;  // standard form
+  bool rev;      // x is not in standard form
+};
+
+__device__ __forceinline__ WindowKmer window_kmer(const QueryBatch& q, uint32_t qi, uint64_t p,
+                                                  int k) {
+  WindowKmer w;
+  w.x = kmer_at(q.words, q.base_off[qi] + p, k);
+  const uint64_t rc = revcomp(w.x, k);
+  w.rev = rc < w.x;
+  w.key = w.rev ? rc : w.x;
+  return w;
+}
+
+// A window's bucket: its table meta, flags (kWinRev, kWinFiltered,
+// kWinTrivial), hits (the bucket's entries less the query's own position) and
+// the own entry's bucket index (kWinTrivial on a built index).
+struct WindowProbe {
+  uint64_t meta;
+  uint32_t hits;
+  uint32_t self;
+  uint8_t flags;
+};
+
+__device__ __forceinline__ WindowProbe probe_window(const DeviceIndex& idx, const QueryBatch& q,
+                                                    uint32_t qi, uint64_t p,
+                                                    uint32_t* __restrict__ q_tie) {
+  const WindowKmer km = window_kmer(q, qi, p, idx.k);
+  bool found;
+  const uint64_t meta = table_probe(idx.table, idx.cap, km.key, &found);
+  uint32_t c = 0, self = 0;
+  uint8_t fl = km.rev ? kWinRev : 0;
+  if (found && (meta & kRepetitiveBit)) {
+    fl |= kWinFiltered;
+  } else if (found) {
+    c = static_cast<uint32_t>((meta >> 40) & ((1ULL << kCountBits) - 1));
+    if (q_tie && (meta & kDupIdsBit) && q_tie[qi] == 0) atomicOr(q_tie + qi, 1u);
+    const int32_t qdi = q.qdi[qi];
+    if (c > 0 && qdi >= 0) {
+      // Is the query's own window among the bucket entries?  Stored form of
+      // the self hit: (qdi, p), or flipped when the lookup flips.
+      uint64_t want;
+      if (idx.transform && km.rev) {
+        const uint32_t sid = static_cast<uint32_t>(qdi) ^ 1u;
+        const int32_t slen = idx.slot_len[sid >> 1];
+        const int64_t sp = static_cast<int64_t>(slen) - static_cast<int64_t>(p) - idx.k;
+        want = sp >= 0 ? ((static_cast<uint64_t>(sid) << 32) | static_cast<uint32_t>(sp)) : ~0ULL;
+      } else {
+        want = (static_cast<uint64_t>(qdi) << 32) | static_cast<uint32_t>(p);
+      }
+      const uint64_t off = meta & kOffsetMask;
+      uint32_t self_hits = 0;
+      if (idx.transform) {
+        // built buckets are sorted by (stored id, stored position), entries
+        // unique.  A query that is an indexed target finds its own entry
+        // where the index recorded it (checked: a query sequence that
+        // differs from the indexed one searches as any other)
+        bool known = false;
+        uint32_t at = 0;
+        if (idx.self_at && !(qdi & 1)) {
+          const uint32_t slot = static_cast<uint32_t>(qdi) >> 1;
+          const uint64_t w0 = idx.win_off[slot];
+          if (w0 + p < idx.win_off[slot + 1]) {
+            const uint32_t g = idx.self_at[w0 + p];
+            if (g < c && __ldg(idx.pos + off + g) == want) {
+              known = true;
+              at = g;
+            }
+          }
+        }
+        if (!known) {
+          uint32_t lo = 0, hi = c;
+          while (lo < hi) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (__ldg(idx.pos + off + mid) < want)
+              lo = mid + 1;
+            else
+              hi = mid;
+          }
+          known = lo < c && __ldg(idx.pos + off + lo) == want;
+          at = lo;
+        }
+        self_hits = known ? 1u : 0u;
+        if (self_hits) self = at;
+      } else {
+        // explicit entries keep input order and may repeat
+        for (uint32_t e = 0; e < c; ++e) self_hits += __ldg(idx.pos + off + e) == want;
+      }
+      if (self_hits) {
+        c -= self_hits;
+        fl |= kWinTrivial;
+      }
+    }
+  }
+  return WindowProbe{meta, c, self, fl};
+}
+
+}  // namespace cuflye

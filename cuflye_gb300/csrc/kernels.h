@@ -108,6 +108,12 @@ struct DeviceIndex {
   // bucket when that k-mer is solid (other windows: any value)
   uint32_t* self_at = nullptr;
   uint64_t* win_off = nullptr;
+  // optional (built indexes of an odd k, when memory allows): the bases around
+  // each stored entry's k-mer, one byte an entry in bucket order, and the
+  // packed targets with each slot's first base (the run path, runs.cu)
+  uint8_t* nbr = nullptr;
+  uint64_t* twords = nullptr;
+  uint64_t* tbase = nullptr;
 };
 
 // Window enumeration over packed targets: keys = standard forms, vals =
@@ -240,8 +246,8 @@ struct MatchTile {
 
 // Per query with two or more hits: flagged queries (q_tie, keys may repeat)
 // are listed for the emulated sort; the others get ntiles[q] radix tiles.
-// tile_flagged: the flagged queries get the tiles (their sorted order up to
-// the order among equal keys) and nothing is listed.
+// tile_flagged: the flagged queries (q_tie null: all of them) get the tiles
+// (their sorted order up to the order among equal keys) and nothing is listed.
 cudaError_t match_plan(const uint64_t* q_off, const uint32_t* q_tie, uint32_t nq, uint32_t* ntiles,
                        uint64_t* emu_begin, uint64_t* emu_end, uint32_t* emu_count,
                        cudaStream_t s, bool tile_flagged = false);
@@ -433,8 +439,5 @@ cudaError_t rows_scatter(const OverlapRow* pool, uint32_t npool, const uint32_t*
                          const uint64_t* kept_off, OverlapRow* rows, cudaStream_t s);
 cudaError_t query_group_offsets(const GroupInfo* groups, uint64_t ngroups, uint32_t nq,
                                 uint64_t* q_group_off, cudaStream_t s);
-// Rows of each query after compaction: out[q] = kept_off[qg[q + 1]] - kept_off[qg[q]].
-cudaError_t query_row_counts(const uint64_t* q_group_off, const uint64_t* kept_off, uint32_t nq,
-                             uint64_t* out, cudaStream_t s);
 
 }  // namespace cuflye

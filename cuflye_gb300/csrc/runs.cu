@@ -1,0 +1,737 @@
+// runs.cu — candidate hits found, sorted and filtered as runs.
+//
+// Hits of one (query, target) pair come in runs at consecutive cur and ext
+// positions: a window's hit (id, pos) continues the run of the window before
+// it exactly when that window is solid and the base before the k-mer is the
+// same in query and target.  So the index keeps, for every stored entry, the
+// bases around its k-mer (one byte), and a query window finds the runs that
+// start in its bucket by comparing bytes; a hit inside a run costs that byte
+// and is never written.  A run's length is how far the packed query and target
+// agree, cut at the query's next window that is not solid.
+//
+// The runs are sorted like hits (radix sort by ext id of runs generated in
+// window order), grouped by ext id, and each group's prefilter is decided from
+// its runs.  run_chain.cu chains them.
+//
+// Measured on all reads of a 5 Mb genome at 40x (HiFi, k = 17: 7.2e9 hits in
+// 36e6 runs, 64 GiB budget): hit generation 183 -> 16.7 ms, KmerMatch sort 54 ->
+// 4 ms, groups 51 -> 19 ms, DP 50 -> 4 ms, backtrack 27 -> 4 ms against writing,
+// sorting and chaining every hit (the hit path, which remains for what the run
+// path leaves open and for indexes without its tables).  At 6 % error (3 Mb
+// genome, 30x ONT reads: 4.7e8 hits in 59e6 runs) 50 -> 25 ms.  One read: 1.0 ->
+// 0.41 ms, its groups' serial scans being as many times shorter as its runs are
+// long.
+//
+// Needs an odd k: an even k has k-mers equal to their own reverse complement,
+// stored on one strand only, so that a run on the other strand has holes.
+#include <algorithm>
+#include <climits>
+#include <cstdint>
+
+#include "common.cuh"
+#include "hits.cuh"
+#include "kernels.h"
+#include "runs.h"
+
+namespace cuflye {
+namespace {
+
+inline unsigned grid(uint64_t n, int b) {
+  return static_cast<unsigned>((n + b - 1) / b > 0 ? (n + b - 1) / b : 1);
+}
+
+// Window flags of the run path, beside kWinRev, kWinFiltered and kWinTrivial:
+// the k-mer is solid; the base before the window; it is the query's first.
+constexpr uint8_t kWinSolid = 8;
+constexpr int kWinBaseShift = 4;
+constexpr uint8_t kWinFirst = 64;
+
+__device__ __forceinline__ uint32_t base_at(const uint64_t* __restrict__ words, uint64_t g) {
+  return static_cast<uint32_t>(__ldg(words + (g >> 5)) >> (62 - 2 * (g & 31))) & 3u;
+}
+
+// 32 bases from base g on (g >= 0; two words).
+__device__ __forceinline__ uint64_t bases32(const uint64_t* __restrict__ words, uint64_t g) {
+  const uint64_t hi = __ldg(words + (g >> 5));
+  const uint32_t s = static_cast<uint32_t>(g & 31u);
+  return s ? (hi << (2 * s)) | (__ldg(words + (g >> 5) + 1) >> (64 - 2 * s)) : hi;
+}
+
+__global__ void neighbour_kernel(const uint64_t* __restrict__ pos, uint64_t n,
+                                 const uint64_t* __restrict__ words,
+                                 const uint64_t* __restrict__ base_off,
+                                 const int32_t* __restrict__ slot_len, int k,
+                                 uint8_t* __restrict__ nbr) {
+  const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const uint64_t v = pos[i];
+  const uint32_t sid = static_cast<uint32_t>(v >> 32);
+  const int32_t sp = static_cast<int32_t>(v & 0xffffffffu);
+  const int32_t len = slot_len[sid >> 1];
+  const uint64_t b = base_off[sid >> 1];
+  const int32_t p = (sid & 1u) ? len - sp - k : sp;  // the window on the forward strand
+  uint32_t before = 4, after = 4;
+  if (p > 0) before = base_at(words, b + static_cast<uint64_t>(p) - 1);
+  if (p + k < len) after = base_at(words, b + static_cast<uint64_t>(p) + k);
+  if (sid & 1u) {
+    const uint32_t x = before;
+    before = after == 4 ? 4u : 3u - after;
+    after = x == 4 ? 4u : 3u - x;
+  }
+  nbr[i] = static_cast<uint8_t>(before | (after << 4));
+}
+
+// One thread per window, blocks of whole 32-window tiles.
+__global__ void __launch_bounds__(256) probe_kernel(
+    DeviceIndex idx, QueryBatch q, uint64_t* __restrict__ wmeta, uint8_t* __restrict__ wflags,
+    uint32_t* __restrict__ wself, uint32_t* __restrict__ cbits, uint32_t* __restrict__ fbits,
+    uint32_t* __restrict__ tile_filt, unsigned long long* __restrict__ hit_total) {
+  __shared__ uint32_t wsum[8];
+  const uint64_t w = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  uint32_t hits = 0;
+  uint8_t fl = 0;
+  if (w < q.nwin) {
+    const uint32_t qi = query_of(q.win_off, q.nq, w);
+    const uint64_t p = w - q.win_off[qi];
+    const WindowProbe x = probe_window(idx, q, qi, p, nullptr);
+    fl = x.flags;
+    hits = x.hits;
+    const uint32_t raw = static_cast<uint32_t>((x.meta >> 40) & ((1ULL << kCountBits) - 1));
+    if (!(fl & kWinFiltered) && raw > 0) fl |= kWinSolid;
+    if (p == 0)
+      fl |= kWinFirst;
+    else
+      fl |= static_cast<uint8_t>(base_at(q.words, q.base_off[qi] + p - 1) << kWinBaseShift);
+    if (fl & kWinTrivial) wself[w] = x.self;
+    wmeta[w] = x.meta;
+    wflags[w] = fl;
+  }
+  const uint32_t cb = __ballot_sync(0xffffffffu, fl & kWinSolid);
+  const uint32_t fb = __ballot_sync(0xffffffffu, fl & kWinFiltered);
+  const uint32_t sum = __reduce_add_sync(0xffffffffu, hits);
+  if (lane == 0) {
+    if (w < q.nwin) {
+      cbits[w >> 5] = cb;
+      fbits[w >> 5] = fb;
+      tile_filt[w >> 5] = __popc(fb);
+    }
+    wsum[threadIdx.x >> 5] = sum;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned long long s = 0;
+    for (int i = 0; i < 8; ++i) s += wsum[i];
+    if (s) atomicAdd(hit_total + (blockIdx.x & 63u), s);
+  }
+}
+
+// What a bucket entry's neighbour nibble must be for its hit to continue the
+// run of the window before, and where the nibble sits in the entry's byte:
+// the base before the window, on the entry's strand (the complement of it
+// after the k-mer when the lookup flips).  7 matches no entry.
+struct RunTest {
+  uint32_t expect;
+  int shift;
+};
+
+__device__ __forceinline__ RunTest run_test(uint8_t fl, uint8_t prev_fl) {
+  uint32_t e = 7;
+  if (!(fl & kWinFirst) && (prev_fl & kWinSolid)) e = (fl >> kWinBaseShift) & 3u;
+  if (!(fl & kWinRev)) return RunTest{e, 0};
+  return RunTest{e == 7 ? 7u : 3u - e, 4};
+}
+
+__device__ __forceinline__ uint32_t bucket_size(uint8_t fl, uint64_t meta) {
+  return (fl & kWinSolid) ? static_cast<uint32_t>((meta >> 40) & ((1ULL << kCountBits) - 1)) : 0u;
+}
+
+// Bytes lo..3 of a word (lo in 0..4) as a mask.
+__device__ __forceinline__ uint32_t bytes_from(int lo) {
+  return lo >= 4 ? 0u : 0xffffffffu << (8 * lo);
+}
+
+// Run starts of each window: one thread a window, 16 entries a load (a bucket
+// of 36 entries is 3 to 4 loads that do not wait for one another; bound by the
+// latency of these scattered loads).
+__global__ void __launch_bounds__(256) start_count_kernel(
+    DeviceIndex idx, QueryBatch q, const uint64_t* __restrict__ wmeta,
+    const uint8_t* __restrict__ wflags, const uint32_t* __restrict__ wself,
+    uint32_t* __restrict__ nstart, uint32_t* __restrict__ tile_start) {
+  const uint64_t w = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  uint32_t fl = 0, c = 0, ns = 0;
+  uint64_t meta = 0;
+  if (w < q.nwin) {
+    fl = wflags[w];
+    meta = wmeta[w];
+    c = bucket_size(static_cast<uint8_t>(fl), meta);
+  }
+  uint32_t pf = __shfl_up_sync(0xffffffffu, fl, 1);
+  if (lane == 0) pf = w > 0 && w < q.nwin ? wflags[w - 1] : 0u;
+  if (c > 0) {
+    const RunTest rt = run_test(static_cast<uint8_t>(fl), static_cast<uint8_t>(pf));
+    const uint64_t off = meta & kOffsetMask;
+    if (rt.expect == 7) {
+      ns = c - ((fl & kWinTrivial) ? 1u : 0u);
+    } else {
+      const uint32_t pat = rt.expect * 0x01010101u;
+      const uint64_t end = off + c;
+      const uint4* nb = reinterpret_cast<const uint4*>(idx.nbr);
+#pragma unroll 2
+      for (uint64_t ch = off >> 4; ch <= (end - 1) >> 4; ++ch) {
+        const uint4 x = __ldg(nb + ch);
+        const int64_t lo = static_cast<int64_t>(off) - static_cast<int64_t>(ch * 16);
+        const int64_t hi = static_cast<int64_t>(end) - static_cast<int64_t>(ch * 16);
+        const uint32_t xs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+          const uint32_t y = ((xs[s] >> rt.shift) & 0x0f0f0f0fu) ^ pat;
+          uint32_t m = (y + 0x7f7f7f7fu) & 0x80808080u;  // bytes that differ
+          const int l = static_cast<int>(lo - 4 * s), h = static_cast<int>(hi - 4 * s);
+          if (l > 0) m &= bytes_from(l);
+          if (h < 4) m &= ~bytes_from(h < 0 ? 0 : h);
+          ns += __popc(m);
+        }
+      }
+      if (fl & kWinTrivial) {  // the query's own position is no hit
+        const uint32_t b = __ldg(idx.nbr + off + wself[w]);
+        if (((b >> rt.shift) & 15u) != rt.expect) --ns;
+      }
+    }
+  }
+  const uint32_t sum = __reduce_add_sync(0xffffffffu, ns);
+  if (w < q.nwin) {
+    nstart[w] = ns;
+    if (lane == 0) tile_start[w >> 5] = sum;
+  }
+}
+
+__global__ void query_offsets_kernel(QueryBatch q, const uint32_t* __restrict__ nstart,
+                                     const uint64_t* __restrict__ tile_off,
+                                     const uint32_t* __restrict__ fbits,
+                                     const uint64_t* __restrict__ ftile_off,
+                                     uint64_t* __restrict__ q_off, uint64_t* __restrict__ f_off) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i > q.nq) return;
+  const uint64_t w = q.win_off[i], t = w >> 5;
+  const uint32_t r = static_cast<uint32_t>(w & 31);
+  uint64_t o = tile_off[t], f = ftile_off[t];
+  if (r) {  // inside a tile
+    for (uint32_t j = 0; j < r; ++j) o += nstart[t * 32 + j];
+    f += __popc(fbits[t] & ((1u << r) - 1u));
+  }
+  q_off[i] = o;
+  f_off[i] = f;
+}
+
+// A warp writes its 32 windows' run starts, one window at a time with all
+// lanes on the bucket's entries: most windows start no run and are skipped, and
+// the first window after a hole in the query starts a run in every entry.
+__global__ void __launch_bounds__(256) start_emit_kernel(
+    DeviceIndex idx, QueryBatch q, const uint64_t* __restrict__ wmeta,
+    const uint8_t* __restrict__ wflags, const uint32_t* __restrict__ wself,
+    const uint32_t* __restrict__ nstart, const uint64_t* __restrict__ tile_off,
+    const uint32_t* __restrict__ fbits, const uint64_t* __restrict__ ftile_off,
+    uint64_t* __restrict__ keys, uint32_t* __restrict__ vals, int32_t* __restrict__ fpos) {
+  const uint64_t w = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const uint32_t lt = (1u << lane) - 1u;
+  uint32_t ns = 0, fl = 0, fb = 0;
+  if (w < q.nwin) {
+    ns = nstart[w];
+    fb = fbits[w >> 5];
+  }
+  const bool filtered = (fb >> lane) & 1u;
+  uint32_t p = 0;
+  if (ns || filtered) {
+    const uint32_t qi = query_of(q.win_off, q.nq, w);
+    p = static_cast<uint32_t>(w - q.win_off[qi]);
+    if (filtered) fpos[ftile_off[w >> 5] + __popc(fb & lt)] = static_cast<int32_t>(p);
+  }
+  unsigned todo = __ballot_sync(0xffffffffu, ns > 0);
+  if (!todo) return;
+  uint64_t meta = 0;
+  uint32_t self = kNoLink;
+  RunTest rt{7, 0};
+  if (ns) {
+    fl = wflags[w];
+    meta = wmeta[w];
+    rt = run_test(static_cast<uint8_t>(fl), w > 0 ? wflags[w - 1] : 0);
+    if (fl & kWinTrivial) self = wself[w];
+  }
+  uint64_t out = tile_off[w >> 5];
+  while (todo) {
+    const int src = __ffs(todo) - 1;
+    todo &= todo - 1;
+    const uint64_t wm = __shfl_sync(0xffffffffu, meta, src);
+    const uint32_t wp = __shfl_sync(0xffffffffu, p, src);
+    const uint32_t wf = __shfl_sync(0xffffffffu, fl, src);
+    const uint32_t ws = __shfl_sync(0xffffffffu, self, src);
+    const uint32_t we = __shfl_sync(0xffffffffu, rt.expect, src);
+    const int wsh = __shfl_sync(0xffffffffu, rt.shift, src);
+    const uint64_t off = wm & kOffsetMask;
+    const uint32_t c = bucket_size(static_cast<uint8_t>(wf), wm);
+    for (uint32_t e0 = 0; e0 < c; e0 += 32) {
+      const uint32_t e = e0 + lane;
+      const bool start = e < c && e != ws &&
+                         ((static_cast<uint32_t>(__ldg(idx.nbr + off + e)) >> wsh) & 15u) != we;
+      const unsigned m = __ballot_sync(0xffffffffu, start);
+      if (start) {
+        const uint64_t sv = __ldg(idx.pos + off + e);
+        uint32_t id = static_cast<uint32_t>(sv >> 32);
+        int32_t pos = static_cast<int32_t>(sv & 0xffffffffu);
+        if (wf & kWinRev) {
+          pos = idx.slot_len[id >> 1] - pos - idx.k;
+          id ^= 1u;
+        }
+        const uint64_t d = out + __popc(m & lt);
+        keys[d] = (static_cast<uint64_t>(id) << 32) | wp;
+        vals[d] = static_cast<uint32_t>(pos);
+      }
+      out += __popc(m);
+    }
+  }
+}
+
+// Hits of the run that starts at window p of query qi and position pos of
+// target strand id: the windows over which query and target agree, up to most,
+// and up to the query's next window that is not solid.
+__device__ __forceinline__ int32_t run_length(const RunTables& t, uint64_t qbase, uint64_t w0,
+                                              uint64_t tbase, int32_t tlen, bool rev, int32_t p,
+                                              int32_t pos, int32_t most) {
+  const int32_t k = t.idx.k;
+  int32_t m = 0;  // agreeing bases after the first window
+  while (m < most - 1) {
+    const int32_t x = pos + k + m;
+    const uint64_t qb = bases32(t.qb.words, qbase + static_cast<uint64_t>(p) + k + m);
+    uint64_t tb;
+    if (!rev) {
+      tb = bases32(t.idx.twords, tbase + static_cast<uint64_t>(x));
+    } else {
+      // bases x .. x + 31 of the reverse strand: the reverse complement of
+      // the 32 forward bases that end before len - x
+      const int64_t s = static_cast<int64_t>(tbase) + tlen - 32 - x;
+      const uint64_t f = s >= 0 ? bases32(t.idx.twords, static_cast<uint64_t>(s))
+                                : bases32(t.idx.twords, 0) >> (2 * -s);
+      tb = revcomp(f, 32);
+    }
+    const uint64_t diff = qb ^ tb;
+    const int32_t same = diff ? __clzll(static_cast<long long>(diff)) >> 1 : 32;
+    // solid bits of windows p + 1 + m .. p + 32 + m
+    const uint64_t b = w0 + static_cast<uint64_t>(p) + 1 + m;
+    const uint32_t c0 = __ldg(t.cbits + (b >> 5));
+    const uint32_t c1 = (b & 31) ? __ldg(t.cbits + (b >> 5) + 1) : 0u;
+    const uint32_t holes = ~__funnelshift_r(c0, c1, static_cast<uint32_t>(b & 31));
+    const int32_t solid = holes ? __ffs(holes) - 1 : 32;
+    const int32_t step = min(same, solid);
+    m += step;
+    if (step < 32) break;
+  }
+  return min(m + 1, most);
+}
+
+__device__ __forceinline__ int run_class(uint32_t npieces) {
+  return npieces > 1024 ? 0 : npieces > 256 ? 1 : npieces > 64 ? 2 : npieces > 16 ? 3 : 4;
+}
+
+// Pieces of a group whose n runs (a, b, l by lane, from run i on) follow one
+// another along its axis: slot piece0 holds element 0, the next slot the rest
+// of its run, then one run a slot.
+__device__ __forceinline__ void store_run_piece(const RunTables& t, uint64_t slot, uint32_t i,
+                                                int32_t a, int32_t b, int32_t l) {
+  if (i == 0) {
+    // (the first slot goes unused when the first run is element 0 alone)
+    t.pa[slot] = a;
+    t.pb[slot] = b;
+    t.pl[slot] = 1;
+    const int32_t rest = l > 1 ? 1 : 0;
+    t.pa[slot + 1] = a + rest;
+    t.pb[slot + 1] = b + rest;
+    t.pl[slot + 1] = l - rest;
+  } else {
+    t.pa[slot + 1 + i] = a;
+    t.pb[slot + 1 + i] = b;
+    t.pl[slot + 1 + i] = l;
+  }
+}
+
+constexpr int kGroupWarps = 8;
+
+__global__ void __launch_bounds__(kGroupWarps * 32) run_groups_kernel(RunTables t, ChainParams p) {
+  __shared__ uint32_t scls[kGroupWarps], sslot[kGroupWarps];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint64_t G = *t.ngroups;
+  constexpr uint32_t kNone = 255;
+  for (uint64_t g0 = static_cast<uint64_t>(blockIdx.x) * kGroupWarps; g0 < G;
+       g0 += static_cast<uint64_t>(gridDim.x) * kGroupWarps) {
+    const uint64_t g = g0 + warp;
+    uint32_t cls = kNone;
+    if (g < G) {
+      const GroupInfo gi = t.bounds[g];
+      const uint64_t end = g + 1 < G ? t.bounds[g + 1].start : t.nruns;
+      const uint32_t n = static_cast<uint32_t>(end - gi.start);
+      const uint32_t slot = gi.ext_di >> 1;
+      const bool rev = gi.ext_di & 1u;
+      const int32_t tlen = t.idx.slot_len[slot];
+      const uint64_t tbase = t.idx.tbase[slot];
+      const uint64_t qbase = t.qb.base_off[gi.query];
+      const uint64_t w0 = t.qb.win_off[gi.query];
+      const int32_t qwin = static_cast<int32_t>(t.qb.win_off[gi.query + 1] - w0);
+      const int32_t cur_len = t.qinfo[gi.query].len;
+      const bool es = tlen > cur_len;
+      const uint64_t pslot = gi.start + g;
+      uint32_t hits = 0, distinct = 0;
+      int32_t mn = INT_MAX, mx = INT_MIN, first_c = 0, first_l = 0;
+      int32_t end_c = 0, end_e = 0;  // ends of the runs so far (cur: greatest; ext: the last one's)
+      bool ties = false, rising = true;
+      for (uint32_t i0 = 0; i0 < n; i0 += 32) {
+        const uint32_t i = i0 + lane;
+        const bool in = i < n;
+        int32_t c = 0, e = 0, l = 0;
+        if (in) {
+          c = static_cast<int32_t>(t.keys[gi.start + i] & 0xffffffffu);
+          e = static_cast<int32_t>(t.vals[gi.start + i]);
+          l = run_length(t, qbase, w0, tbase, tlen, rev, c, e,
+                         min(qwin - c, tlen - t.idx.k + 1 - e));
+          t.rlen[gi.start + i] = static_cast<uint32_t>(l);
+          store_run_piece(t, pslot, i, es ? e : c, es ? c : e, l);
+          hits += l;
+          mn = min(mn, e);
+          mx = max(mx, e + l - 1);
+        }
+        if (i0 == 0) {
+          first_c = __shfl_sync(0xffffffffu, c, 0);
+          first_l = __shfl_sync(0xffffffffu, l, 0);
+        }
+        // greatest end of the runs before this one, and the last one's ext end
+        int32_t inc = in ? c + l : 0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+          if (lane >= o) inc = max(inc, y);
+        }
+        int32_t before = __shfl_up_sync(0xffffffffu, inc, 1);
+        before = lane == 0 ? end_c : max(before, end_c);
+        int32_t pe = __shfl_up_sync(0xffffffffu, e + l, 1);
+        if (lane == 0) pe = end_e;
+        if (in) {
+          distinct += max(0, c + l - max(c, before));
+          ties |= c < before;
+          rising &= e >= pe;
+        }
+        end_c = max(end_c, __shfl_sync(0xffffffffu, inc, 31));
+        end_e = __shfl_sync(0xffffffffu, e + l, 31);  // used when more runs follow
+      }
+      hits = __reduce_add_sync(0xffffffffu, hits);
+      distinct = __reduce_add_sync(0xffffffffu, distinct);
+      mn = __reduce_min_sync(0xffffffffu, mn);
+      mx = __reduce_max_sync(0xffffffffu, mx);
+      ties = __any_sync(0xffffffffu, ties);
+      rising = __all_sync(0xffffffffu, rising);
+      const uint32_t uniq = distinct - (first_c == 0 ? 1u : 0u);
+      if (prefilter_keeps(uniq, first_c, end_c - 1, mn, mx, cur_len, tlen, p)) {
+        const bool ready = es ? rising : !ties;
+        RunGroup rg{};
+        rg.run0 = gi.start;
+        rg.nruns = n;
+        rg.piece0 = pslot + (first_l > 1 ? 0u : 1u);
+        rg.npieces = n + (first_l > 1 ? 1u : 0u);
+        rg.nhits = hits;
+        rg.query = gi.query;
+        rg.ext_di = gi.ext_di;
+        rg.ext_len = tlen;
+        rg.flags = (es ? kRunExt : 0u) | (ties ? kRunCurTies : 0u);
+        if (lane == 0) t.groups[g] = rg;
+        if (ready)
+          cls = static_cast<uint32_t>(run_class(rg.npieces));
+        else
+          cls = kRunClasses + (n <= 32 ? 0u : 1u);
+        if (es) cls |= 256u;
+      }
+    }
+    if (lane == 0) scls[warp] = cls;
+    __syncthreads();
+    if (threadIdx.x < kRunClasses + 2) {  // one counter update a list and block
+      uint32_t m = 0;
+      for (int w = 0; w < kGroupWarps; ++w) m += (scls[w] & 255u) == threadIdx.x;
+      if (m) {
+        uint32_t s = atomicAdd(t.counts + kRcList + threadIdx.x, m);
+        for (int w = 0; w < kGroupWarps; ++w)
+          if ((scls[w] & 255u) == threadIdx.x) sslot[w] = s++;
+      }
+    } else if (threadIdx.x == 32) {
+      uint32_t m = 0;
+      for (int w = 0; w < kGroupWarps; ++w) m += scls[w] >> 8;
+      if (m) atomicAdd(t.counts + kRcExt, m);
+    }
+    __syncthreads();
+    if (lane == 0 && cls != kNone) {
+      const uint32_t k = cls & 255u;
+      uint32_t* list = k < kRunClasses ? t.lists + k * t.max_groups
+                                       : t.sort_lists + (k - kRunClasses) * t.max_groups;
+      list[sslot[warp]] = static_cast<uint32_t>(g);
+    }
+  }
+}
+
+// ---------------------------------------------------------------- open groups
+
+__global__ void open_info_kernel(RunTables t, uint32_t nopen, OpenInfo* __restrict__ out) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nopen) return;
+  const uint32_t g = t.open_list[i];
+  const RunGroup& rg = t.groups[g];
+  out[i] = OpenInfo{g, rg.query, rg.nhits, rg.flags};
+}
+
+// Cur positions that hits of an open group share, as (sub-batch query, key):
+// where a run (in cur order) starts before the greatest end of the ones before.
+__global__ void tie_keys_kernel(RunTables t, OpenBatch o, uint64_t* __restrict__ tie_q,
+                                uint64_t* __restrict__ tie_key, uint32_t* __restrict__ count,
+                                uint32_t cap) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= o.n || o.src_q[i] == kNoLink) return;
+  const RunGroup rg = t.groups[o.list[i]];
+  uint32_t end = 0;
+  for (uint32_t r = 0; r < rg.nruns; ++r) {
+    const uint64_t key = t.keys[rg.run0 + r];
+    const uint32_t c = static_cast<uint32_t>(key), e = c + t.rlen[rg.run0 + r];
+    for (uint32_t x = c; x < min(e, end); ++x) {
+      const uint32_t s = atomicAdd(count, 1u);
+      if (s < cap) {
+        tie_q[s] = o.src_q[i];
+        tie_key[s] = key + (x - c);
+      }
+    }
+    end = max(end, e);
+  }
+}
+
+// The open groups' hits in KmerMatch order: from their runs, or (groups that
+// repeat a cur position) from their query's sorted hits.
+__global__ void expand_kernel(RunTables t, OpenBatch o, uint64_t* __restrict__ keys,
+                              uint32_t* __restrict__ vals, GroupInfo* __restrict__ groups,
+                              uint32_t* __restrict__ ext_list, uint32_t* __restrict__ dp_list,
+                              uint32_t* __restrict__ counts) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
+  for (uint32_t li = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; li < o.n; li += nwarps) {
+    const RunGroup rg = t.groups[o.list[li]];
+    uint64_t d = o.off[li];
+    if (lane == 0) {
+      GroupInfo gi{};
+      gi.start = d;
+      gi.n = rg.nhits;
+      gi.query = rg.query;
+      gi.ext_di = rg.ext_di;
+      gi.ext_len = rg.ext_len;
+      gi.survive = 1;
+      gi.ext_sorted = (rg.flags & kRunExt) ? 1 : 0;
+      groups[li] = gi;
+      dp_list[atomicAdd(counts + 1, 1u)] = li;
+      if (gi.ext_sorted) ext_list[atomicAdd(counts + 0, 1u)] = li;
+    }
+    const uint32_t sq = o.src_q[li];
+    if (sq != kNoLink) {
+      uint64_t lo = o.sorted_off[sq], hi = o.sorted_off[sq + 1];
+      const uint64_t end = hi, first = static_cast<uint64_t>(rg.ext_di) << 32;
+      while (lo < hi) {
+        const uint64_t mid = (lo + hi) >> 1;
+        if (o.sorted_keys[mid] < first)
+          lo = mid + 1;
+        else
+          hi = mid;
+      }
+      for (uint32_t j = lane; j < rg.nhits && lo + j < end; j += 32) {
+        keys[d + j] = o.sorted_keys[lo + j];
+        vals[d + j] = o.sorted_vals[lo + j];
+      }
+      continue;
+    }
+    for (uint32_t i = 0; i < rg.nruns; ++i) {
+      const uint64_t key = t.keys[rg.run0 + i];
+      const uint32_t e = t.vals[rg.run0 + i], l = t.rlen[rg.run0 + i];
+      for (uint32_t j = lane; j < l; j += 32) {
+        keys[d + j] = key + j;
+        vals[d + j] = e + j;
+      }
+      d += l;
+    }
+  }
+}
+
+// Rows of a batch of open groups join the pool under their run groups.
+__global__ void append_rows_kernel(const OverlapRow* __restrict__ from,
+                                   const uint32_t* __restrict__ nfrom,
+                                   const uint32_t* __restrict__ list,
+                                   OverlapRow* __restrict__ pool, uint64_t pool_cap,
+                                   uint32_t* __restrict__ pool_count, DeviceStatus* st) {
+  const uint32_t n = *nfrom;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    OverlapRow r = from[i];
+    r.group = list[r.group];
+    const uint32_t d = atomicAdd(pool_count, 1u);
+    if (d < pool_cap)
+      pool[d] = r;
+    else
+      raise_status(st, kDevProposalOverflow, 1, static_cast<int64_t>(r.group));
+  }
+}
+
+__global__ void fold_rows_kernel(const uint32_t* __restrict__ open_list, uint32_t nopen,
+                                 const uint32_t* __restrict__ rows,
+                                 uint32_t* __restrict__ group_rows) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < nopen) group_rows[open_list[i]] = rows[i];
+}
+
+__global__ void scatter_rows_kernel(const OverlapRow* __restrict__ pool,
+                                    const uint32_t* __restrict__ npool,
+                                    const uint32_t* __restrict__ kept,
+                                    const uint64_t* __restrict__ kept_off,
+                                    OverlapRow* __restrict__ rows) {
+  const uint32_t n = *npool;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const OverlapRow r = pool[i];
+    if (r.rank < kept[r.group]) rows[kept_off[r.group] + r.rank] = r;
+  }
+}
+
+__global__ void query_groups_kernel(const GroupInfo* __restrict__ bounds,
+                                    const uint64_t* __restrict__ ngroups, uint32_t nq,
+                                    uint64_t* __restrict__ qg) {
+  const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q > nq) return;
+  uint64_t lo = 0, hi = *ngroups;
+  while (lo < hi) {
+    const uint64_t mid = (lo + hi) >> 1;
+    if (bounds[mid].query < q)
+      lo = mid + 1;
+    else
+      hi = mid;
+  }
+  qg[q] = lo;
+}
+
+}  // namespace
+
+cudaError_t index_neighbours(const uint64_t* pos, uint64_t npos, const uint64_t* words,
+                             const uint64_t* base_off, const int32_t* slot_len, int k,
+                             uint8_t* nbr, cudaStream_t s) {
+  if (npos == 0) return cudaSuccess;
+  count_launch();
+  neighbour_kernel<<<grid(npos, 256), 256, 0, s>>>(pos, npos, words, base_off, slot_len, k, nbr);
+  return cudaGetLastError();
+}
+
+cudaError_t runs_probe(const DeviceIndex& idx, const QueryBatch& q, uint64_t* wmeta,
+                       uint8_t* wflags, uint32_t* wself, uint32_t* cbits, uint32_t* fbits,
+                       uint32_t* tile_filt, unsigned long long* hit_total, cudaStream_t s) {
+  if (q.nwin == 0) return cudaSuccess;
+  count_launch();
+  probe_kernel<<<grid(q.nwin, 256), 256, 0, s>>>(idx, q, wmeta, wflags, wself, cbits, fbits,
+                                                 tile_filt, hit_total);
+  return cudaGetLastError();
+}
+
+cudaError_t runs_count(const DeviceIndex& idx, const QueryBatch& q, const uint64_t* wmeta,
+                       const uint8_t* wflags, const uint32_t* wself, uint32_t* nstart,
+                       uint32_t* tile_start, cudaStream_t s) {
+  if (q.nwin == 0) return cudaSuccess;
+  count_launch();
+  start_count_kernel<<<grid(q.nwin, 256), 256, 0, s>>>(idx, q, wmeta, wflags, wself, nstart,
+                                                       tile_start);
+  return cudaGetLastError();
+}
+
+cudaError_t runs_query_offsets(const QueryBatch& q, const uint32_t* nstart,
+                               const uint64_t* tile_off, const uint32_t* fbits,
+                               const uint64_t* ftile_off, uint64_t* q_off, uint64_t* f_off,
+                               cudaStream_t s) {
+  count_launch();
+  query_offsets_kernel<<<grid(q.nq + 1ull, 128), 128, 0, s>>>(q, nstart, tile_off, fbits,
+                                                              ftile_off, q_off, f_off);
+  return cudaGetLastError();
+}
+
+cudaError_t runs_emit(const DeviceIndex& idx, const QueryBatch& q, const uint64_t* wmeta,
+                      const uint8_t* wflags, const uint32_t* wself, const uint32_t* nstart,
+                      const uint64_t* tile_off, const uint32_t* fbits, const uint64_t* ftile_off,
+                      uint64_t* keys, uint32_t* vals, int32_t* fpos, cudaStream_t s) {
+  if (q.nwin == 0) return cudaSuccess;
+  count_launch();
+  start_emit_kernel<<<grid(q.nwin, 256), 256, 0, s>>>(idx, q, wmeta, wflags, wself, nstart,
+                                                      tile_off, fbits, ftile_off, keys, vals,
+                                                      fpos);
+  return cudaGetLastError();
+}
+
+cudaError_t runs_groups(const RunTables& t, const ChainParams& p, int num_sms, cudaStream_t s) {
+  if (t.max_groups == 0) return cudaSuccess;
+  count_launch();
+  const uint64_t blocks = (t.max_groups + kGroupWarps - 1) / kGroupWarps;
+  run_groups_kernel<<<static_cast<unsigned>(std::min<uint64_t>(blocks, 64ull * num_sms)),
+                      kGroupWarps * 32, 0, s>>>(t, p);
+  return cudaGetLastError();
+}
+
+cudaError_t runs_open_info(const RunTables& t, uint32_t nopen, OpenInfo* out, cudaStream_t s) {
+  if (nopen == 0) return cudaSuccess;
+  count_launch();
+  open_info_kernel<<<grid(nopen, 256), 256, 0, s>>>(t, nopen, out);
+  return cudaGetLastError();
+}
+
+cudaError_t runs_tie_keys(const RunTables& t, const OpenBatch& o, uint64_t* tie_q,
+                          uint64_t* tie_key, uint32_t* count, uint32_t cap, cudaStream_t s) {
+  if (o.n == 0) return cudaSuccess;
+  count_launch();
+  tie_keys_kernel<<<grid(o.n, 64), 64, 0, s>>>(t, o, tie_q, tie_key, count, cap);
+  return cudaGetLastError();
+}
+
+cudaError_t runs_expand(const RunTables& t, const OpenBatch& o, uint64_t* keys, uint32_t* vals,
+                        GroupInfo* groups, uint32_t* ext_list, uint32_t* dp_list,
+                        uint32_t* counts, int num_sms, cudaStream_t s) {
+  if (o.n == 0) return cudaSuccess;
+  count_launch();
+  expand_kernel<<<static_cast<unsigned>(std::min<uint64_t>(grid(o.n * 32ull, 256),
+                                                           16ull * num_sms)),
+                  256, 0, s>>>(t, o, keys, vals, groups, ext_list, dp_list, counts);
+  return cudaGetLastError();
+}
+
+cudaError_t runs_append_rows(const OverlapRow* from, const uint32_t* nfrom, const uint32_t* list,
+                             OverlapRow* pool, uint64_t pool_cap, uint32_t* pool_count,
+                             DeviceStatus* st, int num_sms, cudaStream_t s) {
+  count_launch();
+  append_rows_kernel<<<num_sms, 256, 0, s>>>(from, nfrom, list, pool, pool_cap, pool_count, st);
+  return cudaGetLastError();
+}
+
+cudaError_t runs_fold_rows(const uint32_t* open_list, uint32_t nopen, const uint32_t* rows,
+                           uint32_t* group_rows, cudaStream_t s) {
+  if (nopen == 0) return cudaSuccess;
+  count_launch();
+  fold_rows_kernel<<<grid(nopen, 256), 256, 0, s>>>(open_list, nopen, rows, group_rows);
+  return cudaGetLastError();
+}
+
+cudaError_t runs_scatter_rows(const OverlapRow* pool, const uint32_t* npool, uint64_t max_pool,
+                              const uint32_t* kept, const uint64_t* kept_off, OverlapRow* rows,
+                              cudaStream_t s) {
+  if (max_pool == 0) return cudaSuccess;
+  count_launch();
+  scatter_rows_kernel<<<std::min(grid(max_pool, 256), 2048u), 256, 0, s>>>(pool, npool, kept,
+                                                                          kept_off, rows);
+  return cudaGetLastError();
+}
+
+cudaError_t runs_query_groups(const RunTables& t, uint64_t* qg, cudaStream_t s) {
+  count_launch();
+  query_groups_kernel<<<grid(t.qb.nq + 1ull, 128), 128, 0, s>>>(t.bounds, t.ngroups, t.qb.nq, qg);
+  return cudaGetLastError();
+}
+
+}  // namespace cuflye

@@ -205,15 +205,18 @@ cuflye_status cuflye_overlaps(cuflye_ctx* ctx, size_t n, const int64_t* query_id
  * 1 gives the plain one-read-per-launch path. */
 cuflye_status cuflye_set_batch_queries(cuflye_ctx* ctx, size_t queries_per_pass);
 
-/* Sorted emission (no counterpart in the reference; on by default): overlap
- * and read-to-graph calls on a built index write each query's candidate hits
- * straight into the order of Flye's KmerMatch sort, one block per query, and
- * decide most target groups' prefilter on the way, instead of writing them
- * in generation order and sorting.  The rows are the same either way.  1
- * (the default) takes it for passes whose windows average at least 6 hits
- * and that hold at least two queries per SM, where it pays off; sparser
- * passes (reads against a genome or a graph) and small ones (the one-read
- * path) emit and sort.  2 takes it for every pass, 0 for none (for comparison).  A pass
+/* How overlap and read-to-graph calls on a built index find and sort their
+ * hits (no counterpart in the reference).  The rows are the same either way.
+ * 1 (the default): as runs of hits at consecutive positions, found, sorted and
+ * chained without writing the hits, where the index holds the tables for it
+ * (an odd k, and memory for about 1.3 bytes an entry and base beside the index);
+ * groups whose result depends on an order of equal keys take the hit path.
+ * Without the tables, passes whose windows average at least 6 hits and that
+ * hold at least two queries per SM take the sorted emission, others emit and
+ * sort.  2: the sorted emission for every pass (each query's hits written
+ * straight into the order of Flye's KmerMatch sort, one block per query, with
+ * most target groups' prefilter decided on the way).  0: hits written in
+ * generation order and sorted (for comparison).  A sorted-emission pass
  * holding a query that hits more than 2,048 distinct targets takes the emit
  * + sort path by itself (counted in cuflye_last_sort_stats, entry 7). */
 cuflye_status cuflye_set_sorted_emission(cuflye_ctx* ctx, int enable);
@@ -493,7 +496,9 @@ cuflye_status cuflye_last_timing(const cuflye_ctx* ctx, double* stage_ms, uint64
  * std::sort; the others take the libstdc++-order sort.  counts[0] / [1]:
  * queries whose KmerMatch sort ran plain / libstdc++-order; [2] / [3]:
  * ext-sorted groups put in ext-pos order plain (most already are) /
- * libstdc++-order; [4]: groups whose backtrack picked its starts by score
+ * libstdc++-order (on the run path [1] counts the queries whose hits were
+ * sorted for the groups that need their order, and [2] and [4] every group
+ * chained over its runs); [4]: groups whose backtrack picked its starts by score
  * itself; [5]: 0 (no score order is sorted ahead of the backtrack); [6]:
  * groups whose backtrack ran again in the libstdc++ order because equal
  * scores could change their result; [7]: passes that left the sorted

@@ -1,0 +1,111 @@
+"""GPU: the run path (hits found, sorted and chained as runs, the default on a
+built index of an odd k) against the hit path and the oracle, row for row,
+divergence bits included.  The cases put run and tile edges everywhere: reads
+of every length around the 32-window tiles, reads that end at a target's ends,
+tandem arrays (equal positions at every sort point, split runs, groups and
+queries left to the hit path), long targets out of ext order and noisy reads."""
+
+import numpy as np
+import pytest
+
+from test_gpu_parity import oracle_index, overlap_tuples_gpu, overlap_tuples_oracle
+
+pytestmark = pytest.mark.gpu
+
+VARIANTS = ({}, {"only_max_ext": 0}, {"only_max_ext": 0, "check_overhang": 0, "min_overlap": 100},
+            {"max_overlaps": 3}, {"max_jump": 40, "max_gap": 10})
+
+
+def _check(gpu, oracle_mod, targets, queries, k, min_freq, max_freq, params, variants=VARIANTS):
+    from cuflye_gb300.backend import OverlapParams
+    oracle_mod.set_stable(False)
+    idx, _ = oracle_index(oracle_mod, targets, k, min_freq, max_freq)
+    gpu.build_index(targets, k, min_freq, max_freq)
+    b = oracle_mod.SeqBatch(queries.ids, queries.offsets, queries.bases.tobytes())
+    rows = 0
+    for variant in variants:
+        pv = dict(params, kmer_size=k, **variant)
+        runs = gpu.overlaps(queries, OverlapParams.make(**pv))
+        gpu.set_sorted_emission(0)
+        try:
+            hits = gpu.overlaps(queries, OverlapParams.make(**pv))
+        finally:
+            gpu.set_sorted_emission(1)
+        exp = oracle_mod.overlaps(idx, b, oracle_mod.default_params(**pv))
+        assert runs.tobytes() == hits.tobytes(), variant
+        assert overlap_tuples_gpu(runs) == overlap_tuples_oracle(exp), variant
+        rows += len(runs)
+    return rows
+
+
+@pytest.mark.parametrize("k", [11, 15, 16, 17, 31])
+def test_read_lengths_around_tiles(gpu, oracle_mod, k):
+    """Reads whose windows end just before, at and after a 32-window tile,
+    some of them a target's very ends, both strands, one base apart."""
+    from cuflye_gb300 import synth
+    rng = np.random.default_rng(k)
+    genome = synth.random_genome(rng, 3000)
+    lengths = [k - 1, k, k + 1, k + 30, k + 31, k + 32, k + 62, k + 63, k + 64, k + 65, 400, 900]
+    seqs = []
+    for n in lengths:
+        for s in (0, 1, 31, 32, 33, 500, len(genome) - n):
+            seqs.append(genome[s:s + n])
+    seqs += [genome[:1500], genome[1400:], synth.revcomp(genome[700:2200])]
+    for i in range(0, len(seqs), 3):
+        seqs[i] = synth.revcomp(seqs[i])
+    for i in range(0, len(seqs), 4):
+        seqs[i] = synth.mutate(rng, seqs[i], 0.01, 0.003, 0.003)
+    reads = synth.ReadSet.from_strings(np.arange(1, len(seqs) + 1), [x.tobytes() for x in seqs])
+    params = dict(synth.OVERLAP_PARAMS, min_overlap=40)
+    assert _check(gpu, oracle_mod, reads, reads, k, 1, 1000, params) > 0
+
+
+@pytest.mark.parametrize("seed", [1, 2, 3, 4, 5, 6])
+def test_tandem_arrays(gpu, oracle_mod, seed):
+    from cuflye_gb300 import synth
+    wl = synth.tandem_case(20 + seed, genome_len=10_000, coverage=4.0, arrays=1,
+                           copy_div=(0.0, 0.01, 0.04, 0.1, 0.2, 0.02)[seed - 1])
+    assert _check(gpu, oracle_mod, wl.reads, wl.reads, wl.k, wl.min_freq, 1000, wl.params) > 0
+
+
+@pytest.mark.parametrize("sub,indel", [(0.0, 0.0), (0.002, 0.001), (0.02, 0.02), (0.05, 0.03)])
+def test_error_rates(gpu, oracle_mod, sub, indel):
+    from cuflye_gb300 import synth
+    wl = synth.small_overlap_case(31, genome_len=50_000, coverage=8.0, sub=sub, ins=indel,
+                                  dele=indel, repeat=True)
+    _check(gpu, oracle_mod, wl.reads, wl.reads, wl.k, 1, wl.max_freq, wl.params)
+
+
+def test_long_targets_and_strands(gpu, oracle_mod):
+    """Groups sorted by ext pos, queries under positive, negative and unknown
+    ids, and an indexed id whose sequence differs from the indexed one."""
+    from cuflye_gb300 import synth
+    rng = np.random.default_rng(77)
+    sw = synth.serving_workload(seed=9, genome_len=1_500_000, n_queries=40, piece=400_000)
+    q = sw.queries
+    seqs = [np.frombuffer(q.seq(i), dtype=np.uint8) for i in range(q.n)]
+    t0 = np.frombuffer(sw.targets.seq(0), dtype=np.uint8)[1000:31_000]
+    seqs += [t0, synth.revcomp(t0), synth.mutate(rng, t0, 0.02, 0.01, 0.01)]
+    ids = list(q.ids) + [1, -1, 2]
+    qs = synth.ReadSet.from_strings(np.array(ids, dtype=np.int64), [x.tobytes() for x in seqs])
+    assert _check(gpu, oracle_mod, sw.targets, qs, sw.k, 1, 32, sw.params, VARIANTS[:3]) > 0
+
+
+def test_run_path_is_taken(gpu):
+    """The default takes runs (its algorithmic sort bytes count runs, far fewer
+    than hits); an even k has no run tables."""
+    from cuflye_gb300 import synth
+    from cuflye_gb300.backend import OverlapParams
+    wl = synth.small_overlap_case(5, genome_len=60_000, sub=0.001, ins=0.0, dele=0.0)
+    for k, fewer in ((15, True), (16, False)):
+        gpu.build_index(wl.reads, k, 2, 40)
+        p = OverlapParams.make(**dict(wl.params, kmer_size=k))
+        gpu.overlaps(wl.reads, p)
+        runs = gpu.last_timing()[1][1]
+        gpu.set_sorted_emission(0)
+        try:
+            gpu.overlaps(wl.reads, p)
+        finally:
+            gpu.set_sorted_emission(1)
+        hits = gpu.last_timing()[1][1]
+        assert (runs * 4 < hits) == fewer
