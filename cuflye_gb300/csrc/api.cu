@@ -432,14 +432,14 @@ BuiltIndex build_one_range(cuflye_ctx* c, const WindowSet& w, const std::vector<
     CUFLYE_CHECK(cudaMemcpyAsync(win_off, w.win_off, (static_cast<uint64_t>(w.nslots) + 1) * 8,
                                  cudaMemcpyDeviceToDevice, st));
   CUFLYE_CHECK(index_copy_positions(r.vals, r.run_id, r.run_start, r.cls, r.kept_off, w.nwin,
-                                    bi.pos, st, self_at, win_off, w.slot_len, w.k));
+                                    bi.pos, true, st, self_at, win_off, w.slot_len, w.k));
   bi.self_at = self_at;
   bi.win_off = win_off;
   bi.cap = 16;
   while (bi.cap < 2 * r.nruns) bi.cap <<= 1;
   bi.table = buf<TableEntry>(c, "ix_table", bi.cap);
   CUFLYE_CHECK(cudaMemsetAsync(bi.table, 0xff, bi.cap * sizeof(TableEntry), st));
-  CUFLYE_CHECK(index_insert(r.keys, r.vals, r.run_start, r.cls, r.kept_off, r.nruns, 0, true,
+  CUFLYE_CHECK(index_insert(r.keys, bi.pos, r.run_start, r.cls, r.kept_off, r.nruns, 0, true,
                             bi.table, bi.cap, c->status, st));
   check_device_status(c);
   bi.npos = r.npos;
@@ -566,9 +566,9 @@ BuiltIndex build_key_ranges(cuflye_ctx* c, const WindowSet& w, const std::vector
           throw Error(CUFLYE_ERR_CUDA, "k-mer index build: a key range's positions overrun "
                                        "the counted total");
         CUFLYE_CHECK(index_copy_positions(r.vals, r.run_id, r.run_start, r.cls, r.kept_off, r.nw,
-                                          bi.pos + base, st));
-        CUFLYE_CHECK(index_insert(r.keys, r.vals, r.run_start, r.cls, r.kept_off, r.nruns, base,
-                                  true, bi.table, bi.cap, c->status, st));
+                                          bi.pos + base, false, st));
+        CUFLYE_CHECK(index_insert(r.keys, bi.pos + base, r.run_start, r.cls, r.kept_off, r.nruns,
+                                  base, true, bi.table, bi.cap, c->status, st));
         written += r.npos;
       });
   if (written != npos)
@@ -693,19 +693,21 @@ void build_index(cuflye_ctx* c, int k, size_t n, const int64_t* ids, const int64
   CUFLYE_CHECK(cudaMemcpyAsync(d_signed, c->slot_signed_h.data(), n * 8, cudaMemcpyHostToDevice,
                                st));
   const WindowSet ws{words, d_base, d_win, d_len, static_cast<uint32_t>(n), nwin, k};
-  // LSD digits: position bytes, stored-id bytes, key bytes
-  std::vector<int> digits;
+  // LSD digits: position bytes, stored-id bytes, key bytes; windows enumerated
+  // in order (one range) need the key bytes only
+  std::vector<int> digits, key_digits;
   const int pbytes = (bits_for(static_cast<uint64_t>(maxlen)) + 7) / 8;
   const int dbytes = (bits_for(2 * n) + 7) / 8;
   const int kbytes = (2 * k + 7) / 8;
   for (int d = 0; d < pbytes; ++d) digits.push_back(d);
   for (int d = 0; d < dbytes; ++d) digits.push_back(4 + d);
   for (int d = 0; d < kbytes; ++d) digits.push_back(8 + d);
+  for (int d = 0; d < kbytes; ++d) key_digits.push_back(8 + d);
   BuiltIndex bi;
   bool ranges = c->build_window_cap != 0 && nwin > c->build_window_cap;
   if (!ranges) {
     try {
-      bi = build_one_range(c, ws, digits, min_freq, max_freq);
+      bi = build_one_range(c, ws, key_digits, min_freq, max_freq);
       c->build_ranges = 1;
     } catch (const Error& e) {
       if (e.code != CUFLYE_ERR_BUDGET) throw;
@@ -801,11 +803,11 @@ void build_index_entries(cuflye_ctx* c, int k, size_t n, const int64_t* tids, co
   uint64_t* kept_off = buf<uint64_t>(c, "ib_keptoff", nruns + 1);
   const uint64_t npos = scan_u32(c, kept, kept_off, nruns, "ib_scan");
   uint64_t* pos = buf<uint64_t>(c, "ix_pos", npos);
-  CUFLYE_CHECK(index_copy_positions(vals, run_id, run_start, cls, kept_off, nn, pos, st));
+  CUFLYE_CHECK(index_copy_positions(vals, run_id, run_start, cls, kept_off, nn, pos, false, st));
   const uint64_t cap = table_capacity(nruns + nrep);
   TableEntry* table = buf<TableEntry>(c, "ix_table", cap);
   CUFLYE_CHECK(cudaMemsetAsync(table, 0xff, cap * sizeof(TableEntry), st));
-  CUFLYE_CHECK(index_insert(keys, vals, run_start, cls, kept_off, nruns, 0, false, table, cap,
+  CUFLYE_CHECK(index_insert(keys, pos, run_start, cls, kept_off, nruns, 0, false, table, cap,
                             c->status, st));
   if (nrep) {
     uint64_t* d_rep = buf<uint64_t>(c, "ib_rep", nrep);

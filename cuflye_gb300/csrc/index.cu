@@ -10,13 +10,16 @@
 // order.  Lookups serve isRepetitive / kmerFreq / iterKmerPos as called at
 // patches/flye/2.9.6/0002-cuflye-candidate-backend-seam.patch:55-80.
 //
-// Construction: enumerate windows -> stable LSD radix sort of
-// (key | stored id | stored position) -> run detection -> solid positions
-// copied in run order -> open-addressing insert (linear probing, load <= 1/2,
-// the table sized at twice its entries).
+// Construction: enumerate windows in (target, position) order -> stable LSD
+// radix sort by key -> run detection -> solid positions copied in (stored id,
+// stored position) order -> open-addressing insert (linear probing, load <=
+// 1/2, the table sized at twice its entries).  Within a run the sort keeps
+// window order, which is the bucket's order but for the entries of one target:
+// those of its reverse strand come after the others, in reverse.
 // When the windows do not fit the memory budget at once, the same steps run
-// per contiguous key range (ranges cut from a histogram of key prefixes), in
-// two passes: the first counts each prefix's solid positions and table
+// per contiguous key range (ranges cut from a histogram of key prefixes; a
+// range's windows are appended in no order, and the sort orders them by stored
+// id and position as well), in two passes: the first counts each prefix's solid positions and table
 // entries, the second writes every range's positions at its prefix's offset
 // in the final array and inserts its runs into the final table.  The
 // position array is then the same as one range's.
@@ -170,12 +173,14 @@ __global__ void classify_runs_kernel(const uint64_t* __restrict__ run_start, uin
   }
 }
 
+// window_order: the runs are in (target, window) order, not in bucket order.
 __global__ void copy_positions_kernel(const uint64_t* __restrict__ vals,
                                       const uint64_t* __restrict__ flags_scan,
                                       const uint64_t* __restrict__ run_start,
                                       const uint8_t* __restrict__ cls,
                                       const uint64_t* __restrict__ kept_off, uint64_t n,
-                                      uint64_t* __restrict__ pos, uint32_t* __restrict__ self_at,
+                                      uint64_t* __restrict__ pos, bool window_order,
+                                      uint32_t* __restrict__ self_at,
                                       const uint64_t* __restrict__ win_off,
                                       const int32_t* __restrict__ slot_len, int k) {
   const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -187,7 +192,21 @@ __global__ void copy_positions_kernel(const uint64_t* __restrict__ vals,
   while (run_start[r] > i) --r;
   if (cls[r] != 1) return;
   const uint64_t v = vals[i];
-  pos[kept_off[r] + (i - run_start[r])] = v;
+  const uint64_t r0 = run_start[r], r1 = run_start[r + 1];
+  uint64_t at = i - r0;
+  if (window_order) {
+    // among the run's entries of this target: forward ones as they come, then
+    // the reverse strand's from the last to the first (a window further on in
+    // the target is nearer to the reverse strand's start)
+    const uint64_t t = v >> 33;
+    const bool rev = (v >> 32) & 1u;
+    uint64_t ahead = 0, later = 0;  // entries that go before this one, either side of it
+    uint64_t lo = i, hi = i + 1;
+    for (; lo > r0 && (vals[lo - 1] >> 33) == t; --lo) ahead += !((vals[lo - 1] >> 32) & 1u);
+    for (; hi < r1 && (vals[hi] >> 33) == t; ++hi) later += rev || !((vals[hi] >> 32) & 1u);
+    at = (lo - r0) + ahead + (rev ? later : 0u);
+  }
+  pos[kept_off[r] + at] = v;
   if (self_at) {
     // the window this entry came from: its forward position in its target
     const uint32_t sid = static_cast<uint32_t>(v >> 32);
@@ -195,7 +214,7 @@ __global__ void copy_positions_kernel(const uint64_t* __restrict__ vals,
     const int64_t sp = static_cast<int64_t>(v & 0xffffffffu);
     const int64_t p = (sid & 1u) ? static_cast<int64_t>(slot_len[slot]) - sp - k : sp;
     const uint64_t w = win_off[slot] + static_cast<uint64_t>(p);
-    if (p >= 0 && w < win_off[slot + 1]) self_at[w] = static_cast<uint32_t>(i - run_start[r]);
+    if (p >= 0 && w < win_off[slot + 1]) self_at[w] = static_cast<uint32_t>(at);
   }
 }
 
@@ -220,13 +239,11 @@ __device__ bool table_insert(TableEntry* table, uint64_t cap, uint64_t key, uint
 }
 
 // Table word of run r (class 1 solid or 2 repetitive) whose positions start
-// at pos_off in the position array.  vals: the run's entries, (stored id <<
-// 32) | stored position.  With sorted_ids the entries of a run are in (id,
-// position) order and a repeated id shows as two neighbours; otherwise
-// (explicit entries in input order) every run of two or more entries is
-// marked.
-__device__ __forceinline__ uint64_t run_meta(const uint64_t* __restrict__ vals, uint64_t r0,
-                                             uint64_t freq, uint8_t cls, uint64_t pos_off,
+// at pos_off in the position array.  bucket: the run's entries, (stored id <<
+// 32) | stored position.  With sorted_ids they are in (id, position) order and
+// a repeated id shows as two neighbours; otherwise (explicit entries in input
+// order) every run of two or more entries is marked.
+__device__ __forceinline__ uint64_t run_meta(const uint64_t* __restrict__ bucket, uint64_t freq, uint8_t cls, uint64_t pos_off,
                                              bool sorted_ids) {
   if (cls == 2) {
     const uint64_t c = freq < ((1ULL << kCountBits) - 1) ? freq : ((1ULL << kCountBits) - 1);
@@ -235,13 +252,13 @@ __device__ __forceinline__ uint64_t run_meta(const uint64_t* __restrict__ vals, 
   uint64_t meta = (pos_off & kOffsetMask) | (freq << 40);
   bool dup = !sorted_ids && freq > 1;
   for (uint64_t e = 1; sorted_ids && e < freq && !dup; ++e)
-    dup = (vals[r0 + e] >> 32) == (vals[r0 + e - 1] >> 32);
+    dup = (bucket[e] >> 32) == (bucket[e - 1] >> 32);
   if (dup) meta |= kDupIdsBit;
   return meta;
 }
 
 __global__ void insert_kernel(const uint64_t* __restrict__ keys,
-                              const uint64_t* __restrict__ vals,
+                              const uint64_t* __restrict__ pos,
                               const uint64_t* __restrict__ run_start,
                               const uint8_t* __restrict__ cls,
                               const uint64_t* __restrict__ kept_off, uint64_t nruns,
@@ -251,7 +268,7 @@ __global__ void insert_kernel(const uint64_t* __restrict__ keys,
   if (r >= nruns || cls[r] == 0) return;
   const uint64_t r0 = run_start[r];
   const uint64_t meta =
-      run_meta(vals, r0, run_start[r + 1] - r0, cls[r], pos_base + kept_off[r], sorted_ids);
+      run_meta(pos + kept_off[r], run_start[r + 1] - r0, cls[r], pos_base + kept_off[r], sorted_ids);
   if (!table_insert(table, cap, keys[r0], meta, false)) raise_status(st, kDevTableFull, 0, r);
 }
 
@@ -376,22 +393,23 @@ cudaError_t index_classify_runs(const uint64_t* run_start, uint64_t nruns, uint3
 cudaError_t index_copy_positions(const uint64_t* vals, const uint64_t* run_id,
                                  const uint64_t* run_start, const uint8_t* cls,
                                  const uint64_t* kept_off, uint64_t n, uint64_t* pos,
-                                 cudaStream_t s, uint32_t* self_at, const uint64_t* win_off,
-                                 const int32_t* slot_len, int k) {
+                                 bool window_order, cudaStream_t s, uint32_t* self_at,
+                                 const uint64_t* win_off, const int32_t* slot_len, int k) {
   if (n == 0) return cudaSuccess;
   count_launch();
   copy_positions_kernel<<<grid(n, 256), 256, 0, s>>>(vals, run_id, run_start, cls, kept_off, n,
-                                                     pos, self_at, win_off, slot_len, k);
+                                                     pos, window_order, self_at, win_off,
+                                                     slot_len, k);
   return cudaGetLastError();
 }
 
-cudaError_t index_insert(const uint64_t* keys, const uint64_t* vals, const uint64_t* run_start,
+cudaError_t index_insert(const uint64_t* keys, const uint64_t* pos, const uint64_t* run_start,
                          const uint8_t* cls, const uint64_t* kept_off, uint64_t nruns,
                          uint64_t pos_base, bool sorted_ids, TableEntry* table, uint64_t cap,
                          DeviceStatus* st, cudaStream_t s) {
   if (nruns == 0) return cudaSuccess;
   count_launch();
-  insert_kernel<<<grid(nruns, 256), 256, 0, s>>>(keys, vals, run_start, cls, kept_off, nruns,
+  insert_kernel<<<grid(nruns, 256), 256, 0, s>>>(keys, pos, run_start, cls, kept_off, nruns,
                                                  pos_base, sorted_ids, table, cap, st);
   return cudaGetLastError();
 }

@@ -144,17 +144,19 @@ cudaError_t index_enumerate_range(const uint64_t* words, const uint64_t* base_of
 cudaError_t index_classify_runs(const uint64_t* run_start, uint64_t nruns, uint32_t min_freq,
                                 uint32_t max_freq, uint32_t* kept, uint8_t* cls,
                                 unsigned long long* tally, cudaStream_t s);
+// Solid runs' entries into pos, in (stored id, stored position) order.
+// window_order: the runs hold them in (target, window) order instead.
 cudaError_t index_copy_positions(const uint64_t* vals, const uint64_t* run_id,
                                  const uint64_t* run_start, const uint8_t* cls,
                                  const uint64_t* kept_off, uint64_t n, uint64_t* pos,
-                                 cudaStream_t s, uint32_t* self_at = nullptr,
+                                 bool window_order, cudaStream_t s, uint32_t* self_at = nullptr,
                                  const uint64_t* win_off = nullptr,
                                  const int32_t* slot_len = nullptr, int k = 0);
 // Table insert of every solid and repetitive run, a solid run's positions
-// at pos_base + kept_off of the position array.  Solid buckets that list
+// at pos + kept_off (pos_base + kept_off of the position array).  Solid buckets that list
 // one stored id twice get kDupIdsBit (sorted_ids: runs are in (id, position)
 // order; otherwise every run of two or more entries is marked).
-cudaError_t index_insert(const uint64_t* keys, const uint64_t* vals, const uint64_t* run_start,
+cudaError_t index_insert(const uint64_t* keys, const uint64_t* pos, const uint64_t* run_start,
                          const uint8_t* cls, const uint64_t* kept_off, uint64_t nruns,
                          uint64_t pos_base, bool sorted_ids, TableEntry* table, uint64_t cap,
                          DeviceStatus* st, cudaStream_t s);
