@@ -824,10 +824,10 @@ cudaError_t runs_order(const RunTables& t, int num_sms, cudaStream_t s) {
   if (e != cudaSuccess) return e;
   count_launch();
   mid<<<static_cast<unsigned>(std::min<uint64_t>(t.max_groups, 8ull * num_sms)), 128,
-        sizeof(OrderSmem<512, 2048>), s>>>(t, t.counts + kRcWork);
+        sizeof(OrderSmem<512, 2048>), s>>>(t, t.counts + kRcWork + 1);
   count_launch();
   big<<<static_cast<unsigned>(std::min<uint64_t>(t.max_groups, num_sms)), 512,
-        sizeof(OrderSmem<4096, 8192>), s>>>(t, t.counts + kRcWork + 1);
+        sizeof(OrderSmem<4096, 8192>), s>>>(t, t.counts + kRcWork + 2);
   return cudaGetLastError();
 }
 
@@ -844,7 +844,7 @@ cudaError_t runs_dp(const RunTables& t, const ChainParams& p, int num_sms, int p
   const uint64_t need = (t.max_groups + kWarpsPerBlock - 1) / kWarpsPerBlock;
   count_launch();
   run_dp_kernel<<<static_cast<unsigned>(std::min(blocks, need)), kWarpsPerBlock * 32, 0, s>>>(
-      t, p, t.counts + kRcWork + 2);
+      t, p, t.counts + kRcWork + 3);
   return cudaGetLastError();
 }
 
@@ -858,7 +858,7 @@ cudaError_t runs_backtrack(const RunTables& t, const ChainParams& p, const uint6
   count_launch();
   run_backtrack_kernel<<<static_cast<unsigned>(std::min(blocks, need)), kWarpsPerBlock * 32, 0,
                          s>>>(t, p, f_off, fpos, logt, pool, pool_cap, group_rows, st,
-                              t.counts + kRcWork + 3);
+                              t.counts + kRcWork + 4);
   return cudaGetLastError();
 }
 

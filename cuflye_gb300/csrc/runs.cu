@@ -294,9 +294,24 @@ __global__ void __launch_bounds__(256) start_emit_kernel(
   }
 }
 
-// Hits of the run that starts at window p of query qi and position pos of
-// target strand id: the windows over which query and target agree, up to most,
-// and up to the query's next window that is not solid.
+// Agreement of query and target over the next 32 bases from base k of a
+// window on (m windows into a run): bases that agree, and the query's
+// consecutive solid windows from the next one on, 32 at most.
+__device__ __forceinline__ int32_t agree(uint64_t qb, uint64_t tb, uint32_t solid_bits) {
+  const uint64_t diff = qb ^ tb;
+  const int32_t same = diff ? __clzll(static_cast<long long>(diff)) >> 1 : 32;
+  const uint32_t holes = ~solid_bits;
+  return min(same, holes ? __ffs(holes) - 1 : 32);
+}
+
+constexpr int kWide = 2;  // 32-base blocks of a wide step
+
+// Hits of the run that starts at window p of a query (first base qbase, first
+// window w0) and position pos of a target strand: the windows over which the
+// two agree, up to most, and up to the query's next window that is not solid.
+// The first 32 bases alone decide most runs of noisy reads; longer runs go on
+// 64 bases at a time, all loads issued together (a step is bound by the latency
+// of its scattered loads; 96 or 128 bases cost more registers than they gain).
 __device__ __forceinline__ int32_t run_length(const RunTables& t, uint64_t qbase, uint64_t w0,
                                               uint64_t tbase, int32_t tlen, bool rev, int32_t p,
                                               int32_t pos, int32_t most) {
@@ -304,29 +319,63 @@ __device__ __forceinline__ int32_t run_length(const RunTables& t, uint64_t qbase
   int32_t m = 0;  // agreeing bases after the first window
   while (m < most - 1) {
     const int32_t x = pos + k + m;
-    const uint64_t qb = bases32(t.qb.words, qbase + static_cast<uint64_t>(p) + k + m);
-    uint64_t tb;
-    if (!rev) {
-      tb = bases32(t.idx.twords, tbase + static_cast<uint64_t>(x));
-    } else {
-      // bases x .. x + 31 of the reverse strand: the reverse complement of
-      // the 32 forward bases that end before len - x
-      const int64_t s = static_cast<int64_t>(tbase) + tlen - 32 - x;
-      const uint64_t f = s >= 0 ? bases32(t.idx.twords, static_cast<uint64_t>(s))
-                                : bases32(t.idx.twords, 0) >> (2 * -s);
-      tb = revcomp(f, 32);
+    const uint64_t q0 = qbase + static_cast<uint64_t>(p) + k + m;
+    const uint64_t b = w0 + static_cast<uint64_t>(p) + 1 + m;  // the next window
+    const uint32_t bs = static_cast<uint32_t>(b & 31);
+    if (m == 0 || m + 32 * kWide >= most) {
+      uint64_t tb;
+      if (!rev) {
+        tb = bases32(t.idx.twords, tbase + static_cast<uint64_t>(x));
+      } else {
+        // bases x .. x + 31 of the reverse strand: the reverse complement of
+        // the 32 forward bases that end before len - x
+        const int64_t s = static_cast<int64_t>(tbase) + tlen - 32 - x;
+        const uint64_t f = s >= 0 ? bases32(t.idx.twords, static_cast<uint64_t>(s))
+                                  : bases32(t.idx.twords, 0) >> (2 * -s);
+        tb = revcomp(f, 32);
+      }
+      const uint32_t c0 = __ldg(t.cbits + (b >> 5));
+      const uint32_t c1 = bs ? __ldg(t.cbits + (b >> 5) + 1) : 0u;
+      const int32_t step = agree(bases32(t.qb.words, q0), tb, __funnelshift_r(c0, c1, bs));
+      m += step;
+      if (step < 32) break;
+      continue;
     }
-    const uint64_t diff = qb ^ tb;
-    const int32_t same = diff ? __clzll(static_cast<long long>(diff)) >> 1 : 32;
-    // solid bits of windows p + 1 + m .. p + 32 + m
-    const uint64_t b = w0 + static_cast<uint64_t>(p) + 1 + m;
-    const uint32_t c0 = __ldg(t.cbits + (b >> 5));
-    const uint32_t c1 = (b & 31) ? __ldg(t.cbits + (b >> 5) + 1) : 0u;
-    const uint32_t holes = ~__funnelshift_r(c0, c1, static_cast<uint32_t>(b & 31));
-    const int32_t solid = holes ? __ffs(holes) - 1 : 32;
-    const int32_t step = min(same, solid);
-    m += step;
-    if (step < 32) break;
+    // all 32 * kWide bases and windows lie inside query and target
+    const uint64_t s0 = rev ? tbase + static_cast<uint64_t>(tlen - 32 * kWide - x)
+                            : tbase + static_cast<uint64_t>(x);
+    const uint32_t qs = static_cast<uint32_t>(q0 & 31), ts = static_cast<uint32_t>(s0 & 31);
+    uint64_t qw[kWide + 1], tw[kWide + 1];
+    uint32_t cw[kWide + 1];
+#pragma unroll
+    for (int u = 0; u < kWide; ++u) {
+      qw[u] = __ldg(t.qb.words + (q0 >> 5) + u);
+      tw[u] = __ldg(t.idx.twords + (s0 >> 5) + u);
+      cw[u] = __ldg(t.cbits + (b >> 5) + u);
+    }
+    qw[kWide] = qs ? __ldg(t.qb.words + (q0 >> 5) + kWide) : 0;
+    tw[kWide] = ts ? __ldg(t.idx.twords + (s0 >> 5) + kWide) : 0;
+    cw[kWide] = bs ? __ldg(t.cbits + (b >> 5) + kWide) : 0;
+    int32_t got = 0;
+#pragma unroll
+    for (int u = 0; u < kWide; ++u) {
+      const uint64_t qb = qs ? (qw[u] << (2 * qs)) | (qw[u + 1] >> (64 - 2 * qs)) : qw[u];
+      const int v = rev ? kWide - 1 - u : u;  // the reverse strand's blocks come last first
+      uint64_t tb = tw[0], tn = tw[1];
+#pragma unroll
+      for (int y = 1; y < kWide; ++y) {
+        if (v == y) {
+          tb = tw[y];
+          tn = tw[y + 1];
+        }
+      }
+      if (ts) tb = (tb << (2 * ts)) | (tn >> (64 - 2 * ts));
+      if (rev) tb = revcomp(tb, 32);
+      const int32_t step = agree(qb, tb, __funnelshift_r(cw[u], cw[u + 1], bs));
+      if (got == 32 * u) got += step;
+    }
+    m += got;
+    if (got < 32 * kWide) break;
   }
   return min(m + 1, most);
 }
@@ -358,16 +407,30 @@ __device__ __forceinline__ void store_run_piece(const RunTables& t, uint64_t slo
 
 constexpr int kGroupWarps = 8;
 
-__global__ void __launch_bounds__(kGroupWarps * 32) run_groups_kernel(RunTables t, ChainParams p) {
-  __shared__ uint32_t scls[kGroupWarps], sslot[kGroupWarps];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+// A warp a group.  Warps take chunks of consecutive groups from a counter and
+// list a chunk's survivors with one counter update a list.  A warp's lanes
+// wait for its longest run, so the kernel is bound by the latency of that
+// chain and wants warps: four blocks an SM (64 registers).  1.0e6 groups of 36
+// runs of 200 hits: 7.2 ms (17.9 with a barrier between a block's warps for a
+// shared counter update, and 32 bases a step); 2.7e5 groups of 218 runs of 8
+// hits: 1.6 ms (3.0).
+__global__ void __launch_bounds__(kGroupWarps * 32, 4) run_groups_kernel(RunTables t, ChainParams p,
+                                                                      uint32_t chunk,
+                                                                      uint32_t* work) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t lt = (1u << lane) - 1u;
   const uint64_t G = *t.ngroups;
-  constexpr uint32_t kNone = 255;
-  for (uint64_t g0 = static_cast<uint64_t>(blockIdx.x) * kGroupWarps; g0 < G;
-       g0 += static_cast<uint64_t>(gridDim.x) * kGroupWarps) {
-    const uint64_t g = g0 + warp;
-    uint32_t cls = kNone;
-    if (g < G) {
+  constexpr uint32_t kNone = kRunClasses + 2;
+  for (;;) {
+    uint32_t item = 0;
+    if (lane == 0) item = atomicAdd(work, chunk);
+    const uint64_t g0 = __shfl_sync(0xffffffffu, item, 0);
+    if (g0 >= G) break;
+    const uint32_t m = static_cast<uint32_t>(min(static_cast<uint64_t>(chunk), G - g0));
+    uint32_t cls = kNone;  // of group g0 + lane
+    bool ext = false;
+    for (uint32_t u = 0; u < m; ++u) {
+      const uint64_t g = g0 + u;
       const GroupInfo gi = t.bounds[g];
       const uint64_t end = g + 1 < G ? t.bounds[g + 1].start : t.nruns;
       const uint32_t n = static_cast<uint32_t>(end - gi.start);
@@ -400,6 +463,7 @@ __global__ void __launch_bounds__(kGroupWarps * 32) run_groups_kernel(RunTables 
           mn = min(mn, e);
           mx = max(mx, e + l - 1);
         }
+        __syncwarp();
         if (i0 == 0) {
           first_c = __shfl_sync(0xffffffffu, c, 0);
           first_l = __shfl_sync(0xffffffffu, l, 0);
@@ -443,35 +507,26 @@ __global__ void __launch_bounds__(kGroupWarps * 32) run_groups_kernel(RunTables 
         rg.ext_len = tlen;
         rg.flags = (es ? kRunExt : 0u) | (ties ? kRunCurTies : 0u);
         if (lane == 0) t.groups[g] = rg;
-        if (ready)
-          cls = static_cast<uint32_t>(run_class(rg.npieces));
-        else
-          cls = kRunClasses + (n <= 32 ? 0u : 1u);
-        if (es) cls |= 256u;
+        if (lane == static_cast<int>(u)) {
+          cls = ready ? static_cast<uint32_t>(run_class(rg.npieces))
+                      : kRunClasses + (n <= 32 ? 0u : 1u);
+          ext = es;
+        }
       }
     }
-    if (lane == 0) scls[warp] = cls;
-    __syncthreads();
-    if (threadIdx.x < kRunClasses + 2) {  // one counter update a list and block
-      uint32_t m = 0;
-      for (int w = 0; w < kGroupWarps; ++w) m += (scls[w] & 255u) == threadIdx.x;
-      if (m) {
-        uint32_t s = atomicAdd(t.counts + kRcList + threadIdx.x, m);
-        for (int w = 0; w < kGroupWarps; ++w)
-          if ((scls[w] & 255u) == threadIdx.x) sslot[w] = s++;
-      }
-    } else if (threadIdx.x == 32) {
-      uint32_t m = 0;
-      for (int w = 0; w < kGroupWarps; ++w) m += scls[w] >> 8;
-      if (m) atomicAdd(t.counts + kRcExt, m);
-    }
-    __syncthreads();
-    if (lane == 0 && cls != kNone) {
-      const uint32_t k = cls & 255u;
+#pragma unroll
+    for (uint32_t k = 0; k < kNone; ++k) {
+      const unsigned b = __ballot_sync(0xffffffffu, cls == k);
+      if (!b) continue;
+      uint32_t at = 0;
+      if (lane == 0) at = atomicAdd(t.counts + kRcList + k, __popc(b));
+      at = __shfl_sync(0xffffffffu, at, 0);
       uint32_t* list = k < kRunClasses ? t.lists + k * t.max_groups
                                        : t.sort_lists + (k - kRunClasses) * t.max_groups;
-      list[sslot[warp]] = static_cast<uint32_t>(g);
+      if (cls == k) list[at + __popc(b & lt)] = static_cast<uint32_t>(g0) + lane;
     }
+    const unsigned eb = __ballot_sync(0xffffffffu, ext);
+    if (lane == 0 && eb) atomicAdd(t.counts + kRcExt, __popc(eb));
   }
 }
 
@@ -669,10 +724,20 @@ cudaError_t runs_emit(const DeviceIndex& idx, const QueryBatch& q, const uint64_
 
 cudaError_t runs_groups(const RunTables& t, const ChainParams& p, int num_sms, cudaStream_t s) {
   if (t.max_groups == 0) return cudaSuccess;
+  int per_sm = 0;
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, run_groups_kernel,
+                                                                kGroupWarps * 32, 0);
+  if (e != cudaSuccess) return e;
+  // chunks of up to 32 groups, at least eight a resident warp (few groups: one
+  // each, so that they run side by side)
+  const uint64_t warps = static_cast<uint64_t>(std::max(per_sm, 1)) * num_sms * kGroupWarps;
+  const uint32_t chunk =
+      static_cast<uint32_t>(std::min<uint64_t>(32, std::max<uint64_t>(1, t.max_groups / (8 * warps))));
+  const uint64_t need = (t.max_groups + chunk - 1) / chunk;
   count_launch();
-  const uint64_t blocks = (t.max_groups + kGroupWarps - 1) / kGroupWarps;
-  run_groups_kernel<<<static_cast<unsigned>(std::min<uint64_t>(blocks, 64ull * num_sms)),
-                      kGroupWarps * 32, 0, s>>>(t, p);
+  run_groups_kernel<<<static_cast<unsigned>(std::min((need + kGroupWarps - 1) / kGroupWarps,
+                                                     warps / kGroupWarps)),
+                      kGroupWarps * 32, 0, s>>>(t, p, chunk, t.counts + kRcWork);
   return cudaGetLastError();
 }
 

@@ -47,8 +47,8 @@ enum : int {
   kRcOpen = kRcSort + 2,              // groups left to the hit path
   kRcExt = kRcOpen + 1,               // surviving ext-axis groups
   kRcPool = kRcExt + 1,               // rows in the pool
-  kRcWork = kRcPool + 1,              // 4: work counters
-  kRcWords = kRcWork + 4,             // (an even number)
+  kRcWork = kRcPool + 1,              // 5: work counters
+  kRcWords = kRcWork + 6,             // (an even number)
 };
 
 struct RunTables {
