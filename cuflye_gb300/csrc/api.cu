@@ -1156,8 +1156,8 @@ void run_runs(cuflye_ctx* c, PassState& ps) {
   uint64_t* ftile_off = buf<uint64_t>(c, "n_ftoff", nt + 1);
   unsigned long long* total = buf<unsigned long long>(c, "n_total", 64);
   CUFLYE_CHECK(cudaMemsetAsync(total, 0, 64 * sizeof(unsigned long long), st));
-  CUFLYE_CHECK(runs_probe(c->idx, ps.qb, wmeta, wflags, wself, cbits, fbits, tfilt, total, st));
-  CUFLYE_CHECK(runs_count(c->idx, ps.qb, wmeta, wflags, wself, nstart, tstart, st));
+  CUFLYE_CHECK(runs_count(c->idx, ps.qb, wmeta, wflags, wself, nstart, cbits, fbits, tfilt, tstart,
+                          total, st));
   scan_u32_async(c, tstart, tile_off, nt, "n_scan");
   scan_u32_async(c, tfilt, ftile_off, nt, "n_scan2");
   ps.q_off = buf<uint64_t>(c, "n_qoff", nq + 1);

@@ -38,6 +38,32 @@ __device__ __forceinline__ WindowKmer window_kmer(const QueryBatch& q, uint32_t 
   return w;
 }
 
+// Where a query's own window would be stored: (dense id, position) of the
+// entry that is the self hit, flipped when the lookup flips (~0: none).
+__device__ __forceinline__ uint64_t self_entry(const DeviceIndex& idx, int32_t qdi, uint64_t p,
+                                               bool rev) {
+  if (!(idx.transform && rev)) return (static_cast<uint64_t>(qdi) << 32) | static_cast<uint32_t>(p);
+  const uint32_t sid = static_cast<uint32_t>(qdi) ^ 1u;
+  const int32_t slen = idx.slot_len[sid >> 1];
+  const int64_t sp = static_cast<int64_t>(slen) - static_cast<int64_t>(p) - idx.k;
+  return sp >= 0 ? ((static_cast<uint64_t>(sid) << 32) | static_cast<uint32_t>(sp)) : ~0ULL;
+}
+
+// Index of entry `want` in a built bucket of c entries (sorted by (stored id,
+// stored position), entries unique), or c.
+__device__ __forceinline__ uint32_t bucket_find(const DeviceIndex& idx, uint64_t off, uint32_t c,
+                                                uint64_t want) {
+  uint32_t lo = 0, hi = c;
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (__ldg(idx.pos + off + mid) < want)
+      lo = mid + 1;
+    else
+      hi = mid;
+  }
+  return lo < c && __ldg(idx.pos + off + lo) == want ? lo : c;
+}
+
 // A window's bucket: its table meta, flags (kWinRev, kWinFiltered,
 // kWinTrivial), hits (the bucket's entries less the query's own position) and
 // the own entry's bucket index (kWinTrivial on a built index).
@@ -63,17 +89,8 @@ __device__ __forceinline__ WindowProbe probe_window(const DeviceIndex& idx, cons
     if (q_tie && (meta & kDupIdsBit) && q_tie[qi] == 0) atomicOr(q_tie + qi, 1u);
     const int32_t qdi = q.qdi[qi];
     if (c > 0 && qdi >= 0) {
-      // Is the query's own window among the bucket entries?  Stored form of
-      // the self hit: (qdi, p), or flipped when the lookup flips.
-      uint64_t want;
-      if (idx.transform && km.rev) {
-        const uint32_t sid = static_cast<uint32_t>(qdi) ^ 1u;
-        const int32_t slen = idx.slot_len[sid >> 1];
-        const int64_t sp = static_cast<int64_t>(slen) - static_cast<int64_t>(p) - idx.k;
-        want = sp >= 0 ? ((static_cast<uint64_t>(sid) << 32) | static_cast<uint32_t>(sp)) : ~0ULL;
-      } else {
-        want = (static_cast<uint64_t>(qdi) << 32) | static_cast<uint32_t>(p);
-      }
+      // is the query's own window among the bucket entries?
+      const uint64_t want = self_entry(idx, qdi, p, km.rev);
       const uint64_t off = meta & kOffsetMask;
       uint32_t self_hits = 0;
       if (idx.transform) {
@@ -95,16 +112,8 @@ __device__ __forceinline__ WindowProbe probe_window(const DeviceIndex& idx, cons
           }
         }
         if (!known) {
-          uint32_t lo = 0, hi = c;
-          while (lo < hi) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (__ldg(idx.pos + off + mid) < want)
-              lo = mid + 1;
-            else
-              hi = mid;
-          }
-          known = lo < c && __ldg(idx.pos + off + lo) == want;
-          at = lo;
+          at = bucket_find(idx, off, c, want);
+          known = at < c;
         }
         self_hits = known ? 1u : 0u;
         if (self_hits) self = at;

@@ -41,10 +41,12 @@ inline unsigned grid(uint64_t n, int b) {
 }
 
 // Window flags of the run path, beside kWinRev, kWinFiltered and kWinTrivial:
-// the k-mer is solid; the base before the window; it is the query's first.
+// the k-mer is solid; the base before the window; it is the query's first; the
+// window before is solid (as far as a run could continue from it).
 constexpr uint8_t kWinSolid = 8;
 constexpr int kWinBaseShift = 4;
 constexpr uint8_t kWinFirst = 64;
+constexpr uint8_t kWinPrevSolid = 128;
 
 __device__ __forceinline__ uint32_t base_at(const uint64_t* __restrict__ words, uint64_t g) {
   return static_cast<uint32_t>(__ldg(words + (g >> 5)) >> (62 - 2 * (g & 31))) & 3u;
@@ -81,51 +83,6 @@ __global__ void neighbour_kernel(const uint64_t* __restrict__ pos, uint64_t n,
   nbr[i] = static_cast<uint8_t>(before | (after << 4));
 }
 
-// One thread per window, blocks of whole 32-window tiles.
-__global__ void __launch_bounds__(256) probe_kernel(
-    DeviceIndex idx, QueryBatch q, uint64_t* __restrict__ wmeta, uint8_t* __restrict__ wflags,
-    uint32_t* __restrict__ wself, uint32_t* __restrict__ cbits, uint32_t* __restrict__ fbits,
-    uint32_t* __restrict__ tile_filt, unsigned long long* __restrict__ hit_total) {
-  __shared__ uint32_t wsum[8];
-  const uint64_t w = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int lane = threadIdx.x & 31;
-  uint32_t hits = 0;
-  uint8_t fl = 0;
-  if (w < q.nwin) {
-    const uint32_t qi = query_of(q.win_off, q.nq, w);
-    const uint64_t p = w - q.win_off[qi];
-    const WindowProbe x = probe_window(idx, q, qi, p, nullptr);
-    fl = x.flags;
-    hits = x.hits;
-    const uint32_t raw = static_cast<uint32_t>((x.meta >> 40) & ((1ULL << kCountBits) - 1));
-    if (!(fl & kWinFiltered) && raw > 0) fl |= kWinSolid;
-    if (p == 0)
-      fl |= kWinFirst;
-    else
-      fl |= static_cast<uint8_t>(base_at(q.words, q.base_off[qi] + p - 1) << kWinBaseShift);
-    if (fl & kWinTrivial) wself[w] = x.self;
-    wmeta[w] = x.meta;
-    wflags[w] = fl;
-  }
-  const uint32_t cb = __ballot_sync(0xffffffffu, fl & kWinSolid);
-  const uint32_t fb = __ballot_sync(0xffffffffu, fl & kWinFiltered);
-  const uint32_t sum = __reduce_add_sync(0xffffffffu, hits);
-  if (lane == 0) {
-    if (w < q.nwin) {
-      cbits[w >> 5] = cb;
-      fbits[w >> 5] = fb;
-      tile_filt[w >> 5] = __popc(fb);
-    }
-    wsum[threadIdx.x >> 5] = sum;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned long long s = 0;
-    for (int i = 0; i < 8; ++i) s += wsum[i];
-    if (s) atomicAdd(hit_total + (blockIdx.x & 63u), s);
-  }
-}
-
 // What a bucket entry's neighbour nibble must be for its hit to continue the
 // run of the window before, and where the nibble sits in the entry's byte:
 // the base before the window, on the entry's strand (the complement of it
@@ -135,75 +92,169 @@ struct RunTest {
   int shift;
 };
 
-__device__ __forceinline__ RunTest run_test(uint8_t fl, uint8_t prev_fl) {
+__device__ __forceinline__ RunTest run_test(uint8_t fl, bool prev_solid) {
   uint32_t e = 7;
-  if (!(fl & kWinFirst) && (prev_fl & kWinSolid)) e = (fl >> kWinBaseShift) & 3u;
+  if (!(fl & kWinFirst) && prev_solid) e = (fl >> kWinBaseShift) & 3u;
   if (!(fl & kWinRev)) return RunTest{e, 0};
   return RunTest{e == 7 ? 7u : 3u - e, 4};
 }
 
-__device__ __forceinline__ uint32_t bucket_size(uint8_t fl, uint64_t meta) {
-  return (fl & kWinSolid) ? static_cast<uint32_t>((meta >> 40) & ((1ULL << kCountBits) - 1)) : 0u;
+__device__ __forceinline__ uint32_t bucket_size(uint64_t meta) {
+  return static_cast<uint32_t>((meta >> 40) & ((1ULL << kCountBits) - 1));
 }
 
-// Bytes lo..3 of a word (lo in 0..4) as a mask.
-__device__ __forceinline__ uint32_t bytes_from(int lo) {
-  return lo >= 4 ? 0u : 0xffffffffu << (8 * lo);
+// Which of 16 entries' nibbles differ from the pattern: bit 8 j + 7 - s for
+// entry 4 s + j (byte j of word s), so that one popcount counts them all.
+__device__ __forceinline__ uint32_t differ16(uint4 x, int shift, uint32_t pat) {
+  auto word = [&](uint32_t w) {
+    return ((((w >> shift) & 0x0f0f0f0fu) ^ pat) + 0x7f7f7f7fu) & 0x80808080u;
+  };
+  return word(x.x) | (word(x.y) >> 1) | (word(x.z) >> 2) | (word(x.w) >> 3);
+}
+// The entries from lo on (0..16) in that order of bits.
+__device__ __forceinline__ uint32_t entries_from(uint32_t lo) {
+  const uint32_t s = lo >> 2, top = 0x80u >> s;
+  return lo >= 16 ? 0u
+                  : ((top - 1u) & 0xf0u) * 0x01010101u |
+                        ((top * 0x01010101u) & (0xffffffffu << (8 * (lo & 3u))));
 }
 
-// Run starts of each window: one thread a window, 16 entries a load (a bucket
-// of 36 entries is 3 to 4 loads that do not wait for one another; bound by the
-// latency of these scattered loads).
-__global__ void __launch_bounds__(256) start_count_kernel(
-    DeviceIndex idx, QueryBatch q, const uint64_t* __restrict__ wmeta,
-    const uint8_t* __restrict__ wflags, const uint32_t* __restrict__ wself,
-    uint32_t* __restrict__ nstart, uint32_t* __restrict__ tile_start) {
-  const uint64_t w = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int lane = threadIdx.x & 31;
-  uint32_t fl = 0, c = 0, ns = 0;
-  uint64_t meta = 0;
-  if (w < q.nwin) {
-    fl = wflags[w];
-    meta = wmeta[w];
-    c = bucket_size(static_cast<uint8_t>(fl), meta);
-  }
-  uint32_t pf = __shfl_up_sync(0xffffffffu, fl, 1);
-  if (lane == 0) pf = w > 0 && w < q.nwin ? wflags[w - 1] : 0u;
-  if (c > 0) {
-    const RunTest rt = run_test(static_cast<uint8_t>(fl), static_cast<uint8_t>(pf));
-    const uint64_t off = meta & kOffsetMask;
-    if (rt.expect == 7) {
-      ns = c - ((fl & kWinTrivial) ? 1u : 0u);
-    } else {
-      const uint32_t pat = rt.expect * 0x01010101u;
-      const uint64_t end = off + c;
-      const uint4* nb = reinterpret_cast<const uint4*>(idx.nbr);
-#pragma unroll 2
-      for (uint64_t ch = off >> 4; ch <= (end - 1) >> 4; ++ch) {
-        const uint4 x = __ldg(nb + ch);
-        const int64_t lo = static_cast<int64_t>(off) - static_cast<int64_t>(ch * 16);
-        const int64_t hi = static_cast<int64_t>(end) - static_cast<int64_t>(ch * 16);
-        const uint32_t xs[4] = {x.x, x.y, x.z, x.w};
+// Entries of the bucket [off, off + c) that start a run (the query's own
+// entry among them): 16 entries a load, four loads issued together.
+__device__ __forceinline__ uint32_t count_starts(const DeviceIndex& idx, uint64_t off, uint32_t c,
+                                                 RunTest rt) {
+  const uint32_t pat = rt.expect * 0x01010101u;
+  const uint4* nb = reinterpret_cast<const uint4*>(idx.nbr);
+  const uint64_t c0 = off >> 4, c1 = (off + c - 1) >> 4;
+  const uint32_t head = entries_from(static_cast<uint32_t>(off & 15)),
+                 tail = ~entries_from(static_cast<uint32_t>((off + c - 1) & 15) + 1);
+  uint32_t ns = 0;
+  for (uint64_t b = c0; b <= c1; b += 4) {
+    uint4 x[4];
 #pragma unroll
-        for (int s = 0; s < 4; ++s) {
-          const uint32_t y = ((xs[s] >> rt.shift) & 0x0f0f0f0fu) ^ pat;
-          uint32_t m = (y + 0x7f7f7f7fu) & 0x80808080u;  // bytes that differ
-          const int l = static_cast<int>(lo - 4 * s), h = static_cast<int>(hi - 4 * s);
-          if (l > 0) m &= bytes_from(l);
-          if (h < 4) m &= ~bytes_from(h < 0 ? 0 : h);
-          ns += __popc(m);
-        }
-      }
-      if (fl & kWinTrivial) {  // the query's own position is no hit
-        const uint32_t b = __ldg(idx.nbr + off + wself[w]);
-        if (((b >> rt.shift) & 15u) != rt.expect) --ns;
+    for (int u = 0; u < 4; ++u)
+      if (b + u <= c1) x[u] = __ldg(nb + b + u);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (b + u <= c1) {
+        uint32_t m = differ16(x[u], rt.shift, pat);
+        if (b + u == c0) m &= head;
+        if (b + u == c1) m &= tail;
+        ns += __popc(m);
       }
     }
   }
-  const uint32_t sum = __reduce_add_sync(0xffffffffu, ns);
+  return ns;
+}
+
+// A window's table word, its own entry's place in the bucket and the flags.
+// The query's own position is an entry exactly when the indexed sequence has
+// the query's k-mer there, which a look at the packed target tells (in step
+// with the query's own bases, where reading the entry is a scattered load).
+__device__ __forceinline__ uint8_t probe_run_window(const DeviceIndex& idx, const QueryBatch& q,
+                                                    uint32_t qi, uint64_t p, uint64_t& meta,
+                                                    uint32_t& self) {
+  const WindowKmer km = window_kmer(q, qi, p, idx.k);
+  bool found;
+  meta = table_probe(idx.table, idx.cap, km.key, &found);
+  uint8_t fl = km.rev ? kWinRev : 0;
+  if (!found) return fl;
+  if (meta & kRepetitiveBit) return fl | kWinFiltered;
+  fl |= kWinSolid;
+  const int32_t qdi = q.qdi[qi];
+  if (qdi < 0) return fl;
+  const uint32_t slot = static_cast<uint32_t>(qdi) >> 1;
+  const int64_t last = static_cast<int64_t>(idx.slot_len[slot]) - idx.k;
+  const int64_t f = (qdi & 1) ? last - static_cast<int64_t>(p) : static_cast<int64_t>(p);
+  if (f < 0 || f > last) return fl;
+  const uint64_t y = kmer_at(idx.twords, idx.tbase[slot] + static_cast<uint64_t>(f), idx.k);
+  if (((qdi & 1) ? revcomp(y, idx.k) : y) != km.x) return fl;
+  self = idx.self_at ? idx.self_at[idx.win_off[slot] + static_cast<uint64_t>(f)]
+                     : bucket_find(idx, meta & kOffsetMask, bucket_size(meta),
+                                   self_entry(idx, qdi, p, km.rev));
+  return fl | kWinTrivial;
+}
+
+constexpr int kProbeBlock = 256;
+
+// One thread per window, blocks of whole 32-window tiles: the table probe, then
+// the run starts in the window's bucket.  Bound by the probe's scattered
+// loads (a table slot and two to three sectors of neighbours a window), which
+// is why both share a kernel: the counting of one warp hides the other's loads.
+__global__ void __launch_bounds__(kProbeBlock) probe_kernel(
+    DeviceIndex idx, QueryBatch q, uint64_t* __restrict__ wmeta, uint8_t* __restrict__ wflags,
+    uint32_t* __restrict__ wself, uint32_t* __restrict__ nstart, uint32_t* __restrict__ cbits,
+    uint32_t* __restrict__ fbits, uint32_t* __restrict__ tile_filt,
+    uint32_t* __restrict__ tile_start, unsigned long long* __restrict__ hit_total) {
+  __shared__ uint32_t wsum[kProbeBlock / 32];
+  __shared__ bool solid[kProbeBlock + 1];  // of the windows before and in the block
+  const uint64_t w = static_cast<uint64_t>(blockIdx.x) * kProbeBlock + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  uint64_t meta = 0;
+  uint32_t self = kNoLink;
+  uint8_t fl = 0;
+  if (w < q.nwin) {
+    const uint32_t qi = query_of(q.win_off, q.nq, w);
+    const uint64_t p = w - q.win_off[qi];
+    fl = probe_run_window(idx, q, qi, p, meta, self);
+    if (p == 0)
+      fl |= kWinFirst;
+    else
+      fl |= static_cast<uint8_t>(base_at(q.words, q.base_off[qi] + p - 1) << kWinBaseShift);
+    if (threadIdx.x == 0) {
+      bool before = false;
+      if (p > 0) {  // the last window of the block before
+        bool found;
+        const uint64_t m = table_probe(idx.table, idx.cap,
+                                       window_kmer(q, qi, p - 1, idx.k).key, &found);
+        before = found && !(m & kRepetitiveBit);
+      }
+      solid[0] = before;
+    }
+  }
+  solid[threadIdx.x + 1] = fl & kWinSolid;
+  __syncthreads();
+  uint32_t ns = 0, hits = 0;
+  if (fl & kWinSolid) {
+    const RunTest rt = run_test(fl, solid[threadIdx.x]);
+    if (rt.expect != 7) fl |= kWinPrevSolid;
+    const uint64_t off = meta & kOffsetMask;
+    const uint32_t c = bucket_size(meta), own = self != kNoLink ? 1u : 0u;
+    hits = c - own;
+    if (rt.expect == 7) {
+      ns = hits;
+    } else {
+      ns = count_starts(idx, off, c, rt);
+      // the query's own position is no hit
+      if (own && ((static_cast<uint32_t>(__ldg(idx.nbr + off + self)) >> rt.shift) & 15u) !=
+                     rt.expect)
+        --ns;
+    }
+  }
+  const uint32_t cb = __ballot_sync(0xffffffffu, fl & kWinSolid);
+  const uint32_t fb = __ballot_sync(0xffffffffu, fl & kWinFiltered);
+  const uint32_t starts = __reduce_add_sync(0xffffffffu, ns);
+  const uint32_t sum = __reduce_add_sync(0xffffffffu, hits);
   if (w < q.nwin) {
     nstart[w] = ns;
-    if (lane == 0) tile_start[w >> 5] = sum;
+    if (ns) {  // what the emission reads
+      wmeta[w] = meta;
+      wflags[w] = fl;
+      wself[w] = self;
+    }
+    if (lane == 0) {
+      cbits[w >> 5] = cb;
+      fbits[w >> 5] = fb;
+      tile_filt[w >> 5] = __popc(fb);
+      tile_start[w >> 5] = starts;
+    }
+  }
+  if (lane == 0) wsum[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned long long s = 0;
+    for (int i = 0; i < kProbeBlock / 32; ++i) s += wsum[i];
+    if (s) atomicAdd(hit_total + (blockIdx.x & 63u), s);
   }
 }
 
@@ -225,9 +276,9 @@ __global__ void query_offsets_kernel(QueryBatch q, const uint32_t* __restrict__ 
   f_off[i] = f;
 }
 
-// A warp writes its 32 windows' run starts, one window at a time with all
-// lanes on the bucket's entries: most windows start no run and are skipped, and
-// the first window after a hole in the query starts a run in every entry.
+// A warp writes its 32 windows' run starts.  The entries of the windows that
+// start runs (few windows do) are numbered through and taken 32 at a time, so
+// the lanes are busy whether a bucket holds two entries or two hundred.
 __global__ void __launch_bounds__(256) start_emit_kernel(
     DeviceIndex idx, QueryBatch q, const uint64_t* __restrict__ wmeta,
     const uint8_t* __restrict__ wflags, const uint32_t* __restrict__ wself,
@@ -237,7 +288,7 @@ __global__ void __launch_bounds__(256) start_emit_kernel(
   const uint64_t w = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
   const uint32_t lt = (1u << lane) - 1u;
-  uint32_t ns = 0, fl = 0, fb = 0;
+  uint32_t ns = 0, fb = 0;
   if (w < q.nwin) {
     ns = nstart[w];
     fb = fbits[w >> 5];
@@ -249,48 +300,56 @@ __global__ void __launch_bounds__(256) start_emit_kernel(
     p = static_cast<uint32_t>(w - q.win_off[qi]);
     if (filtered) fpos[ftile_off[w >> 5] + __popc(fb & lt)] = static_cast<int32_t>(p);
   }
-  unsigned todo = __ballot_sync(0xffffffffu, ns > 0);
-  if (!todo) return;
-  uint64_t meta = 0;
-  uint32_t self = kNoLink;
-  RunTest rt{7, 0};
+  if (!__any_sync(0xffffffffu, ns > 0)) return;
+  uint64_t off = 0;
+  uint32_t self = kNoLink, c = 0, test = 0;  // test: expected nibble | shift << 3 | rev << 6
   if (ns) {
-    fl = wflags[w];
-    meta = wmeta[w];
-    rt = run_test(static_cast<uint8_t>(fl), w > 0 ? wflags[w - 1] : 0);
-    if (fl & kWinTrivial) self = wself[w];
+    const uint8_t fl = wflags[w];
+    const uint64_t meta = wmeta[w];
+    const RunTest rt = run_test(fl, fl & kWinPrevSolid);
+    test = rt.expect | static_cast<uint32_t>(rt.shift) << 3 | ((fl & kWinRev) ? 64u : 0u);
+    self = wself[w];
+    off = meta & kOffsetMask;
+    c = bucket_size(meta);
   }
+  uint32_t upto = c;  // entries of this window and the ones before
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, upto, o);
+    if (lane >= o) upto += y;
+  }
+  const uint32_t total = __shfl_sync(0xffffffffu, upto, 31);
   uint64_t out = tile_off[w >> 5];
-  while (todo) {
-    const int src = __ffs(todo) - 1;
-    todo &= todo - 1;
-    const uint64_t wm = __shfl_sync(0xffffffffu, meta, src);
+  for (uint32_t e0 = 0; e0 < total; e0 += 32) {
+    const uint32_t j = e0 + lane;
+    int src = 0;  // the window of entry j: the first whose count exceeds j
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      if (__shfl_sync(0xffffffffu, upto, src + o - 1) <= j) src += o;
+    const uint32_t end = __shfl_sync(0xffffffffu, upto, src);
+    const uint32_t n = __shfl_sync(0xffffffffu, c, src);
+    const uint64_t wo = __shfl_sync(0xffffffffu, off, src);
     const uint32_t wp = __shfl_sync(0xffffffffu, p, src);
-    const uint32_t wf = __shfl_sync(0xffffffffu, fl, src);
+    const uint32_t wt = __shfl_sync(0xffffffffu, test, src);
     const uint32_t ws = __shfl_sync(0xffffffffu, self, src);
-    const uint32_t we = __shfl_sync(0xffffffffu, rt.expect, src);
-    const int wsh = __shfl_sync(0xffffffffu, rt.shift, src);
-    const uint64_t off = wm & kOffsetMask;
-    const uint32_t c = bucket_size(static_cast<uint8_t>(wf), wm);
-    for (uint32_t e0 = 0; e0 < c; e0 += 32) {
-      const uint32_t e = e0 + lane;
-      const bool start = e < c && e != ws &&
-                         ((static_cast<uint32_t>(__ldg(idx.nbr + off + e)) >> wsh) & 15u) != we;
-      const unsigned m = __ballot_sync(0xffffffffu, start);
-      if (start) {
-        const uint64_t sv = __ldg(idx.pos + off + e);
-        uint32_t id = static_cast<uint32_t>(sv >> 32);
-        int32_t pos = static_cast<int32_t>(sv & 0xffffffffu);
-        if (wf & kWinRev) {
-          pos = idx.slot_len[id >> 1] - pos - idx.k;
-          id ^= 1u;
-        }
-        const uint64_t d = out + __popc(m & lt);
-        keys[d] = (static_cast<uint64_t>(id) << 32) | wp;
-        vals[d] = static_cast<uint32_t>(pos);
+    const uint32_t e = j - (end - n);
+    const bool start =
+        j < total && e != ws &&
+        ((static_cast<uint32_t>(__ldg(idx.nbr + wo + e)) >> ((wt >> 3) & 7u)) & 15u) != (wt & 7u);
+    const unsigned m = __ballot_sync(0xffffffffu, start);
+    if (start) {
+      const uint64_t sv = __ldg(idx.pos + wo + e);
+      uint32_t id = static_cast<uint32_t>(sv >> 32);
+      int32_t pos = static_cast<int32_t>(sv & 0xffffffffu);
+      if (wt & 64u) {
+        pos = idx.slot_len[id >> 1] - pos - idx.k;
+        id ^= 1u;
       }
-      out += __popc(m);
+      const uint64_t d = out + __popc(m & lt);
+      keys[d] = (static_cast<uint64_t>(id) << 32) | wp;
+      vals[d] = static_cast<uint32_t>(pos);
     }
+    out += __popc(m);
   }
 }
 
@@ -680,23 +739,14 @@ cudaError_t index_neighbours(const uint64_t* pos, uint64_t npos, const uint64_t*
   return cudaGetLastError();
 }
 
-cudaError_t runs_probe(const DeviceIndex& idx, const QueryBatch& q, uint64_t* wmeta,
-                       uint8_t* wflags, uint32_t* wself, uint32_t* cbits, uint32_t* fbits,
-                       uint32_t* tile_filt, unsigned long long* hit_total, cudaStream_t s) {
+cudaError_t runs_count(const DeviceIndex& idx, const QueryBatch& q, uint64_t* wmeta,
+                       uint8_t* wflags, uint32_t* wself, uint32_t* nstart, uint32_t* cbits,
+                       uint32_t* fbits, uint32_t* tile_filt, uint32_t* tile_start,
+                       unsigned long long* hit_total, cudaStream_t s) {
   if (q.nwin == 0) return cudaSuccess;
   count_launch();
-  probe_kernel<<<grid(q.nwin, 256), 256, 0, s>>>(idx, q, wmeta, wflags, wself, cbits, fbits,
-                                                 tile_filt, hit_total);
-  return cudaGetLastError();
-}
-
-cudaError_t runs_count(const DeviceIndex& idx, const QueryBatch& q, const uint64_t* wmeta,
-                       const uint8_t* wflags, const uint32_t* wself, uint32_t* nstart,
-                       uint32_t* tile_start, cudaStream_t s) {
-  if (q.nwin == 0) return cudaSuccess;
-  count_launch();
-  start_count_kernel<<<grid(q.nwin, 256), 256, 0, s>>>(idx, q, wmeta, wflags, wself, nstart,
-                                                       tile_start);
+  probe_kernel<<<grid(q.nwin, kProbeBlock), kProbeBlock, 0, s>>>(
+      idx, q, wmeta, wflags, wself, nstart, cbits, fbits, tile_filt, tile_start, hit_total);
   return cudaGetLastError();
 }
 
