@@ -434,9 +434,42 @@ __device__ __forceinline__ void scan_round(const Candidate& c, int32_t ax, bool 
   ended = bm != 0;
 }
 
-// One warp a group.  The last 32 pieces live in the warp's registers (piece j
-// in lane j mod 32), so most scans read no memory; older pieces are scanned
-// only while the highest score among them could still beat the best found.
+// Inclusive scans over the warp.
+__device__ __forceinline__ int32_t scan_add(int32_t x) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  return x;
+}
+__device__ __forceinline__ int32_t scan_max(int32_t x) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x = max(x, y);
+  }
+  return x;
+}
+
+constexpr int32_t kNoScore = -(1 << 30);
+
+// One warp a group, 32 pieces (a chunk) at a time.
+//
+// In a chain each piece links to the end of the one before it, and no other
+// piece can do better: the piece before is visited first, and an older one
+// scores its end plus k at most.  So the warp scores a stretch of pieces as if
+// that were so with one prefix sum, checks it with one prefix maximum (the
+// greatest end before each piece's predecessor), and keeps what comes before the
+// first piece that fails.  That piece is scanned: against the 32 pieces before
+// it, which the warp's registers hold (piece j in lane j mod 32), and against
+// older ones only while the greatest end among them could still beat the best
+// found.
+//
+// Bound by issue: a scan costs about 100 instructions a piece, a stretch
+// about 4.
 __global__ void __launch_bounds__(kWarpsPerBlock * 32) run_dp_kernel(RunTables t, ChainParams p,
                                                                      uint32_t* work) {
   const int lane = threadIdx.x & 31;
@@ -447,9 +480,12 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) run_dp_kernel(RunTables t
     const uint64_t base = g.piece0;
     const uint32_t n = g.npieces;
     const bool ties = g.flags & kRunTies;
-    int32_t ra = 0, rb = 0, rl = 0, rs = 0;  // the ring: this lane's latest piece
-    int32_t older = 0;                       // highest score of the pieces before the ring's
-    int32_t na = 0, nb = 0, nl = 0;          // the next 32 pieces, loaded ahead
+    int32_t qa = 0, qb = 0, ql = 0, qs = 0;  // the chunk before: this lane's piece
+    int32_t qmax = kNoScore;     // greatest end of that chunk's pieces before this lane's
+    int32_t older = kNoScore;    // greatest end of the pieces before that chunk
+    int32_t na = 0, nb = 0, nl = 0;  // the next chunk, loaded ahead
+    int32_t s_prev = 0, e_prev = 0;  // score and end of the piece before the next one
+    int32_t big = kNoScore;          // greatest end of the pieces before that one
     bool open = false;
     if (lane < static_cast<int>(n)) {
       na = t.pa[base + lane];
@@ -458,64 +494,126 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) run_dp_kernel(RunTables t
     }
     for (uint32_t i0 = 0; i0 < n && !open; i0 += 32) {
       const int32_t ca = na, cb = nb, cl = nl;
+      int32_t cs = 0;
       if (i0 + 32 + lane < n) {
         na = t.pa[base + i0 + 32 + lane];
         nb = t.pb[base + i0 + 32 + lane];
         nl = t.pl[base + i0 + 32 + lane];
       }
-      int32_t ms = 0, mo = 0;
-      uint32_t mk = kNoLink;
       const uint32_t len = min(32u, n - i0);
-      for (uint32_t u = 0; u < len; ++u) {
+      uint32_t mk = kNoLink;
+      int32_t mo = 0;
+      // this piece after the end of the one before it: the score it would gain
+      int32_t a1 = __shfl_up_sync(0xffffffffu, ca, 1), b1 = __shfl_up_sync(0xffffffffu, cb, 1),
+              l1 = __shfl_up_sync(0xffffffffu, cl, 1);
+      const int32_t la = __shfl_sync(0xffffffffu, qa, 31), lb = __shfl_sync(0xffffffffu, qb, 31),
+                    ll = __shfl_sync(0xffffffffu, ql, 31);
+      if (lane == 0) {
+        a1 = la;
+        b1 = lb;
+        l1 = ll;
+      }
+      const Candidate pre = candidate(i0 + lane > 0, ca, cb, a1, b1, l1, 0, p);
+      const int32_t gain = pre.score;
+      bool ok = lane < static_cast<int>(len) && pre.score != INT_MIN && pre.off == l1 - 1;
+      if (ties) {  // neither in a cluster nor after one
+        int32_t a2 = __shfl_up_sync(0xffffffffu, a1, 1);
+        const int32_t q30 = __shfl_sync(0xffffffffu, qa, 30);
+        if (lane == 0) a2 = q30;
+        ok = ok && ca != a1 && (a1 != a2 || i0 + lane < 2);
+      }
+      const unsigned okm = __ballot_sync(0xffffffffu, ok);
+      uint32_t u = 0;
+      if (i0 == 0) {  // element 0 of the group: score 0, no link
+        s_prev = 0;
+        e_prev = 0;
+        u = 1;
+      }
+      while (u < len && !open) {
+        const unsigned stop = ~okm & (0xffffffffu << u);
+        const uint32_t r = stop ? static_cast<uint32_t>(__ffs(stop) - 1) : 32u;
+        if (r >= u + 3) {  // a stretch worth its scans
+          const bool in = lane >= static_cast<int>(u) && lane < static_cast<int>(r);
+          const int32_t s = s_prev + scan_add(in ? gain : 0);
+          const int32_t e = s + cl - 1;
+          const int32_t em = scan_max(in ? e : kNoScore);
+          const int32_t em2 = __shfl_up_sync(0xffffffffu, em, 2);
+          int32_t before = big;
+          if (lane > static_cast<int>(u)) before = max(before, e_prev);
+          if (lane > static_cast<int>(u) + 1) before = max(before, em2);
+          const bool holds = in && s > p.k && (pre.ends || before + p.k <= s);
+          const unsigned fail = ~__ballot_sync(0xffffffffu, holds) & (0xffffffffu << u);
+          const uint32_t f = fail ? static_cast<uint32_t>(__ffs(fail) - 1) : 32u;
+          if (f > u) {
+            if (in && lane < static_cast<int>(f)) {
+              cs = s;
+              mk = i0 + lane - 1;
+              mo = l1 - 1;
+              if (ties) t.ps[base + i0 + lane] = s;
+            }
+            const int32_t ef1 = __shfl_sync(0xffffffffu, e, static_cast<int>(f - 1));
+            const int32_t emf = __shfl_sync(0xffffffffu, em, static_cast<int>(max(f, 2u) - 2));
+            big = max(big, e_prev);
+            if (f >= u + 2) big = max(big, emf);
+            e_prev = ef1;
+            s_prev = __shfl_sync(0xffffffffu, s, static_cast<int>(f - 1));
+            u = f;
+            if (ties) __syncwarp();
+            continue;
+          }
+        }
+        // scan piece i0 + u
         const uint32_t i = i0 + u;
         const int32_t ai = __shfl_sync(0xffffffffu, ca, u);
         const int32_t bi = __shfl_sync(0xffffffffu, cb, u);
         const int32_t li_ = __shfl_sync(0xffffffffu, cl, u);
-        int32_t si = 0, off = 0;
-        uint32_t link = kNoLink;
-        if (i > 0) {
-          const bool valid = lane < static_cast<int>(i);
-          const Candidate c = candidate(valid, ai, bi, ra, rb, rl, rs, p);
-          int32_t best = 0;
-          uint32_t bestj = kNoLink;
-          int32_t bestoff = 0;
-          bool ended = false;
-          // a tie cluster astride two rounds belongs to the later one: the
-          // oldest pieces of this round that share the next one's position
-          uint32_t held = 0;
-          const uint32_t s0 = (i - 1) & 31;  // the lane of piece i - 1
-          if (ties || __any_sync(0xffffffffu, c.ends)) {
-            // in scan order: position d is the lane of piece i - 1 - d
-            const int src = static_cast<int>((s0 - lane) & 31);
-            Candidate o;
-            o.score = __shfl_sync(0xffffffffu, c.score, src);
-            o.off = __shfl_sync(0xffffffffu, c.off, src);
-            o.ends = __shfl_sync(0xffffffffu, c.ends, src);
-            const int32_t oax = __shfl_sync(0xffffffffu, ra, src);
-            bool ov = lane < static_cast<int>(min(i, 32u));
-            if (ties && i > 32) {
-              const bool hold = oax == t.pa[base + i - 33];
-              held = __popc(__ballot_sync(0xffffffffu, hold));
-              if (hold) {
-                ov = false;
-                o.score = INT_MIN;
-                o.ends = false;
-              }
-            }
-            scan_round(o, oax, ov, ties, i - 1 - lane, best, bestj, bestoff, ended, open);
-          } else {
-            const int32_t m = __reduce_max_sync(0xffffffffu, c.score);
-            if (m > 0) {
-              const unsigned bal = __ballot_sync(0xffffffffu, c.score == m);
-              // bit d of the rotated word: the lane of piece i - 1 - d
-              const unsigned rev = __brev(bal);
-              const uint32_t d = __ffs(__funnelshift_r(rev, rev, 31 - s0)) - 1;
-              best = m;
-              bestj = i - 1 - d;
-              bestoff = __shfl_sync(0xffffffffu, c.off, static_cast<int>((s0 - d) & 31));
+        const bool now = lane < static_cast<int>(u);  // the ring: this chunk's pieces so far
+        const int32_t ra = now ? ca : qa, rb = now ? cb : qb, rl = now ? cl : ql,
+                      rs = now ? cs : qs;
+        const bool valid = now || i0 > 0;
+        const Candidate c = candidate(valid, ai, bi, ra, rb, rl, rs, p);
+        int32_t best = 0;
+        uint32_t bestj = kNoLink;
+        int32_t bestoff = 0;
+        bool ended = false;
+        // a tie cluster astride two rounds belongs to the later one: the
+        // oldest pieces of this round that share the next one's position
+        uint32_t held = 0;
+        const uint32_t s0 = (i - 1) & 31;  // the lane of piece i - 1
+        if (ties || __any_sync(0xffffffffu, c.ends)) {
+          // in scan order: position d is the lane of piece i - 1 - d
+          const int src = static_cast<int>((s0 - lane) & 31);
+          Candidate o;
+          o.score = __shfl_sync(0xffffffffu, c.score, src);
+          o.off = __shfl_sync(0xffffffffu, c.off, src);
+          o.ends = __shfl_sync(0xffffffffu, c.ends, src);
+          const int32_t oax = __shfl_sync(0xffffffffu, ra, src);
+          bool ov = lane < static_cast<int>(min(i, 32u));
+          if (ties && i > 32) {
+            const bool hold = oax == t.pa[base + i - 33];
+            held = __popc(__ballot_sync(0xffffffffu, hold));
+            if (hold) {
+              ov = false;
+              o.score = INT_MIN;
+              o.ends = false;
             }
           }
-          if (i > 32 && !ended && (held || older + p.k > best)) {
+          scan_round(o, oax, ov, ties, i - 1 - lane, best, bestj, bestoff, ended, open);
+        } else {
+          const int32_t m = __reduce_max_sync(0xffffffffu, c.score);
+          if (m > 0) {
+            const unsigned bal = __ballot_sync(0xffffffffu, c.score == m);
+            // bit d of the rotated word: the lane of piece i - 1 - d
+            const unsigned rev = __brev(bal);
+            const uint32_t d = __ffs(__funnelshift_r(rev, rev, 31 - s0)) - 1;
+            best = m;
+            bestj = i - 1 - d;
+            bestoff = __shfl_sync(0xffffffffu, c.off, static_cast<int>((s0 - d) & 31));
+          }
+        }
+        if (i > 32 && !ended) {
+          const int32_t past = max(older, __shfl_sync(0xffffffffu, qmax, static_cast<int>(u)));
+          if (held || past + p.k > best) {
             // beyond the jump along the axis from some piece on?  (held pieces
             // are the oldest: lane order d >= 32 - held)
             const uint32_t d = (s0 - lane) & 31;
@@ -525,14 +623,14 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) run_dp_kernel(RunTables t
               more = false;
             }
             for (int32_t c0 = static_cast<int32_t>(i + held) - 33; more && c0 >= 0;) {
-              const int32_t j = c0 - lane;
-              bool v = j >= 0;
+              const int32_t jj = c0 - lane;
+              bool v = jj >= 0;
               int32_t a = 0, b = 0, l = 0, s = 0;
               if (v) {
-                a = t.pa[base + j];
-                b = t.pb[base + j];
-                l = t.pl[base + j];
-                s = __ldcg(t.ps + base + j);
+                a = t.pa[base + jj];
+                b = t.pb[base + jj];
+                l = t.pl[base + jj];
+                s = __ldcg(t.ps + base + jj);
               }
               held = 0;
               if (ties && c0 >= 32) {
@@ -542,54 +640,56 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) run_dp_kernel(RunTables t
                 if (held == 32) open = true;
               }
               const Candidate x = candidate(v, ai, bi, a, b, l, s, p);
-              scan_round(x, a, v, ties, static_cast<uint32_t>(j), best, bestj, bestoff, ended,
+              scan_round(x, a, v, ties, static_cast<uint32_t>(jj), best, bestj, bestoff, ended,
                          open);
               if (ended || open || __any_sync(0xffffffffu, v && ai - a > p.max_jump) ||
-                  (held == 0 && older + p.k <= best))
+                  (held == 0 && past + p.k <= best))
                 break;
               c0 -= 32 - static_cast<int32_t>(held);
             }
           }
-          si = max(best, p.k);
-          if (best > p.k) {
-            link = bestj;
-            off = bestoff;
-          }
-          if (ties) {
-            if (i == 1 && ai == __shfl_sync(0xffffffffu, ra, 0)) open = true;
-            // the cluster so far: could the elements inside one of two pieces
-            // link into the other (one axis position back, so on a lower
-            // second position)?
-            const bool mate = valid && ra == ai;
-            const int32_t d = bi - rb, jd = abs(d);
-            const float pen = jd > p.gap_jump_threshold ? p.large_gap_penalty : p.small_gap_penalty;
-            const int32_t gc = __float2int_rz(__fmul_rn(pen, static_cast<float>(jd)));
-            const bool close = jd <= p.max_gap && jd + 1 < p.max_jump;
-            const bool unsafe = mate && li_ > 1 && close && !(d > 0 ? si > rs - gc : rs > si - gc);
-            const unsigned mates = __ballot_sync(0xffffffffu, mate);
-            if (__any_sync(0xffffffffu, unsafe) || mates == 0xffffffffu) open = true;
-          }
         }
-        const int32_t gone = __shfl_sync(0xffffffffu, rs + rl - 1, static_cast<int>(u));
-        if (i >= 32) older = max(older, gone);
+        const int32_t si = max(best, p.k);
+        if (ties) {
+          if (i == 1 && ai == __shfl_sync(0xffffffffu, ra, 0)) open = true;
+          // the cluster so far: could the elements inside one of two pieces
+          // link into the other (one axis position back, so on a lower second
+          // position)?
+          const bool mate = valid && ra == ai;
+          const int32_t d = bi - rb, jd = abs(d);
+          const float pen = jd > p.gap_jump_threshold ? p.large_gap_penalty : p.small_gap_penalty;
+          const int32_t gc = __float2int_rz(__fmul_rn(pen, static_cast<float>(jd)));
+          const bool close = jd <= p.max_gap && jd + 1 < p.max_jump;
+          const bool unsafe = mate && li_ > 1 && close && !(d > 0 ? si > rs - gc : rs > si - gc);
+          const unsigned mates = __ballot_sync(0xffffffffu, mate);
+          if (__any_sync(0xffffffffu, unsafe) || mates == 0xffffffffu) open = true;
+        }
         if (lane == static_cast<int>(u)) {
-          ra = ai;
-          rb = bi;
-          rl = li_;
-          rs = si;
-          ms = si;
-          mk = link;
-          mo = off;
+          cs = si;
+          mk = best > p.k ? bestj : kNoLink;
+          mo = best > p.k ? bestoff : 0;
           if (ties) t.ps[base + i] = si;  // a held piece is read back before the chunk's store
         }
         if (ties) __syncwarp();
+        big = max(big, e_prev);
+        s_prev = si;
+        e_prev = si + li_ - 1;
+        ++u;
       }
       if (lane < static_cast<int>(len)) {
-        t.ps[base + i0 + lane] = ms;
+        t.ps[base + i0 + lane] = cs;
         t.pk[base + i0 + lane] = mk;
         t.po[base + i0 + lane] = mo;
       }
       __syncwarp();
+      older = max(older, __reduce_max_sync(0xffffffffu, i0 > 0 ? qs + ql - 1 : kNoScore));
+      qa = ca;
+      qb = cb;
+      ql = cl;
+      qs = cs;
+      const int32_t em = scan_max(cs + cl - 1);
+      qmax = __shfl_up_sync(0xffffffffu, em, 1);
+      if (lane == 0) qmax = kNoScore;
     }
     if (open && lane == 0) {
       t.groups[gidx].flags = g.flags | kRunOpen;
