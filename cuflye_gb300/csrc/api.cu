@@ -905,7 +905,8 @@ void emit_generation_order(cuflye_ctx* c, PassState& ps) {
 constexpr uint64_t kRunBytesPerWindow = 40;
 // Buffers sized by the windows of a pass's run (reused by the next pass).
 const char* const kPerWindowBuffers[] = {"q_ascii", "q_words",  "w_cnt",     "w_filt", "w_meta",
-                                         "w_flags", "w_hitoff", "w_filtoff", "w_scan", "w_self"};
+                                         "w_flags", "w_hitoff", "w_filtoff", "w_scan", "w_self",
+                                         "w_recs"};
 
 // Bytes of the buffers that a pass of this kind reuses from the last one.
 uint64_t reusable_bytes(const cuflye_ctx* c, bool runs, bool windows) {
@@ -1144,9 +1145,7 @@ void run_runs(cuflye_ctx* c, PassState& ps) {
   const uint64_t nwin = ps.nwin, nt = (nwin + 31) / 32;
   cudaStream_t st = c->stream;
   ps.runs = true;
-  uint64_t* wmeta = buf<uint64_t>(c, "w_meta", nwin);
-  uint8_t* wflags = buf<uint8_t>(c, "w_flags", nwin);
-  uint32_t* wself = buf<uint32_t>(c, "w_self", nwin);
+  uint4* recs = buf<uint4>(c, "w_recs", nwin);
   uint32_t* nstart = buf<uint32_t>(c, "w_cnt", nwin);
   uint32_t* cbits = buf<uint32_t>(c, "n_cbits", nt + 2);
   uint32_t* fbits = buf<uint32_t>(c, "n_fbits", nt);
@@ -1156,8 +1155,7 @@ void run_runs(cuflye_ctx* c, PassState& ps) {
   uint64_t* ftile_off = buf<uint64_t>(c, "n_ftoff", nt + 1);
   unsigned long long* total = buf<unsigned long long>(c, "n_total", 64);
   CUFLYE_CHECK(cudaMemsetAsync(total, 0, 64 * sizeof(unsigned long long), st));
-  CUFLYE_CHECK(runs_count(c->idx, ps.qb, wmeta, wflags, wself, nstart, cbits, fbits, tfilt, tstart,
-                          total, st));
+  CUFLYE_CHECK(runs_count(c->idx, ps.qb, recs, nstart, cbits, fbits, tfilt, tstart, total, st));
   scan_u32_async(c, tstart, tile_off, nt, "n_scan");
   scan_u32_async(c, tfilt, ftile_off, nt, "n_scan2");
   ps.q_off = buf<uint64_t>(c, "n_qoff", nq + 1);
@@ -1208,8 +1206,8 @@ void run_runs(cuflye_ctx* c, PassState& ps) {
   ps.keys = buf<uint64_t>(c, "n_keys", ps.units);
   ps.vals = buf<uint32_t>(c, "n_vals", ps.units);
   ps.fpos = buf<int32_t>(c, "n_fpos", ps.nfilt);
-  CUFLYE_CHECK(runs_emit(c->idx, ps.qb, wmeta, wflags, wself, nstart, tile_off, fbits, ftile_off,
-                         ps.keys, ps.vals, ps.fpos, st));
+  CUFLYE_CHECK(runs_emit(c->idx, ps.qb, recs, nstart, tile_off, fbits, ftile_off, ps.keys, ps.vals,
+                         ps.fpos, st));
   ps.cbits = cbits;
 }
 

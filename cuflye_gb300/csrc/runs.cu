@@ -40,13 +40,7 @@ inline unsigned grid(uint64_t n, int b) {
   return static_cast<unsigned>((n + b - 1) / b > 0 ? (n + b - 1) / b : 1);
 }
 
-// Window flags of the run path, beside kWinRev, kWinFiltered and kWinTrivial:
-// the k-mer is solid; the base before the window; it is the query's first; the
-// window before is solid (as far as a run could continue from it).
-constexpr uint8_t kWinSolid = 8;
-constexpr int kWinBaseShift = 4;
-constexpr uint8_t kWinFirst = 64;
-constexpr uint8_t kWinPrevSolid = 128;
+constexpr uint8_t kWinSolid = 8;  // window flag beside kWinRev and kWinFiltered
 
 __device__ __forceinline__ uint32_t base_at(const uint64_t* __restrict__ words, uint64_t g) {
   return static_cast<uint32_t>(__ldg(words + (g >> 5)) >> (62 - 2 * (g & 31))) & 3u;
@@ -84,20 +78,19 @@ __global__ void neighbour_kernel(const uint64_t* __restrict__ pos, uint64_t n,
 }
 
 // What a bucket entry's neighbour nibble must be for its hit to continue the
-// run of the window before, and where the nibble sits in the entry's byte:
-// the base before the window, on the entry's strand (the complement of it
-// after the k-mer when the lookup flips).  7 matches no entry.
+// run of the window before (7 matches no entry), and where the nibble sits in
+// the entry's byte: the base before the window, on the entry's strand (the
+// complement of it after the k-mer when the lookup flips).
 struct RunTest {
   uint32_t expect;
-  int shift;
+  int shift;  // 0, or 4 when the lookup flips
 };
 
-__device__ __forceinline__ RunTest run_test(uint8_t fl, bool prev_solid) {
-  uint32_t e = 7;
-  if (!(fl & kWinFirst) && prev_solid) e = (fl >> kWinBaseShift) & 3u;
-  if (!(fl & kWinRev)) return RunTest{e, 0};
-  return RunTest{e == 7 ? 7u : 3u - e, 4};
-}
+// What the emission reads of a window that starts runs or is filtered:
+// {table word (8 bytes), the window's position in its query, own entry | expect
+// << 22 | flip << 25}.  Own entry: its place in the bucket, kNoSelf without one.
+constexpr uint32_t kNoSelf = (1u << kCountBits) - 1;
+static_assert(kCountBits == 22, "bucket places take 22 bits of a window record");
 
 __device__ __forceinline__ uint32_t bucket_size(uint64_t meta) {
   return static_cast<uint32_t>((meta >> 40) & ((1ULL << kCountBits) - 1));
@@ -158,6 +151,7 @@ __device__ __forceinline__ uint8_t probe_run_window(const DeviceIndex& idx, cons
   bool found;
   meta = table_probe(idx.table, idx.cap, km.key, &found);
   uint8_t fl = km.rev ? kWinRev : 0;
+  self = kNoSelf;
   if (!found) return fl;
   if (meta & kRepetitiveBit) return fl | kWinFiltered;
   fl |= kWinSolid;
@@ -172,7 +166,7 @@ __device__ __forceinline__ uint8_t probe_run_window(const DeviceIndex& idx, cons
   self = idx.self_at ? idx.self_at[idx.win_off[slot] + static_cast<uint64_t>(f)]
                      : bucket_find(idx, meta & kOffsetMask, bucket_size(meta),
                                    self_entry(idx, qdi, p, km.rev));
-  return fl | kWinTrivial;
+  return fl;
 }
 
 constexpr int kProbeBlock = 256;
@@ -181,32 +175,42 @@ constexpr int kProbeBlock = 256;
 // the run starts in the window's bucket.  Bound by the probe's scattered
 // loads (a table slot and two to three sectors of neighbours a window), which
 // is why both share a kernel: the counting of one warp hides the other's loads.
-__global__ void __launch_bounds__(kProbeBlock) probe_kernel(
-    DeviceIndex idx, QueryBatch q, uint64_t* __restrict__ wmeta, uint8_t* __restrict__ wflags,
-    uint32_t* __restrict__ wself, uint32_t* __restrict__ nstart, uint32_t* __restrict__ cbits,
-    uint32_t* __restrict__ fbits, uint32_t* __restrict__ tile_filt,
+__global__ void __launch_bounds__(kProbeBlock, 6) probe_kernel(
+    DeviceIndex idx, QueryBatch q, uint4* __restrict__ recs, uint32_t* __restrict__ nstart,
+    uint32_t* __restrict__ cbits, uint32_t* __restrict__ fbits, uint32_t* __restrict__ tile_filt,
     uint32_t* __restrict__ tile_start, unsigned long long* __restrict__ hit_total) {
   __shared__ uint32_t wsum[kProbeBlock / 32];
+  __shared__ uint32_t ends[2];             // queries of the block's first and last windows
   __shared__ bool solid[kProbeBlock + 1];  // of the windows before and in the block
-  const uint64_t w = static_cast<uint64_t>(blockIdx.x) * kProbeBlock + threadIdx.x;
+  const uint64_t w0 = static_cast<uint64_t>(blockIdx.x) * kProbeBlock, w = w0 + threadIdx.x;
   const int lane = threadIdx.x & 31;
-  uint64_t meta = 0;
-  uint32_t self = kNoLink;
+  if (threadIdx.x == 0)
+    ends[0] = query_of(q.win_off, q.nq, w0);
+  else if (threadIdx.x == 32)
+    ends[1] = query_of(q.win_off, q.nq, min(w0 + kProbeBlock, q.nwin) - 1);
+  __syncthreads();
+  uint64_t meta = 0, p = 0;
+  uint32_t self = kNoSelf, left = 7;
   uint8_t fl = 0;
   if (w < q.nwin) {
-    const uint32_t qi = query_of(q.win_off, q.nq, w);
-    const uint64_t p = w - q.win_off[qi];
-    fl = probe_run_window(idx, q, qi, p, meta, self);
-    if (p == 0)
-      fl |= kWinFirst;
-    else
-      fl |= static_cast<uint8_t>(base_at(q.words, q.base_off[qi] + p - 1) << kWinBaseShift);
+    uint32_t lo = ends[0], hi = ends[1];  // most blocks lie within one query
+    while (lo < hi) {
+      const uint32_t mid = (lo + hi + 1) >> 1;
+      if (__ldg(q.win_off + mid) <= w)
+        lo = mid;
+      else
+        hi = mid - 1;
+    }
+    p = w - q.win_off[lo];
+    fl = probe_run_window(idx, q, lo, p, meta, self);
+    if (p > 0) left = base_at(q.words, q.base_off[lo] + p - 1);
     if (threadIdx.x == 0) {
+      // the last window of the block before: could a run continue from it?
       bool before = false;
-      if (p > 0) {  // the last window of the block before
+      if (p > 0) {
         bool found;
-        const uint64_t m = table_probe(idx.table, idx.cap,
-                                       window_kmer(q, qi, p - 1, idx.k).key, &found);
+        const uint64_t m =
+            table_probe(idx.table, idx.cap, window_kmer(q, lo, p - 1, idx.k).key, &found);
         before = found && !(m & kRepetitiveBit);
       }
       solid[0] = before;
@@ -215,11 +219,11 @@ __global__ void __launch_bounds__(kProbeBlock) probe_kernel(
   solid[threadIdx.x + 1] = fl & kWinSolid;
   __syncthreads();
   uint32_t ns = 0, hits = 0;
+  RunTest rt{7, (fl & kWinRev) ? 4 : 0};
   if (fl & kWinSolid) {
-    const RunTest rt = run_test(fl, solid[threadIdx.x]);
-    if (rt.expect != 7) fl |= kWinPrevSolid;
+    if (left != 7 && solid[threadIdx.x]) rt.expect = rt.shift ? 3u - left : left;
     const uint64_t off = meta & kOffsetMask;
-    const uint32_t c = bucket_size(meta), own = self != kNoLink ? 1u : 0u;
+    const uint32_t c = bucket_size(meta), own = self != kNoSelf ? 1u : 0u;
     hits = c - own;
     if (rt.expect == 7) {
       ns = hits;
@@ -237,11 +241,10 @@ __global__ void __launch_bounds__(kProbeBlock) probe_kernel(
   const uint32_t sum = __reduce_add_sync(0xffffffffu, hits);
   if (w < q.nwin) {
     nstart[w] = ns;
-    if (ns) {  // what the emission reads
-      wmeta[w] = meta;
-      wflags[w] = fl;
-      wself[w] = self;
-    }
+    if (ns || (fl & kWinFiltered))
+      recs[w] = make_uint4(static_cast<uint32_t>(meta), static_cast<uint32_t>(meta >> 32),
+                           static_cast<uint32_t>(p),
+                           self | rt.expect << 22 | static_cast<uint32_t>(rt.shift) << 23);
     if (lane == 0) {
       cbits[w >> 5] = cb;
       fbits[w >> 5] = fb;
@@ -280,8 +283,7 @@ __global__ void query_offsets_kernel(QueryBatch q, const uint32_t* __restrict__ 
 // start runs (few windows do) are numbered through and taken 32 at a time, so
 // the lanes are busy whether a bucket holds two entries or two hundred.
 __global__ void __launch_bounds__(256) start_emit_kernel(
-    DeviceIndex idx, QueryBatch q, const uint64_t* __restrict__ wmeta,
-    const uint8_t* __restrict__ wflags, const uint32_t* __restrict__ wself,
+    DeviceIndex idx, QueryBatch q, const uint4* __restrict__ recs,
     const uint32_t* __restrict__ nstart, const uint64_t* __restrict__ tile_off,
     const uint32_t* __restrict__ fbits, const uint64_t* __restrict__ ftile_off,
     uint64_t* __restrict__ keys, uint32_t* __restrict__ vals, int32_t* __restrict__ fpos) {
@@ -294,24 +296,13 @@ __global__ void __launch_bounds__(256) start_emit_kernel(
     fb = fbits[w >> 5];
   }
   const bool filtered = (fb >> lane) & 1u;
-  uint32_t p = 0;
-  if (ns || filtered) {
-    const uint32_t qi = query_of(q.win_off, q.nq, w);
-    p = static_cast<uint32_t>(w - q.win_off[qi]);
-    if (filtered) fpos[ftile_off[w >> 5] + __popc(fb & lt)] = static_cast<int32_t>(p);
-  }
+  uint4 rec = make_uint4(0, 0, 0, 0);
+  if (ns || filtered) rec = recs[w];
+  const uint32_t p = rec.z;
+  if (filtered) fpos[ftile_off[w >> 5] + __popc(fb & lt)] = static_cast<int32_t>(p);
   if (!__any_sync(0xffffffffu, ns > 0)) return;
-  uint64_t off = 0;
-  uint32_t self = kNoLink, c = 0, test = 0;  // test: expected nibble | shift << 3 | rev << 6
-  if (ns) {
-    const uint8_t fl = wflags[w];
-    const uint64_t meta = wmeta[w];
-    const RunTest rt = run_test(fl, fl & kWinPrevSolid);
-    test = rt.expect | static_cast<uint32_t>(rt.shift) << 3 | ((fl & kWinRev) ? 64u : 0u);
-    self = wself[w];
-    off = meta & kOffsetMask;
-    c = bucket_size(meta);
-  }
+  const uint64_t meta = (static_cast<uint64_t>(rec.y) << 32) | rec.x, off = meta & kOffsetMask;
+  const uint32_t test = rec.w, c = ns ? bucket_size(meta) : 0;
   uint32_t upto = c;  // entries of this window and the ones before
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -331,17 +322,17 @@ __global__ void __launch_bounds__(256) start_emit_kernel(
     const uint64_t wo = __shfl_sync(0xffffffffu, off, src);
     const uint32_t wp = __shfl_sync(0xffffffffu, p, src);
     const uint32_t wt = __shfl_sync(0xffffffffu, test, src);
-    const uint32_t ws = __shfl_sync(0xffffffffu, self, src);
     const uint32_t e = j - (end - n);
     const bool start =
-        j < total && e != ws &&
-        ((static_cast<uint32_t>(__ldg(idx.nbr + wo + e)) >> ((wt >> 3) & 7u)) & 15u) != (wt & 7u);
+        j < total && e != (wt & kNoSelf) &&
+        ((static_cast<uint32_t>(__ldg(idx.nbr + wo + e)) >> ((wt >> 23) & 4u)) & 15u) !=
+            ((wt >> 22) & 7u);
     const unsigned m = __ballot_sync(0xffffffffu, start);
     if (start) {
       const uint64_t sv = __ldg(idx.pos + wo + e);
       uint32_t id = static_cast<uint32_t>(sv >> 32);
       int32_t pos = static_cast<int32_t>(sv & 0xffffffffu);
-      if (wt & 64u) {
+      if (wt >> 25) {
         pos = idx.slot_len[id >> 1] - pos - idx.k;
         id ^= 1u;
       }
@@ -739,14 +730,13 @@ cudaError_t index_neighbours(const uint64_t* pos, uint64_t npos, const uint64_t*
   return cudaGetLastError();
 }
 
-cudaError_t runs_count(const DeviceIndex& idx, const QueryBatch& q, uint64_t* wmeta,
-                       uint8_t* wflags, uint32_t* wself, uint32_t* nstart, uint32_t* cbits,
-                       uint32_t* fbits, uint32_t* tile_filt, uint32_t* tile_start,
-                       unsigned long long* hit_total, cudaStream_t s) {
+cudaError_t runs_count(const DeviceIndex& idx, const QueryBatch& q, uint4* recs, uint32_t* nstart,
+                       uint32_t* cbits, uint32_t* fbits, uint32_t* tile_filt,
+                       uint32_t* tile_start, unsigned long long* hit_total, cudaStream_t s) {
   if (q.nwin == 0) return cudaSuccess;
   count_launch();
   probe_kernel<<<grid(q.nwin, kProbeBlock), kProbeBlock, 0, s>>>(
-      idx, q, wmeta, wflags, wself, nstart, cbits, fbits, tile_filt, tile_start, hit_total);
+      idx, q, recs, nstart, cbits, fbits, tile_filt, tile_start, hit_total);
   return cudaGetLastError();
 }
 
@@ -760,15 +750,14 @@ cudaError_t runs_query_offsets(const QueryBatch& q, const uint32_t* nstart,
   return cudaGetLastError();
 }
 
-cudaError_t runs_emit(const DeviceIndex& idx, const QueryBatch& q, const uint64_t* wmeta,
-                      const uint8_t* wflags, const uint32_t* wself, const uint32_t* nstart,
-                      const uint64_t* tile_off, const uint32_t* fbits, const uint64_t* ftile_off,
-                      uint64_t* keys, uint32_t* vals, int32_t* fpos, cudaStream_t s) {
+cudaError_t runs_emit(const DeviceIndex& idx, const QueryBatch& q, const uint4* recs,
+                      const uint32_t* nstart, const uint64_t* tile_off, const uint32_t* fbits,
+                      const uint64_t* ftile_off, uint64_t* keys, uint32_t* vals, int32_t* fpos,
+                      cudaStream_t s) {
   if (q.nwin == 0) return cudaSuccess;
   count_launch();
-  start_emit_kernel<<<grid(q.nwin, 256), 256, 0, s>>>(idx, q, wmeta, wflags, wself, nstart,
-                                                      tile_off, fbits, ftile_off, keys, vals,
-                                                      fpos);
+  start_emit_kernel<<<grid(q.nwin, 256), 256, 0, s>>>(idx, q, recs, nstart, tile_off, fbits,
+                                                      ftile_off, keys, vals, fpos);
   return cudaGetLastError();
 }
 

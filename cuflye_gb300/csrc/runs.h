@@ -88,24 +88,23 @@ cudaError_t index_neighbours(const uint64_t* pos, uint64_t npos, const uint64_t*
                              const uint64_t* base_off, const int32_t* slot_len, int k,
                              uint8_t* nbr, cudaStream_t s);
 
-// Per window its run starts (nstart), and for windows that have some the table
-// meta, flags and own entry; per 32 windows the run starts, and the bits of
+// Per window its run starts (nstart), and a record (recs) for runs_emit where
+// it has some or is filtered; per 32 windows the run starts, and the bits of
 // solid and of filtered windows; hit totals spread over 64 words of hit_total
 // (zeroed by the caller).
-cudaError_t runs_count(const DeviceIndex& idx, const QueryBatch& q, uint64_t* wmeta,
-                       uint8_t* wflags, uint32_t* wself, uint32_t* nstart, uint32_t* cbits,
-                       uint32_t* fbits, uint32_t* tile_filt, uint32_t* tile_start,
-                       unsigned long long* hit_total, cudaStream_t s);
+cudaError_t runs_count(const DeviceIndex& idx, const QueryBatch& q, uint4* recs, uint32_t* nstart,
+                       uint32_t* cbits, uint32_t* fbits, uint32_t* tile_filt,
+                       uint32_t* tile_start, unsigned long long* hit_total, cudaStream_t s);
 // Each query's first run and first filtered position (nq + 1 entries each).
 cudaError_t runs_query_offsets(const QueryBatch& q, const uint32_t* nstart,
                                const uint64_t* tile_off, const uint32_t* fbits,
                                const uint64_t* ftile_off, uint64_t* q_off, uint64_t* f_off,
                                cudaStream_t s);
 // The run starts in window order, then bucket order, and the filtered positions.
-cudaError_t runs_emit(const DeviceIndex& idx, const QueryBatch& q, const uint64_t* wmeta,
-                      const uint8_t* wflags, const uint32_t* wself, const uint32_t* nstart,
-                      const uint64_t* tile_off, const uint32_t* fbits, const uint64_t* ftile_off,
-                      uint64_t* keys, uint32_t* vals, int32_t* fpos, cudaStream_t s);
+cudaError_t runs_emit(const DeviceIndex& idx, const QueryBatch& q, const uint4* recs,
+                      const uint32_t* nstart, const uint64_t* tile_off, const uint32_t* fbits,
+                      const uint64_t* ftile_off, uint64_t* keys, uint32_t* vals, int32_t* fpos,
+                      cudaStream_t s);
 
 // Run lengths, group prefilter, and the pieces of groups whose runs are in
 // order already; the other survivors are listed for runs_order.
