@@ -890,7 +890,8 @@ const char* const kPerHitBuffers[] = {"h_keys",  "h_vals",   "h_kmers", "s_l",  
 // Buffers sized by the run count of a pass on the run path.
 const char* const kPerRunBuffers[] = {"n_keys", "n_vals", "n_akeys", "n_avals", "n_rlen", "n_pa",
                                       "n_pb",   "n_pl",   "n_ps",    "n_pk",    "n_po",   "n_pd",
-                                      "n_pm",   "m_tiles", "m_counts", "n_tcount", "n_toffg"};
+                                      "n_pm",   "n_pp",   "n_pe",    "m_tiles", "m_counts", "n_tcount",
+                                      "n_toffg"};
 
 // The pass's hits in Flye's generation order (and the filtered positions).
 void emit_generation_order(cuflye_ctx* c, PassState& ps) {
@@ -1134,9 +1135,9 @@ bool run_path(const cuflye_ctx* c, const ChainParams& cp) {
 }
 
 // Device bytes per run: sorted pairs and their second buffer (24), length
-// (4), pieces with score, link and walk state (40 and half as much for cut
-// ones), and about as much for the per-group tables.
-constexpr uint64_t kRunBytes = 128;
+// (4), pieces with score, link and walk state (48 and half as much for cut
+// ones), and the per-group tables.
+constexpr uint64_t kRunBytes = 144;
 
 // Counts ps's run starts (queries uploaded): the longest prefix of the queries
 // whose runs fit in device memory stays in ps, sorted out but not written.
@@ -1614,7 +1615,8 @@ GroupRows chain_groups(cuflye_ctx* c, uint64_t* keys, uint32_t* vals, uint64_t H
     c->hits_flagged += c->emit_tally[0];
     c->hits_prefiltered += c->emit_tally[1];
   }
-  const uint64_t pool_cap = 8ull * survivors + 1024;
+  // (a row a group beyond eight: one that max_divergence drops later)
+  const uint64_t pool_cap = 9ull * survivors + 1024;
   OverlapRow* pool = buf<OverlapRow>(c, "o_pool", pool_cap);
   uint32_t* pool_count = buf<uint32_t>(c, "o_poolcount", 1);
   uint32_t* group_rows = buf<uint32_t>(c, "o_grows", G);
@@ -1638,6 +1640,7 @@ GroupRows chain_groups(cuflye_ctx* c, uint64_t* keys, uint32_t* vals, uint64_t H
                                nullptr, nullptr, qinfo, f_off, fpos, slot_signed, c->logt,
                                cp, pool, pool_cap, pool_count, group_rows, c->status, G32, gmaps,
                                gmap_words, work, c->shape.backtrack_blocks_per_sm, st));
+  CUFLYE_CHECK(chain_open_rows(pool, pool_cap, pool_count, c->logt, cp, group_rows, c->num_sms, st));
   return GroupRows{pool, pool_count, pool_cap, group_rows};
 }
 
@@ -1896,6 +1899,8 @@ ChainRows chain_runs(cuflye_ctx* c, PassState& ps, const ChainParams& cp) {
   t.pk = buf<uint32_t>(c, "n_pk", P);
   t.po = buf<int32_t>(c, "n_po", P);
   t.pd = buf<int32_t>(c, "n_pd", P);
+  t.pp = buf<int32_t>(c, "n_pp", P);
+  t.pe = buf<int32_t>(c, "n_pe", P);
   t.pm = buf<uint32_t>(c, "n_pm", 3 * P);
   t.lists = buf<uint32_t>(c, "n_lists", kRunClasses * G);
   t.sort_lists = buf<uint32_t>(c, "n_slists", 2 * G);
@@ -1922,10 +1927,13 @@ ChainRows chain_runs(cuflye_ctx* c, PassState& ps, const ChainParams& cp) {
   }
   CUFLYE_CHECK(runs_dp(t, cp, c->num_sms, c->shape.dp_blocks_per_sm, st));
   mark(c, 3);
-  const uint64_t pool_cap = 8ull * survivors + 1024;
+  // (a row a group beyond eight: one that max_divergence drops later)
+  const uint64_t pool_cap = 9ull * survivors + 1024;
   OverlapRow* pool = buf<OverlapRow>(c, "n_pool", pool_cap);
   CUFLYE_CHECK(runs_backtrack(t, cp, ps.f_off, ps.fpos, c->logt, pool, pool_cap, group_rows,
                               c->status, c->num_sms, c->shape.backtrack_blocks_per_sm, st));
+  CUFLYE_CHECK(chain_open_rows(pool, pool_cap, t.counts + kRcPool, c->logt, cp, group_rows,
+                               c->num_sms, st));
   // 4. max_overlaps + compaction in group order
   uint64_t* qg = buf<uint64_t>(c, "n_qg", nq + 1);
   uint64_t* kept_off = buf<uint64_t>(c, "n_keptoff", G + 1);

@@ -639,14 +639,14 @@ __device__ void walk_maps(const uint32_t* link, const uint32_t* step, uint32_t* 
   }
 }
 
-// The overlap of one walked chain (start s0 back to first): overlapTest,
-// then the k-mer divergence; kept proposals are appended to props.
+// The overlap of one walked chain (start s0 back to first): overlapTest, then
+// the k-mer divergence (whole warp); kept proposals are appended to lane 0's props.
 __device__ __forceinline__ void add_proposal(
     const uint64_t* __restrict__ keys, const uint32_t* __restrict__ vals,
     const int32_t* __restrict__ score, uint64_t b, uint32_t s0, int32_t first, int32_t clen,
     const QueryInfo& qi, int64_t ext_signed, const GroupInfo& g, const int32_t* fq, uint32_t nf,
-    const LogfTable& logt, const ChainParams& p, DeviceStatus* st, uint32_t gidx, Prop* props,
-    int& np, bool& overflow) {
+    const ChainParams& p, DeviceStatus* st, uint32_t gidx, Prop* props, int& np,
+    bool& overflow) {
   const bool swapped = g.ext_sorted == 1;
   const int32_t k = p.k;
   int32_t c0, e0, c1, e1;
@@ -659,7 +659,7 @@ __device__ __forceinline__ void add_proposal(
   o.ee = e1 + k - 1;
   o.score = score[b + s0] - score[b + first] + k - 1;
   o.clen = clen;
-  keep_proposal(o, qi, ext_signed, g.ext_len, fq, nf, logt, p, st, gidx, props, np, overflow);
+  keep_proposal(o, qi, ext_signed, g.ext_len, fq, nf, p, st, gidx, props, np, overflow);
 }
 
 __global__ void __launch_bounds__(kBtWarps * 32, 4) backtrack_kernel(
@@ -776,8 +776,8 @@ __global__ void __launch_bounds__(kBtWarps * 32, 4) backtrack_kernel(
       bool met = false;
       walk_maps(lk, sp, dn, bt + b, static_cast<int32_t>(mi), first, clen, remaining, nullptr,
                 met);
-      if (lane == 0 && !overflow)
-        add_proposal(keys, vals, score, b, mi, first, clen, qi, ext_signed, g, fq, nf, logt, p, st,
+      if (!overflow)
+        add_proposal(keys, vals, score, b, mi, first, clen, qi, ext_signed, g, fq, nf, p, st,
                      gidx, props, np, overflow);
       __syncwarp();
       continue;
@@ -806,9 +806,9 @@ __global__ void __launch_bounds__(kBtWarps * 32, 4) backtrack_kernel(
           clash = true;
           break;
         }
-        if (lane == 0 && !overflow)
-          add_proposal(keys, vals, score, b, s0, first, clen, qi, ext_signed, g, fq, nf, logt, p,
-                       st, gidx, props, np, overflow);
+        if (!overflow)
+          add_proposal(keys, vals, score, b, s0, first, clen, qi, ext_signed, g, fq, nf, p, st,
+                       gidx, props, np, overflow);
         __syncwarp();
       }
     }
@@ -843,8 +843,8 @@ __global__ void __launch_bounds__(kBtWarps * 32, 4) backtrack_kernel(
       bool met = false;
       walk_maps(lk, sp, dn, bt + b, static_cast<int32_t>(s0), first, clen, remaining, nullptr,
                 met);
-      if (lane == 0 && !overflow)
-        add_proposal(keys, vals, score, b, s0, first, clen, qi, ext_signed, g, fq, nf, logt, p, st,
+      if (!overflow)
+        add_proposal(keys, vals, score, b, s0, first, clen, qi, ext_signed, g, fq, nf, p, st,
                      gidx, props, np, overflow);
       __syncwarp();
       if (remaining == 0) break;
@@ -864,8 +864,24 @@ __global__ void __launch_bounds__(kBtWarps * 32, 4) backtrack_kernel(
     group_rows[gidx] = 0;
     continue;
   }
-  finish_group(props, np, qi, g.query, g.ext_di, g.ext_len, gidx, p, pool, pool_cap, pool_count,
-               group_rows, st);
+  finish_group(props, np, qi, g.query, g.ext_di, g.ext_len, gidx, logt, p, pool, pool_cap,
+               pool_count, group_rows, st);
+  }
+}
+
+// The divergence of the rows that backtracks left open, a thread each; rows
+// over max_divergence are dropped.
+__global__ void open_rows_kernel(OverlapRow* __restrict__ pool, uint64_t pool_cap,
+                                 const uint32_t* __restrict__ pool_count, LogfTable logt,
+                                 ChainParams p, uint32_t* __restrict__ group_rows) {
+  const uint32_t n = static_cast<uint32_t>(min(static_cast<uint64_t>(*pool_count), pool_cap));
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    if (!(pool[i].rank & kRankOpen)) continue;
+    const float d = fdiv(flye_logf(pool[i].div, logt), static_cast<float>(p.k));
+    const bool kept = d < p.max_divergence;
+    pool[i].div = d;
+    pool[i].rank = kept ? 0u : kRankDropped;
+    if (!kept) group_rows[pool[i].group] = 0;
   }
 }
 
@@ -1088,6 +1104,15 @@ cudaError_t chain_backtrack(const uint64_t* keys, const uint32_t* vals, const in
       keys, vals, score, bt, order, groups, list, list_count, top, redo_list, redo_count,
       qinfo, f_off, fpos, slot_signed, logt,
       p, pool, pool_cap, pool_count, group_rows, st, gmaps, gmap_words, work);
+  return cudaGetLastError();
+}
+
+cudaError_t chain_open_rows(OverlapRow* pool, uint64_t pool_cap, const uint32_t* pool_count,
+                            const LogfTable& logt, const ChainParams& p, uint32_t* group_rows,
+                            int num_sms, cudaStream_t s) {
+  count_launch();
+  open_rows_kernel<<<static_cast<unsigned>(std::min<uint64_t>(grid(pool_cap, 128), 8ull * num_sms)),
+                     128, 0, s>>>(pool, pool_cap, pool_count, logt, p, group_rows);
   return cudaGetLastError();
 }
 

@@ -434,6 +434,11 @@ cudaError_t chain_backtrack(const uint64_t* keys, const uint32_t* vals, const in
                             uint32_t* pool_count, uint32_t* group_rows, DeviceStatus* st,
                             uint32_t max_groups, uint32_t* gmaps, uint64_t gmap_words,
                             uint32_t* work, int per_sm, cudaStream_t s);
+// After the backtracks of a pool: the divergence of its groups' only rows, and
+// the max_divergence filter on them (group_rows is corrected).
+cudaError_t chain_open_rows(OverlapRow* pool, uint64_t pool_cap, const uint32_t* pool_count,
+                            const LogfTable& logt, const ChainParams& p, uint32_t* group_rows,
+                            int num_sms, cudaStream_t s);
 // max_overlaps cutoff and group-order compaction of the pooled rows.
 cudaError_t rows_limit(const uint32_t* group_rows, const uint64_t* q_group_off, uint32_t nq,
                        int32_t max_overlaps, uint32_t* kept_rows, cudaStream_t s);

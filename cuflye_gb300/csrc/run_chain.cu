@@ -707,48 +707,81 @@ struct WalkSmem {
   uint32_t link[kWalkCap];
   int32_t off[kWalkCap];
   int32_t done[kWalkCap];
+  int32_t upto[kWalkCap];
+  int32_t end[kWalkCap];
 };
 
 struct WalkTables {
-  const uint32_t* link;
-  const int32_t* off;
-  int32_t* done;
-  uint32_t* marks;  // tie rounds: {round, least, greatest} offset walked, per piece
+  const uint32_t* link;  // per piece: the piece its first element links to (kNoLink: none) ...
+  const int32_t* off;    // ... and the element of it
+  int32_t* done;         // elements cleared, from the first on
+  int32_t* upto;         // elements of the pieces up to this one
+  int32_t* end;          // score of the last element, kNoScore if it has no link
+  uint32_t* marks;       // tie rounds: {round, least, greatest} offset walked, per piece
+  __device__ __forceinline__ int32_t before(uint32_t i) const { return i ? upto[i - 1] : 0; }
+  __device__ __forceinline__ int32_t len(uint32_t i) const { return upto[i] - before(i); }
 };
+
+// Marks offsets lo .. hi of piece r walked in a tie round.
+__device__ __forceinline__ void mark_walked(const WalkTables& w, uint32_t r, uint32_t round,
+                                            int32_t lo, int32_t hi) {
+  uint32_t* m = w.marks + 3ull * r;
+  const bool mine = m[0] == round;
+  m[1] = static_cast<uint32_t>(mine ? min(static_cast<int32_t>(m[1]), lo) : lo);
+  m[2] = static_cast<uint32_t>(mine ? max(static_cast<int32_t>(m[2]), hi) : hi);
+  m[0] = round;
+}
 
 // Walk from element off of piece r: first element, chain length as Flye's walk
 // counts them; what it visits becomes cleared.  round > 0: visited elements
 // are marked, and `met` tells whether the walk ended on a linked element
-// marked in the same round.
+// marked in the same round.  Pieces that link to the end of the piece before
+// and are not yet cleared are passed 32 at a time.
 __device__ __forceinline__ void walk_pieces(const WalkTables& w, uint32_t r, int32_t off,
                                             uint32_t round, uint32_t& fr, int32_t& fo,
                                             int32_t& clen, bool& met) {
   const int lane = threadIdx.x & 31;
   clen = 0;
   for (;;) {
+    const int32_t j = static_cast<int32_t>(r) - lane;
+    bool pass = false;
+    int32_t l = 0;
+    if (j > 0) {
+      l = w.len(j);
+      pass = w.link[j] == static_cast<uint32_t>(j - 1) && w.off[j] == w.len(j - 1) - 1 &&
+             w.done[j] == 0;
+    }
+    const unsigned held = ~__ballot_sync(0xffffffffu, pass);
+    const int np = held ? __ffs(held) - 1 : 32;  // pieces passed
+    if (np > 0) {
+      if (lane < np) {
+        const int32_t top = lane == 0 ? off : l - 1;
+        w.done[j] = top + 1;
+        if (round) mark_walked(w, static_cast<uint32_t>(j), round, 0, top);
+      }
+      clen += off + 1 + w.before(r) - w.before(r - np + 1);
+      __syncwarp();
+      r -= np;
+      off = w.len(r) - 1;
+      if (np == 32) continue;
+    }
+    // piece r: down to z, and there stop if z is cleared or has no link
     const int32_t d = w.done[r];
     const uint32_t link = w.link[r];
-    // the walk goes down to z and stops there if z is cleared or not linked
     const int32_t z = off < d ? off : d > 0 ? d - 1 : 0;
-    const bool cleared = d > 0;
     const bool linked = z > 0 || link != kNoLink;
-    const bool stop = cleared || !linked;
+    const bool stop = d > 0 || !linked;
     clen += off - z + 1;
-    if (round) {
+    if (round && stop) {
       const uint32_t* m = w.marks + 3ull * r;
-      const bool mine = m[0] == round;
-      const int32_t lo = mine ? static_cast<int32_t>(m[1]) : INT_MAX;
-      const int32_t hi = mine ? static_cast<int32_t>(m[2]) : -1;
-      if (stop) met = linked && z >= lo && z <= hi;
-      __syncwarp();
-      if (lane == 0) {
-        w.marks[3ull * r] = round;
-        w.marks[3ull * r + 1] = static_cast<uint32_t>(min(lo, z));
-        w.marks[3ull * r + 2] = static_cast<uint32_t>(max(hi, off));
-      }
+      met = linked && m[0] == round && z >= static_cast<int32_t>(m[1]) &&
+            z <= static_cast<int32_t>(m[2]);
     }
     __syncwarp();
-    if (lane == 0 && off >= d) w.done[r] = off + 1;
+    if (lane == 0) {
+      if (off >= d) w.done[r] = off + 1;
+      if (round) mark_walked(w, r, round, z, off);
+    }
     __syncwarp();
     if (stop) {
       fr = r;
@@ -760,6 +793,9 @@ __device__ __forceinline__ void walk_pieces(const WalkTables& w, uint32_t r, int
   }
 }
 
+// One warp a group.  Bound by the latency of each group's chain (tables loaded,
+// walks, the searches of a proposal), so everything a walk reads is staged in
+// shared memory, and the searches probe 32 places a round.
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, 4) run_backtrack_kernel(
     RunTables t, ChainParams p, const uint64_t* __restrict__ f_off,
     const int32_t* __restrict__ fpos, LogfTable logt, OverlapRow* __restrict__ pool,
@@ -780,18 +816,32 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 4) run_backtrack_kernel(
                                                : t.idx.slot_signed[g.ext_di >> 1];
     const int32_t* fq = fpos + f_off[g.query];
     const uint32_t nf = static_cast<uint32_t>(f_off[g.query + 1] - f_off[g.query]);
-    WalkTables w{sw.link, sw.off, sw.done, t.pm + 3 * base};
-    if (n <= kWalkCap) {
-      for (uint32_t i = lane; i < n; i += 32) {
-        sw.link[i] = t.pk[base + i];
-        sw.off[i] = t.po[base + i];
-        sw.done[i] = 0;
-      }
-    } else {
+    const bool small = n <= kWalkCap;
+    WalkTables w{sw.link, sw.off, sw.done, sw.upto, sw.end, t.pm + 3 * base};
+    if (!small) {
       w.link = t.pk + base;
       w.off = t.po + base;
       w.done = t.pd + base;
-      for (uint32_t i = lane; i < n; i += 32) t.pd[base + i] = 0;
+      w.upto = t.pp + base;
+      w.end = t.pe + base;
+    }
+    int32_t total = 0;
+    for (uint32_t i0 = 0; i0 < n; i0 += 32) {
+      const uint32_t i = i0 + lane;
+      const bool in = i < n;
+      const int32_t l = in ? t.pl[base + i] : 0;
+      const int32_t upto = scan_add(l);
+      if (in) {
+        const uint32_t link = t.pk[base + i];
+        if (small) {
+          sw.link[i] = link;
+          sw.off[i] = t.po[base + i];
+        }
+        w.done[i] = 0;
+        w.upto[i] = total + upto;
+        w.end[i] = l >= 2 || link != kNoLink ? t.ps[base + i] + l - 1 : kNoScore;
+      }
+      total += __shfl_sync(0xffffffffu, upto, 31);
     }
     __syncwarp();
     Prop props[kMaxProposals];
@@ -799,8 +849,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 4) run_backtrack_kernel(
     bool overflow = false, ambiguous = false, multi = false;
     uint32_t round = 0;
     auto propose = [&](uint32_t r, uint32_t fr, int32_t fo, int32_t clen) {
-      if (lane != 0 || overflow) return;
-      const int32_t l1 = t.pl[base + r] - 1;
+      if (overflow) return;
+      const int32_t l1 = w.len(r) - 1;
       const int32_t a0 = t.pa[base + fr] + fo, b0 = t.pb[base + fr] + fo;
       const int32_t a1 = t.pa[base + r] + l1, b1 = t.pb[base + r] + l1;
       Prop o;
@@ -808,9 +858,9 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 4) run_backtrack_kernel(
       o.ce = (es ? b1 : a1) + p.k - 1;
       o.eb = es ? a0 : b0;
       o.ee = (es ? a1 : b1) + p.k - 1;
-      o.score = (t.ps[base + r] + l1) - (t.ps[base + fr] + fo) + p.k - 1;
+      o.score = w.end[r] - (t.ps[base + fr] + fo) + p.k - 1;
       o.clen = clen;
-      keep_proposal(o, qi, ext_signed, g.ext_len, fq, nf, logt, p, st, gidx, props, np, overflow);
+      keep_proposal(o, qi, ext_signed, g.ext_len, fq, nf, p, st, gidx, props, np, overflow);
     };
     // Starts by score: the live linked element of the highest score next, always
     // the end of a piece.  Ends sharing the top score are walked in order; see
@@ -819,9 +869,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 4) run_backtrack_kernel(
       int32_t bs = INT_MIN;
       uint32_t bi = kNoLink, bc = 0;
       for (uint32_t i = lane; i < n; i += 32) {
-        const int32_t l = t.pl[base + i];
-        if (w.done[i] >= l || (l < 2 && w.link[i] == kNoLink)) continue;
-        const int32_t s = t.ps[base + i] + l - 1;
+        const int32_t s = w.end[i];
+        if (s == kNoScore || w.done[i] >= w.len(i)) continue;
         if (s > bs) {
           bs = s;
           bi = i;
@@ -838,7 +887,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 4) run_backtrack_kernel(
       int32_t fo = 0, clen = 0;
       bool met = false;
       if (mc == 1) {
-        walk_pieces(w, mi, t.pl[base + mi] - 1, 0, fr, fo, clen, met);
+        walk_pieces(w, mi, w.len(mi) - 1, 0, fr, fo, clen, met);
         propose(mi, fr, fo, clen);
         __syncwarp();
         continue;
@@ -855,16 +904,13 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 4) run_backtrack_kernel(
       for (uint32_t i0 = mi & ~31u; i0 < n && left > 0 && !clash; i0 += 32) {
         const uint32_t i = i0 + lane;
         bool tied = false;
-        if (i < n) {
-          const int32_t l = t.pl[base + i];
-          tied = w.done[i] < l && (l >= 2 || w.link[i] != kNoLink) && t.ps[base + i] + l - 1 == ms;
-        }
+        if (i < n) tied = w.end[i] == ms && w.done[i] < w.len(i);
         unsigned tm = __ballot_sync(0xffffffffu, tied);
         while (tm && !clash) {
           const uint32_t r = i0 + __ffs(tm) - 1;
           tm &= tm - 1;
           --left;
-          const int32_t l = t.pl[base + r];
+          const int32_t l = w.len(r);
           if (w.done[r] >= l) {  // cleared by an earlier walk of this round
             clash = true;
             break;
@@ -900,7 +946,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 4) run_backtrack_kernel(
     } else if (overflow) {
       group_rows[gidx] = 0;
     } else {
-      finish_group(props, np, qi, g.query, g.ext_di, g.ext_len, gidx, p, pool, pool_cap,
+      finish_group(props, np, qi, g.query, g.ext_di, g.ext_len, gidx, logt, p, pool, pool_cap,
                    t.counts + kRcPool, group_rows, st);
     }
   }

@@ -31,6 +31,7 @@
 #include "common.cuh"
 #include "hits.cuh"
 #include "kernels.h"
+#include "proposals.cuh"
 #include "runs.h"
 
 namespace cuflye {
@@ -675,6 +676,7 @@ __global__ void append_rows_kernel(const OverlapRow* __restrict__ from,
   const uint32_t n = *nfrom;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     OverlapRow r = from[i];
+    if (r.rank == kRankDropped) continue;
     r.group = list[r.group];
     const uint32_t d = atomicAdd(pool_count, 1u);
     if (d < pool_cap)

@@ -72,7 +72,9 @@ struct RunTables {
   int32_t* ps = nullptr;   // score of the piece's first element
   uint32_t* pk = nullptr;  // its link: piece of the group (kNoLink: none) ...
   int32_t* po = nullptr;   // ... and offset in it
-  int32_t* pd = nullptr;   // elements cleared by the backtrack (pieces beyond shared memory)
+  // the backtrack's tables of groups beyond shared memory: elements cleared,
+  // elements up to each piece, end scores
+  int32_t *pd = nullptr, *pp = nullptr, *pe = nullptr;
   uint32_t* pm = nullptr;  // tie-round marks, 3 words a piece
   uint32_t* lists = nullptr;       // kRunClasses * max_groups
   uint32_t* sort_lists = nullptr;  // 2 * max_groups
