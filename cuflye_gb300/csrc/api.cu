@@ -1901,7 +1901,7 @@ ChainRows chain_runs(cuflye_ctx* c, PassState& ps, const ChainParams& cp) {
   t.pd = buf<int32_t>(c, "n_pd", P);
   t.pp = buf<int32_t>(c, "n_pp", P);
   t.pe = buf<int32_t>(c, "n_pe", P);
-  t.pm = buf<uint32_t>(c, "n_pm", 3 * P);
+  t.pm = buf<uint32_t>(c, "n_pm", 2 * P);
   t.lists = buf<uint32_t>(c, "n_lists", kRunClasses * G);
   t.sort_lists = buf<uint32_t>(c, "n_slists", 2 * G);
   t.open_list = buf<uint32_t>(c, "n_open", G);

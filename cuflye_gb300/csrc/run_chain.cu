@@ -487,6 +487,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) run_dp_kernel(RunTables t
     int32_t s_prev = 0, e_prev = 0;  // score and end of the piece before the next one
     int32_t big = kNoScore;          // greatest end of the pieces before that one
     bool open = false;
+    uint32_t first_tied = 0;  // pieces in a tie cluster at the first position
     if (lane < static_cast<int>(n)) {
       na = t.pa[base + lane];
       nb = t.pb[base + lane];
@@ -524,9 +525,22 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) run_dp_kernel(RunTables t
       }
       const unsigned okm = __ballot_sync(0xffffffffu, ok);
       uint32_t u = 0;
-      if (i0 == 0) {  // element 0 of the group: score 0, no link
-        s_prev = 0;
-        e_prev = 0;
+      if (i0 == 0) {
+        // Element 0 of the group: score 0, no link.  In a tie cluster at the
+        // group's first position any piece may be it; they score k, and if one
+        // of them becomes a link (with score 0 it never would) the group stays
+        // open
+        const int32_t at0 = __shfl_sync(0xffffffffu, ca, 0);
+        const bool at_first = lane < static_cast<int>(len) && ca == at0;
+        first_tied = __popc(__ballot_sync(0xffffffffu, at_first));
+        if (first_tied == 1) first_tied = 0;
+        s_prev = first_tied ? p.k : 0;
+        e_prev = s_prev;
+        if (lane == 0) {
+          cs = s_prev;
+          if (ties) t.ps[base] = s_prev;
+        }
+        if (ties) __syncwarp();
         u = 1;
       }
       while (u < len && !open) {
@@ -651,7 +665,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) run_dp_kernel(RunTables t
         }
         const int32_t si = max(best, p.k);
         if (ties) {
-          if (i == 1 && ai == __shfl_sync(0xffffffffu, ra, 0)) open = true;
+          if (best > p.k && bestj < first_tied) open = true;
           // the cluster so far: could the elements inside one of two pieces
           // link into the other (one axis position back, so on a lower second
           // position)?
@@ -717,25 +731,25 @@ struct WalkTables {
   int32_t* done;         // elements cleared, from the first on
   int32_t* upto;         // elements of the pieces up to this one
   int32_t* end;          // score of the last element, kNoScore if it has no link
-  uint32_t* marks;       // tie rounds: {round, least, greatest} offset walked, per piece
+  uint32_t* marks;       // per piece: the last tie round that walked it, and
+                         // what was cleared of it before that round
   __device__ __forceinline__ int32_t before(uint32_t i) const { return i ? upto[i - 1] : 0; }
   __device__ __forceinline__ int32_t len(uint32_t i) const { return upto[i] - before(i); }
 };
 
-// Marks offsets lo .. hi of piece r walked in a tie round.
+// Notes that a tie round walks piece r, d of whose elements are cleared.
 __device__ __forceinline__ void mark_walked(const WalkTables& w, uint32_t r, uint32_t round,
-                                            int32_t lo, int32_t hi) {
-  uint32_t* m = w.marks + 3ull * r;
-  const bool mine = m[0] == round;
-  m[1] = static_cast<uint32_t>(mine ? min(static_cast<int32_t>(m[1]), lo) : lo);
-  m[2] = static_cast<uint32_t>(mine ? max(static_cast<int32_t>(m[2]), hi) : hi);
+                                            int32_t d) {
+  uint32_t* m = w.marks + 2ull * r;
+  if (m[0] != round) m[1] = static_cast<uint32_t>(d);
   m[0] = round;
 }
 
 // Walk from element off of piece r: first element, chain length as Flye's walk
-// counts them; what it visits becomes cleared.  round > 0: visited elements
-// are marked, and `met` tells whether the walk ended on a linked element
-// marked in the same round.  Pieces that link to the end of the piece before
+// counts them; what it visits becomes cleared.  round > 0: `met` tells whether
+// the walk ended on a linked element that another walk of the round cleared (an
+// element cleared before the round ends every walk that reaches it, as one
+// without a link does).  Pieces that link to the end of the piece before
 // and are not yet cleared are passed 32 at a time.
 __device__ __forceinline__ void walk_pieces(const WalkTables& w, uint32_t r, int32_t off,
                                             uint32_t round, uint32_t& fr, int32_t& fo,
@@ -757,7 +771,7 @@ __device__ __forceinline__ void walk_pieces(const WalkTables& w, uint32_t r, int
       if (lane < np) {
         const int32_t top = lane == 0 ? off : l - 1;
         w.done[j] = top + 1;
-        if (round) mark_walked(w, static_cast<uint32_t>(j), round, 0, top);
+        if (round) mark_walked(w, static_cast<uint32_t>(j), round, 0);
       }
       clen += off + 1 + w.before(r) - w.before(r - np + 1);
       __syncwarp();
@@ -773,14 +787,13 @@ __device__ __forceinline__ void walk_pieces(const WalkTables& w, uint32_t r, int
     const bool stop = d > 0 || !linked;
     clen += off - z + 1;
     if (round && stop) {
-      const uint32_t* m = w.marks + 3ull * r;
-      met = linked && m[0] == round && z >= static_cast<int32_t>(m[1]) &&
-            z <= static_cast<int32_t>(m[2]);
+      const uint32_t* m = w.marks + 2ull * r;
+      met = linked && z < d && m[0] == round && z >= static_cast<int32_t>(m[1]);
     }
     __syncwarp();
     if (lane == 0) {
       if (off >= d) w.done[r] = off + 1;
-      if (round) mark_walked(w, r, round, z, off);
+      if (round) mark_walked(w, r, round, d);
     }
     __syncwarp();
     if (stop) {
@@ -817,7 +830,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 4) run_backtrack_kernel(
     const int32_t* fq = fpos + f_off[g.query];
     const uint32_t nf = static_cast<uint32_t>(f_off[g.query + 1] - f_off[g.query]);
     const bool small = n <= kWalkCap;
-    WalkTables w{sw.link, sw.off, sw.done, sw.upto, sw.end, t.pm + 3 * base};
+    WalkTables w{sw.link, sw.off, sw.done, sw.upto, sw.end, t.pm + 2 * base};
     if (!small) {
       w.link = t.pk + base;
       w.off = t.po + base;
@@ -894,7 +907,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 4) run_backtrack_kernel(
       }
       // a tie round over the mc live ends of score ms
       if (round == 0) {
-        for (uint32_t i = lane; i < n; i += 32) w.marks[3ull * i] = 0;
+        for (uint32_t i = lane; i < n; i += 32) w.marks[2ull * i] = 0;
         __syncwarp();
       }
       ++round;

@@ -75,7 +75,7 @@ struct RunTables {
   // the backtrack's tables of groups beyond shared memory: elements cleared,
   // elements up to each piece, end scores
   int32_t *pd = nullptr, *pp = nullptr, *pe = nullptr;
-  uint32_t* pm = nullptr;  // tie-round marks, 3 words a piece
+  uint32_t* pm = nullptr;  // tie-round marks, 2 words a piece
   uint32_t* lists = nullptr;       // kRunClasses * max_groups
   uint32_t* sort_lists = nullptr;  // 2 * max_groups
   uint32_t* open_list = nullptr;   // max_groups
