@@ -250,19 +250,11 @@ void scan_u32_async(cuflye_ctx* c, const uint32_t* in, uint64_t* out, uint64_t n
                     const char* temp_name) {
   uint64_t* temp = buf<uint64_t>(c, temp_name, scan_temp_words(n));
   CUFLYE_CHECK(exclusive_scan_u32_to_u64(in, out, n, temp, c->stream));
-  const uint64_t ntiles = scan_temp_words(n) - 1;
-  CUFLYE_CHECK(cudaMemcpyAsync(out + n, temp + (n ? ntiles : 0), sizeof(uint64_t),
-                               cudaMemcpyDeviceToDevice, c->stream));
 }
 
 uint64_t scan_u32(cuflye_ctx* c, const uint32_t* in, uint64_t* out, uint64_t n,
                   const char* temp_name) {
-  uint64_t* temp = buf<uint64_t>(c, temp_name, scan_temp_words(n));
-  CUFLYE_CHECK(exclusive_scan_u32_to_u64(in, out, n, temp, c->stream));
-  // out[n] = total
-  const uint64_t ntiles = scan_temp_words(n) - 1;
-  CUFLYE_CHECK(cudaMemcpyAsync(out + n, temp + (n ? ntiles : 0), sizeof(uint64_t),
-                               cudaMemcpyDeviceToDevice, c->stream));
+  scan_u32_async(c, in, out, n, temp_name);
   return read_scalar(c, out + n);
 }
 
@@ -873,7 +865,7 @@ struct PassState {
   // run path: the pass's runs instead of hits; nhits counts those of its hits
   // that the hit path chains
   bool runs = false;
-  uint64_t run_hits = 0;
+  uint64_t run_hits = 0, longest = 0;  // hits in runs; runs of the longest query
   const uint32_t* cbits = nullptr;  // per 32 windows: the solid ones
   std::vector<uint64_t> base_off_h, win_off_h;  // nq + 1
   std::vector<int32_t> qdi_h;
@@ -890,8 +882,7 @@ const char* const kPerHitBuffers[] = {"h_keys",  "h_vals",   "h_kmers", "s_l",  
 // Buffers sized by the run count of a pass on the run path.
 const char* const kPerRunBuffers[] = {"n_keys", "n_vals", "n_akeys", "n_avals", "n_rlen", "n_pa",
                                       "n_pb",   "n_pl",   "n_ps",    "n_pk",    "n_po",   "n_pd",
-                                      "n_pm",   "n_pp",   "n_pe",    "m_tiles", "m_counts", "n_tcount",
-                                      "n_toffg"};
+                                      "n_pm",   "n_pp",   "n_pe",    "m_tiles", "m_counts"};
 
 // The pass's hits in Flye's generation order (and the filtered positions).
 void emit_generation_order(cuflye_ctx* c, PassState& ps) {
@@ -1154,24 +1145,24 @@ void run_runs(cuflye_ctx* c, PassState& ps) {
   uint32_t* tstart = buf<uint32_t>(c, "n_tstart", nt);
   uint64_t* tile_off = buf<uint64_t>(c, "n_toff", nt + 1);
   uint64_t* ftile_off = buf<uint64_t>(c, "n_ftoff", nt + 1);
-  unsigned long long* total = buf<unsigned long long>(c, "n_total", 64);
-  CUFLYE_CHECK(cudaMemsetAsync(total, 0, 64 * sizeof(unsigned long long), st));
+  // 64 partial sums of hits, the totals of runs_query_offsets
+  unsigned long long* total = buf<unsigned long long>(c, "n_total", 67);
+  CUFLYE_CHECK(cudaMemsetAsync(total, 0, 67 * sizeof(unsigned long long), st));
   CUFLYE_CHECK(runs_count(c->idx, ps.qb, recs, nstart, cbits, fbits, tfilt, tstart, total, st));
-  scan_u32_async(c, tstart, tile_off, nt, "n_scan");
-  scan_u32_async(c, tfilt, ftile_off, nt, "n_scan2");
+  CUFLYE_CHECK(exclusive_scan_pair(tstart, tile_off, tfilt, ftile_off, nt,
+                                   buf<uint64_t>(c, "n_scan", scan_temp_words(nt)), st));
   ps.q_off = buf<uint64_t>(c, "n_qoff", nq + 1);
   ps.f_off = buf<uint64_t>(c, "n_foff", nq + 1);
   CUFLYE_CHECK(runs_query_offsets(ps.qb, nstart, tile_off, fbits, ftile_off, ps.q_off, ps.f_off,
-                                  st));
+                                  total + 64, st));
   ReadBack rb{c};
-  const uint64_t* nr = rb.add(tile_off + nt);
-  const uint64_t* nf = rb.add(ftile_off + nt);
-  const unsigned long long* nh = rb.add(total, 64);
+  const unsigned long long* nh = rb.add(total, 67);
   rb.read_all();
   uint64_t hits = 0;
   for (int i = 0; i < 64; ++i) hits += nh[i];
-  ps.units = *nr;
-  ps.nfilt = *nf;
+  ps.longest = nh[64];
+  ps.units = nh[65];
+  ps.nfilt = nh[66];
   const uint64_t limit = effective_budget(c);
   const uint64_t used = c->in_use - reusable_bytes(c, true, false);
   const uint64_t free_b = limit > used ? limit - used : 0;
@@ -1843,41 +1834,50 @@ ChainRows chain_runs(cuflye_ctx* c, PassState& ps, const ChainParams& cp) {
   const uint32_t nq = ps.nq;
   uint64_t* sstats = buf<uint64_t>(c, "x_sortstats", kSortStats);
   mark(c, 0);
-  // 1. the runs in (ext id, cur pos) order: a stable radix sort by ext id of
-  // each query's runs (generated in cur-pos order).  Tiles of kMatchTile runs
-  // within a query: at most this many, the unused ones empty
-  uint32_t* ntiles = buf<uint32_t>(c, "m_ntiles", nq);
-  uint64_t* mtile_off = buf<uint64_t>(c, "m_tileoff", nq + 1);
-  const uint64_t NT = NR / kMatchTile + nq;
+  // 1. the runs in (ext id, cur pos) order.  Queries of up to kRunSortCap runs
+  // are sorted on chip; longer ones by radix passes over tiles of kMatchTile
+  // runs (at most NT tiles, the unused ones empty)
   int id_bits = 0;
   while (id_bits < 32 && ((2ull * c->idx.nslots - 1) >> id_bits) != 0) ++id_bits;
-  MatchTile* tiles = buf<MatchTile>(c, "m_tiles", NT);
-  uint32_t* mcounts = buf<uint32_t>(c, "m_counts", 256 * NT);
-  uint64_t* akeys = buf<uint64_t>(c, "n_akeys", NR);
-  uint32_t* avals = buf<uint32_t>(c, "n_avals", NR);
-  CUFLYE_CHECK(cudaMemsetAsync(tiles, 0, NT * sizeof(MatchTile), st));
-  CUFLYE_CHECK(match_plan(ps.q_off, nullptr, nq, ntiles, nullptr, nullptr, nullptr, st, true));
-  scan_u32_async(c, ntiles, mtile_off, nq, "m_scan");
-  CUFLYE_CHECK(match_tiles(ps.q_off, ntiles, mtile_off, nq, tiles, st));
-  CUFLYE_CHECK(match_radix(ps.keys, ps.vals, akeys, avals, tiles, static_cast<uint32_t>(NT),
-                           ps.q_off, ntiles, mtile_off, nq, id_bits, mcounts, c->num_sms,
-                           c->shape.scatter_blocks_per_sm, st));
+  if (ps.longest > kRunSortCap) {
+    uint32_t* ntiles = buf<uint32_t>(c, "m_ntiles", nq);
+    uint64_t* mtile_off = buf<uint64_t>(c, "m_tileoff", nq + 1);
+    const uint64_t NT = NR / kMatchTile + std::min<uint64_t>(nq, NR / kRunSortCap) + 1;
+    MatchTile* tiles = buf<MatchTile>(c, "m_tiles", NT);
+    uint32_t* mcounts = buf<uint32_t>(c, "m_counts", 256 * NT);
+    uint64_t* akeys = buf<uint64_t>(c, "n_akeys", NR);
+    uint32_t* avals = buf<uint32_t>(c, "n_avals", NR);
+    CUFLYE_CHECK(cudaMemsetAsync(tiles, 0, NT * sizeof(MatchTile), st));
+    CUFLYE_CHECK(match_plan(ps.q_off, nullptr, nq, ntiles, nullptr, nullptr, nullptr, st, true,
+                            kRunSortCap));
+    scan_u32_async(c, ntiles, mtile_off, nq, "m_scan");
+    CUFLYE_CHECK(match_tiles(ps.q_off, ntiles, mtile_off, nq, tiles, st));
+    CUFLYE_CHECK(match_radix(ps.keys, ps.vals, akeys, avals, tiles, static_cast<uint32_t>(NT),
+                             ps.q_off, ntiles, mtile_off, nq, id_bits, mcounts, c->num_sms,
+                             c->shape.scatter_blocks_per_sm, st));
+  }
+  // counters, the spare slots' cursor, the sort's work counter: zeroed at once
+  uint32_t* words = buf<uint32_t>(c, "n_words", kRcWords + 4);
+  static_assert(kRcWords % 2 == 0, "the cursor after the counters is 8-byte aligned");
+  CUFLYE_CHECK(cudaMemsetAsync(words, 0, (kRcWords + 4) * 4, st));
+  uint32_t* q_groups = buf<uint32_t>(c, "n_qgroups", nq);
+  CUFLYE_CHECK(runs_sort(ps.q_off, nq, ps.keys, ps.vals, id_bits, q_groups, words + kRcWords + 2,
+                         c->num_sms, st));
   mark(c, 1);
   // 2. groups.  Small passes size everything by their runs (a group has at
   // least one) and read nothing back before the rows; large ones read the
   // number of groups, then of survivors
-  const uint64_t gtiles = (NR + kGroupTile - 1) / kGroupTile;
-  uint32_t* gtcount = buf<uint32_t>(c, "n_tcount", gtiles);
-  uint64_t* gtoff = buf<uint64_t>(c, "n_toffg", gtiles + 1);
-  CUFLYE_CHECK(groups_count(ps.keys, ps.q_off, nq, NR, gtcount, st));
-  scan_u32_async(c, gtcount, gtoff, gtiles, "n_scan");
+  uint64_t* qg = buf<uint64_t>(c, "n_qg", nq + 1);  // first group of each query
+  scan_u32_async(c, q_groups, qg, nq, "n_scan");
   constexpr uint64_t kSmallPass = 1u << 15;
   const bool small = NR <= kSmallPass;
   RunTables t;
-  t.max_groups = small ? NR : read_scalar(c, gtoff + gtiles);
+  t.max_groups = small ? NR : read_scalar(c, qg + nq);
   const uint64_t G = t.max_groups;
   GroupInfo* bounds = buf<GroupInfo>(c, "n_bounds", G);
-  CUFLYE_CHECK(groups_write(ps.keys, ps.q_off, nq, NR, gtoff, bounds, st));
+  CUFLYE_CHECK(runs_bounds(ps.q_off, nq, ps.keys, qg, bounds, c->num_sms, st));
+  t.counts = words;
+  t.spare_cursor = reinterpret_cast<unsigned long long*>(words + kRcWords);
   t.idx = c->idx;
   t.qb = ps.qb;
   t.qinfo = ps.qinfo;
@@ -1886,7 +1886,7 @@ ChainRows chain_runs(cuflye_ctx* c, PassState& ps, const ChainParams& cp) {
   t.vals = ps.vals;
   t.nruns = NR;
   t.bounds = bounds;
-  t.ngroups = gtoff + gtiles;
+  t.ngroups = qg + nq;
   t.rlen = buf<uint32_t>(c, "n_rlen", NR);
   t.groups = buf<RunGroup>(c, "n_groups", G);
   t.spare0 = NR + G;
@@ -1906,12 +1906,6 @@ ChainRows chain_runs(cuflye_ctx* c, PassState& ps, const ChainParams& cp) {
   t.sort_lists = buf<uint32_t>(c, "n_slists", 2 * G);
   t.open_list = buf<uint32_t>(c, "n_open", G);
   uint32_t* group_rows = buf<uint32_t>(c, "n_grows", G);
-  // counters and the spare slots' cursor: zeroed at once
-  uint32_t* words = buf<uint32_t>(c, "n_words", kRcWords + 2);
-  static_assert(kRcWords % 2 == 0, "the cursor after the counters is 8-byte aligned");
-  t.counts = words;
-  t.spare_cursor = reinterpret_cast<unsigned long long*>(words + kRcWords);
-  CUFLYE_CHECK(cudaMemsetAsync(words, 0, (kRcWords + 2) * 4, st));
   CUFLYE_CHECK(cudaMemsetAsync(group_rows, 0, std::max<uint64_t>(G, 1) * 4, st));
   CUFLYE_CHECK(runs_groups(t, cp, c->num_sms, st));
   CUFLYE_CHECK(runs_order(t, c->num_sms, st));
@@ -1935,10 +1929,8 @@ ChainRows chain_runs(cuflye_ctx* c, PassState& ps, const ChainParams& cp) {
   CUFLYE_CHECK(chain_open_rows(pool, pool_cap, t.counts + kRcPool, c->logt, cp, group_rows,
                                c->num_sms, st));
   // 4. max_overlaps + compaction in group order
-  uint64_t* qg = buf<uint64_t>(c, "n_qg", nq + 1);
   uint64_t* kept_off = buf<uint64_t>(c, "n_keptoff", G + 1);
   uint32_t* kept = group_rows;
-  CUFLYE_CHECK(runs_query_groups(t, qg, st));
   auto compact = [&]() {
     if (cp.max_overlaps > 0) {
       kept = buf<uint32_t>(c, "n_kept", G);

@@ -14,12 +14,14 @@ void count_launch();
 unsigned long long launches_total();
 
 // ---------------------------------------------------------------- scan
-// Exclusive prefix sums (out may alias in).  temp needs scan_temp_words(n) words.
+// Exclusive prefix sums: out[i] for i in [0, n], out[n] the total.  temp needs
+// scan_temp_words(n) words.
 size_t scan_temp_words(uint64_t n);
 cudaError_t exclusive_scan_u32_to_u64(const uint32_t* in, uint64_t* out, uint64_t n,
                                       uint64_t* temp, cudaStream_t s);
-cudaError_t exclusive_scan_u64(const uint64_t* in, uint64_t* out, uint64_t n, uint64_t* temp,
-                               cudaStream_t s);
+// Two scans of the same length.
+cudaError_t exclusive_scan_pair(const uint32_t* in0, uint64_t* out0, const uint32_t* in1,
+                                uint64_t* out1, uint64_t n, uint64_t* temp, cudaStream_t s);
 
 // ---------------------------------------------------------------- sort
 size_t segsort_smem_bytes();
@@ -249,10 +251,11 @@ struct MatchTile {
 // Per query with two or more hits: flagged queries (q_tie, keys may repeat)
 // are listed for the emulated sort; the others get ntiles[q] radix tiles.
 // tile_flagged: the flagged queries (q_tie null: all of them) get the tiles
-// (their sorted order up to the order among equal keys) and nothing is listed.
+// with more than `over` hits (their sorted order up to the order among equal
+// keys) and nothing is listed.
 cudaError_t match_plan(const uint64_t* q_off, const uint32_t* q_tie, uint32_t nq, uint32_t* ntiles,
                        uint64_t* emu_begin, uint64_t* emu_end, uint32_t* emu_count,
-                       cudaStream_t s, bool tile_flagged = false);
+                       cudaStream_t s, bool tile_flagged = false, uint32_t over = 1);
 // tile_off: exclusive scan of ntiles.
 cudaError_t match_tiles(const uint64_t* q_off, const uint32_t* ntiles, const uint64_t* tile_off,
                         uint32_t nq, MatchTile* tiles, cudaStream_t s);

@@ -155,7 +155,7 @@ uint64_t radix_tiles(uint64_t n) { return (n + kRadixTile - 1) / kRadixTile; }
 // The scratch: 256 counts a tile, their offsets (8 bytes each), the scan's.
 size_t radix_hist_words(uint64_t n) {
   const uint64_t c = 256 * radix_tiles(n);
-  return 3 * c + 2 * scan_temp_words(c) + 2;
+  return 3 * c + 2 * scan_temp_words(c) + 4;
 }
 
 cudaError_t radix_sort_pairs(uint64_t* keys, uint64_t* vals, uint64_t* keys_alt,
@@ -166,7 +166,7 @@ cudaError_t radix_sort_pairs(uint64_t* keys, uint64_t* vals, uint64_t* keys_alt,
   const uint32_t ntiles = static_cast<uint32_t>(nt);
   const uint64_t c = 256 * nt;  // even: the offsets are 8-byte aligned
   uint64_t* offs = reinterpret_cast<uint64_t*>(hist + c);
-  uint64_t* temp = offs + c;
+  uint64_t* temp = offs + c + 1;
   cudaError_t e = cudaFuncSetAttribute(radix_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(sizeof(RadixSmem)));
   if (e != cudaSuccess) return e;

@@ -262,22 +262,38 @@ __global__ void __launch_bounds__(kProbeBlock, 6) probe_kernel(
   }
 }
 
+// First run and first filtered position of each query; in totals the most runs
+// of a query, and all runs and filtered positions.
 __global__ void query_offsets_kernel(QueryBatch q, const uint32_t* __restrict__ nstart,
                                      const uint64_t* __restrict__ tile_off,
                                      const uint32_t* __restrict__ fbits,
                                      const uint64_t* __restrict__ ftile_off,
-                                     uint64_t* __restrict__ q_off, uint64_t* __restrict__ f_off) {
+                                     uint64_t* __restrict__ q_off, uint64_t* __restrict__ f_off,
+                                     unsigned long long* __restrict__ totals) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i > q.nq) return;
-  const uint64_t w = q.win_off[i], t = w >> 5;
-  const uint32_t r = static_cast<uint32_t>(w & 31);
-  uint64_t o = tile_off[t], f = ftile_off[t];
-  if (r) {  // inside a tile
-    for (uint32_t j = 0; j < r; ++j) o += nstart[t * 32 + j];
-    f += __popc(fbits[t] & ((1u << r) - 1u));
+  auto first_run = [&](uint64_t w) {
+    uint64_t o = tile_off[w >> 5];
+    for (uint64_t j = w & ~31ull; j < w; ++j) o += nstart[j];  // inside a tile
+    return o;
+  };
+  uint64_t o = 0;
+  if (i <= q.nq) {
+    const uint64_t w = q.win_off[i], t = w >> 5;
+    const uint32_t r = static_cast<uint32_t>(w & 31);
+    o = first_run(w);
+    q_off[i] = o;
+    const uint64_t f = ftile_off[t] + (r ? __popc(fbits[t] & ((1u << r) - 1u)) : 0);
+    f_off[i] = f;
+    if (i == q.nq) {
+      totals[1] = o;
+      totals[2] = f;
+    }
   }
-  q_off[i] = o;
-  f_off[i] = f;
+  uint64_t next = __shfl_down_sync(0xffffffffu, o, 1);
+  if ((threadIdx.x & 31) == 31 && i < q.nq) next = first_run(q.win_off[i + 1]);
+  uint32_t n = i < q.nq ? static_cast<uint32_t>(next - o) : 0u;
+  n = __reduce_max_sync(0xffffffffu, n);
+  if ((threadIdx.x & 31) == 0 && n) atomicMax(totals, static_cast<unsigned long long>(n));
 }
 
 // A warp writes its 32 windows' run starts.  The entries of the windows that
@@ -342,6 +358,191 @@ __global__ void __launch_bounds__(256) start_emit_kernel(
       vals[d] = static_cast<uint32_t>(pos);
     }
     out += __popc(m);
+  }
+}
+
+// ---------------------------------------------------------------- sort, groups
+
+constexpr int kSortBlock = 512;
+constexpr int kSortWarps = kSortBlock / 32;
+constexpr int kSortItems = static_cast<int>(kRunSortCap / kSortBlock);
+
+struct SortSmem {
+  uint64_t key[kRunSortCap];
+  uint32_t val[kRunSortCap];
+  uint32_t wc[kSortWarps][256];  // per-warp digit counts, then offsets
+  uint32_t dbase[256];
+  uint32_t ws[8];
+  uint32_t item;
+};
+
+// A block a query: its runs (in cur-pos order) into (ext id, cur pos) order by a
+// stable LSD radix sort of the ext ids, 8 bits a pass, and the number of its
+// groups.  The runs stay on chip from load to store, where passes over device
+// memory (match_radix, which longer queries take beforehand) move them twice a
+// digit and launch three kernels for it.
+__global__ void __launch_bounds__(kSortBlock, 2)
+    sort_queries_kernel(const uint64_t* __restrict__ q_off, uint32_t nq,
+                        uint64_t* __restrict__ keys, uint32_t* __restrict__ vals, int id_bits,
+                        uint32_t* __restrict__ q_groups, uint32_t* __restrict__ work) {
+  extern __shared__ __align__(16) unsigned char sort_raw[];
+  SortSmem& sm = *reinterpret_cast<SortSmem*>(sort_raw);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t lt = (1u << lane) - 1u;
+  for (;;) {
+    if (threadIdx.x == 0) sm.item = atomicAdd(work, 1u);
+    __syncthreads();
+    const uint32_t q = sm.item;
+    if (q >= nq) break;
+    const uint64_t b = q_off[q];
+    const uint64_t len = q_off[q + 1] - b;
+    const bool whole = len <= kRunSortCap;
+    const uint32_t n = whole ? static_cast<uint32_t>(len) : 0u;
+    // warp w owns per_warp consecutive runs
+    const uint32_t per_warp = ((n + kSortBlock - 1) / kSortBlock) * 32;
+    const int rounds = static_cast<int>(per_warp / 32);
+    const uint32_t j0 = warp * per_warp + lane;
+    uint64_t k[kSortItems];
+    uint32_t v[kSortItems], rk[kSortItems];
+#pragma unroll
+    for (int r = 0; r < kSortItems; ++r) {
+      const uint32_t j = j0 + r * 32;
+      const bool in = r < rounds && j < n;
+      k[r] = in ? keys[b + j] : 0;
+      v[r] = in ? vals[b + j] : 0;
+    }
+    for (int shift = 32; n > 1 && shift < 32 + id_bits; shift += 8) {
+      for (int i = threadIdx.x; i < kSortWarps * 256; i += kSortBlock) (&sm.wc[0][0])[i] = 0;
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < kSortItems; ++r) {
+        if (r >= rounds) break;
+        const bool in = j0 + r * 32 < n;
+        const uint32_t d = in ? static_cast<uint32_t>(k[r] >> shift) & 0xffu : 256u;
+        const uint32_t peers = __match_any_sync(0xffffffffu, d);
+        const int leader = __ffs(peers) - 1;
+        uint32_t base = 0;
+        if (in && lane == leader) {
+          base = sm.wc[warp][d];
+          sm.wc[warp][d] = base + __popc(peers);
+        }
+        base = __shfl_sync(0xffffffffu, base, leader);
+        rk[r] = base + __popc(peers & lt);
+        __syncwarp();
+      }
+      __syncthreads();
+      uint32_t tot = 0, inc = 0;
+      if (threadIdx.x < 256) {
+#pragma unroll
+        for (int w = 0; w < kSortWarps; ++w) {
+          const uint32_t c = sm.wc[w][threadIdx.x];
+          sm.wc[w][threadIdx.x] = tot;
+          tot += c;
+        }
+        inc = tot;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+          if (lane >= o) inc += u;
+        }
+        if (lane == 31) sm.ws[warp] = inc;
+      }
+      __syncthreads();
+      if (threadIdx.x < 256) {
+        uint32_t before = 0;
+        for (int w = 0; w < warp; ++w) before += sm.ws[w];
+        sm.dbase[threadIdx.x] = before + inc - tot;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < kSortItems; ++r) {
+        if (r < rounds && j0 + r * 32 < n) {
+          const uint32_t d = static_cast<uint32_t>(k[r] >> shift) & 0xffu;
+          const uint32_t o = sm.dbase[d] + sm.wc[warp][d] + rk[r];
+          sm.key[o] = k[r];
+          sm.val[o] = v[r];
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < kSortItems; ++r) {
+        const uint32_t j = j0 + r * 32;
+        if (r < rounds && j < n) {
+          k[r] = sm.key[j];
+          v[r] = sm.val[j];
+        }
+      }
+    }
+    // in order now (in shared memory, a query of one run in k[0]; longer
+    // queries in device memory): write, count the groups
+    uint32_t heads = 0;
+    if (whole) {
+#pragma unroll
+      for (int r = 0; r < kSortItems; ++r) {
+        const uint32_t j = j0 + r * 32;
+        if (r < rounds && j < n) {
+          if (n > 1) {
+            keys[b + j] = k[r];
+            vals[b + j] = v[r];
+          }
+          heads += j == 0 || (k[r] >> 32) != (sm.key[j - 1] >> 32);
+        }
+      }
+    } else {
+      for (uint64_t j = threadIdx.x; j < len; j += kSortBlock)
+        heads += j == 0 || (keys[b + j] >> 32) != (keys[b + j - 1] >> 32);
+    }
+    heads = __reduce_add_sync(0xffffffffu, heads);
+    __syncthreads();  // sm.key and sm.item are read
+    if (lane == 0) sm.wc[0][warp] = heads;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      uint32_t g = 0;
+      for (int w = 0; w < kSortWarps; ++w) g += sm.wc[0][w];
+      q_groups[q] = g;
+    }
+    __syncthreads();
+  }
+}
+
+// The groups of each query: runs of one ext id among its sorted runs.
+__global__ void __launch_bounds__(256) bounds_kernel(const uint64_t* __restrict__ q_off,
+                                                     uint32_t nq,
+                                                     const uint64_t* __restrict__ keys,
+                                                     const uint64_t* __restrict__ q_group,
+                                                     GroupInfo* __restrict__ bounds) {
+  __shared__ uint32_t wsum[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (uint32_t q = blockIdx.x; q < nq; q += gridDim.x) {
+    const uint64_t b = q_off[q], n = q_off[q + 1] - b;
+    uint64_t g = q_group[q];
+    for (uint64_t t0 = 0; t0 < n; t0 += 256) {
+      const uint64_t j = t0 + threadIdx.x;
+      uint32_t id = 0;
+      bool head = false;
+      if (j < n) {
+        id = static_cast<uint32_t>(keys[b + j] >> 32);
+        head = j == 0 || id != static_cast<uint32_t>(keys[b + j - 1] >> 32);
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, head);
+      if (lane == 0) wsum[warp] = __popc(m);
+      __syncthreads();
+      uint32_t before = 0, all = 0;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) {
+        before += w < warp ? wsum[w] : 0u;
+        all += wsum[w];
+      }
+      if (head) {
+        GroupInfo gi{};
+        gi.start = b + j;
+        gi.query = q;
+        gi.ext_di = id;
+        bounds[g + before + __popc(m & ((1u << lane) - 1u))] = gi;
+      }
+      g += all;
+      __syncthreads();
+    }
   }
 }
 
@@ -705,22 +906,6 @@ __global__ void scatter_rows_kernel(const OverlapRow* __restrict__ pool,
   }
 }
 
-__global__ void query_groups_kernel(const GroupInfo* __restrict__ bounds,
-                                    const uint64_t* __restrict__ ngroups, uint32_t nq,
-                                    uint64_t* __restrict__ qg) {
-  const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q > nq) return;
-  uint64_t lo = 0, hi = *ngroups;
-  while (lo < hi) {
-    const uint64_t mid = (lo + hi) >> 1;
-    if (bounds[mid].query < q)
-      lo = mid + 1;
-    else
-      hi = mid;
-  }
-  qg[q] = lo;
-}
-
 }  // namespace
 
 cudaError_t index_neighbours(const uint64_t* pos, uint64_t npos, const uint64_t* words,
@@ -745,10 +930,10 @@ cudaError_t runs_count(const DeviceIndex& idx, const QueryBatch& q, uint4* recs,
 cudaError_t runs_query_offsets(const QueryBatch& q, const uint32_t* nstart,
                                const uint64_t* tile_off, const uint32_t* fbits,
                                const uint64_t* ftile_off, uint64_t* q_off, uint64_t* f_off,
-                               cudaStream_t s) {
+                               unsigned long long* totals, cudaStream_t s) {
   count_launch();
   query_offsets_kernel<<<grid(q.nq + 1ull, 128), 128, 0, s>>>(q, nstart, tile_off, fbits,
-                                                              ftile_off, q_off, f_off);
+                                                              ftile_off, q_off, f_off, totals);
   return cudaGetLastError();
 }
 
@@ -760,6 +945,29 @@ cudaError_t runs_emit(const DeviceIndex& idx, const QueryBatch& q, const uint4* 
   count_launch();
   start_emit_kernel<<<grid(q.nwin, 256), 256, 0, s>>>(idx, q, recs, nstart, tile_off, fbits,
                                                       ftile_off, keys, vals, fpos);
+  return cudaGetLastError();
+}
+
+cudaError_t runs_sort(const uint64_t* q_off, uint32_t nq, uint64_t* keys, uint32_t* vals,
+                      int id_bits, uint32_t* q_groups, uint32_t* work, int num_sms,
+                      cudaStream_t s) {
+  if (nq == 0) return cudaSuccess;
+  const cudaError_t e =
+      cudaFuncSetAttribute(sort_queries_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           static_cast<int>(sizeof(SortSmem)));
+  if (e != cudaSuccess) return e;
+  count_launch();
+  sort_queries_kernel<<<static_cast<unsigned>(std::min<uint64_t>(nq, 2ull * num_sms)), kSortBlock,
+                        sizeof(SortSmem), s>>>(q_off, nq, keys, vals, id_bits, q_groups, work);
+  return cudaGetLastError();
+}
+
+cudaError_t runs_bounds(const uint64_t* q_off, uint32_t nq, const uint64_t* keys,
+                        const uint64_t* q_group, GroupInfo* bounds, int num_sms, cudaStream_t s) {
+  if (nq == 0) return cudaSuccess;
+  count_launch();
+  bounds_kernel<<<static_cast<unsigned>(std::min<uint64_t>(nq, 8ull * num_sms)), 256, 0, s>>>(
+      q_off, nq, keys, q_group, bounds);
   return cudaGetLastError();
 }
 
@@ -831,12 +1039,6 @@ cudaError_t runs_scatter_rows(const OverlapRow* pool, const uint32_t* npool, uin
   count_launch();
   scatter_rows_kernel<<<std::min(grid(max_pool, 256), 2048u), 256, 0, s>>>(pool, npool, kept,
                                                                           kept_off, rows);
-  return cudaGetLastError();
-}
-
-cudaError_t runs_query_groups(const RunTables& t, uint64_t* qg, cudaStream_t s) {
-  count_launch();
-  query_groups_kernel<<<grid(t.qb.nq + 1ull, 128), 128, 0, s>>>(t.bounds, t.ngroups, t.qb.nq, qg);
   return cudaGetLastError();
 }
 

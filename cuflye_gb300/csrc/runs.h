@@ -97,17 +97,29 @@ cudaError_t index_neighbours(const uint64_t* pos, uint64_t npos, const uint64_t*
 cudaError_t runs_count(const DeviceIndex& idx, const QueryBatch& q, uint4* recs, uint32_t* nstart,
                        uint32_t* cbits, uint32_t* fbits, uint32_t* tile_filt,
                        uint32_t* tile_start, unsigned long long* hit_total, cudaStream_t s);
-// Each query's first run and first filtered position (nq + 1 entries each).
+// Each query's first run and first filtered position (nq + 1 entries each);
+// totals[0] (zeroed by the caller): the most runs of a query, [1] and [2]: all
+// runs and filtered positions.
 cudaError_t runs_query_offsets(const QueryBatch& q, const uint32_t* nstart,
                                const uint64_t* tile_off, const uint32_t* fbits,
                                const uint64_t* ftile_off, uint64_t* q_off, uint64_t* f_off,
-                               cudaStream_t s);
+                               unsigned long long* totals, cudaStream_t s);
 // The run starts in window order, then bucket order, and the filtered positions.
 cudaError_t runs_emit(const DeviceIndex& idx, const QueryBatch& q, const uint4* recs,
                       const uint32_t* nstart, const uint64_t* tile_off, const uint32_t* fbits,
                       const uint64_t* ftile_off, uint64_t* keys, uint32_t* vals, int32_t* fpos,
                       cudaStream_t s);
 
+// The runs of every query of up to kRunSortCap runs sorted by ext id, in place
+// and stable (longer ones come sorted, by match_radix), and the groups of each
+// query.  *work zeroed by the caller.
+constexpr uint32_t kRunSortCap = 4096;
+cudaError_t runs_sort(const uint64_t* q_off, uint32_t nq, uint64_t* keys, uint32_t* vals,
+                      int id_bits, uint32_t* q_groups, uint32_t* work, int num_sms,
+                      cudaStream_t s);
+// Start, query and ext id of each group; q_group: the scan of q_groups.
+cudaError_t runs_bounds(const uint64_t* q_off, uint32_t nq, const uint64_t* keys,
+                        const uint64_t* q_group, GroupInfo* bounds, int num_sms, cudaStream_t s);
 // Run lengths, group prefilter, and the pieces of groups whose runs are in
 // order already; the other survivors are listed for runs_order.
 cudaError_t runs_groups(const RunTables& t, const ChainParams& p, int num_sms, cudaStream_t s);
@@ -155,7 +167,5 @@ cudaError_t runs_fold_rows(const uint32_t* list, uint32_t n, const uint32_t* row
 cudaError_t runs_scatter_rows(const OverlapRow* pool, const uint32_t* npool, uint64_t max_pool,
                               const uint32_t* kept, const uint64_t* kept_off, OverlapRow* rows,
                               cudaStream_t s);
-// First group of each query (nq + 1), by a search of the group bounds.
-cudaError_t runs_query_groups(const RunTables& t, uint64_t* qg, cudaStream_t s);
 
 }  // namespace cuflye

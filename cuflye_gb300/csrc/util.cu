@@ -73,6 +73,57 @@ __global__ void scan_sums(uint64_t* sums, uint64_t ntiles) {
   if (threadIdx.x == 0) sums[ntiles] = carry;
 }
 
+// Short arrays: one block a scan (the second's for a pair of them), so that a
+// small call pays one launch, not three.
+constexpr int kSmallBlock = 1024;
+constexpr uint64_t kSmallScan = 32768;
+
+__global__ void __launch_bounds__(kSmallBlock) scan_small(const uint32_t* __restrict__ in0,
+                                                          uint64_t* __restrict__ out0,
+                                                          const uint32_t* __restrict__ in1,
+                                                          uint64_t* __restrict__ out1,
+                                                          uint32_t n) {
+  __shared__ uint64_t ws[kSmallBlock / 32];
+  const uint32_t* __restrict__ in = blockIdx.x ? in1 : in0;
+  uint64_t* __restrict__ out = blockIdx.x ? out1 : out0;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint64_t carry = 0;
+  for (uint32_t t0 = 0; t0 < n; t0 += kSmallBlock * 4) {
+    const uint32_t a = t0 + threadIdx.x * 4;
+    uint32_t v[4];
+    uint64_t s = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      v[j] = a + j < n ? in[a + j] : 0u;
+      s += v[j];
+    }
+    uint64_t inc = s;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint64_t o = __shfl_up_sync(0xffffffffu, inc, d);
+      if (lane >= d) inc += o;
+    }
+    if (lane == 31) ws[warp] = inc;
+    __syncthreads();
+    uint64_t before = carry, all = 0;
+#pragma unroll
+    for (int w = 0; w < kSmallBlock / 32; ++w) {
+      const uint64_t x = ws[w];
+      before += w < warp ? x : 0;
+      all += x;
+    }
+    uint64_t run = before + inc - s;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (a + j < n) out[a + j] = run;
+      run += v[j];
+    }
+    carry += all;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) out[n] = carry;
+}
+
 template <typename In>
 __global__ void scan_downsweep(const In* __restrict__ in, uint64_t* __restrict__ out, uint64_t n,
                                const uint64_t* __restrict__ sums) {
@@ -110,6 +161,7 @@ __global__ void scan_downsweep(const In* __restrict__ in, uint64_t* __restrict__
     if (i < n) out[i] = run;
     run += v[j];
   }
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[n] = sums[gridDim.x];
 }
 
 __global__ void pack_kernel(const uint8_t* __restrict__ ascii, uint64_t nbases,
@@ -144,31 +196,33 @@ __global__ void pack_kernel(const uint8_t* __restrict__ ascii, uint64_t nbases,
 
 size_t scan_temp_words(uint64_t n) { return (n + kScanTile - 1) / kScanTile + 1; }
 
-template <typename In>
-static cudaError_t run_scan(const In* in, uint64_t* out, uint64_t n, uint64_t* temp,
-                            cudaStream_t s) {
-  if (n == 0) {
-    cudaMemsetAsync(temp, 0, sizeof(uint64_t), s);
+cudaError_t exclusive_scan_u32_to_u64(const uint32_t* in, uint64_t* out, uint64_t n,
+                                      uint64_t* temp, cudaStream_t s) {
+  if (n == 0) return cudaMemsetAsync(out, 0, sizeof(uint64_t), s);
+  if (n <= kSmallScan) {
+    count_launch();
+    scan_small<<<1, kSmallBlock, 0, s>>>(in, out, in, out, static_cast<uint32_t>(n));
     return cudaGetLastError();
   }
   const uint64_t ntiles = (n + kScanTile - 1) / kScanTile;
   count_launch();
-  scan_tile_sums<In><<<static_cast<unsigned>(ntiles), kScanBlock, 0, s>>>(in, n, temp);
+  scan_tile_sums<uint32_t><<<static_cast<unsigned>(ntiles), kScanBlock, 0, s>>>(in, n, temp);
   count_launch();
   scan_sums<<<1, 1024, 0, s>>>(temp, ntiles);
   count_launch();
-  scan_downsweep<In><<<static_cast<unsigned>(ntiles), kScanBlock, 0, s>>>(in, out, n, temp);
+  scan_downsweep<uint32_t><<<static_cast<unsigned>(ntiles), kScanBlock, 0, s>>>(in, out, n, temp);
   return cudaGetLastError();
 }
 
-cudaError_t exclusive_scan_u32_to_u64(const uint32_t* in, uint64_t* out, uint64_t n,
-                                      uint64_t* temp, cudaStream_t s) {
-  return run_scan<uint32_t>(in, out, n, temp, s);
-}
-
-cudaError_t exclusive_scan_u64(const uint64_t* in, uint64_t* out, uint64_t n, uint64_t* temp,
-                               cudaStream_t s) {
-  return run_scan<uint64_t>(in, out, n, temp, s);
+cudaError_t exclusive_scan_pair(const uint32_t* in0, uint64_t* out0, const uint32_t* in1,
+                                uint64_t* out1, uint64_t n, uint64_t* temp, cudaStream_t s) {
+  if (n == 0 || n > kSmallScan) {
+    const cudaError_t e = exclusive_scan_u32_to_u64(in0, out0, n, temp, s);
+    return e != cudaSuccess ? e : exclusive_scan_u32_to_u64(in1, out1, n, temp, s);
+  }
+  count_launch();
+  scan_small<<<2, kSmallBlock, 0, s>>>(in0, out0, in1, out1, static_cast<uint32_t>(n));
+  return cudaGetLastError();
 }
 
 cudaError_t pack_bases(const uint8_t* ascii, uint64_t nbases, uint64_t* words, cudaStream_t s) {

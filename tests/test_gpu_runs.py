@@ -109,3 +109,37 @@ def test_run_path_is_taken(gpu):
             gpu.set_sorted_emission(1)
         hits = gpu.last_timing()[1][1]
         assert (runs * 4 < hits) == fewer
+
+
+def test_queries_around_the_sort_capacity(gpu, oracle_mod):
+    """Queries of a few runs up to more than a block sorts on chip (4096)."""
+    from cuflye_gb300 import synth
+    from cuflye_gb300.backend import OverlapParams
+    rng = np.random.default_rng(4096)
+    genome = synth.random_genome(rng, 2000)
+    seqs = [synth.mutate(rng, genome[:n], 0.04, 0.01, 0.01)
+            for n in np.linspace(60, 2000, 160).astype(int)]
+    reads = synth.ReadSet.from_strings(np.arange(1, len(seqs) + 1), [x.tobytes() for x in seqs])
+    params = dict(synth.OVERLAP_PARAMS, min_overlap=200)
+    assert _check(gpu, oracle_mod, reads, reads, 11, 1, 1000, params, VARIANTS[:2]) > 0
+    runs = []
+    for i in (0, reads.n - 1):
+        one = synth.ReadSet.from_strings(np.array([i + 1]), [reads.seq(i)])
+        gpu.overlaps(one, OverlapParams.make(**dict(params, kmer_size=11)))
+        runs.append(gpu.last_timing()[1][1] // 8)
+    assert runs[0] < 4096 < runs[1]
+
+
+@pytest.mark.parametrize("nq", [1, 8191, 8193, 32767, 32768, 32769])
+def test_query_counts_around_the_scans(gpu, oracle_mod, nq):
+    """Scans of one block (up to 32768 entries) and of three kernels."""
+    from cuflye_gb300 import synth
+    rng = np.random.default_rng(nq)
+    genome = synth.random_genome(rng, 30_000)
+    at = rng.integers(0, len(genome) - 60, size=nq)
+    reads = synth.ReadSet.from_strings(
+        np.arange(100, 100 + nq), [genome[s:s + 60].tobytes() for s in at])
+    targets = synth.ReadSet.from_strings(
+        np.arange(1, 31), [genome[i:i + 1000].tobytes() for i in range(0, 30_000, 1000)])
+    params = dict(synth.OVERLAP_PARAMS, min_overlap=40)
+    assert _check(gpu, oracle_mod, targets, reads, 15, 1, 100, params, VARIANTS[1:2]) > 0
