@@ -325,15 +325,16 @@ struct BuiltIndex {
   uint64_t cap = 0;
   uint64_t* pos = nullptr;
   uint64_t npos = 0, nsolid = 0, nrep = 0;
-  uint32_t* self_at = nullptr;  // one-range builds, when memory allows
+  // one-range builds, when memory allows
+  uint4* windows = nullptr;
   uint64_t* win_off = nullptr;
+  uint8_t* nbr = nullptr;
 };
 
 // Scratch of one key range's build.
 const char* const kBuildScratch[] = {"ib_keys", "ib_vals",  "ib_keys2",    "ib_vals2",
-                                     "ib_hist", "ib_flags", "ib_runid",    "ib_runstart",
-                                     "ib_kept", "ib_cls",   "ib_keptoff",  "ib_scan",
-                                     "ib_count"};
+                                     "ib_hist", "ib_flags", "ib_kept",     "ib_cls",
+                                     "ib_keptoff", "ib_scan", "ib_count"};
 
 void release_build_scratch(cuflye_ctx* c) {
   for (const char* t : kBuildScratch) release(c, t);
@@ -347,18 +348,22 @@ struct KeyRuns {
   uint64_t* run_start;
   uint8_t* cls;
   uint64_t* kept_off;
+  uint32_t* free_words;      // nw words that nothing needs any more
+  uint32_t* free_run_words;  // nruns words
   uint64_t nw, nruns, npos, nsolid, nrep;
 };
 
-// Sorts the windows in ib_keys / ib_vals (the alternates ib_keys2 / ib_vals2
-// already sized), finds their runs and classifies them (solid, repetitive).
+// Sorts the windows in ib_keys / ib_vals (with the alternates ib_keys2 / ib_vals2
+// already sized, nw + 1 words each), finds their runs and classifies them
+// (solid, repetitive).  The run tables take the two arrays that the sort ends
+// without.
 KeyRuns sort_and_classify(cuflye_ctx* c, uint64_t nw, const std::vector<int>& digits,
                           uint32_t min_freq, uint32_t max_freq) {
   cudaStream_t st = c->stream;
-  uint64_t* keys = buf<uint64_t>(c, "ib_keys", nw);
-  uint64_t* vals = buf<uint64_t>(c, "ib_vals", nw);
-  uint64_t* keys2 = buf<uint64_t>(c, "ib_keys2", nw);
-  uint64_t* vals2 = buf<uint64_t>(c, "ib_vals2", nw);
+  uint64_t* keys = buf<uint64_t>(c, "ib_keys", nw + 1);
+  uint64_t* vals = buf<uint64_t>(c, "ib_vals", nw + 1);
+  uint64_t* keys2 = buf<uint64_t>(c, "ib_keys2", nw + 1);
+  uint64_t* vals2 = buf<uint64_t>(c, "ib_vals2", nw + 1);
   uint32_t* hist = buf<uint32_t>(c, "ib_hist", radix_hist_words(nw));
   int in_alt = 0;
   if (nw)
@@ -369,10 +374,10 @@ KeyRuns sort_and_classify(cuflye_ctx* c, uint64_t nw, const std::vector<int>& di
     std::swap(vals, vals2);
   }
   uint32_t* flags = buf<uint32_t>(c, "ib_flags", nw);
-  uint64_t* run_id = buf<uint64_t>(c, "ib_runid", nw + 1);
+  uint64_t* run_id = keys2;
   CUFLYE_CHECK(index_mark_runs(keys, nw, flags, st));
   const uint64_t nruns = scan_u32(c, flags, run_id, nw, "ib_scan");
-  uint64_t* run_start = buf<uint64_t>(c, "ib_runstart", nruns + 1);
+  uint64_t* run_start = vals2;
   CUFLYE_CHECK(index_run_starts(flags, run_id, nw, nruns, run_start, st));
   uint32_t* kept = buf<uint32_t>(c, "ib_kept", nruns);
   uint8_t* cls = buf<uint8_t>(c, "ib_cls", nruns);
@@ -383,11 +388,28 @@ KeyRuns sort_and_classify(cuflye_ctx* c, uint64_t nw, const std::vector<int>& di
   unsigned long long t[2];
   CUFLYE_CHECK(cudaMemcpyAsync(t, tally, sizeof(t), cudaMemcpyDeviceToHost, st));
   sync(c);
-  return KeyRuns{keys, vals, run_id, run_start, cls, kept_off, nw, nruns, npos, t[0], t[1]};
+  return KeyRuns{keys, vals, run_id, run_start, cls,   kept_off, flags, kept,
+                 nw,   nruns, npos,  t[0],      t[1]};
 }
 
 // Table slots for `entries` keys: twice as many (load 1/2), at least 16.
 uint64_t table_capacity(uint64_t entries) { return std::max<uint64_t>(16, 2 * entries); }
+
+// The run path's byte an entry (the bases around its k-mer), or null.  Kept for
+// an odd k (an even k has k-mers that equal their reverse complement) and while
+// it takes at most a quarter of the memory the index leaves (1 byte an entry
+// beside 8 and its share of the table; without it a pass runs on hits).
+uint8_t* neighbour_bytes(cuflye_ctx* c, int k, uint64_t npos) {
+  const uint64_t limit = effective_budget(c);
+  const uint64_t left = limit > c->in_use ? limit - c->in_use : 0;
+  if (k % 2 == 0 || npos + 16 > left / 4) return nullptr;
+  try {
+    return buf<uint8_t>(c, "ix_nbr", npos + 32);
+  } catch (const Error& e) {
+    if (e.code != CUFLYE_ERR_BUDGET) throw;
+    return nullptr;
+  }
+}
 
 // All windows at once.  This build fits the memory with room to spare, so
 // its table takes the power of two at or above twice every run (solid,
@@ -396,43 +418,53 @@ BuiltIndex build_one_range(cuflye_ctx* c, const WindowSet& w, const std::vector<
                            uint32_t min_freq, uint32_t max_freq) {
   cudaStream_t st = c->stream;
   // the four sort arrays first: a build that cannot hold them fails before any work
-  uint64_t* keys = buf<uint64_t>(c, "ib_keys", w.nwin);
-  uint64_t* vals = buf<uint64_t>(c, "ib_vals", w.nwin);
-  buf<uint64_t>(c, "ib_keys2", w.nwin);
-  buf<uint64_t>(c, "ib_vals2", w.nwin);
+  uint64_t* keys = buf<uint64_t>(c, "ib_keys", w.nwin + 1);
+  uint64_t* vals = buf<uint64_t>(c, "ib_vals", w.nwin + 1);
+  buf<uint64_t>(c, "ib_keys2", w.nwin + 1);
+  buf<uint64_t>(c, "ib_vals2", w.nwin + 1);
   CUFLYE_CHECK(index_enumerate(w.words, w.base_off, w.win_off, w.slot_len, w.nslots, w.nwin,
                                w.k, keys, vals, st));
   const KeyRuns r = sort_and_classify(c, w.nwin, digits, min_freq, max_freq);
   if (r.npos >= (1ull << 40)) throw Error(CUFLYE_ERR_UNSUPPORTED, "index larger than 2^40 entries");
   BuiltIndex bi;
   bi.pos = buf<uint64_t>(c, "ix_pos", r.npos);
-  // each indexed window's own bucket entry (4 bytes a window), when memory
-  // allows: hit counting then finds a query's own entry with one load
-  uint32_t* self_at = nullptr;
-  uint64_t* win_off = nullptr;
-  try {
-    self_at = buf<uint32_t>(c, "ix_selfat", w.nwin);
-    win_off = buf<uint64_t>(c, "ix_winoff", static_cast<uint64_t>(w.nslots) + 1);
-  } catch (const Error& e) {
-    if (e.code != CUFLYE_ERR_BUDGET) throw;
-    release(c, "ix_selfat");
-    release(c, "ix_winoff");
-    self_at = nullptr;
-    win_off = nullptr;
-  }
-  if (win_off)
-    CUFLYE_CHECK(cudaMemcpyAsync(win_off, w.win_off, (static_cast<uint64_t>(w.nslots) + 1) * 8,
-                                 cudaMemcpyDeviceToDevice, st));
-  CUFLYE_CHECK(index_copy_positions(r.vals, r.run_id, r.run_start, r.cls, r.kept_off, w.nwin,
-                                    bi.pos, true, st, self_at, win_off, w.slot_len, w.k));
-  bi.self_at = self_at;
-  bi.win_off = win_off;
   bi.cap = 16;
   while (bi.cap < 2 * r.nruns) bi.cap <<= 1;
   bi.table = buf<TableEntry>(c, "ix_table", bi.cap);
+  bi.nbr = neighbour_bytes(c, w.k, r.npos);
+  // every indexed window's record (16 bytes), while they take at most a quarter
+  // of the memory the build leaves
+  uint32_t* place = nullptr;
+  const uint64_t limit = effective_budget(c);
+  const uint64_t left = limit > c->in_use ? limit - c->in_use : 0;
+  if (w.nwin * sizeof(uint4) <= left / 4) {
+    try {
+      bi.windows = buf<uint4>(c, "ix_windows", w.nwin);
+      bi.win_off = buf<uint64_t>(c, "ix_winoff", static_cast<uint64_t>(w.nslots) + 1);
+      place = r.free_words;
+      CUFLYE_CHECK(cudaMemcpyAsync(bi.win_off, w.win_off,
+                                   (static_cast<uint64_t>(w.nslots) + 1) * 8,
+                                   cudaMemcpyDeviceToDevice, st));
+    } catch (const Error& e) {
+      if (e.code != CUFLYE_ERR_BUDGET) throw;
+      release(c, "ix_windows");
+      release(c, "ix_winoff");
+      bi.windows = nullptr;
+      bi.win_off = nullptr;
+    }
+  }
   CUFLYE_CHECK(cudaMemsetAsync(bi.table, 0xff, bi.cap * sizeof(TableEntry), st));
+  CUFLYE_CHECK(index_copy_positions(r.vals, r.run_id, r.run_start, r.cls, r.kept_off, w.nwin,
+                                    bi.pos, true, st, place));
+  if (bi.nbr)
+    CUFLYE_CHECK(index_neighbours(bi.pos, r.npos, w.words, w.base_off, w.slot_len, w.k, bi.nbr, st));
   CUFLYE_CHECK(index_insert(r.keys, bi.pos, r.run_start, r.cls, r.kept_off, r.nruns, 0, true,
-                            bi.table, bi.cap, c->status, st));
+                            bi.table, bi.cap, c->status, st,
+                            bi.windows ? r.free_run_words : nullptr, bi.nbr));
+  if (bi.windows)
+    CUFLYE_CHECK(index_window_records(r.vals, r.run_id, r.run_start, r.kept_off, r.cls,
+                                      r.free_run_words, place, w.nwin, bi.win_off, w.slot_len, w.k,
+                                      bi.windows, st));
   check_device_status(c);
   bi.npos = r.npos;
   bi.nsolid = r.nsolid;
@@ -440,9 +472,10 @@ BuiltIndex build_one_range(cuflye_ctx* c, const WindowSet& w, const std::vector<
   return bi;
 }
 
-// Device bytes one window of a key range needs while the range is built:
-// the radix sort's two key/value pairs (32), run flag and id (12) and the
-// run tables (21, at most one run per window), with margin.
+// Device bytes one window of a key range needs while the range is built: the
+// radix sort's two key/value pairs (32; the run ids and starts take one of
+// them), the run flag (4) and the run tables (13, at most one run per window),
+// with margin.
 constexpr uint64_t kRangeBytesPerWindow = 72;
 constexpr int kPrefixBits = 14;
 
@@ -477,10 +510,10 @@ uint64_t for_each_key_range(cuflye_ctx* c, const WindowSet& w, const std::vector
     const uint64_t hi = static_cast<uint64_t>(e) << shift;
     b = e;
     if (nw == 0) continue;
-    uint64_t* keys = buf<uint64_t>(c, "ib_keys", nw);
-    uint64_t* vals = buf<uint64_t>(c, "ib_vals", nw);
-    buf<uint64_t>(c, "ib_keys2", nw);
-    buf<uint64_t>(c, "ib_vals2", nw);
+    uint64_t* keys = buf<uint64_t>(c, "ib_keys", nw + 1);
+    uint64_t* vals = buf<uint64_t>(c, "ib_vals", nw + 1);
+    buf<uint64_t>(c, "ib_keys2", nw + 1);
+    buf<uint64_t>(c, "ib_vals2", nw + 1);
     unsigned long long* count = buf<unsigned long long>(c, "ib_count", 4);
     CUFLYE_CHECK(index_enumerate_range(w.words, w.base_off, w.win_off, w.slot_len, w.nslots,
                                        w.nwin, w.k, lo, hi, keys, vals, count, nw, st));
@@ -583,32 +616,23 @@ void drop_run_tables(cuflye_ctx* c) {
   c->idx.tbase = nullptr;
 }
 
-// Kept for an odd k (an even k has k-mers that equal their reverse
-// complement) and while they take at most a quarter of the memory the index
-// leaves (1 byte an entry, 1/4 byte a base: beside the 8 bytes of an entry
-// and its share of the table they shorten a pass by a few per cent at most).
+// A build in one range has the bytes already (its records need them).
 void keep_run_tables(cuflye_ctx* c, const BuiltIndex& bi, int k, const int32_t* d_len) {
-  const uint64_t limit = effective_budget(c);
-  const uint64_t left = limit > c->in_use ? limit - c->in_use : 0;
-  if (k % 2 == 0 || bi.npos + 16 > left / 4) return;
-  try {
-    uint8_t* nbr = buf<uint8_t>(c, "ix_nbr", bi.npos + 32);
-    auto keep = [&](const char* from, const char* to) {
-      // the scratch buffer becomes part of the index
-      release(c, to);
-      c->bufs[to] = c->bufs[from];
-      c->bufs.erase(from);
-      return c->bufs[to].p;
-    };
-    c->idx.twords = static_cast<uint64_t*>(keep("ib_words", "ix_words"));
-    c->idx.tbase = static_cast<uint64_t*>(keep("ib_base", "ix_base"));
+  uint8_t* nbr = bi.nbr ? bi.nbr : neighbour_bytes(c, k, bi.npos);
+  if (!nbr) return;
+  auto keep = [&](const char* from, const char* to) {
+    // the scratch buffer becomes part of the index
+    release(c, to);
+    c->bufs[to] = c->bufs[from];
+    c->bufs.erase(from);
+    return c->bufs[to].p;
+  };
+  c->idx.twords = static_cast<uint64_t*>(keep("ib_words", "ix_words"));
+  c->idx.tbase = static_cast<uint64_t*>(keep("ib_base", "ix_base"));
+  if (!bi.nbr)
     CUFLYE_CHECK(index_neighbours(bi.pos, bi.npos, c->idx.twords, c->idx.tbase, d_len, k, nbr,
                                   c->stream));
-    c->idx.nbr = nbr;
-  } catch (const Error& e) {
-    if (e.code != CUFLYE_ERR_BUDGET) throw;
-    drop_run_tables(c);
-  }
+  c->idx.nbr = nbr;
 }
 
 void build_index(cuflye_ctx* c, int k, size_t n, const int64_t* ids, const int64_t* offsets,
@@ -654,10 +678,10 @@ void build_index(cuflye_ctx* c, int k, size_t n, const int64_t* ids, const int64
   // the previous index's arrays go first (has_index is false from here on)
   release(c, "ix_pos");
   release(c, "ix_table");
-  release(c, "ix_selfat");
+  release(c, "ix_windows");
   release(c, "ix_winoff");
   drop_run_tables(c);
-  c->idx.self_at = nullptr;
+  c->idx.windows = nullptr;
   c->idx.win_off = nullptr;
   // bases packed in chunks of 256 MiB (a multiple of 32 bases: chunks start on
   // word boundaries; each chunk's trailing pad word is overwritten by the next)
@@ -707,8 +731,7 @@ void build_index(cuflye_ctx* c, int k, size_t n, const int64_t* ids, const int64
       release_build_scratch(c);
       release(c, "ix_pos");
       release(c, "ix_table");
-      release(c, "ix_selfat");
-      release(c, "ix_winoff");
+      for (const char* t : {"ix_windows", "ix_winoff", "ix_nbr"}) release(c, t);
       ranges = true;
     }
   }
@@ -725,7 +748,7 @@ void build_index(cuflye_ctx* c, int k, size_t n, const int64_t* ids, const int64
   c->idx.slot_len = d_len;
   c->idx.slot_signed = d_signed;
   c->idx.nslots = static_cast<uint32_t>(n);
-  c->idx.self_at = bi.self_at;
+  c->idx.windows = bi.windows;
   c->idx.win_off = bi.win_off;
   c->idx.nkeys = bi.nsolid + bi.nrep;
   c->idx.nrep = bi.nrep;
@@ -813,10 +836,10 @@ void build_index_entries(cuflye_ctx* c, int k, size_t n, const int64_t* tids, co
     release(c, t);
   c->idx.k = k;
   c->idx.transform = false;
-  release(c, "ix_selfat");
+  release(c, "ix_windows");
   release(c, "ix_winoff");
   drop_run_tables(c);
-  c->idx.self_at = nullptr;
+  c->idx.windows = nullptr;
   c->idx.win_off = nullptr;
   c->idx.table = table;
   c->idx.cap = cap;
@@ -1148,7 +1171,8 @@ void run_runs(cuflye_ctx* c, PassState& ps) {
   // 64 partial sums of hits, the totals of runs_query_offsets
   unsigned long long* total = buf<unsigned long long>(c, "n_total", 67);
   CUFLYE_CHECK(cudaMemsetAsync(total, 0, 67 * sizeof(unsigned long long), st));
-  CUFLYE_CHECK(runs_count(c->idx, ps.qb, recs, nstart, cbits, fbits, tfilt, tstart, total, st));
+  CUFLYE_CHECK(runs_count(c->idx, ps.qb, recs, nstart, cbits, fbits, tfilt, tstart, total,
+                          c->num_sms, st));
   CUFLYE_CHECK(exclusive_scan_pair(tstart, tile_off, tfilt, ftile_off, nt,
                                    buf<uint64_t>(c, "n_scan", scan_temp_words(nt)), st));
   ps.q_off = buf<uint64_t>(c, "n_qoff", nq + 1);

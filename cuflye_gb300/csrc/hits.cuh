@@ -22,6 +22,23 @@ __device__ __forceinline__ uint32_t query_of(const uint64_t* __restrict__ win_of
   return lo;
 }
 
+// The same by a whole warp, 32 candidates a step: three loads in a row where
+// the halving search has thirteen (13 thousand queries).
+__device__ __forceinline__ uint32_t query_of_warp(const uint64_t* __restrict__ win_off,
+                                                  uint32_t nq, uint64_t w) {
+  const uint32_t lane = threadIdx.x & 31;
+  uint32_t lo = 0, n = nq;  // the answer is in [lo, lo + n)
+  while (n > 1) {
+    const uint32_t step = (n + 31) / 32, at = lane * step;
+    const unsigned m =
+        __ballot_sync(0xffffffffu, at < n && __ldg(win_off + lo + at) <= w) | 1u;
+    const uint32_t j = 31 - __clz(m);
+    lo += j * step;
+    n = min(step, n - j * step);
+  }
+  return lo;
+}
+
 struct WindowKmer {
   uint64_t x;    // forward k-mer (Kmer::numRepr)
   uint64_t key;  // standard form
@@ -64,6 +81,34 @@ __device__ __forceinline__ uint32_t bucket_find(const DeviceIndex& idx, uint64_t
   return lo < c && __ldg(idx.pos + off + lo) == want ? lo : c;
 }
 
+constexpr uint32_t kPlaceMask = (1u << kCountBits) - 1;
+
+// Position of query window p on the forward strand of its target (dense id
+// qdi); negative or past the target's last window when it is not one of them.
+__device__ __forceinline__ int64_t forward_window(const DeviceIndex& idx, int32_t qdi,
+                                                  uint64_t p) {
+  const int64_t f = static_cast<int64_t>(p);
+  return (qdi & 1) ? static_cast<int64_t>(idx.slot_len[static_cast<uint32_t>(qdi) >> 1]) - idx.k - f
+                   : f;
+}
+
+// Whether the indexed sequence of dense id qdi has the query's k-mer x at the
+// query's position p: its own position is an entry of x's bucket exactly then
+// (a look at the packed target, in step with the query's own bases).  rec: the
+// index's record of the target's window, if it keeps any (loaded beside the
+// target's bases, not after the comparison).
+__device__ __forceinline__ bool own_window(const DeviceIndex& idx, int32_t qdi, uint64_t p,
+                                           uint64_t x, uint4& rec) {
+  rec = make_uint4(0, 0, 0, 0);
+  if (qdi < 0 || !idx.twords) return false;
+  const uint32_t slot = static_cast<uint32_t>(qdi) >> 1;
+  const int64_t f = forward_window(idx, qdi, p);
+  if (f < 0 || f + idx.k > idx.slot_len[slot]) return false;
+  if (idx.windows) rec = __ldg(idx.windows + idx.win_off[slot] + static_cast<uint64_t>(f));
+  const uint64_t y = kmer_at(idx.twords, idx.tbase[slot] + static_cast<uint64_t>(f), idx.k);
+  return ((qdi & 1) ? revcomp(y, idx.k) : y) == x;
+}
+
 // A window's bucket: its table meta, flags (kWinRev, kWinFiltered,
 // kWinTrivial), hits (the bucket's entries less the query's own position) and
 // the own entry's bucket index (kWinTrivial on a built index).
@@ -78,8 +123,11 @@ __device__ __forceinline__ WindowProbe probe_window(const DeviceIndex& idx, cons
                                                     uint32_t qi, uint64_t p,
                                                     uint32_t* __restrict__ q_tie) {
   const WindowKmer km = window_kmer(q, qi, p, idx.k);
-  bool found;
-  const uint64_t meta = table_probe(idx.table, idx.cap, km.key, &found);
+  uint4 rec;
+  const bool recorded = own_window(idx, q.qdi[qi], p, km.x, rec) && idx.windows;
+  bool found = rec.w & kWindowFound;
+  const uint64_t meta = recorded ? static_cast<uint64_t>(rec.y) << 32 | rec.x
+                                 : table_probe(idx.table, idx.cap, km.key, &found);
   uint32_t c = 0, self = 0;
   uint8_t fl = km.rev ? kWinRev : 0;
   if (found && (meta & kRepetitiveBit)) {
@@ -98,17 +146,14 @@ __device__ __forceinline__ WindowProbe probe_window(const DeviceIndex& idx, cons
         // unique.  A query that is an indexed target finds its own entry
         // where the index recorded it (checked: a query sequence that
         // differs from the indexed one searches as any other)
-        bool known = false;
-        uint32_t at = 0;
-        if (idx.self_at && !(qdi & 1)) {
+        bool known = recorded;
+        uint32_t at = rec.z & kPlaceMask;
+        if (!known && idx.windows && !(qdi & 1)) {
           const uint32_t slot = static_cast<uint32_t>(qdi) >> 1;
           const uint64_t w0 = idx.win_off[slot];
           if (w0 + p < idx.win_off[slot + 1]) {
-            const uint32_t g = idx.self_at[w0 + p];
-            if (g < c && __ldg(idx.pos + off + g) == want) {
-              known = true;
-              at = g;
-            }
+            at = idx.windows[w0 + p].z & kPlaceMask;
+            known = at < c && __ldg(idx.pos + off + at) == want;
           }
         }
         if (!known) {

@@ -173,23 +173,28 @@ __global__ void classify_runs_kernel(const uint64_t* __restrict__ run_start, uin
   }
 }
 
+// flags_scan holds the exclusive scan of run-start flags: the run of element i
+// is the number of run starts at or before i, minus one.
+__device__ __forceinline__ uint64_t run_of(const uint64_t* __restrict__ flags_scan,
+                                           const uint64_t* __restrict__ run_start, uint64_t i) {
+  uint64_t r = flags_scan[i];
+  if (r >= 1 && run_start[r] > i) r -= 1;
+  while (run_start[r] > i) --r;
+  return r;
+}
+
 // window_order: the runs are in (target, window) order, not in bucket order.
+// place (optional): each solid element's place in its bucket.
 __global__ void copy_positions_kernel(const uint64_t* __restrict__ vals,
                                       const uint64_t* __restrict__ flags_scan,
                                       const uint64_t* __restrict__ run_start,
                                       const uint8_t* __restrict__ cls,
                                       const uint64_t* __restrict__ kept_off, uint64_t n,
                                       uint64_t* __restrict__ pos, bool window_order,
-                                      uint32_t* __restrict__ self_at,
-                                      const uint64_t* __restrict__ win_off,
-                                      const int32_t* __restrict__ slot_len, int k) {
+                                      uint32_t* __restrict__ place) {
   const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  // flags_scan holds the exclusive scan of run-start flags: the run of
-  // element i is the number of run starts at or before i, minus one.
-  uint64_t r = flags_scan[i];
-  if (r >= 1 && run_start[r] > i) r -= 1;
-  while (run_start[r] > i) --r;
+  const uint64_t r = run_of(flags_scan, run_start, i);
   if (cls[r] != 1) return;
   const uint64_t v = vals[i];
   const uint64_t r0 = run_start[r], r1 = run_start[r + 1];
@@ -207,15 +212,42 @@ __global__ void copy_positions_kernel(const uint64_t* __restrict__ vals,
     at = (lo - r0) + ahead + (rev ? later : 0u);
   }
   pos[kept_off[r] + at] = v;
-  if (self_at) {
-    // the window this entry came from: its forward position in its target
-    const uint32_t sid = static_cast<uint32_t>(v >> 32);
-    const uint32_t slot = sid >> 1;
-    const int64_t sp = static_cast<int64_t>(v & 0xffffffffu);
-    const int64_t p = (sid & 1u) ? static_cast<int64_t>(slot_len[slot]) - sp - k : sp;
-    const uint64_t w = win_off[slot] + static_cast<uint64_t>(p);
-    if (p >= 0 && w < win_off[slot + 1]) self_at[w] = static_cast<uint32_t>(at);
+  if (place) place[i] = static_cast<uint32_t>(at);
+}
+
+// The record of every window (DeviceIndex::windows).  Bound by its
+// scattered 16-byte stores, one a window, in bucket order.
+__global__ void window_records_kernel(const uint64_t* __restrict__ vals,
+                                      const uint64_t* __restrict__ flags_scan,
+                                      const uint64_t* __restrict__ run_start,
+                                      const uint64_t* __restrict__ meta,
+                                      const uint8_t* __restrict__ sides,
+                                      const uint32_t* __restrict__ others,
+                                      const uint32_t* __restrict__ place, uint64_t n,
+                                      const uint64_t* __restrict__ win_off,
+                                      const int32_t* __restrict__ slot_len, int k,
+                                      uint4* __restrict__ windows) {
+  const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const uint64_t r = run_of(flags_scan, run_start, i);
+  const uint64_t m = meta[r], v = vals[i];
+  uint4 rec = make_uint4(0, 0, 0, 0);
+  if (m != kNoMeta) {
+    rec.x = static_cast<uint32_t>(m);
+    rec.y = static_cast<uint32_t>(m >> 32);
+    rec.w = kWindowFound;
+    if (!(m & kRepetitiveBit)) {
+      rec.z = place[i] | static_cast<uint32_t>(sides[r]) << kCountBits;
+      rec.w |= others[r];
+    }
   }
+  // the window this entry came from: its forward position in its target
+  const uint32_t sid = static_cast<uint32_t>(v >> 32);
+  const uint32_t slot = sid >> 1;
+  const int64_t sp = static_cast<int64_t>(v & 0xffffffffu);
+  const int64_t p = (sid & 1u) ? static_cast<int64_t>(slot_len[slot]) - sp - k : sp;
+  const uint64_t w = win_off[slot] + static_cast<uint64_t>(p);
+  if (p >= 0 && w < win_off[slot + 1]) windows[w] = rec;
 }
 
 __device__ bool table_insert(TableEntry* table, uint64_t cap, uint64_t key, uint64_t meta,
@@ -257,18 +289,62 @@ __device__ __forceinline__ uint64_t run_meta(const uint64_t* __restrict__ bucket
   return meta;
 }
 
+// What most entries of a bucket have before (bits 0-2) and after (3-5) their
+// k-mer, and how many have something else (before: bits 0-11, after: 16-27); 7s
+// for a bucket too large for the counters.
+__device__ __forceinline__ uint8_t bucket_sides(const uint8_t* __restrict__ nbr, uint64_t n,
+                                                uint32_t& others) {
+  others = 0;
+  if (n >= 4096) return 63;
+  uint64_t before = 0, after = 0;  // five counters of 12 bits
+  for (uint64_t e = 0; e < n; ++e) {
+    const uint32_t x = nbr[e];
+    before += 1ull << (12 * (x & 7u));
+    after += 1ull << (12 * (x >> 4));
+  }
+  auto most = [&](uint64_t counts, int at) {
+    uint32_t best = 0, side = 0;
+#pragma unroll
+    for (uint32_t v = 0; v < 5; ++v) {
+      const uint32_t c = static_cast<uint32_t>(counts >> (12 * v)) & 4095u;
+      if (c > best) {
+        best = c;
+        side = v;
+      }
+    }
+    others |= (static_cast<uint32_t>(n) - best) << at;
+    return side;
+  };
+  const uint32_t b = most(before, 0), a = most(after, 16);
+  return static_cast<uint8_t>(b | a << 3);
+}
+
+// records (optional): takes what most entries have beside their k-mers, with
+// the counts of the others (bucket_sides); the runs' table words (kNoMeta: not
+// in the table) then replace kept_off and the sides cls, for
+// window_records_kernel.  nbr: optional.
 __global__ void insert_kernel(const uint64_t* __restrict__ keys,
                               const uint64_t* __restrict__ pos,
-                              const uint64_t* __restrict__ run_start,
-                              const uint8_t* __restrict__ cls,
-                              const uint64_t* __restrict__ kept_off, uint64_t nruns,
-                              uint64_t pos_base, bool sorted_ids, TableEntry* table,
-                              uint64_t cap, DeviceStatus* st) {
+                              const uint64_t* __restrict__ run_start, uint8_t* cls,
+                              uint64_t* kept_off, uint64_t nruns, uint64_t pos_base,
+                              bool sorted_ids, TableEntry* table, uint64_t cap, DeviceStatus* st,
+                              uint32_t* __restrict__ records,
+                              const uint8_t* __restrict__ nbr) {
   const uint64_t r = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (r >= nruns || cls[r] == 0) return;
-  const uint64_t r0 = run_start[r];
-  const uint64_t meta =
-      run_meta(pos + kept_off[r], run_start[r + 1] - r0, cls[r], pos_base + kept_off[r], sorted_ids);
+  if (r >= nruns) return;
+  const uint8_t cl = cls[r];
+  if (cl == 0) {
+    if (records) kept_off[r] = kNoMeta;
+    return;
+  }
+  const uint64_t r0 = run_start[r], off = kept_off[r], n = run_start[r + 1] - r0;
+  const uint64_t meta = run_meta(pos + off, n, cl, pos_base + off, sorted_ids);
+  if (records) {
+    kept_off[r] = meta;
+    uint32_t others = 0;
+    cls[r] = nbr && cl == 1 ? bucket_sides(nbr + off, n, others) : static_cast<uint8_t>(63);
+    records[r] = others;
+  }
   if (!table_insert(table, cap, keys[r0], meta, false)) raise_status(st, kDevTableFull, 0, r);
 }
 
@@ -393,24 +469,36 @@ cudaError_t index_classify_runs(const uint64_t* run_start, uint64_t nruns, uint3
 cudaError_t index_copy_positions(const uint64_t* vals, const uint64_t* run_id,
                                  const uint64_t* run_start, const uint8_t* cls,
                                  const uint64_t* kept_off, uint64_t n, uint64_t* pos,
-                                 bool window_order, cudaStream_t s, uint32_t* self_at,
-                                 const uint64_t* win_off, const int32_t* slot_len, int k) {
+                                 bool window_order, cudaStream_t s, uint32_t* place) {
   if (n == 0) return cudaSuccess;
   count_launch();
   copy_positions_kernel<<<grid(n, 256), 256, 0, s>>>(vals, run_id, run_start, cls, kept_off, n,
-                                                     pos, window_order, self_at, win_off,
-                                                     slot_len, k);
+                                                     pos, window_order, place);
   return cudaGetLastError();
 }
 
 cudaError_t index_insert(const uint64_t* keys, const uint64_t* pos, const uint64_t* run_start,
-                         const uint8_t* cls, const uint64_t* kept_off, uint64_t nruns,
-                         uint64_t pos_base, bool sorted_ids, TableEntry* table, uint64_t cap,
-                         DeviceStatus* st, cudaStream_t s) {
+                         uint8_t* cls, uint64_t* kept_off, uint64_t nruns, uint64_t pos_base,
+                         bool sorted_ids, TableEntry* table, uint64_t cap, DeviceStatus* st,
+                         cudaStream_t s, uint32_t* records, const uint8_t* nbr) {
   if (nruns == 0) return cudaSuccess;
   count_launch();
   insert_kernel<<<grid(nruns, 256), 256, 0, s>>>(keys, pos, run_start, cls, kept_off, nruns,
-                                                 pos_base, sorted_ids, table, cap, st);
+                                                 pos_base, sorted_ids, table, cap, st, records,
+                                                 nbr);
+  return cudaGetLastError();
+}
+
+cudaError_t index_window_records(const uint64_t* vals, const uint64_t* run_id,
+                                 const uint64_t* run_start, const uint64_t* meta,
+                                 const uint8_t* sides, const uint32_t* others,
+                                 const uint32_t* place, uint64_t n, const uint64_t* win_off,
+                                 const int32_t* slot_len, int k, uint4* windows,
+                                 cudaStream_t s) {
+  if (n == 0) return cudaSuccess;
+  count_launch();
+  window_records_kernel<<<grid(n, 256), 256, 0, s>>>(vals, run_id, run_start, meta, sides, others,
+                                                     place, n, win_off, slot_len, k, windows);
   return cudaGetLastError();
 }
 

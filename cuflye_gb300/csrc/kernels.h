@@ -105,10 +105,16 @@ struct DeviceIndex {
   int64_t* slot_signed = nullptr;  // signed id per dense slot
   uint32_t nslots = 0;
   uint64_t nkeys = 0, nrep = 0;
-  // optional (one-range builds): per window of the indexed targets (slot
-  // order, win_off per slot), the index of its own entry in its k-mer's
-  // bucket when that k-mer is solid (other windows: any value)
-  uint32_t* self_at = nullptr;
+  // optional (one-range builds, when memory allows): per window of the indexed
+  // targets (slot order, win_off per slot) its k-mer's table word (x, y), its
+  // own entry's place in the bucket (z, low kCountBits bits) with what most of
+  // the bucket's entries have before and after the k-mer (3 bits each, a nibble
+  // of nbr; 7: not known), and whether the table holds the k-mer (w, bit 31)
+  // with how many entries have something else before (bits 0-11) and after
+  // (16-27).
+  // A query that is an indexed target reads its windows' records in a row
+  // where a table probe is a scattered load, and most of their neighbours too
+  uint4* windows = nullptr;
   uint64_t* win_off = nullptr;
   // optional (built indexes of an odd k, when memory allows): the bases around
   // each stored entry's k-mer, one byte an entry in bucket order, and the
@@ -148,20 +154,31 @@ cudaError_t index_classify_runs(const uint64_t* run_start, uint64_t nruns, uint3
                                 unsigned long long* tally, cudaStream_t s);
 // Solid runs' entries into pos, in (stored id, stored position) order.
 // window_order: the runs hold them in (target, window) order instead.
+// place (optional): each solid element's place in its bucket.
 cudaError_t index_copy_positions(const uint64_t* vals, const uint64_t* run_id,
                                  const uint64_t* run_start, const uint8_t* cls,
                                  const uint64_t* kept_off, uint64_t n, uint64_t* pos,
-                                 bool window_order, cudaStream_t s, uint32_t* self_at = nullptr,
-                                 const uint64_t* win_off = nullptr,
-                                 const int32_t* slot_len = nullptr, int k = 0);
+                                 bool window_order, cudaStream_t s, uint32_t* place = nullptr);
 // Table insert of every solid and repetitive run, a solid run's positions
 // at pos + kept_off (pos_base + kept_off of the position array).  Solid buckets that list
 // one stored id twice get kDupIdsBit (sorted_ids: runs are in (id, position)
 // order; otherwise every run of two or more entries is marked).
 cudaError_t index_insert(const uint64_t* keys, const uint64_t* pos, const uint64_t* run_start,
-                         const uint8_t* cls, const uint64_t* kept_off, uint64_t nruns,
-                         uint64_t pos_base, bool sorted_ids, TableEntry* table, uint64_t cap,
-                         DeviceStatus* st, cudaStream_t s);
+                         uint8_t* cls, uint64_t* kept_off, uint64_t nruns, uint64_t pos_base,
+                         bool sorted_ids, TableEntry* table, uint64_t cap, DeviceStatus* st,
+                         cudaStream_t s, uint32_t* records = nullptr,
+                         const uint8_t* nbr = nullptr);
+// Window records (DeviceIndex::windows) from index_insert's (records, a word a
+// run: it takes the counts of others, and kept_off and cls then hold the run's
+// table word, kNoMeta for none, and sides).
+constexpr uint64_t kNoMeta = ~0ull;
+constexpr uint32_t kWindowFound = 1u << 31;
+cudaError_t index_window_records(const uint64_t* vals, const uint64_t* run_id,
+                                 const uint64_t* run_start, const uint64_t* meta,
+                                 const uint8_t* sides, const uint32_t* others,
+                                 const uint32_t* place, uint64_t n, const uint64_t* win_off,
+                                 const int32_t* slot_len, int k, uint4* windows,
+                                 cudaStream_t s);
 // Per key prefix (key >> shift) of sorted runs: solid positions into
 // npos_bin, solid and repetitive runs into nent_bin (both accumulate).
 cudaError_t index_bin_totals(const uint64_t* keys, const uint64_t* run_start, const uint8_t* cls,

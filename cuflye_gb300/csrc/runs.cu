@@ -141,119 +141,147 @@ __device__ __forceinline__ uint32_t count_starts(const DeviceIndex& idx, uint64_
   return ns;
 }
 
-// A window's table word, its own entry's place in the bucket and the flags.
-// The query's own position is an entry exactly when the indexed sequence has
-// the query's k-mer there, which a look at the packed target tells (in step
-// with the query's own bases, where reading the entry is a scattered load).
+// What most entries of a window's bucket have on the side that tells whether
+// they continue a run (a nibble's value, 7: not known), and how many differ.
+struct BucketSide {
+  uint32_t most, others;
+};
+
+// A window's table word, its own entry's place in the bucket, the bucket's side
+// and the flags.
 __device__ __forceinline__ uint8_t probe_run_window(const DeviceIndex& idx, const QueryBatch& q,
                                                     uint32_t qi, uint64_t p, uint64_t& meta,
-                                                    uint32_t& self) {
+                                                    uint32_t& self, BucketSide& side) {
   const WindowKmer km = window_kmer(q, qi, p, idx.k);
-  bool found;
-  meta = table_probe(idx.table, idx.cap, km.key, &found);
+  const int32_t qdi = q.qdi[qi];
+  uint4 rec;
+  const bool own = own_window(idx, qdi, p, km.x, rec), recorded = own && idx.windows;
+  bool found = rec.w & kWindowFound;
+  meta = recorded ? static_cast<uint64_t>(rec.y) << 32 | rec.x
+                  : table_probe(idx.table, idx.cap, km.key, &found);
   uint8_t fl = km.rev ? kWinRev : 0;
   self = kNoSelf;
+  side = BucketSide{7, 0};
   if (!found) return fl;
   if (meta & kRepetitiveBit) return fl | kWinFiltered;
   fl |= kWinSolid;
-  const int32_t qdi = q.qdi[qi];
-  if (qdi < 0) return fl;
-  const uint32_t slot = static_cast<uint32_t>(qdi) >> 1;
-  const int64_t last = static_cast<int64_t>(idx.slot_len[slot]) - idx.k;
-  const int64_t f = (qdi & 1) ? last - static_cast<int64_t>(p) : static_cast<int64_t>(p);
-  if (f < 0 || f > last) return fl;
-  const uint64_t y = kmer_at(idx.twords, idx.tbase[slot] + static_cast<uint64_t>(f), idx.k);
-  if (((qdi & 1) ? revcomp(y, idx.k) : y) != km.x) return fl;
-  self = idx.self_at ? idx.self_at[idx.win_off[slot] + static_cast<uint64_t>(f)]
-                     : bucket_find(idx, meta & kOffsetMask, bucket_size(meta),
-                                   self_entry(idx, qdi, p, km.rev));
+  if (recorded) {
+    self = rec.z & kPlaceMask;
+    side.most = rec.z >> (kCountBits + (km.rev ? 3 : 0)) & 7u;
+    side.others = rec.w >> (km.rev ? 16 : 0) & 0xfffu;
+  } else if (own) {
+    self = bucket_find(idx, meta & kOffsetMask, bucket_size(meta),
+                       self_entry(idx, qdi, p, km.rev));
+  }
   return fl;
+}
+
+// The base before the query's own window p in its target (4: the target's end):
+// what its entry's nibble says, in step with the query's bases.
+__device__ __forceinline__ uint32_t own_before(const DeviceIndex& idx, int32_t qdi, uint64_t p) {
+  const uint32_t slot = static_cast<uint32_t>(qdi) >> 1;
+  const int64_t f = forward_window(idx, qdi, p);
+  const uint64_t b = idx.tbase[slot];
+  if (!(qdi & 1)) return f > 0 ? base_at(idx.twords, b + static_cast<uint64_t>(f) - 1) : 4u;
+  const int64_t after = f + idx.k;
+  return after < idx.slot_len[slot]
+             ? 3u - base_at(idx.twords, b + static_cast<uint64_t>(after)) : 4u;
 }
 
 constexpr int kProbeBlock = 256;
 
-// One thread per window, blocks of whole 32-window tiles: the table probe, then
-// the run starts in the window's bucket.  Bound by the probe's scattered
-// loads (a table slot and two to three sectors of neighbours a window), which
-// is why both share a kernel: the counting of one warp hides the other's loads.
+// One thread per window, blocks of whole 32-window tiles, `rounds` block widths of
+// windows a block: the table probe (or the index's record of the window), then
+// the run starts in the window's bucket.  Bound by latency: a chain of loads
+// (the block's query, its target, bases, then a table slot and neighbours, all
+// scattered, for a query that is no target of the index).
 __global__ void __launch_bounds__(kProbeBlock, 6) probe_kernel(
-    DeviceIndex idx, QueryBatch q, uint4* __restrict__ recs, uint32_t* __restrict__ nstart,
-    uint32_t* __restrict__ cbits, uint32_t* __restrict__ fbits, uint32_t* __restrict__ tile_filt,
-    uint32_t* __restrict__ tile_start, unsigned long long* __restrict__ hit_total) {
+    DeviceIndex idx, QueryBatch q, int rounds, uint4* __restrict__ recs,
+    uint32_t* __restrict__ nstart, uint32_t* __restrict__ cbits, uint32_t* __restrict__ fbits,
+    uint32_t* __restrict__ tile_filt, uint32_t* __restrict__ tile_start,
+    unsigned long long* __restrict__ hit_total) {
   __shared__ uint32_t wsum[kProbeBlock / 32];
   __shared__ uint32_t ends[2];             // queries of the block's first and last windows
   __shared__ bool solid[kProbeBlock + 1];  // of the windows before and in the block
-  const uint64_t w0 = static_cast<uint64_t>(blockIdx.x) * kProbeBlock, w = w0 + threadIdx.x;
+  const uint64_t w0 = static_cast<uint64_t>(blockIdx.x) * kProbeBlock * rounds;
+  const uint64_t w1 = min(w0 + static_cast<uint64_t>(kProbeBlock) * rounds, q.nwin);
   const int lane = threadIdx.x & 31;
-  if (threadIdx.x == 0)
-    ends[0] = query_of(q.win_off, q.nq, w0);
-  else if (threadIdx.x == 32)
-    ends[1] = query_of(q.win_off, q.nq, min(w0 + kProbeBlock, q.nwin) - 1);
+  if (threadIdx.x < 64) {
+    const uint32_t e = query_of_warp(q.win_off, q.nq, threadIdx.x < 32 ? w0 : w1 - 1);
+    if (lane == 0) ends[threadIdx.x >> 5] = e;
+  }
   __syncthreads();
-  uint64_t meta = 0, p = 0;
-  uint32_t self = kNoSelf, left = 7;
-  uint8_t fl = 0;
-  if (w < q.nwin) {
-    uint32_t lo = ends[0], hi = ends[1];  // most blocks lie within one query
-    while (lo < hi) {
-      const uint32_t mid = (lo + hi + 1) >> 1;
-      if (__ldg(q.win_off + mid) <= w)
-        lo = mid;
-      else
-        hi = mid - 1;
-    }
-    p = w - q.win_off[lo];
-    fl = probe_run_window(idx, q, lo, p, meta, self);
-    if (p > 0) left = base_at(q.words, q.base_off[lo] + p - 1);
-    if (threadIdx.x == 0) {
-      // the last window of the block before: could a run continue from it?
-      bool before = false;
-      if (p > 0) {
-        bool found;
-        const uint64_t m =
-            table_probe(idx.table, idx.cap, window_kmer(q, lo, p - 1, idx.k).key, &found);
-        before = found && !(m & kRepetitiveBit);
+  uint32_t lo = ends[0], block_hits = 0;
+  for (uint64_t b0 = w0; b0 < w1; b0 += kProbeBlock) {
+    const uint64_t w = b0 + threadIdx.x;
+    uint64_t meta = 0, p = 0;
+    uint32_t self = kNoSelf, left = 7;
+    BucketSide side{7, 0};
+    uint8_t fl = 0;
+    if (w < w1) {
+      uint32_t hi = ends[1];  // most blocks lie within one query
+      while (lo < hi) {
+        const uint32_t mid = (lo + hi + 1) >> 1;
+        if (__ldg(q.win_off + mid) <= w)
+          lo = mid;
+        else
+          hi = mid - 1;
       }
-      solid[0] = before;
+      p = w - q.win_off[lo];
+      fl = probe_run_window(idx, q, lo, p, meta, self, side);
+      if (p > 0) left = base_at(q.words, q.base_off[lo] + p - 1);
+      if (threadIdx.x == 0 && b0 == w0) {
+        // the last window of the block before: could a run continue from it?
+        bool before = false;
+        if (p > 0) {
+          uint64_t m;
+          uint32_t a;
+          BucketSide b;
+          before = probe_run_window(idx, q, lo, p - 1, m, a, b) & kWinSolid;
+        }
+        solid[0] = before;
+      }
     }
-  }
-  solid[threadIdx.x + 1] = fl & kWinSolid;
-  __syncthreads();
-  uint32_t ns = 0, hits = 0;
-  RunTest rt{7, (fl & kWinRev) ? 4 : 0};
-  if (fl & kWinSolid) {
-    if (left != 7 && solid[threadIdx.x]) rt.expect = rt.shift ? 3u - left : left;
-    const uint64_t off = meta & kOffsetMask;
-    const uint32_t c = bucket_size(meta), own = self != kNoSelf ? 1u : 0u;
-    hits = c - own;
-    if (rt.expect == 7) {
-      ns = hits;
-    } else {
-      ns = count_starts(idx, off, c, rt);
-      // the query's own position is no hit
-      if (own && ((static_cast<uint32_t>(__ldg(idx.nbr + off + self)) >> rt.shift) & 15u) !=
-                     rt.expect)
-        --ns;
+    solid[threadIdx.x + 1] = fl & kWinSolid;
+    __syncthreads();
+    const bool continues = solid[threadIdx.x];
+    uint32_t ns = 0, hits = 0;
+    RunTest rt{7, (fl & kWinRev) ? 4 : 0};
+    if (fl & kWinSolid) {
+      if (left != 7 && continues) rt.expect = rt.shift ? 3u - left : left;
+      const uint64_t off = meta & kOffsetMask;
+      const uint32_t c = bucket_size(meta), own = self != kNoSelf ? 1u : 0u;
+      hits = c - own;
+      if (side.most != 7 && side.most != rt.expect && side.others == 0) rt.expect = 7;
+      if (rt.expect == 7) {
+        ns = hits;
+      } else {
+        ns = side.most == rt.expect ? side.others : count_starts(idx, off, c, rt);
+        // the query's own position is no hit
+        if (ns && own && own_before(idx, q.qdi[lo], p) != left) --ns;
+      }
     }
-  }
-  const uint32_t cb = __ballot_sync(0xffffffffu, fl & kWinSolid);
-  const uint32_t fb = __ballot_sync(0xffffffffu, fl & kWinFiltered);
-  const uint32_t starts = __reduce_add_sync(0xffffffffu, ns);
-  const uint32_t sum = __reduce_add_sync(0xffffffffu, hits);
-  if (w < q.nwin) {
-    nstart[w] = ns;
-    if (ns || (fl & kWinFiltered))
-      recs[w] = make_uint4(static_cast<uint32_t>(meta), static_cast<uint32_t>(meta >> 32),
-                           static_cast<uint32_t>(p),
-                           self | rt.expect << 22 | static_cast<uint32_t>(rt.shift) << 23);
-    if (lane == 0) {
-      cbits[w >> 5] = cb;
-      fbits[w >> 5] = fb;
-      tile_filt[w >> 5] = __popc(fb);
-      tile_start[w >> 5] = starts;
+    const uint32_t cb = __ballot_sync(0xffffffffu, fl & kWinSolid);
+    const uint32_t fb = __ballot_sync(0xffffffffu, fl & kWinFiltered);
+    const uint32_t starts = __reduce_add_sync(0xffffffffu, ns);
+    block_hits += __reduce_add_sync(0xffffffffu, hits);
+    if (w < w1) {
+      nstart[w] = ns;
+      if (ns || (fl & kWinFiltered))
+        recs[w] = make_uint4(static_cast<uint32_t>(meta), static_cast<uint32_t>(meta >> 32),
+                             static_cast<uint32_t>(p),
+                             self | rt.expect << 22 | static_cast<uint32_t>(rt.shift) << 23);
+      if (lane == 0) {
+        cbits[w >> 5] = cb;
+        fbits[w >> 5] = fb;
+        tile_filt[w >> 5] = __popc(fb);
+        tile_start[w >> 5] = starts;
+      }
     }
+    __syncthreads();  // solid is read
+    if (threadIdx.x == kProbeBlock - 1) solid[0] = fl & kWinSolid;
   }
-  if (lane == 0) wsum[threadIdx.x >> 5] = sum;
+  if (lane == 0) wsum[threadIdx.x >> 5] = block_hits;
   __syncthreads();
   if (threadIdx.x == 0) {
     unsigned long long s = 0;
@@ -340,10 +368,10 @@ __global__ void __launch_bounds__(256) start_emit_kernel(
     const uint32_t wp = __shfl_sync(0xffffffffu, p, src);
     const uint32_t wt = __shfl_sync(0xffffffffu, test, src);
     const uint32_t e = j - (end - n);
-    const bool start =
-        j < total && e != (wt & kNoSelf) &&
-        ((static_cast<uint32_t>(__ldg(idx.nbr + wo + e)) >> ((wt >> 23) & 4u)) & 15u) !=
-            ((wt >> 22) & 7u);
+    const uint32_t expect = (wt >> 22) & 7u;
+    bool start = j < total && e != (wt & kNoSelf);
+    if (start && expect != 7)
+      start = ((static_cast<uint32_t>(__ldg(idx.nbr + wo + e)) >> ((wt >> 23) & 4u)) & 15u) != expect;
     const unsigned m = __ballot_sync(0xffffffffu, start);
     if (start) {
       const uint64_t sv = __ldg(idx.pos + wo + e);
@@ -919,11 +947,15 @@ cudaError_t index_neighbours(const uint64_t* pos, uint64_t npos, const uint64_t*
 
 cudaError_t runs_count(const DeviceIndex& idx, const QueryBatch& q, uint4* recs, uint32_t* nstart,
                        uint32_t* cbits, uint32_t* fbits, uint32_t* tile_filt,
-                       uint32_t* tile_start, unsigned long long* hit_total, cudaStream_t s) {
+                       uint32_t* tile_start, unsigned long long* hit_total, int num_sms,
+                       cudaStream_t s) {
   if (q.nwin == 0) return cudaSuccess;
+  // up to eight rounds a block, as long as the blocks fill the chip four times
+  const int rounds = static_cast<int>(std::clamp<uint64_t>(
+      q.nwin / (4ull * 6 * num_sms * kProbeBlock), 1, 8));
   count_launch();
-  probe_kernel<<<grid(q.nwin, kProbeBlock), kProbeBlock, 0, s>>>(
-      idx, q, recs, nstart, cbits, fbits, tile_filt, tile_start, hit_total);
+  probe_kernel<<<grid(q.nwin, kProbeBlock * rounds), kProbeBlock, 0, s>>>(
+      idx, q, rounds, recs, nstart, cbits, fbits, tile_filt, tile_start, hit_total);
   return cudaGetLastError();
 }
 

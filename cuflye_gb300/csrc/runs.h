@@ -96,7 +96,8 @@ cudaError_t index_neighbours(const uint64_t* pos, uint64_t npos, const uint64_t*
 // (zeroed by the caller).
 cudaError_t runs_count(const DeviceIndex& idx, const QueryBatch& q, uint4* recs, uint32_t* nstart,
                        uint32_t* cbits, uint32_t* fbits, uint32_t* tile_filt,
-                       uint32_t* tile_start, unsigned long long* hit_total, cudaStream_t s);
+                       uint32_t* tile_start, unsigned long long* hit_total, int num_sms,
+                       cudaStream_t s);
 // Each query's first run and first filtered position (nq + 1 entries each);
 // totals[0] (zeroed by the caller): the most runs of a query, [1] and [2]: all
 // runs and filtered positions.

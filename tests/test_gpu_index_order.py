@@ -45,3 +45,35 @@ def test_bucket_order(gpu, oracle_mod, n, k):
     assert len(rec) > 0
     assert cand_tuples_gpu(rec) == cand_tuples_oracle(exp)
     assert filt["pos"].tolist() == exp["filtered_pos"].tolist()
+
+
+@pytest.mark.parametrize("k", [11, 15, 16, 31])
+def test_window_records_change_no_result(built_lib, k):
+    """An index built at once keeps a record a target window, one built in key
+    ranges does not: hits and rows are the same, for targets around a block of
+    windows (and shorter than a k-mer), their reverse strands, and sequences
+    that differ from the indexed ones."""
+    from cuflye_gb300 import synth
+    from cuflye_gb300.backend import CudaBackend, OverlapParams
+    rng = np.random.default_rng(100 + k)
+    genome = synth.random_genome(rng, 1200)
+    seqs = [genome[s:s + n] for s in (0, 100) for n in (k - 1, k, k + 1, 255 + k, 256 + k, 600)]
+    seqs += [synth.mutate(rng, genome, 0.02, 0.005, 0.005) for _ in range(4)]
+    targets = synth.ReadSet.from_strings(np.arange(1, len(seqs) + 1), [x.tobytes() for x in seqs])
+    other = [synth.revcomp(x) for x in seqs] + [synth.mutate(rng, x, 0.05, 0.0, 0.0) for x in seqs[-4:]]
+    ids = [-i for i in range(1, len(seqs) + 1)] + list(range(len(seqs) - 3, len(seqs) + 1))
+    queries = synth.ReadSet.from_strings(np.array(ids), [x.tobytes() for x in other])
+    p = OverlapParams.make(**dict(synth.OVERLAP_PARAMS, min_overlap=100, kmer_size=k,
+                                  only_max_ext=0))
+    got = []
+    for ranges in (False, True):
+        with CudaBackend(device=0) as be:
+            if ranges:
+                be.set_index_build_windows(3000)
+            be.build_index(targets, k, 2, 1000)
+            assert (be.last_index_ranges() > 1) == ranges
+            for q in (targets, queries):
+                cand, filt = be.candidates(q)
+                got.append((cand.tobytes(), filt.tobytes(), be.overlaps(q, p).tobytes()))
+    assert got[:2] == got[2:]
+    assert all(len(x[0]) and len(x[2]) for x in got)
