@@ -69,6 +69,11 @@ struct cuflye_ctx {
   std::string err;
   std::map<std::string, DevBuf> bufs;
   uint64_t in_use = 0, peak = 0;
+  // released buffers kept for the next allocation of about their size, oldest
+  // first: at most 1/16 of the budget (or of the device), given back when
+  // memory runs short and by cuflye_trim
+  std::vector<DevBuf> spare;
+  uint64_t spare_bytes = 0, spare_limit = 0;
   DeviceStatus* status = nullptr;
   // index
   bool has_index = false;
@@ -117,6 +122,40 @@ namespace {
 constexpr int kStages = 7;
 constexpr int kSortStats = 7;
 
+struct AllocTimer {
+  cuflye_ctx* c;
+  std::chrono::steady_clock::time_point t0 = std::chrono::steady_clock::now();
+  ~AllocTimer() {
+    c->alloc_ms +=
+        std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+  }
+};
+
+// Gives the oldest spare buffers back until at most `most` bytes are kept.
+void drop_spares(cuflye_ctx* c, uint64_t most) {
+  size_t n = 0;
+  while (n < c->spare.size() && c->spare_bytes > most) {
+    cudaFree(c->spare[n].p);
+    c->spare_bytes -= c->spare[n++].cap;
+  }
+  c->spare.erase(c->spare.begin(), c->spare.begin() + static_cast<std::ptrdiff_t>(n));
+}
+
+// A buffer out of use: kept as a spare, or freed when it is beyond the limit.
+// Whoever takes it next uses it on the context's stream (the side streams join
+// that one before a call's next step), so after what was launched on it here.
+void retire(cuflye_ctx* c, const DevBuf& b) {
+  if (!b.p) return;
+  c->in_use -= b.cap;
+  if (b.cap > c->spare_limit) {
+    cudaFree(b.p);
+    return;
+  }
+  drop_spares(c, c->spare_limit - b.cap);
+  c->spare.push_back(b);
+  c->spare_bytes += b.cap;
+}
+
 template <typename T>
 T* buf(cuflye_ctx* c, const std::string& name, uint64_t count) {
   const size_t bytes = std::max<size_t>(static_cast<size_t>(count) * sizeof(T), 16);
@@ -135,23 +174,45 @@ T* buf(cuflye_ctx* c, const std::string& name, uint64_t count) {
                       std::to_string(bytes) + " bytes; in use " + std::to_string(c->in_use) +
                       " of CUFLYE_CUDA_MEMORY_BUDGET_BYTES=" + std::to_string(c->budget));
   }
-  const size_t alloc = (c->budget && c->in_use - b.cap + want > c->budget) ? bytes : want;
-  const auto t0 = std::chrono::steady_clock::now();
-  struct AllocTimer {
-    cuflye_ctx* c;
-    std::chrono::steady_clock::time_point t0;
-    ~AllocTimer() {
-      c->alloc_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() -
-                                                               t0).count();
-    }
-  } timer{c, t0};
-  if (b.p) CUFLYE_CHECK(cudaFree(b.p));
-  c->in_use -= b.cap;
+  size_t alloc = (c->budget && c->in_use - b.cap + want > c->budget) ? bytes : want;
+  AllocTimer timer{c};
+  retire(c, b);
   b.p = nullptr;
   b.cap = 0;
+  // the smallest spare that is large enough and at most a quarter too large
+  auto best = c->spare.end();
+  for (auto it = c->spare.begin(); it != c->spare.end(); ++it)
+    if (it->cap >= alloc && it->cap - alloc <= alloc / 4 &&
+        (!c->budget || c->in_use + it->cap <= c->budget) &&
+        (best == c->spare.end() || it->cap < best->cap))
+      best = it;
+  if (best != c->spare.end()) {
+    b = *best;
+    c->spare.erase(best);
+    c->spare_bytes -= b.cap;
+    c->in_use += b.cap;
+    c->peak = std::max(c->peak, c->in_use);
+    return static_cast<T*>(b.p);
+  }
+  // a build's scratch comes in steps of a sixteenth, so that the next build's
+  // fits it
+  if (name.compare(0, 3, "ib_") == 0 && alloc >= (1u << 20)) {
+    size_t step = 1;
+    while (step * 32 <= alloc) step *= 2;
+    const size_t up = (alloc + step - 1) / step * step;
+    if (!c->budget || c->in_use + up <= c->budget) alloc = up;
+  }
+  if (c->budget && c->in_use + c->spare_bytes + alloc > c->budget)
+    drop_spares(c, c->budget - c->in_use - alloc);
   cudaError_t e = cudaMalloc(&b.p, alloc);
+  if (e == cudaErrorMemoryAllocation && !c->spare.empty()) {
+    cudaGetLastError();
+    drop_spares(c, 0);
+    e = cudaMalloc(&b.p, alloc);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
+    b.p = nullptr;
     throw Error(CUFLYE_ERR_BUDGET, "cudaMalloc of " + std::to_string(alloc) + " bytes for '" +
                                        name + "' failed: " + cudaGetErrorString(e));
   }
@@ -164,11 +225,8 @@ T* buf(cuflye_ctx* c, const std::string& name, uint64_t count) {
 void release(cuflye_ctx* c, const std::string& name) {
   auto it = c->bufs.find(name);
   if (it == c->bufs.end()) return;
-  const auto t0 = std::chrono::steady_clock::now();
-  if (it->second.p) cudaFree(it->second.p);
-  c->alloc_ms +=
-      std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-  c->in_use -= it->second.cap;
+  AllocTimer timer{c};
+  retire(c, it->second);
   c->bufs.erase(it);
 }
 
@@ -302,7 +360,7 @@ uint64_t effective_budget(cuflye_ctx* c) {
   if (c->budget) return c->budget;
   size_t free_b = 0, total_b = 0;
   CUFLYE_CHECK(cudaMemGetInfo(&free_b, &total_b));
-  const uint64_t cap = static_cast<uint64_t>(free_b) + c->in_use;
+  const uint64_t cap = static_cast<uint64_t>(free_b) + c->in_use + c->spare_bytes;
   const uint64_t margin = 8ull << 30;
   return cap > margin ? cap - margin : cap / 2;
 }
@@ -2265,6 +2323,9 @@ cuflye_status cuflye_open(int device, uint64_t memory_budget_bytes, cuflye_ctx**
     CUFLYE_CHECK(cudaSetDevice(device));
     CUFLYE_CHECK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
     CUFLYE_CHECK(cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device));
+    size_t free_b = 0, total_b = 0;
+    CUFLYE_CHECK(cudaMemGetInfo(&free_b, &total_b));
+    c->spare_limit = (c->budget ? c->budget : total_b) / 16;
     CUFLYE_CHECK(cudaMallocHost(&c->back, kBackBytes));
     CUFLYE_CHECK(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
     CUFLYE_CHECK(cudaStreamCreateWithFlags(&c->side2, cudaStreamNonBlocking));
@@ -2357,6 +2418,7 @@ void cuflye_close(cuflye_ctx* c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   for (auto& kv : c->bufs)
     if (kv.second.p) cudaFree(kv.second.p);
+  drop_spares(c, 0);
   if (c->side) cudaStreamSynchronize(c->side);
   if (c->side2) cudaStreamSynchronize(c->side2);
   for (auto& e : c->clock) cudaEventDestroy(e);
@@ -3094,6 +3156,7 @@ cuflye_status cuflye_trim(cuflye_ctx* c) {
     if (!keep) names.push_back(n);
   }
   for (const std::string& n : names) release(c, n);
+  drop_spares(c, 0);
   CUFLYE_API_END(c)
 }
 
@@ -3281,6 +3344,7 @@ cuflye_status cuflye_server_open(cuflye_ctx* owner, int workers,
   check_params(owner, params);
   if (workers < 1 || workers > 8) throw Error(CUFLYE_ERR_INVALID, "workers must be in [1, 8]");
   CUFLYE_CHECK(cudaSetDevice(owner->device));
+  drop_spares(owner, 0);
   // the workers share what is left of the budget (or of the free memory)
   uint64_t avail = 0;
   if (owner->budget) {

@@ -77,3 +77,31 @@ def test_window_records_change_no_result(built_lib, k):
                 got.append((cand.tobytes(), filt.tobytes(), be.overlaps(q, p).tobytes()))
     assert got[:2] == got[2:]
     assert all(len(x[0]) and len(x[2]) for x in got)
+
+
+@pytest.mark.parametrize("room", [0.0, 0.02, 1.0])
+def test_rebuilds_reuse_released_buffers(built_lib, room):
+    """Index builds of two sizes in turn, and batches on them, give what a fresh
+    context gives, within a budget that leaves the released buffers no room,
+    little, or enough."""
+    from cuflye_gb300 import synth
+    from cuflye_gb300.backend import CudaBackend, OverlapParams
+    cases = [synth.small_overlap_case(s, genome_len=n, coverage=8.0, sub=0.01, ins=0.002,
+                                      dele=0.002) for s, n in ((3, 60_000), (4, 90_000))]
+    fresh, peak = [], 0
+    for wl in cases:
+        with CudaBackend(device=0, memory_budget_bytes=0) as be:
+            stats = be.build_index(wl.reads, wl.k, wl.min_freq, wl.max_freq)
+            rows = be.overlaps(wl.reads, OverlapParams.make(**wl.params)).tobytes()
+            fresh.append((stats, rows))
+            peak = max(peak, be.memory_stats()[1])
+    budget = int(peak * (1 + room)) + (1 << 20)
+    with CudaBackend(device=0, memory_budget_bytes=budget) as be:
+        for i in (0, 1, 0, 1, 1, 0):
+            wl = cases[i]
+            stats = be.build_index(wl.reads, wl.k, wl.min_freq, wl.max_freq)
+            rows = be.overlaps(wl.reads, OverlapParams.make(**wl.params)).tobytes()
+            assert (stats, rows) == fresh[i]
+        assert be.memory_stats()[1] <= budget
+        be.trim()
+        assert be.overlaps(cases[0].reads, OverlapParams.make(**cases[0].params)).tobytes() == fresh[0][1]
