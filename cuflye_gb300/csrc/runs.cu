@@ -584,78 +584,55 @@ __device__ __forceinline__ int32_t agree(uint64_t qb, uint64_t tb, uint32_t soli
   return min(same, holes ? __ffs(holes) - 1 : 32);
 }
 
-constexpr int kWide = 2;  // 32-base blocks of a wide step
+constexpr int32_t kLongRoom = 96;    // room from which a run's end is looked for from there
+constexpr int32_t kBack = 24;        // windows before the expected end
 
 // Hits of the run that starts at window p of a query (first base qbase, first
 // window w0) and position pos of a target strand: the windows over which the
 // two agree, up to most, and up to the query's next window that is not solid.
-// The first 32 bases alone decide most runs of noisy reads; longer runs go on
-// 64 bases at a time, all loads issued together (a step is bound by the latency
-// of its scattered loads; 96 or 128 bases cost more registers than they gain).
+// The first 32 bases alone decide most runs of noisy reads.
+//
+// room: windows from this run's first to the first of the group's next run (or
+// up to the end of query or target when there is none).  No run starts between,
+// so the hits of this run's diagonal in there are this run's, one after the
+// other: a window of it that is a hit has nothing but hits before it.  A run
+// usually ends k windows before the next one starts (or at the sequences' end),
+// so one that outlasts its first 32 bases is taken up shortly before that place
+// if the window there is a hit: the loads of a long run, which the warp's other
+// lanes wait for, do not grow with its length (runs of 200 hits: all groups of
+// all HiFi reads 7.4 -> 4.0 ms, against 64 bases a step all the way).
 __device__ __forceinline__ int32_t run_length(const RunTables& t, uint64_t qbase, uint64_t w0,
                                               uint64_t tbase, int32_t tlen, bool rev, int32_t p,
-                                              int32_t pos, int32_t most) {
+                                              int32_t pos, int32_t most, int32_t room) {
   const int32_t k = t.idx.k;
+  // bases x .. x + 31 of the target strand
+  auto target32 = [&](int32_t x) {
+    if (!rev) return bases32(t.idx.twords, tbase + static_cast<uint64_t>(x));
+    // the reverse complement of the 32 forward bases that end before len - x
+    const int64_t s = static_cast<int64_t>(tbase) + tlen - 32 - x;
+    const uint64_t f = s >= 0 ? bases32(t.idx.twords, static_cast<uint64_t>(s))
+                              : bases32(t.idx.twords, 0) >> (2 * -s);
+    return revcomp(f, 32);
+  };
   int32_t m = 0;  // agreeing bases after the first window
   while (m < most - 1) {
-    const int32_t x = pos + k + m;
     const uint64_t q0 = qbase + static_cast<uint64_t>(p) + k + m;
     const uint64_t b = w0 + static_cast<uint64_t>(p) + 1 + m;  // the next window
     const uint32_t bs = static_cast<uint32_t>(b & 31);
-    if (m == 0 || m + 32 * kWide >= most) {
-      uint64_t tb;
-      if (!rev) {
-        tb = bases32(t.idx.twords, tbase + static_cast<uint64_t>(x));
-      } else {
-        // bases x .. x + 31 of the reverse strand: the reverse complement of
-        // the 32 forward bases that end before len - x
-        const int64_t s = static_cast<int64_t>(tbase) + tlen - 32 - x;
-        const uint64_t f = s >= 0 ? bases32(t.idx.twords, static_cast<uint64_t>(s))
-                                  : bases32(t.idx.twords, 0) >> (2 * -s);
-        tb = revcomp(f, 32);
-      }
-      const uint32_t c0 = __ldg(t.cbits + (b >> 5));
-      const uint32_t c1 = bs ? __ldg(t.cbits + (b >> 5) + 1) : 0u;
-      const int32_t step = agree(bases32(t.qb.words, q0), tb, __funnelshift_r(c0, c1, bs));
-      m += step;
-      if (step < 32) break;
-      continue;
+    const uint32_t c0 = __ldg(t.cbits + (b >> 5));
+    const uint32_t c1 = bs ? __ldg(t.cbits + (b >> 5) + 1) : 0u;
+    const int32_t step =
+        agree(bases32(t.qb.words, q0), target32(pos + k + m), __funnelshift_r(c0, c1, bs));
+    m += step;
+    if (step < 32) break;
+    if (m == 32 && room > kLongRoom) {
+      const int32_t m0 = (room < most ? room - k : most) - kBack;
+      const uint64_t d =
+          bases32(t.qb.words, qbase + static_cast<uint64_t>(p) + m0) ^ target32(pos + m0);
+      const uint64_t h = w0 + static_cast<uint64_t>(p) + m0;
+      const bool solid = __ldg(t.cbits + (h >> 5)) >> (h & 31) & 1u;
+      if (solid && (d >> (64 - 2 * k)) == 0) m = m0;
     }
-    // all 32 * kWide bases and windows lie inside query and target
-    const uint64_t s0 = rev ? tbase + static_cast<uint64_t>(tlen - 32 * kWide - x)
-                            : tbase + static_cast<uint64_t>(x);
-    const uint32_t qs = static_cast<uint32_t>(q0 & 31), ts = static_cast<uint32_t>(s0 & 31);
-    uint64_t qw[kWide + 1], tw[kWide + 1];
-    uint32_t cw[kWide + 1];
-#pragma unroll
-    for (int u = 0; u < kWide; ++u) {
-      qw[u] = __ldg(t.qb.words + (q0 >> 5) + u);
-      tw[u] = __ldg(t.idx.twords + (s0 >> 5) + u);
-      cw[u] = __ldg(t.cbits + (b >> 5) + u);
-    }
-    qw[kWide] = qs ? __ldg(t.qb.words + (q0 >> 5) + kWide) : 0;
-    tw[kWide] = ts ? __ldg(t.idx.twords + (s0 >> 5) + kWide) : 0;
-    cw[kWide] = bs ? __ldg(t.cbits + (b >> 5) + kWide) : 0;
-    int32_t got = 0;
-#pragma unroll
-    for (int u = 0; u < kWide; ++u) {
-      const uint64_t qb = qs ? (qw[u] << (2 * qs)) | (qw[u + 1] >> (64 - 2 * qs)) : qw[u];
-      const int v = rev ? kWide - 1 - u : u;  // the reverse strand's blocks come last first
-      uint64_t tb = tw[0], tn = tw[1];
-#pragma unroll
-      for (int y = 1; y < kWide; ++y) {
-        if (v == y) {
-          tb = tw[y];
-          tn = tw[y + 1];
-        }
-      }
-      if (ts) tb = (tb << (2 * ts)) | (tn >> (64 - 2 * ts));
-      if (rev) tb = revcomp(tb, 32);
-      const int32_t step = agree(qb, tb, __funnelshift_r(cw[u], cw[u + 1], bs));
-      if (got == 32 * u) got += step;
-    }
-    m += got;
-    if (got < 32 * kWide) break;
   }
   return min(m + 1, most);
 }
@@ -735,8 +712,12 @@ __global__ void __launch_bounds__(kGroupWarps * 32, 4) run_groups_kernel(RunTabl
         if (in) {
           c = static_cast<int32_t>(t.keys[gi.start + i] & 0xffffffffu);
           e = static_cast<int32_t>(t.vals[gi.start + i]);
+          const int32_t most = min(qwin - c, tlen - t.idx.k + 1 - e);
+          const int32_t room =
+              i + 1 < n ? min(static_cast<int32_t>(t.keys[gi.start + i + 1] & 0xffffffffu) - c, most)
+                        : most;
           l = run_length(t, qbase, w0, tbase, tlen, rev, c, e,
-                         min(qwin - c, tlen - t.idx.k + 1 - e));
+                         most, room);
           t.rlen[gi.start + i] = static_cast<uint32_t>(l);
           store_run_piece(t, pslot, i, es ? e : c, es ? c : e, l);
           hits += l;

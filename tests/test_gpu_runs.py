@@ -143,3 +143,34 @@ def test_query_counts_around_the_scans(gpu, oracle_mod, nq):
         np.arange(1, 31), [genome[i:i + 1000].tobytes() for i in range(0, 30_000, 1000)])
     params = dict(synth.OVERLAP_PARAMS, min_overlap=40)
     assert _check(gpu, oracle_mod, targets, reads, 15, 1, 100, params, VARIANTS[1:2]) > 0
+
+
+@pytest.mark.parametrize("k,kind", [(15, "sub"), (15, "ins"), (15, "del"), (31, "sub"), (17, "hole")])
+def test_run_ends_around_the_expected_place(gpu, oracle_mod, k, kind):
+    """Long runs that end at every distance from the group's next run: a second
+    error (or a stretch of repetitive k-mers) at each offset from the first."""
+    from cuflye_gb300 import synth
+    rng = np.random.default_rng(k)
+    target = synth.random_genome(rng, 700)
+    unit = synth.random_genome(rng, 25)
+    filler = [np.concatenate([synth.random_genome(rng, 30), unit] * 8)] if kind == "hole" else []
+    queries = []
+    for d in range(0, 90):
+        s = target.copy()
+        s[250] = ord("ACGT"["TGCA".index(chr(s[250]))])
+        if kind == "sub" and d:
+            s[250 + d] = ord("ACGT"["TGCA".index(chr(s[250 + d]))])
+        elif kind == "ins":
+            s = np.insert(s, 250 - d, s[250 - d])
+        elif kind == "del":
+            s = np.delete(s, 250 + d)
+        elif kind == "hole":
+            s[200 - d:225 - d] = unit
+        queries.append(s if d % 2 else synth.revcomp(s))
+    targets = [target] + filler
+    if kind == "hole":
+        targets.append(queries[7])  # shares the stretch, at one place
+    t = synth.ReadSet.from_strings(np.arange(1, len(targets) + 1), [x.tobytes() for x in targets])
+    q = synth.ReadSet.from_strings(np.arange(50, 50 + len(queries)), [x.tobytes() for x in queries])
+    params = dict(synth.OVERLAP_PARAMS, min_overlap=100)
+    assert _check(gpu, oracle_mod, t, q, k, 1, 6, params, VARIANTS[:2]) >= len(queries)
