@@ -1316,7 +1316,7 @@ SortTasks sort_tasks(cuflye_ctx* c, const std::string& prefix, uint64_t nelems, 
               segsort_pair_reserve(nelems),
               nelems,
               {buf<uint8_t>(c, prefix + "_r0", rb), buf<uint8_t>(c, prefix + "_r1", rb)},
-              buf<uint32_t>(c, prefix + "_rc", 2 * (kSortRounds + 1)),
+              buf<uint32_t>(c, prefix + "_rc", kSortRoundWords),
               c->shape.round_blocks_per_sm};
   t.side = c->side;
   t.side2 = c->side2;

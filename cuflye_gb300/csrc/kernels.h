@@ -32,6 +32,8 @@ size_t segsort_smem_bytes();
 constexpr uint32_t kHeapPackCap = 57344;
 // Rounds of the global phase (partitions of ranges beyond shared memory).
 constexpr int kSortRounds = 64;
+// words of the rounds' counters: two lists a round, their sizes and claims
+constexpr int kSortRoundWords = 4 * (kSortRounds + 1);
 constexpr size_t kRoundItemBytes = 40;  // one range of a global-phase round
 struct SortTasks {
   uint64_t* f;
@@ -41,7 +43,7 @@ struct SortTasks {
   uint32_t pair_reserve;  // top entries kept for heap ranges beyond kHeapPackCap
   uint64_t nelems;        // elements of the call at most (no global phase up to 4,096)
   void* round[2];         // two round lists of segsort_round_bytes(nelems) each
-  uint32_t* round_counts;  // 2 * (kSortRounds + 1) words
+  uint32_t* round_counts;  // kSortRoundWords words
   int round_per_sm = 0;    // blocks per SM of the global phase (1-2; 0: 2)
   // Pruning (optional): segment s's keys that may repeat, sorted, are
   // prune_keys[prune_off[s] .. prune_off[s + 1]).  A global-phase range whose

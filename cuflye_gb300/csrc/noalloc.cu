@@ -55,7 +55,7 @@ constexpr size_t kRoundBytes = (kMaxElems / 4096 + 1) * kRoundItemBytes;  // seg
 constexpr size_t kOffR0 = align256(kOffTd + 4 * kTaskCap);
 constexpr size_t kOffR1 = align256(kOffR0 + kRoundBytes);
 constexpr size_t kOffRc = align256(kOffR1 + kRoundBytes);
-constexpr size_t kScratchBytes = align256(kOffRc + 4 * 2 * (kSortRounds + 1));
+constexpr size_t kScratchBytes = align256(kOffRc + 4 * kSortRoundWords);
 
 constexpr int kMaxDevices = 64;
 std::mutex g_mu;

@@ -10,8 +10,9 @@
 //                             16 warps partition different tasks concurrently
 //                             (level by level), then one thread per leaf task;
 //   * larger:                 partitions in global memory, in rounds over all
-//                             such ranges (one CTA per range), until the ranges
-//                             fit kCap; each is then finished in shared memory.
+//                             such ranges (one CTA per range, a cluster of CTAs
+//                             for the longest), until the ranges fit kCap;
+//                             each is then finished in shared memory.
 // Every partition is a single pass: L stoppers get ranks from the left, R
 // stoppers left ranks too (the k-th R stopper from the right is the
 // (TR - k)-th from the left), so a partition reads its keys once.
@@ -673,8 +674,9 @@ __global__ void __launch_bounds__(kBlock, 3) sort_cta(uint64_t* K, uint32_t* V,
 // ---------------------------------------------------------------- large segments
 //
 // Global phase, in rounds: each launch partitions every range of its round's
-// list (ranges longer than kCap with recursion budget left) in global memory
-// (round_partition), one CTA per range, CTAs taking ranges from a counter.
+// lists (ranges longer than kCap with recursion budget left) in global memory:
+// ranges longer than kWide by a cluster of CTAs each (cluster_partition), the
+// others by one CTA each (round_partition), taken from counters.
 // Children longer than kCap with budget left go to the next round's list,
 // shorter ones to the task list that sort_tasks finishes in shared memory,
 // and children whose budget ran out to the heap lists.  A range's partition
@@ -683,6 +685,8 @@ __global__ void __launch_bounds__(kBlock, 3) sort_cta(uint64_t* K, uint32_t* V,
 
 constexpr int kBigBlock = 512;
 constexpr int kBigPerSm = 2;
+constexpr int kCluster = 8;
+constexpr uint32_t kWide = 16384;
 
 // A range of a round: its elements [f, f + n), depth budget d, segment seg,
 // and the key interval [lo, hi] its elements lie in (the pivots above it).
@@ -716,9 +720,20 @@ __device__ __forceinline__ bool holds_listed_key(const PruneLists& pl, uint32_t 
   return a < pl.off[seg + 1] && pl.keys[a] <= hi;
 }
 
+// Lists a range for the next round: ranges for one CTA from the bottom of out,
+// for a cluster from the top; out_count holds how many of each.
+__device__ __forceinline__ void append_range(const RoundItem& r, RoundItem* out,
+                                             uint32_t* out_count, uint32_t out_cap) {
+  if (r.n > kWide)
+    out[out_cap - 1u - atomicAdd(out_count + 1, 1u)] = r;
+  else
+    out[atomicAdd(out_count, 1u)] = r;
+}
+
 // Where a child range of a global-phase partition goes.
 __device__ __forceinline__ void place_range(const RoundItem& r, RoundItem* out,
-                                            uint32_t* out_count, uint64_t* task_f,
+                                            uint32_t* out_count, uint32_t out_cap,
+                                            uint64_t* task_f,
                                             uint32_t* task_n, int* task_d, uint32_t* task_count,
                                             uint32_t* heap_count, uint32_t* pair_count,
                                             uint32_t task_cap, uint32_t pair_reserve,
@@ -745,31 +760,201 @@ __device__ __forceinline__ void place_range(const RoundItem& r, RoundItem* out,
     task_n[slot] = n;
     task_d[slot] = 0;
   } else {
-    out[atomicAdd(out_count, 1u)] = r;
+    append_range(r, out, out_count, out_cap);
   }
 }
 
-// The round-0 list: the segments longer than kCap with libstdc++'s budget.
+// The round-0 lists: the segments longer than kCap with libstdc++'s budget.
 __global__ void round_seed(const uint64_t* __restrict__ begin, const uint64_t* __restrict__ end,
                            const uint32_t* __restrict__ list, const uint32_t* __restrict__ counts,
-                           RoundItem* __restrict__ out) {
+                           RoundItem* __restrict__ out, uint32_t* out_count,
+                           uint32_t out_cap) {
   const uint32_t cnt = counts[3];
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x) {
     const uint32_t s = list[i];
     const uint32_t n = static_cast<uint32_t>(end[s] - begin[s]);
-    out[i] = RoundItem{begin[s], 0ull, ~0ull, n, isort::depth_limit(n), s, 0u};
+    append_range(RoundItem{begin[s], 0ull, ~0ull, n, isort::depth_limit(n), s, 0u}, out, out_count,
+                 out_cap);
   }
 }
 
-__global__ void __launch_bounds__(kBigBlock, kBigPerSm)
+// A range's partition by a cluster of CTAs, each a slice of it: every CTA ranks
+// its slice's stoppers as round_partition does its tiles' (maps in the slice's
+// own index range), the slices' counts meet in shared memory, and the CTAs
+// share the swaps.  A range of n elements takes one CTA n / 4096 steps in a
+// row: for the first ranges of a long segment that chain was the whole round.
+struct ClusterScratch {
+  uint32_t count[2];                     // this slice's stoppers
+  uint32_t upto[2][kCluster + 1];        // stoppers before each slice
+};
+
+__device__ __forceinline__ uint32_t kth_stopper(const uint32_t* map, const uint32_t* upto,
+                                                uint32_t slice, uint32_t k) {
+  // the k-th (from 0) of all slices
+  uint32_t c = 0;
+#pragma unroll
+  for (int x = 1; x < kCluster; ++x) c += upto[x] <= k;
+  return map[c * slice + (k - upto[c])];
+}
+
+__device__ uint32_t cluster_partition(cooperative_groups::cluster_group cluster, uint64_t* K,
+                                      uint32_t* V, uint32_t* Lr, uint32_t* Rr, uint32_t n,
+                                      RoundScratch<kBigBlock, 8>& rs, ClusterScratch& cs) {
+  using RS = RoundScratch<kBigBlock, 8>;
+  constexpr int kW = RS::kW, kRounds = RS::kR;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const unsigned lt = (1u << lane) - 1u;
+  const uint32_t rank = cluster.block_rank();
+  if (rank == 0 && t == 0) isort::median_to_first(K, V, 0, 1, n / 2, n - 1);
+  cluster.sync();
+  const uint64_t p = K[0];
+  const uint32_t slice = ((n + kCluster - 1) / kCluster + 31) / 32 * 32;
+  const uint32_t f = min(rank * slice, n), l = min(f + slice, n);
+  uint32_t nl = 0, nr = 0;
+  for (uint32_t t0 = f; t0 < l; t0 += kBigBlock * kRounds) {
+    uint64_t k[kRounds];
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+      const uint32_t i = t0 + r * kBigBlock + t;
+      k[r] = i < l ? K[i] : 0;
+    }
+    unsigned bl[kRounds], br[kRounds];
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+      const uint32_t i = t0 + r * kBigBlock + t;
+      bl[r] = __ballot_sync(0xffffffffu, i < l && i > 0 && !(k[r] < p));
+      br[r] = __ballot_sync(0xffffffffu, i < l && !(p < k[r]));
+      if (lane == 0) {
+        rs.cl[r * kW + warp] = __popc(bl[r]);
+        rs.cr[r * kW + warp] = __popc(br[r]);
+      }
+    }
+    __syncthreads();
+    round_scan(rs);
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+      const uint32_t i = t0 + r * kBigBlock + t;
+      if ((bl[r] >> lane) & 1u) Lr[f + nl + rs.cl[r * kW + warp] + __popc(bl[r] & lt)] = i;
+      if ((br[r] >> lane) & 1u) Rr[f + nr + rs.cr[r * kW + warp] + __popc(br[r] & lt)] = i;
+    }
+    nl += rs.tot[0];
+    nr += rs.tot[1];
+    __syncthreads();
+  }
+  if (t == 0) {
+    cs.count[0] = nl;
+    cs.count[1] = nr;
+  }
+  cluster.sync();
+  if (t < 2) {
+    uint32_t s = 0;
+    for (int c = 0; c < kCluster; ++c) {
+      cs.upto[t][c] = s;
+      s += *cluster.map_shared_rank(&cs.count[t], c);
+    }
+    cs.upto[t][kCluster] = s;
+  }
+  __syncthreads();
+  const uint32_t tl = cs.upto[0][kCluster], tr = cs.upto[1][kCluster];
+  auto left = [&](uint32_t k) { return kth_stopper(Lr, cs.upto[0], slice, k); };
+  auto right = [&](uint32_t k) { return kth_stopper(Rr, cs.upto[1], slice, k); };
+  if (warp == 0) {  // round_partition's search for the last swap, in every CTA
+    uint32_t lo = 0, hi = tl < tr ? tl : tr;
+    while (lo < hi) {
+      const uint32_t step = (hi - lo + 31) / 32;
+      const uint32_t k = lo + (lane + 1) * step;
+      const bool ok = k <= hi && left(k - 1) < right(tr - k);
+      const unsigned mask = __ballot_sync(0xffffffffu, ok);
+      if (mask == 0) {
+        hi = lo + step - 1;
+      } else {
+        const uint32_t nlo = lo + (32u - __clz(mask)) * step;
+        hi = (nlo + step - 1 < hi) ? nlo + step - 1 : hi;
+        lo = nlo;
+      }
+    }
+    if (lane == 0) {
+      const uint32_t m = lo;
+      uint32_t cut = m ? right(tr - m) : left(0);
+      if (m && m + 1 <= tl) cut = min(cut, left(m));
+      rs.scalar[0] = m;
+      rs.scalar[1] = cut;
+    }
+  }
+  __syncthreads();
+  const uint32_t m = rs.scalar[0], cut = rs.scalar[1];
+  for (uint32_t q0 = 1 + rank * kBigBlock + t; q0 <= m; q0 += 4 * kCluster * kBigBlock) {
+    uint32_t a[4], b[4];
+    uint64_t ka[4], kb[4];
+    uint32_t va[4], vb[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const uint32_t q = q0 + u * kCluster * kBigBlock;
+      if (q <= m) {
+        a[u] = left(q - 1);
+        b[u] = right(tr - q);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (q0 + u * kCluster * kBigBlock <= m) {
+        ka[u] = K[a[u]];
+        kb[u] = K[b[u]];
+        va[u] = V[a[u]];
+        vb[u] = V[b[u]];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (q0 + u * kCluster * kBigBlock <= m) {
+        K[a[u]] = kb[u];
+        K[b[u]] = ka[u];
+        V[a[u]] = vb[u];
+        V[b[u]] = va[u];
+      }
+    }
+  }
+  return cut;
+}
+
+__global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kBigBlock, kBigPerSm)
     sort_round(uint64_t* K, uint32_t* V, uint32_t* Lg, uint32_t* Rg,
                const RoundItem* __restrict__ in, const uint32_t* __restrict__ in_count,
-               uint32_t* work, RoundItem* out, uint32_t* out_count, uint64_t* task_f,
-               uint32_t* task_n, int* task_d, uint32_t* task_count, uint32_t* heap_count,
-               uint32_t* pair_count, uint32_t task_cap, uint32_t pair_reserve, PruneLists pl) {
+               uint32_t list_cap, uint32_t* work, RoundItem* out, uint32_t* out_count,
+               uint64_t* task_f, uint32_t* task_n, int* task_d, uint32_t* task_count,
+               uint32_t* heap_count, uint32_t* pair_count, uint32_t task_cap,
+               uint32_t pair_reserve, PruneLists pl) {
   __shared__ RoundScratch<kBigBlock, 8> rs;
+  __shared__ ClusterScratch cs;
   __shared__ uint32_t item;
-  const uint32_t cnt = *in_count;
+  // the pivot stays at the range's first slot: the left part holds keys <= it,
+  // the right part keys >= it
+  auto place = [&](const RoundItem& r, uint32_t cut) {
+    const uint64_t p = K[r.f];
+    const RoundItem left{r.f, r.lo, p, cut, r.d - 1, r.seg, 0u};
+    const RoundItem right{r.f + cut, p, r.hi, r.n - cut, r.d - 1, r.seg, 0u};
+    place_range(left, out, out_count, list_cap, task_f, task_n, task_d, task_count, heap_count,
+                pair_count, task_cap, pair_reserve, pl);
+    place_range(right, out, out_count, list_cap, task_f, task_n, task_d, task_count, heap_count,
+                pair_count, task_cap, pair_reserve, pl);
+  };
+  const uint32_t wide = in_count[1];
+  if (wide) {
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    for (;;) {
+      if (cluster.block_rank() == 0 && threadIdx.x == 0) item = atomicAdd(work + 1, 1u);
+      cluster.sync();
+      const uint32_t i = *cluster.map_shared_rank(&item, 0);
+      if (i >= wide) break;
+      const RoundItem r = in[list_cap - 1u - i];
+      const uint32_t cut =
+          cluster_partition(cluster, K + r.f, V + r.f, Lg + r.f, Rg + r.f, r.n, rs, cs);
+      if (cluster.block_rank() == 0 && threadIdx.x == 0) place(r, cut);
+      __syncthreads();
+    }
+    cluster.sync();  // the first CTA's item is read: it may go on and end
+  }
+  const uint32_t cnt = in_count[0];
   for (;;) {
     if (threadIdx.x == 0) item = atomicAdd(work, 1u);
     __syncthreads();
@@ -780,17 +965,7 @@ __global__ void __launch_bounds__(kBigBlock, kBigPerSm)
     // rank maps share the range's index range
     const uint32_t cut =
         round_partition<kBigBlock, uint32_t>(K + r.f, V + r.f, Lg + r.f, Rg + r.f, 0, r.n, rs);
-    if (threadIdx.x == 0) {
-      // the pivot stays at the range's first slot: the left part holds keys
-      // <= it, the right part keys >= it
-      const uint64_t p = K[r.f];
-      const RoundItem left{r.f, r.lo, p, cut, r.d - 1, r.seg, 0u};
-      const RoundItem right{r.f + cut, p, r.hi, r.n - cut, r.d - 1, r.seg, 0u};
-      place_range(left, out, out_count, task_f, task_n, task_d, task_count, heap_count,
-                  pair_count, task_cap, pair_reserve, pl);
-      place_range(right, out, out_count, task_f, task_n, task_d, task_count, heap_count,
-                  pair_count, task_cap, pair_reserve, pl);
-    }
+    if (threadIdx.x == 0) place(r, cut);
     __syncthreads();
   }
 }
@@ -1497,29 +1672,31 @@ cudaError_t segmented_std_sort(uint64_t* keys, uint32_t* vals, uint32_t* lscratc
     // runs out by round 62)
     RoundItem* rl[2] = {static_cast<RoundItem*>(tasks.round[0]),
                         static_cast<RoundItem*>(tasks.round[1])};
-    uint32_t* rcount = tasks.round_counts;                  // list size of round r
-    uint32_t* rwork = tasks.round_counts + kSortRounds + 1;  // claims of round r
-    cudaMemsetAsync(tasks.round_counts, 0, 2 * (kSortRounds + 1) * sizeof(uint32_t), stream);
+    uint32_t* rcount = tasks.round_counts;                        // two list sizes a round
+    uint32_t* rwork = tasks.round_counts + 2 * (kSortRounds + 1);  // and their claims
+    const uint32_t list_cap = static_cast<uint32_t>(tasks.nelems / kCap + 1);
+    cudaMemsetAsync(tasks.round_counts, 0, kSortRoundWords * sizeof(uint32_t), stream);
     count_launch();
     round_seed<<<std::min((nseg + 255) / 256, 1024u), 256, 0, stream>>>(
-        begin, end, lists + 3 * static_cast<size_t>(nseg), counts, rl[0]);
+        begin, end, lists + 3 * static_cast<size_t>(nseg), counts, rl[0], rcount, list_cap);
     // blocks claim ranges from a counter: the grid (round_per_sm blocks per
     // SM, 1-2) changes no result
     const int round_blocks =
         tasks.round_per_sm > 0 ? std::min(tasks.round_per_sm, kBigPerSm) : kBigPerSm;
+    const int round_grid = (num_sms * round_blocks + kCluster - 1) / kCluster * kCluster;
     for (int r = 0; r < kSortRounds; ++r) {
       count_launch();
-      sort_round<<<num_sms * round_blocks, kBigBlock, 0, stream>>>(
-          keys, vals, lscratch, rscratch, rl[r & 1], r == 0 ? counts + 3 : rcount + r, rwork + r,
-          rl[(r + 1) & 1], rcount + r + 1, tasks.f, tasks.n, tasks.d, counts + 4, counts + 5,
+      sort_round<<<round_grid, kBigBlock, 0, stream>>>(
+          keys, vals, lscratch, rscratch, rl[r & 1], rcount + 2 * r, list_cap, rwork + 2 * r,
+          rl[(r + 1) & 1], rcount + 2 * (r + 1), tasks.f, tasks.n, tasks.d, counts + 4, counts + 5,
           counts + 7, tasks.cap, tasks.pair_reserve, PruneLists{tasks.prune_keys, tasks.prune_off});
       if (((r + 1) & r) == 0) {
-        uint32_t next = 0;
-        cudaError_t e = cudaMemcpyAsync(&next, rcount + r + 1, sizeof(next),
+        uint32_t next[2] = {0, 0};
+        cudaError_t e = cudaMemcpyAsync(next, rcount + 2 * (r + 1), sizeof(next),
                                         cudaMemcpyDeviceToHost, stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) return e;
-        if (next == 0) break;
+        if (next[0] == 0 && next[1] == 0) break;
       }
     }
   }
