@@ -37,6 +37,12 @@ constexpr uint32_t kCap = 4096;       // CTA shared-memory segment capacity
 constexpr uint32_t kWarpMax = 512;    // tasks up to this size become warp subtrees
 constexpr uint32_t kTiny = 64;        // segments up to this size: thread kernel
 constexpr uint32_t kWarpSeg = 2048;   // segments up to this size: warp kernel
+// One warp sorts 2048 elements in 220 us, a CTA in 50.  Few segments (at most
+// kFewPerSm an SM), or few long ones (a mean of at most kFewMean), leave the CTA
+// kernel idle while the warps' longest is the call: CTAs take them from
+// kWarpSegFew on.  30 segments of 1000: .44 -> .20 ms; 2000 of 500: .75 -> .50;
+// 611 of 3273, whose CTAs are busy, stay as they are (.84; .89 with kWarpSegFew).
+constexpr uint32_t kFewPerSm = 2, kFewMean = 1024, kWarpSegFew = 512;
 constexpr int kWarpSegWarps = 6;      // warps per CTA in the warp kernel
 constexpr int kMaxWarpTasks = 256;    // warp subtrees per CTA task (<= 2 per partition)
 
@@ -588,8 +594,8 @@ __device__ void cta_load_sort_store(uint64_t* K, uint32_t* V, uint64_t begin, ui
 
 __global__ void classify_segments(const uint64_t* __restrict__ begin,
                                   const uint64_t* __restrict__ end, uint32_t nseg,
-                                  const uint32_t* __restrict__ nseg_dev, uint32_t* lists,
-                                  uint32_t* counts) {
+                                  const uint32_t* __restrict__ nseg_dev, uint32_t warp_max,
+                                  uint32_t* lists, uint32_t* counts) {
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nseg || (nseg_dev && s >= *nseg_dev)) return;
   const uint64_t n = end[s] - begin[s];
@@ -597,7 +603,7 @@ __global__ void classify_segments(const uint64_t* __restrict__ begin,
   int c;
   if (n <= kTiny)
     c = 0;
-  else if (n <= kWarpSeg)
+  else if (n <= warp_max)
     c = 1;
   else if (n <= kCap)
     c = 2;
@@ -627,7 +633,7 @@ struct WarpSlice {
   LeafBuf leaves;
 };
 
-// One warp per segment of (kTiny, kWarpSeg] elements.
+// One warp per segment of up to kWarpSeg elements.
 __global__ void __launch_bounds__(kWarpSegWarps * 32) sort_warp(
     uint64_t* K, uint32_t* V, const uint64_t* __restrict__ begin,
     const uint64_t* __restrict__ end, const uint32_t* __restrict__ list,
@@ -1650,11 +1656,14 @@ cudaError_t segmented_std_sort(uint64_t* keys, uint32_t* vals, uint32_t* lscratc
   cudaStream_t side2 = split ? tasks.side2 : stream;
   cudaMemsetAsync(counts, 0, 10 * sizeof(uint32_t), stream);
   count_launch();
-  classify_segments<<<(nseg + 255) / 256, 256, 0, stream>>>(begin, end, nseg, nseg_dev, lists,
-                                                            counts);
+  const bool few = nseg <= kFewPerSm * static_cast<uint32_t>(num_sms) ||
+                   tasks.nelems <= static_cast<uint64_t>(kFewMean) * nseg;
+  classify_segments<<<(nseg + 255) / 256, 256, 0, stream>>>(
+      begin, end, nseg, nseg_dev, few ? kWarpSegFew : kWarpSeg, lists, counts);
   if (split) {
     cudaError_t e = cudaEventRecord(tasks.fork, stream);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(side, tasks.fork, 0);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(side2, tasks.fork, 0);
     if (e != cudaSuccess) return e;
   }
   count_launch();
@@ -1663,7 +1672,7 @@ cudaError_t segmented_std_sort(uint64_t* keys, uint32_t* vals, uint32_t* lscratc
   sort_warp<<<num_sms, kWarpSegWarps * 32, sizeof(WarpSlice) * kWarpSegWarps, side>>>(
       keys, vals, begin, end, lists + nseg, counts);
   count_launch();
-  sort_cta<<<num_sms * 3, kBlock, sizeof(CtaSmem), side>>>(keys, vals, begin, end,
+  sort_cta<<<num_sms * 3, kBlock, sizeof(CtaSmem), side2>>>(keys, vals, begin, end,
                                                        lists + 2 * static_cast<size_t>(nseg),
                                                        counts);
   if (tasks.nelems > kCap) {
