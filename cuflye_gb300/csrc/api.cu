@@ -521,8 +521,8 @@ BuiltIndex build_one_range(cuflye_ctx* c, const WindowSet& w, const std::vector<
                             bi.windows ? r.free_run_words : nullptr, bi.nbr));
   if (bi.windows)
     CUFLYE_CHECK(index_window_records(r.vals, r.run_id, r.run_start, r.kept_off, r.cls,
-                                      r.free_run_words, place, w.nwin, bi.win_off, w.slot_len, w.k,
-                                      bi.windows, st));
+                                      r.free_run_words, place, w.nwin, bi.nbr, bi.win_off,
+                                      w.slot_len, w.k, bi.windows, st));
   check_device_status(c);
   bi.npos = r.npos;
   bi.nsolid = r.nsolid;

@@ -224,6 +224,7 @@ __global__ void window_records_kernel(const uint64_t* __restrict__ vals,
                                       const uint8_t* __restrict__ sides,
                                       const uint32_t* __restrict__ others,
                                       const uint32_t* __restrict__ place, uint64_t n,
+                                      const uint8_t* __restrict__ nbr,
                                       const uint64_t* __restrict__ win_off,
                                       const int32_t* __restrict__ slot_len, int k,
                                       uint4* __restrict__ windows) {
@@ -231,6 +232,7 @@ __global__ void window_records_kernel(const uint64_t* __restrict__ vals,
   if (i >= n) return;
   const uint64_t r = run_of(flags_scan, run_start, i);
   const uint64_t m = meta[r], v = vals[i];
+  const uint32_t sid = static_cast<uint32_t>(v >> 32);
   uint4 rec = make_uint4(0, 0, 0, 0);
   if (m != kNoMeta) {
     rec.x = static_cast<uint32_t>(m);
@@ -239,10 +241,15 @@ __global__ void window_records_kernel(const uint64_t* __restrict__ vals,
     if (!(m & kRepetitiveBit)) {
       rec.z = place[i] | static_cast<uint32_t>(sides[r]) << kCountBits;
       rec.w |= others[r];
+      if (nbr) {
+        uint32_t x = nbr[(m & kOffsetMask) + place[i]];  // of the entry's strand
+        if (sid & 1u) x = (~x << 4 & 0x30u) | (~x >> 4 & 3u);
+        rec.z |= (x & 3u) << 28 | (x & 0x30u) << 26;
+      }
     }
   }
+  if (sid & 1u) rec.w |= kWindowRev;
   // the window this entry came from: its forward position in its target
-  const uint32_t sid = static_cast<uint32_t>(v >> 32);
   const uint32_t slot = sid >> 1;
   const int64_t sp = static_cast<int64_t>(v & 0xffffffffu);
   const int64_t p = (sid & 1u) ? static_cast<int64_t>(slot_len[slot]) - sp - k : sp;
@@ -492,13 +499,13 @@ cudaError_t index_insert(const uint64_t* keys, const uint64_t* pos, const uint64
 cudaError_t index_window_records(const uint64_t* vals, const uint64_t* run_id,
                                  const uint64_t* run_start, const uint64_t* meta,
                                  const uint8_t* sides, const uint32_t* others,
-                                 const uint32_t* place, uint64_t n, const uint64_t* win_off,
-                                 const int32_t* slot_len, int k, uint4* windows,
-                                 cudaStream_t s) {
+                                 const uint32_t* place, uint64_t n, const uint8_t* nbr,
+                                 const uint64_t* win_off, const int32_t* slot_len, int k,
+                                 uint4* windows, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
   count_launch();
   window_records_kernel<<<grid(n, 256), 256, 0, s>>>(vals, run_id, run_start, meta, sides, others,
-                                                     place, n, win_off, slot_len, k, windows);
+                                                     place, n, nbr, win_off, slot_len, k, windows);
   return cudaGetLastError();
 }
 

@@ -111,8 +111,10 @@ struct DeviceIndex {
   // targets (slot order, win_off per slot) its k-mer's table word (x, y), its
   // own entry's place in the bucket (z, low kCountBits bits) with what most of
   // the bucket's entries have before and after the k-mer (3 bits each, a nibble
-  // of nbr; 7: not known), and whether the table holds the k-mer (w, bit 31)
-  // with how many entries have something else before (bits 0-11) and after
+  // of nbr; 7: not known) and the bases around the window itself (z, bits 28-29
+  // and 30-31; of solid windows, not those off the target's ends), and whether
+  // the table holds the k-mer (w, bit 31) and in its reverse form (bit 30), with
+  // how many entries have something else before (w, bits 0-11) and after
   // (16-27).
   // A query that is an indexed target reads its windows' records in a row
   // where a table probe is a scattered load, and most of their neighbours too
@@ -174,13 +176,13 @@ cudaError_t index_insert(const uint64_t* keys, const uint64_t* pos, const uint64
 // run: it takes the counts of others, and kept_off and cls then hold the run's
 // table word, kNoMeta for none, and sides).
 constexpr uint64_t kNoMeta = ~0ull;
-constexpr uint32_t kWindowFound = 1u << 31;
+constexpr uint32_t kWindowFound = 1u << 31, kWindowRev = 1u << 30;
 cudaError_t index_window_records(const uint64_t* vals, const uint64_t* run_id,
                                  const uint64_t* run_start, const uint64_t* meta,
                                  const uint8_t* sides, const uint32_t* others,
-                                 const uint32_t* place, uint64_t n, const uint64_t* win_off,
-                                 const int32_t* slot_len, int k, uint4* windows,
-                                 cudaStream_t s);
+                                 const uint32_t* place, uint64_t n, const uint8_t* nbr,
+                                 const uint64_t* win_off, const int32_t* slot_len, int k,
+                                 uint4* windows, cudaStream_t s);
 // Per key prefix (key >> shift) of sorted runs: solid positions into
 // npos_bin, solid and repetitive runs into nent_bin (both accumulate).
 cudaError_t index_bin_totals(const uint64_t* keys, const uint64_t* run_start, const uint8_t* cls,

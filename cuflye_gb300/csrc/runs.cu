@@ -147,6 +147,10 @@ struct BucketSide {
   uint32_t most, others;
 };
 
+__device__ __forceinline__ BucketSide record_side(const uint4& rec, bool rev) {
+  return BucketSide{rec.z >> (kCountBits + (rev ? 3 : 0)) & 7u, rec.w >> (rev ? 16 : 0) & 0xfffu};
+}
+
 // A window's table word, its own entry's place in the bucket, the bucket's side
 // and the flags.
 __device__ __forceinline__ uint8_t probe_run_window(const DeviceIndex& idx, const QueryBatch& q,
@@ -167,8 +171,7 @@ __device__ __forceinline__ uint8_t probe_run_window(const DeviceIndex& idx, cons
   fl |= kWinSolid;
   if (recorded) {
     self = rec.z & kPlaceMask;
-    side.most = rec.z >> (kCountBits + (km.rev ? 3 : 0)) & 7u;
-    side.others = rec.w >> (km.rev ? 16 : 0) & 0xfffu;
+    side = record_side(rec, km.rev);
   } else if (own) {
     self = bucket_find(idx, meta & kOffsetMask, bucket_size(meta),
                        self_entry(idx, qdi, p, km.rev));
@@ -186,6 +189,41 @@ __device__ __forceinline__ uint32_t own_before(const DeviceIndex& idx, int32_t q
   const int64_t after = f + idx.k;
   return after < idx.slot_len[slot]
              ? 3u - base_at(idx.twords, b + static_cast<uint64_t>(after)) : 4u;
+}
+
+// Bases x .. x + 31 of a target strand (first base tbase, tlen bases).
+__device__ __forceinline__ uint64_t target_bases32(const uint64_t* __restrict__ words,
+                                                   uint64_t tbase, int32_t tlen, bool rev,
+                                                   int32_t x) {
+  if (!rev) return bases32(words, tbase + static_cast<uint64_t>(x));
+  // the reverse complement of the 32 forward bases that end before len - x
+  const int64_t s = static_cast<int64_t>(tbase) + tlen - 32 - x;
+  const uint64_t f = s >= 0 ? bases32(words, static_cast<uint64_t>(s))
+                            : bases32(words, 0) >> (2 * -s);
+  return revcomp(f, 32);
+}
+
+// Whether windows [w0, w1) of query qi (and the one before) are those of the
+// indexed target of its id, base for base (called by the whole block).  Their
+// records then tell all that a probe would, strand and neighbours included.
+__device__ __forceinline__ bool indexed_windows(const DeviceIndex& idx, const QueryBatch& q,
+                                                uint32_t qi, uint64_t w0, uint64_t w1) {
+  const int32_t qdi = q.qdi[qi];
+  bool differ = true;
+  if (idx.windows && idx.twords && qdi >= 0) {
+    const uint32_t slot = static_cast<uint32_t>(qdi) >> 1;
+    const int32_t len = idx.slot_len[slot];
+    const int64_t p0 = static_cast<int64_t>(w0 - q.win_off[qi]);
+    const int64_t b0 = p0 > 0 ? p0 - 1 : 0, b1 = static_cast<int64_t>(w1 - q.win_off[qi]) + idx.k - 1;
+    differ = b1 > len;
+    for (int64_t x = b0 + 32 * threadIdx.x; !differ && x < b1; x += 32 * blockDim.x) {
+      const uint64_t d = bases32(q.words, q.base_off[qi] + static_cast<uint64_t>(x)) ^
+                         target_bases32(idx.twords, idx.tbase[slot], len, qdi & 1,
+                                        static_cast<int32_t>(x));
+      differ = (b1 - x < 32 ? d >> (64 - 2 * (b1 - x)) : d) != 0;
+    }
+  }
+  return !__syncthreads_or(differ);
 }
 
 constexpr int kProbeBlock = 256;
@@ -212,13 +250,45 @@ __global__ void __launch_bounds__(kProbeBlock, 6) probe_kernel(
   }
   __syncthreads();
   uint32_t lo = ends[0], block_hits = 0;
+  const bool indexed = ends[0] == ends[1] && indexed_windows(idx, q, lo, w0, w1);
+  const uint4* row = nullptr;  // records of the query's target
+  int64_t last = 0;            // the target's last window, for a query that is its reverse
+  bool back = false;
+  if (indexed) {
+    const int32_t qdi = q.qdi[lo];
+    row = idx.windows + idx.win_off[static_cast<uint32_t>(qdi) >> 1];
+    last = static_cast<int64_t>(idx.slot_len[static_cast<uint32_t>(qdi) >> 1]) - idx.k;
+    back = qdi & 1;
+  }
+  const uint64_t q0 = q.win_off[lo];
   for (uint64_t b0 = w0; b0 < w1; b0 += kProbeBlock) {
     const uint64_t w = b0 + threadIdx.x;
     uint64_t meta = 0, p = 0;
     uint32_t self = kNoSelf, left = 7;
     BucketSide side{7, 0};
     uint8_t fl = 0;
-    if (w < w1) {
+    if (w < w1 && indexed) {
+      p = w - q0;
+      const uint4* at = row + (back ? last - static_cast<int64_t>(p) : static_cast<int64_t>(p));
+      const uint4 rec = __ldg(at);
+      meta = static_cast<uint64_t>(rec.y) << 32 | rec.x;
+      const bool rev = ((rec.w & kWindowRev) != 0) != back;
+      if (rev) fl = kWinRev;
+      if (rec.w & kWindowFound) {
+        if (meta & kRepetitiveBit) {
+          fl |= kWinFiltered;
+        } else {
+          fl |= kWinSolid;
+          self = rec.z & kPlaceMask;
+          side = record_side(rec, rev);
+          if (p > 0) left = back ? 3u - (rec.z >> 30) : rec.z >> 28 & 3u;
+        }
+      }
+      if (threadIdx.x == 0 && b0 == w0) {
+        const uint4 r = p > 0 ? __ldg(at + (back ? 1 : -1)) : make_uint4(0, 0, 0, 0);
+        solid[0] = (r.w & kWindowFound) && !(r.y >> 31);
+      }
+    } else if (w < w1) {
       uint32_t hi = ends[1];  // most blocks lie within one query
       while (lo < hi) {
         const uint32_t mid = (lo + hi + 1) >> 1;
@@ -258,7 +328,7 @@ __global__ void __launch_bounds__(kProbeBlock, 6) probe_kernel(
       } else {
         ns = side.most == rt.expect ? side.others : count_starts(idx, off, c, rt);
         // the query's own position is no hit
-        if (ns && own && own_before(idx, q.qdi[lo], p) != left) --ns;
+        if (!indexed && ns && own && own_before(idx, q.qdi[lo], p) != left) --ns;
       }
     }
     const uint32_t cb = __ballot_sync(0xffffffffu, fl & kWinSolid);
@@ -605,14 +675,8 @@ __device__ __forceinline__ int32_t run_length(const RunTables& t, uint64_t qbase
                                               uint64_t tbase, int32_t tlen, bool rev, int32_t p,
                                               int32_t pos, int32_t most, int32_t room) {
   const int32_t k = t.idx.k;
-  // bases x .. x + 31 of the target strand
   auto target32 = [&](int32_t x) {
-    if (!rev) return bases32(t.idx.twords, tbase + static_cast<uint64_t>(x));
-    // the reverse complement of the 32 forward bases that end before len - x
-    const int64_t s = static_cast<int64_t>(tbase) + tlen - 32 - x;
-    const uint64_t f = s >= 0 ? bases32(t.idx.twords, static_cast<uint64_t>(s))
-                              : bases32(t.idx.twords, 0) >> (2 * -s);
-    return revcomp(f, 32);
+    return target_bases32(t.idx.twords, tbase, tlen, rev, x);
   };
   int32_t m = 0;  // agreeing bases after the first window
   while (m < most - 1) {
