@@ -394,9 +394,20 @@ __global__ void query_offsets_kernel(QueryBatch q, const uint32_t* __restrict__ 
   if ((threadIdx.x & 31) == 0 && n) atomicMax(totals, static_cast<unsigned long long>(n));
 }
 
-// A warp writes its 32 windows' run starts.  The entries of the windows that
-// start runs (few windows do) are numbered through and taken 32 at a time, so
-// the lanes are busy whether a bucket holds two entries or two hundred.
+// Which of 16 entries' nibbles differ from the pattern, entry i at bit i.
+__device__ __forceinline__ uint32_t differ_bits16(uint4 x, int shift, uint32_t pat) {
+  auto word = [&](uint32_t w) {  // one bit a byte, gathered by a multiplication
+    const uint32_t d = ((((w >> shift) & 0x0f0f0f0fu) ^ pat) + 0x7f7f7f7fu) >> 7 & 0x01010101u;
+    return d * 0x01020408u >> 24;  // bits 28 up are zero: the sums do not reach them
+  };
+  return word(x.x) | word(x.y) << 4 | word(x.z) << 8 | word(x.w) << 12;
+}
+
+// A warp writes its 32 windows' run starts.  The buckets of the windows that
+// start runs (few windows do) are cut at every 16th entry; the pieces are
+// numbered through and taken a lane each, which compares its 16 neighbour bytes
+// at once, so the lanes are busy whether a bucket holds two entries or two
+// hundred.  Bound by instructions and the scattered entries.
 __global__ void __launch_bounds__(256) start_emit_kernel(
     DeviceIndex idx, QueryBatch q, const uint4* __restrict__ recs,
     const uint32_t* __restrict__ nstart, const uint64_t* __restrict__ tile_off,
@@ -418,7 +429,8 @@ __global__ void __launch_bounds__(256) start_emit_kernel(
   if (!__any_sync(0xffffffffu, ns > 0)) return;
   const uint64_t meta = (static_cast<uint64_t>(rec.y) << 32) | rec.x, off = meta & kOffsetMask;
   const uint32_t test = rec.w, c = ns ? bucket_size(meta) : 0;
-  uint32_t upto = c;  // entries of this window and the ones before
+  const uint32_t pieces = ns ? (static_cast<uint32_t>(off & 15) + c + 15) >> 4 : 0;
+  uint32_t upto = pieces;  // of this window and the ones before
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const uint32_t y = __shfl_up_sync(0xffffffffu, upto, o);
@@ -428,34 +440,50 @@ __global__ void __launch_bounds__(256) start_emit_kernel(
   uint64_t out = tile_off[w >> 5];
   for (uint32_t e0 = 0; e0 < total; e0 += 32) {
     const uint32_t j = e0 + lane;
-    int src = 0;  // the window of entry j: the first whose count exceeds j
+    int src = 0;  // the window of piece j: the first whose count exceeds j
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
       if (__shfl_sync(0xffffffffu, upto, src + o - 1) <= j) src += o;
-    const uint32_t end = __shfl_sync(0xffffffffu, upto, src);
+    const uint32_t before = __shfl_sync(0xffffffffu, upto - pieces, src);
     const uint32_t n = __shfl_sync(0xffffffffu, c, src);
     const uint64_t wo = __shfl_sync(0xffffffffu, off, src);
     const uint32_t wp = __shfl_sync(0xffffffffu, p, src);
     const uint32_t wt = __shfl_sync(0xffffffffu, test, src);
-    const uint32_t e = j - (end - n);
-    const uint32_t expect = (wt >> 22) & 7u;
-    bool start = j < total && e != (wt & kNoSelf);
-    if (start && expect != 7)
-      start = ((static_cast<uint32_t>(__ldg(idx.nbr + wo + e)) >> ((wt >> 23) & 4u)) & 15u) != expect;
-    const unsigned m = __ballot_sync(0xffffffffu, start);
-    if (start) {
-      const uint64_t sv = __ldg(idx.pos + wo + e);
+    // the piece's 16 entries, the first of them (before the bucket's in its first piece)
+    const int32_t first = static_cast<int32_t>((j - before) << 4) - static_cast<int32_t>(wo & 15);
+    uint32_t m = 0;
+    if (j < total) {
+      const uint32_t expect = (wt >> 22) & 7u;
+      m = expect == 7 ? 0xffffu
+                      : differ_bits16(__ldg(reinterpret_cast<const uint4*>(idx.nbr) + (wo >> 4) +
+                                            (j - before)),
+                                      (wt >> 23) & 4u, expect * 0x01010101u);
+      if (first < 0) m &= 0xffffu << -first;
+      const int32_t end = static_cast<int32_t>(n) - first;  // entries of the bucket from here on
+      if (end < 16) m &= (1u << end) - 1u;
+      const uint32_t self = (wt & kNoSelf) - static_cast<uint32_t>(first);
+      if (self < 16) m &= ~(1u << self);  // kNoSelf is beyond every bucket
+    }
+    uint32_t upto_m = __popc(m);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, upto_m, o);
+      if (lane >= o) upto_m += y;
+    }
+    uint64_t d = out + upto_m - __popc(m);
+    out += __shfl_sync(0xffffffffu, upto_m, 31);
+    const uint64_t base = wo + static_cast<uint64_t>(static_cast<int64_t>(first));
+    for (; m; m &= m - 1u, ++d) {
+      const uint64_t sv = __ldg(idx.pos + base + (__ffs(m) - 1));
       uint32_t id = static_cast<uint32_t>(sv >> 32);
       int32_t pos = static_cast<int32_t>(sv & 0xffffffffu);
       if (wt >> 25) {
         pos = idx.slot_len[id >> 1] - pos - idx.k;
         id ^= 1u;
       }
-      const uint64_t d = out + __popc(m & lt);
       keys[d] = (static_cast<uint64_t>(id) << 32) | wp;
       vals[d] = static_cast<uint32_t>(pos);
     }
-    out += __popc(m);
   }
 }
 
