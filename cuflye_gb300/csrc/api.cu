@@ -947,6 +947,9 @@ struct PassState {
   // that the hit path chains
   bool runs = false;
   uint64_t run_hits = 0, longest = 0;  // hits in runs; runs of the longest query
+  uint32_t on_chip = 0;                // runs up to which a query is sorted on chip
+  uint32_t* long_list = nullptr;       // queries that the sort's large form takes
+  const unsigned long long* long_count = nullptr;
   const uint32_t* cbits = nullptr;  // per 32 windows: the solid ones
   std::vector<uint64_t> base_off_h, win_off_h;  // nq + 1
   std::vector<int32_t> qdi_h;
@@ -1227,24 +1230,31 @@ void run_runs(cuflye_ctx* c, PassState& ps) {
   uint64_t* tile_off = buf<uint64_t>(c, "n_toff", nt + 1);
   uint64_t* ftile_off = buf<uint64_t>(c, "n_ftoff", nt + 1);
   // 64 partial sums of hits, the totals of runs_query_offsets
-  unsigned long long* total = buf<unsigned long long>(c, "n_total", 67);
-  CUFLYE_CHECK(cudaMemsetAsync(total, 0, 67 * sizeof(unsigned long long), st));
+  unsigned long long* total = buf<unsigned long long>(c, "n_total", 68);
+  CUFLYE_CHECK(cudaMemsetAsync(total, 0, 68 * sizeof(unsigned long long), st));
   CUFLYE_CHECK(runs_count(c->idx, ps.qb, recs, nstart, cbits, fbits, tfilt, tstart, total,
                           c->num_sms, st));
   CUFLYE_CHECK(exclusive_scan_pair(tstart, tile_off, tfilt, ftile_off, nt,
                                    buf<uint64_t>(c, "n_scan", scan_temp_words(nt)), st));
   ps.q_off = buf<uint64_t>(c, "n_qoff", nq + 1);
+  ps.long_list = buf<uint32_t>(c, "n_qlong", nq);
+  ps.long_count = total + 67;
   ps.f_off = buf<uint64_t>(c, "n_foff", nq + 1);
   CUFLYE_CHECK(runs_query_offsets(ps.qb, nstart, tile_off, fbits, ftile_off, ps.q_off, ps.f_off,
-                                  total + 64, st));
+                                  total + 64, ps.long_list, st));
   ReadBack rb{c};
-  const unsigned long long* nh = rb.add(total, 67);
+  const unsigned long long* nh = rb.add(total, 68);
   rb.read_all();
   uint64_t hits = 0;
   for (int i = 0; i < 64; ++i) hits += nh[i];
   ps.longest = nh[64];
   ps.units = nh[65];
   ps.nfilt = nh[66];
+  // many queries for the sort's large form, and longer ones beside them: the
+  // radix passes that these need take them all (59e6 runs in 3583 queries: 1.27
+  // against 1.39 ms; 36e6 in 13301, none longer: 2.24 against 1.98)
+  const bool large = nh[67] <= 4ull * c->num_sms || ps.longest <= kRunSortLarge;
+  ps.on_chip = large ? kRunSortLarge : kRunSortCap;
   const uint64_t limit = effective_budget(c);
   const uint64_t used = c->in_use - reusable_bytes(c, true, false);
   const uint64_t free_b = limit > used ? limit - used : 0;
@@ -1916,22 +1926,22 @@ ChainRows chain_runs(cuflye_ctx* c, PassState& ps, const ChainParams& cp) {
   const uint32_t nq = ps.nq;
   uint64_t* sstats = buf<uint64_t>(c, "x_sortstats", kSortStats);
   mark(c, 0);
-  // 1. the runs in (ext id, cur pos) order.  Queries of up to kRunSortCap runs
+  // 1. the runs in (ext id, cur pos) order.  Queries of up to ps.on_chip runs
   // are sorted on chip; longer ones by radix passes over tiles of kMatchTile
   // runs (at most NT tiles, the unused ones empty)
   int id_bits = 0;
   while (id_bits < 32 && ((2ull * c->idx.nslots - 1) >> id_bits) != 0) ++id_bits;
-  if (ps.longest > kRunSortCap) {
+  if (ps.longest > ps.on_chip) {
     uint32_t* ntiles = buf<uint32_t>(c, "m_ntiles", nq);
     uint64_t* mtile_off = buf<uint64_t>(c, "m_tileoff", nq + 1);
-    const uint64_t NT = NR / kMatchTile + std::min<uint64_t>(nq, NR / kRunSortCap) + 1;
+    const uint64_t NT = NR / kMatchTile + std::min<uint64_t>(nq, NR / ps.on_chip) + 1;
     MatchTile* tiles = buf<MatchTile>(c, "m_tiles", NT);
     uint32_t* mcounts = buf<uint32_t>(c, "m_counts", 256 * NT);
     uint64_t* akeys = buf<uint64_t>(c, "n_akeys", NR);
     uint32_t* avals = buf<uint32_t>(c, "n_avals", NR);
     CUFLYE_CHECK(cudaMemsetAsync(tiles, 0, NT * sizeof(MatchTile), st));
     CUFLYE_CHECK(match_plan(ps.q_off, nullptr, nq, ntiles, nullptr, nullptr, nullptr, st, true,
-                            kRunSortCap));
+                            ps.on_chip));
     scan_u32_async(c, ntiles, mtile_off, nq, "m_scan");
     CUFLYE_CHECK(match_tiles(ps.q_off, ntiles, mtile_off, nq, tiles, st));
     CUFLYE_CHECK(match_radix(ps.keys, ps.vals, akeys, avals, tiles, static_cast<uint32_t>(NT),
@@ -1943,8 +1953,8 @@ ChainRows chain_runs(cuflye_ctx* c, PassState& ps, const ChainParams& cp) {
   static_assert(kRcWords % 2 == 0, "the cursor after the counters is 8-byte aligned");
   CUFLYE_CHECK(cudaMemsetAsync(words, 0, (kRcWords + 4) * 4, st));
   uint32_t* q_groups = buf<uint32_t>(c, "n_qgroups", nq);
-  CUFLYE_CHECK(runs_sort(ps.q_off, nq, ps.keys, ps.vals, id_bits, q_groups, words + kRcWords + 2,
-                         c->num_sms, st));
+  CUFLYE_CHECK(runs_sort(ps.q_off, nq, ps.longest, ps.on_chip, ps.long_list, ps.long_count, ps.keys,
+                         ps.vals, id_bits, q_groups, words + kRcWords + 2, c->num_sms, st));
   mark(c, 1);
   // 2. groups.  Small passes size everything by their runs (a group has at
   // least one) and read nothing back before the rows; large ones read the

@@ -361,13 +361,15 @@ __global__ void __launch_bounds__(kProbeBlock, 6) probe_kernel(
 }
 
 // First run and first filtered position of each query; in totals the most runs
-// of a query, and all runs and filtered positions.
+// of a query, all runs, all filtered positions, and the number of queries in
+// list: those that the large form of the sort takes.
 __global__ void query_offsets_kernel(QueryBatch q, const uint32_t* __restrict__ nstart,
                                      const uint64_t* __restrict__ tile_off,
                                      const uint32_t* __restrict__ fbits,
                                      const uint64_t* __restrict__ ftile_off,
                                      uint64_t* __restrict__ q_off, uint64_t* __restrict__ f_off,
-                                     unsigned long long* __restrict__ totals) {
+                                     unsigned long long* __restrict__ totals,
+                                     uint32_t* __restrict__ list) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   auto first_run = [&](uint64_t w) {
     uint64_t o = tile_off[w >> 5];
@@ -390,6 +392,7 @@ __global__ void query_offsets_kernel(QueryBatch q, const uint32_t* __restrict__ 
   uint64_t next = __shfl_down_sync(0xffffffffu, o, 1);
   if ((threadIdx.x & 31) == 31 && i < q.nq) next = first_run(q.win_off[i + 1]);
   uint32_t n = i < q.nq ? static_cast<uint32_t>(next - o) : 0u;
+  if (n > kRunSortCap && n <= kRunSortLarge) list[atomicAdd(totals + 3, 1ull)] = i;
   n = __reduce_max_sync(0xffffffffu, n);
   if ((threadIdx.x & 31) == 0 && n) atomicMax(totals, static_cast<unsigned long long>(n));
 }
@@ -489,80 +492,95 @@ __global__ void __launch_bounds__(256) start_emit_kernel(
 
 // ---------------------------------------------------------------- sort, groups
 
-constexpr int kSortBlock = 512;
-constexpr int kSortWarps = kSortBlock / 32;
-constexpr int kSortItems = static_cast<int>(kRunSortCap / kSortBlock);
-
+template <int BLOCK, int ITEMS>
 struct SortSmem {
-  uint64_t key[kRunSortCap];
-  uint32_t val[kRunSortCap];
-  uint32_t wc[kSortWarps][256];  // per-warp digit counts, then offsets
+  static constexpr int kCap = BLOCK * ITEMS;
+  uint32_t id[kCap];
+  uint16_t at[kCap];             // the run's place before the sort
+  uint16_t wc[BLOCK / 32][256];  // per-warp digit counts, then offsets
   uint32_t dbase[256];
   uint32_t ws[8];
+  uint32_t heads[BLOCK / 32];
   uint32_t item;
 };
+using SortSmall = SortSmem<512, 8>;
+using SortLarge = SortSmem<1024, 16>;
+static_assert(SortSmall::kCap == kRunSortCap && SortLarge::kCap == kRunSortLarge,
+              "the sorts' capacities");
 
 // A block a query: its runs (in cur-pos order) into (ext id, cur pos) order by a
 // stable LSD radix sort of the ext ids, 8 bits a pass, and the number of its
-// groups.  The runs stay on chip from load to store, where passes over device
-// memory (match_radix, which longer queries take beforehand) move them twice a
-// digit and launch three kernels for it.
-__global__ void __launch_bounds__(kSortBlock, 2)
-    sort_queries_kernel(const uint64_t* __restrict__ q_off, uint32_t nq,
-                        uint64_t* __restrict__ keys, uint32_t* __restrict__ vals, int id_bits,
-                        uint32_t* __restrict__ q_groups, uint32_t* __restrict__ work) {
+// groups.  Ids and 16-bit places stay on chip; the runs themselves move once,
+// where passes over device memory (match_radix, which queries beyond on_chip runs
+// take beforehand) move them twice a digit and launch three kernels for it.  The
+// small form takes all queries but the listed ones (of more than kRunSortCap and
+// at most kRunSortLarge runs), which the large form takes when on_chip says so.
+// One query of 5000 runs: 60 -> 30 us.
+template <int BLOCK, int ITEMS>
+__global__ void __launch_bounds__(BLOCK, BLOCK > 512 ? 1 : 2)
+    sort_queries_kernel(const uint64_t* __restrict__ q_off, uint32_t nq, uint32_t on_chip,
+                        const uint32_t* __restrict__ list,
+                        const unsigned long long* __restrict__ list_count, uint64_t* keys,
+                        uint32_t* vals, int id_bits, uint32_t* __restrict__ q_groups,
+                        uint32_t* __restrict__ work) {
+  constexpr int kWarps = BLOCK / 32;
+  constexpr bool kLarge = BLOCK > 512;
   extern __shared__ __align__(16) unsigned char sort_raw[];
-  SortSmem& sm = *reinterpret_cast<SortSmem*>(sort_raw);
+  auto& sm = *reinterpret_cast<SortSmem<BLOCK, ITEMS>*>(sort_raw);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t lt = (1u << lane) - 1u;
+  const uint32_t items = kLarge ? static_cast<uint32_t>(*list_count) : nq;
   for (;;) {
     if (threadIdx.x == 0) sm.item = atomicAdd(work, 1u);
     __syncthreads();
-    const uint32_t q = sm.item;
-    if (q >= nq) break;
+    const uint32_t item = sm.item;
+    __syncthreads();
+    if (item >= items) break;
+    const uint32_t q = kLarge ? list[item] : item;
+    if (kLarge && q >= nq) continue;  // the pass was cut after the list was made
     const uint64_t b = q_off[q];
     const uint64_t len = q_off[q + 1] - b;
-    const bool whole = len <= kRunSortCap;
+    if (!kLarge && len > kRunSortCap && len <= on_chip) continue;
+    const bool whole = len <= SortSmem<BLOCK, ITEMS>::kCap;
     const uint32_t n = whole ? static_cast<uint32_t>(len) : 0u;
     // warp w owns per_warp consecutive runs
-    const uint32_t per_warp = ((n + kSortBlock - 1) / kSortBlock) * 32;
+    const uint32_t per_warp = ((n + BLOCK - 1) / BLOCK) * 32;
     const int rounds = static_cast<int>(per_warp / 32);
     const uint32_t j0 = warp * per_warp + lane;
-    uint64_t k[kSortItems];
-    uint32_t v[kSortItems], rk[kSortItems];
+    uint32_t id[ITEMS], at[ITEMS];  // at: the place, and in a pass the rank above it
 #pragma unroll
-    for (int r = 0; r < kSortItems; ++r) {
+    for (int r = 0; r < ITEMS; ++r) {
       const uint32_t j = j0 + r * 32;
-      const bool in = r < rounds && j < n;
-      k[r] = in ? keys[b + j] : 0;
-      v[r] = in ? vals[b + j] : 0;
+      id[r] = r < rounds && j < n ? static_cast<uint32_t>(keys[b + j] >> 32) : 0u;
+      at[r] = j;
     }
-    for (int shift = 32; n > 1 && shift < 32 + id_bits; shift += 8) {
-      for (int i = threadIdx.x; i < kSortWarps * 256; i += kSortBlock) (&sm.wc[0][0])[i] = 0;
+    for (int shift = 0; n > 1 && shift < id_bits; shift += 8) {
+      uint32_t* wc32 = reinterpret_cast<uint32_t*>(&sm.wc[0][0]);
+      for (int i = threadIdx.x; i < kWarps * 128; i += BLOCK) wc32[i] = 0;
       __syncthreads();
 #pragma unroll
-      for (int r = 0; r < kSortItems; ++r) {
+      for (int r = 0; r < ITEMS; ++r) {
         if (r >= rounds) break;
         const bool in = j0 + r * 32 < n;
-        const uint32_t d = in ? static_cast<uint32_t>(k[r] >> shift) & 0xffu : 256u;
+        const uint32_t d = in ? (id[r] >> shift) & 0xffu : 256u;
         const uint32_t peers = __match_any_sync(0xffffffffu, d);
         const int leader = __ffs(peers) - 1;
         uint32_t base = 0;
         if (in && lane == leader) {
           base = sm.wc[warp][d];
-          sm.wc[warp][d] = base + __popc(peers);
+          sm.wc[warp][d] = static_cast<uint16_t>(base + __popc(peers));
         }
         base = __shfl_sync(0xffffffffu, base, leader);
-        rk[r] = base + __popc(peers & lt);
+        at[r] |= (base + __popc(peers & lt)) << 16;
         __syncwarp();
       }
       __syncthreads();
       uint32_t tot = 0, inc = 0;
       if (threadIdx.x < 256) {
 #pragma unroll
-        for (int w = 0; w < kSortWarps; ++w) {
+        for (int w = 0; w < kWarps; ++w) {
           const uint32_t c = sm.wc[w][threadIdx.x];
-          sm.wc[w][threadIdx.x] = tot;
+          sm.wc[w][threadIdx.x] = static_cast<uint16_t>(tot);
           tot += c;
         }
         inc = tot;
@@ -581,94 +599,121 @@ __global__ void __launch_bounds__(kSortBlock, 2)
       }
       __syncthreads();
 #pragma unroll
-      for (int r = 0; r < kSortItems; ++r) {
+      for (int r = 0; r < ITEMS; ++r) {
         if (r < rounds && j0 + r * 32 < n) {
-          const uint32_t d = static_cast<uint32_t>(k[r] >> shift) & 0xffu;
-          const uint32_t o = sm.dbase[d] + sm.wc[warp][d] + rk[r];
-          sm.key[o] = k[r];
-          sm.val[o] = v[r];
+          const uint32_t d = (id[r] >> shift) & 0xffu;
+          const uint32_t o = sm.dbase[d] + sm.wc[warp][d] + (at[r] >> 16);
+          sm.id[o] = id[r];
+          sm.at[o] = static_cast<uint16_t>(at[r]);
         }
       }
       __syncthreads();
 #pragma unroll
-      for (int r = 0; r < kSortItems; ++r) {
+      for (int r = 0; r < ITEMS; ++r) {
         const uint32_t j = j0 + r * 32;
         if (r < rounds && j < n) {
-          k[r] = sm.key[j];
-          v[r] = sm.val[j];
+          id[r] = sm.id[j];
+          at[r] = sm.at[j];
         }
       }
     }
-    // in order now (in shared memory, a query of one run in k[0]; longer
-    // queries in device memory): write, count the groups
-    uint32_t heads = 0;
-    if (whole) {
+    // in order now; longer queries are so in device memory.  Every run is read
+    // before any is written
+    uint32_t heads = n == 1 && threadIdx.x == 0;
+    if (n > 1) {
+      uint32_t x[ITEMS];
 #pragma unroll
-      for (int r = 0; r < kSortItems; ++r) {
+      for (int r = 0; r < ITEMS; ++r)
+        if (r < rounds && j0 + r * 32 < n) x[r] = vals[b + at[r]];
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < ITEMS; ++r)
+        if (r < rounds && j0 + r * 32 < n) vals[b + j0 + r * 32] = x[r];
+#pragma unroll
+      for (int r = 0; r < ITEMS; ++r)
+        if (r < rounds && j0 + r * 32 < n) x[r] = static_cast<uint32_t>(keys[b + at[r]]);
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < ITEMS; ++r) {
         const uint32_t j = j0 + r * 32;
         if (r < rounds && j < n) {
-          if (n > 1) {
-            keys[b + j] = k[r];
-            vals[b + j] = v[r];
-          }
-          heads += j == 0 || (k[r] >> 32) != (sm.key[j - 1] >> 32);
+          keys[b + j] = static_cast<uint64_t>(id[r]) << 32 | x[r];
+          heads += j == 0 || id[r] != sm.id[j - 1];
         }
       }
-    } else {
-      for (uint64_t j = threadIdx.x; j < len; j += kSortBlock)
+    } else if (!whole) {
+      for (uint64_t j = threadIdx.x; j < len; j += BLOCK)
         heads += j == 0 || (keys[b + j] >> 32) != (keys[b + j - 1] >> 32);
     }
     heads = __reduce_add_sync(0xffffffffu, heads);
-    __syncthreads();  // sm.key and sm.item are read
-    if (lane == 0) sm.wc[0][warp] = heads;
+    if (lane == 0) sm.heads[warp] = heads;
     __syncthreads();
     if (threadIdx.x == 0) {
       uint32_t g = 0;
-      for (int w = 0; w < kSortWarps; ++w) g += sm.wc[0][w];
+      for (int w = 0; w < kWarps; ++w) g += sm.heads[w];
       q_groups[q] = g;
     }
-    __syncthreads();
   }
 }
 
-// The groups of each query: runs of one ext id among its sorted runs.
+// The groups of each query: runs of one ext id among its sorted runs.  Bound by
+// the latency of its steps, so a step takes eight runs a thread (59e6 runs in
+// 3583 queries: 450 us with one).
+constexpr int kBoundItems = 8;
+
 __global__ void __launch_bounds__(256) bounds_kernel(const uint64_t* __restrict__ q_off,
                                                      uint32_t nq,
                                                      const uint64_t* __restrict__ keys,
                                                      const uint64_t* __restrict__ q_group,
                                                      GroupInfo* __restrict__ bounds) {
-  __shared__ uint32_t wsum[8];
+  __shared__ uint32_t wsum[2][8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t lt = (1u << lane) - 1u;
   for (uint32_t q = blockIdx.x; q < nq; q += gridDim.x) {
     const uint64_t b = q_off[q], n = q_off[q + 1] - b;
     uint64_t g = q_group[q];
-    for (uint64_t t0 = 0; t0 < n; t0 += 256) {
-      const uint64_t j = t0 + threadIdx.x;
-      uint32_t id = 0;
-      bool head = false;
-      if (j < n) {
-        id = static_cast<uint32_t>(keys[b + j] >> 32);
-        head = j == 0 || id != static_cast<uint32_t>(keys[b + j - 1] >> 32);
+    int side = 0;
+    for (uint64_t t0 = 0; t0 < n; t0 += 256 * kBoundItems, side ^= 1) {
+      // a warp's runs are consecutive
+      const uint64_t j0 = t0 + warp * (32 * kBoundItems) + lane;
+      uint32_t id[kBoundItems];
+      unsigned head[kBoundItems];
+      uint32_t mine = 0;
+#pragma unroll
+      for (int r = 0; r < kBoundItems; ++r) {
+        const uint64_t j = j0 + 32 * r;
+        id[r] = j < n ? static_cast<uint32_t>(keys[b + j] >> 32) : 0u;
       }
-      const unsigned m = __ballot_sync(0xffffffffu, head);
-      if (lane == 0) wsum[warp] = __popc(m);
+#pragma unroll
+      for (int r = 0; r < kBoundItems; ++r) {
+        const uint64_t j = j0 + 32 * r;
+        uint32_t prev = __shfl_up_sync(0xffffffffu, id[r], 1);
+        if (lane == 0 && j > 0 && j < n) prev = static_cast<uint32_t>(keys[b + j - 1] >> 32);
+        head[r] = __ballot_sync(0xffffffffu, j < n && (j == 0 || id[r] != prev));
+        mine += __popc(head[r]);
+      }
+      if (lane == 0) wsum[side][warp] = mine;
       __syncthreads();
       uint32_t before = 0, all = 0;
 #pragma unroll
       for (int w = 0; w < 8; ++w) {
-        before += w < warp ? wsum[w] : 0u;
-        all += wsum[w];
+        before += w < warp ? wsum[side][w] : 0u;
+        all += wsum[side][w];
       }
-      if (head) {
-        GroupInfo gi{};
-        gi.start = b + j;
-        gi.query = q;
-        gi.ext_di = id;
-        bounds[g + before + __popc(m & ((1u << lane) - 1u))] = gi;
+#pragma unroll
+      for (int r = 0; r < kBoundItems; ++r) {
+        if (head[r] >> lane & 1u) {
+          GroupInfo gi{};
+          gi.start = b + j0 + 32 * r;
+          gi.query = q;
+          gi.ext_di = id[r];
+          bounds[g + before + __popc(head[r] & lt)] = gi;
+        }
+        before += __popc(head[r]);
       }
       g += all;
-      __syncthreads();
     }
+    __syncthreads();  // wsum is free for the next query
   }
 }
 
@@ -1035,10 +1080,12 @@ cudaError_t runs_count(const DeviceIndex& idx, const QueryBatch& q, uint4* recs,
 cudaError_t runs_query_offsets(const QueryBatch& q, const uint32_t* nstart,
                                const uint64_t* tile_off, const uint32_t* fbits,
                                const uint64_t* ftile_off, uint64_t* q_off, uint64_t* f_off,
-                               unsigned long long* totals, cudaStream_t s) {
+                               unsigned long long* totals, uint32_t* list,
+                               cudaStream_t s) {
   count_launch();
   query_offsets_kernel<<<grid(q.nq + 1ull, 128), 128, 0, s>>>(q, nstart, tile_off, fbits,
-                                                              ftile_off, q_off, f_off, totals);
+                                                              ftile_off, q_off, f_off, totals,
+                                                              list);
   return cudaGetLastError();
 }
 
@@ -1053,18 +1100,26 @@ cudaError_t runs_emit(const DeviceIndex& idx, const QueryBatch& q, const uint4* 
   return cudaGetLastError();
 }
 
-cudaError_t runs_sort(const uint64_t* q_off, uint32_t nq, uint64_t* keys, uint32_t* vals,
+cudaError_t runs_sort(const uint64_t* q_off, uint32_t nq, uint64_t longest, uint32_t on_chip,
+                      const uint32_t* list,
+                      const unsigned long long* list_count, uint64_t* keys, uint32_t* vals,
                       int id_bits, uint32_t* q_groups, uint32_t* work, int num_sms,
                       cudaStream_t s) {
   if (nq == 0) return cudaSuccess;
-  const cudaError_t e =
-      cudaFuncSetAttribute(sort_queries_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(sizeof(SortSmem)));
-  if (e != cudaSuccess) return e;
-  count_launch();
-  sort_queries_kernel<<<static_cast<unsigned>(std::min<uint64_t>(nq, 2ull * num_sms)), kSortBlock,
-                        sizeof(SortSmem), s>>>(q_off, nq, keys, vals, id_bits, q_groups, work);
-  return cudaGetLastError();
+  auto launch = [&](auto kernel, size_t smem, int block, int per_sm, uint32_t* counter) {
+    const cudaError_t e = cudaFuncSetAttribute(
+        kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return e;
+    count_launch();
+    kernel<<<static_cast<unsigned>(std::min<uint64_t>(nq, static_cast<uint64_t>(per_sm) * num_sms)),
+             block, smem, s>>>(q_off, nq, on_chip, list, list_count, keys, vals, id_bits, q_groups, counter);
+    return cudaGetLastError();
+  };
+  cudaError_t e = cudaSuccess;
+  if (longest > kRunSortCap && on_chip > kRunSortCap)
+    e = launch(sort_queries_kernel<1024, 16>, sizeof(SortLarge), 1024, 1, work + 1);
+  if (e == cudaSuccess) e = launch(sort_queries_kernel<512, 8>, sizeof(SortSmall), 512, 2, work);
+  return e;
 }
 
 cudaError_t runs_bounds(const uint64_t* q_off, uint32_t nq, const uint64_t* keys,

@@ -99,23 +99,28 @@ cudaError_t runs_count(const DeviceIndex& idx, const QueryBatch& q, uint4* recs,
                        uint32_t* tile_start, unsigned long long* hit_total, int num_sms,
                        cudaStream_t s);
 // Each query's first run and first filtered position (nq + 1 entries each);
-// totals[0] (zeroed by the caller): the most runs of a query, [1] and [2]: all
-// runs and filtered positions.
+// totals (zeroed by the caller): [0] the most runs of a query, [1] and [2] all
+// runs and filtered positions, [3] the queries in list (nq words): those of
+// more than kRunSortCap and up to kRunSortLarge runs.
 cudaError_t runs_query_offsets(const QueryBatch& q, const uint32_t* nstart,
                                const uint64_t* tile_off, const uint32_t* fbits,
                                const uint64_t* ftile_off, uint64_t* q_off, uint64_t* f_off,
-                               unsigned long long* totals, cudaStream_t s);
+                               unsigned long long* totals, uint32_t* list,
+                               cudaStream_t s);
 // The run starts in window order, then bucket order, and the filtered positions.
 cudaError_t runs_emit(const DeviceIndex& idx, const QueryBatch& q, const uint4* recs,
                       const uint32_t* nstart, const uint64_t* tile_off, const uint32_t* fbits,
                       const uint64_t* ftile_off, uint64_t* keys, uint32_t* vals, int32_t* fpos,
                       cudaStream_t s);
 
-// The runs of every query of up to kRunSortCap runs sorted by ext id, in place
-// and stable (longer ones come sorted, by match_radix), and the groups of each
-// query.  *work zeroed by the caller.
-constexpr uint32_t kRunSortCap = 4096;
-cudaError_t runs_sort(const uint64_t* q_off, uint32_t nq, uint64_t* keys, uint32_t* vals,
+// The runs of every query of up to on_chip (kRunSortCap or kRunSortLarge) runs
+// sorted by ext id, in place and stable (longer ones come sorted, by match_radix), and the groups of each
+// query.  longest, list, list_count: from runs_query_offsets.  work: two
+// counters, zeroed by the caller.
+constexpr uint32_t kRunSortCap = 4096, kRunSortLarge = 16384;
+cudaError_t runs_sort(const uint64_t* q_off, uint32_t nq, uint64_t longest, uint32_t on_chip,
+                      const uint32_t* list,
+                      const unsigned long long* list_count, uint64_t* keys, uint32_t* vals,
                       int id_bits, uint32_t* q_groups, uint32_t* work, int num_sms,
                       cudaStream_t s);
 // Start, query and ext id of each group; q_group: the scan of q_groups.

@@ -174,3 +174,29 @@ def test_run_ends_around_the_expected_place(gpu, oracle_mod, k, kind):
     q = synth.ReadSet.from_strings(np.arange(50, 50 + len(queries)), [x.tobytes() for x in queries])
     params = dict(synth.OVERLAP_PARAMS, min_overlap=100)
     assert _check(gpu, oracle_mod, t, q, k, 1, 6, params, VARIANTS[:2]) >= len(queries)
+
+
+@pytest.mark.parametrize("passes", [0, 7])
+def test_queries_around_the_large_sort(gpu, oracle_mod, passes):
+    """Queries of up to more runs than the large sort takes on chip (16384), in
+    one pass and in passes."""
+    from cuflye_gb300 import synth
+    from cuflye_gb300.backend import OverlapParams
+    rng = np.random.default_rng(16384)
+    genome = synth.random_genome(rng, 6000)
+    seqs = [synth.mutate(rng, genome[:n], 0.05, 0.01, 0.01)
+            for n in rng.permutation(np.linspace(60, 6000, 160).astype(int))]
+    reads = synth.ReadSet.from_strings(np.arange(1, len(seqs) + 1), [x.tobytes() for x in seqs])
+    params = dict(synth.OVERLAP_PARAMS, min_overlap=200)
+    gpu.set_batch_queries(passes)
+    try:
+        assert _check(gpu, oracle_mod, reads, reads, 11, 1, 1000, params, VARIANTS[:1]) > 0
+    finally:
+        gpu.set_batch_queries(0)
+    runs = []
+    for n in (200, 700, 6000):
+        i = int(np.argmin([abs(len(x) - n) for x in seqs]))
+        one = synth.ReadSet.from_strings(np.array([i + 1]), [reads.seq(i)])
+        gpu.overlaps(one, OverlapParams.make(**dict(params, kmer_size=11)))
+        runs.append(gpu.last_timing()[1][1] // 8)
+    assert runs[0] < 4096 < runs[1] < 16384 < runs[2], runs
