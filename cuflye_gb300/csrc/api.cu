@@ -387,6 +387,8 @@ struct BuiltIndex {
   uint4* windows = nullptr;
   uint64_t* win_off = nullptr;
   uint8_t* nbr = nullptr;
+  uint32_t* filter = nullptr;
+  uint64_t filter_mask = 0;
 };
 
 // Scratch of one key range's build.
@@ -490,6 +492,19 @@ BuiltIndex build_one_range(cuflye_ctx* c, const WindowSet& w, const std::vector<
   while (bi.cap < 2 * r.nruns) bi.cap <<= 1;
   bi.table = buf<TableEntry>(c, "ix_table", bi.cap);
   bi.nbr = neighbour_bytes(c, w.k, r.npos);
+  const uint64_t nkeys = r.nsolid + r.nrep;
+  if (nkeys && nkeys <= kFilterKeys) {
+    uint64_t words = 1;  // 8 to 16 bits a key, as many as kFilterWords hold
+    while (words < kFilterWords && words * 4 < nkeys) words <<= 1;
+    try {
+      bi.filter = buf<uint32_t>(c, "ix_filter", words);
+      bi.filter_mask = words - 1;
+      CUFLYE_CHECK(cudaMemsetAsync(bi.filter, 0, words * 4, st));
+    } catch (const Error& e) {
+      if (e.code != CUFLYE_ERR_BUDGET) throw;
+      bi.filter = nullptr;
+    }
+  }
   // every indexed window's record (16 bytes), while they take at most a quarter
   // of the memory the build leaves
   uint32_t* place = nullptr;
@@ -518,7 +533,8 @@ BuiltIndex build_one_range(cuflye_ctx* c, const WindowSet& w, const std::vector<
     CUFLYE_CHECK(index_neighbours(bi.pos, r.npos, w.words, w.base_off, w.slot_len, w.k, bi.nbr, st));
   CUFLYE_CHECK(index_insert(r.keys, bi.pos, r.run_start, r.cls, r.kept_off, r.nruns, 0, true,
                             bi.table, bi.cap, c->status, st,
-                            bi.windows ? r.free_run_words : nullptr, bi.nbr));
+                            bi.windows ? r.free_run_words : nullptr, bi.nbr, bi.filter,
+                            bi.filter_mask));
   if (bi.windows)
     CUFLYE_CHECK(index_window_records(r.vals, r.run_id, r.run_start, r.kept_off, r.cls,
                                       r.free_run_words, place, w.nwin, bi.nbr, bi.win_off,
@@ -736,10 +752,10 @@ void build_index(cuflye_ctx* c, int k, size_t n, const int64_t* ids, const int64
   // the previous index's arrays go first (has_index is false from here on)
   release(c, "ix_pos");
   release(c, "ix_table");
-  release(c, "ix_windows");
-  release(c, "ix_winoff");
+  for (const char* t : {"ix_windows", "ix_winoff", "ix_filter"}) release(c, t);
   drop_run_tables(c);
   c->idx.windows = nullptr;
+  c->idx.filter = nullptr;
   c->idx.win_off = nullptr;
   // bases packed in chunks of 256 MiB (a multiple of 32 bases: chunks start on
   // word boundaries; each chunk's trailing pad word is overwritten by the next)
@@ -789,7 +805,7 @@ void build_index(cuflye_ctx* c, int k, size_t n, const int64_t* ids, const int64
       release_build_scratch(c);
       release(c, "ix_pos");
       release(c, "ix_table");
-      for (const char* t : {"ix_windows", "ix_winoff", "ix_nbr"}) release(c, t);
+      for (const char* t : {"ix_windows", "ix_winoff", "ix_nbr", "ix_filter"}) release(c, t);
       ranges = true;
     }
   }
@@ -807,6 +823,8 @@ void build_index(cuflye_ctx* c, int k, size_t n, const int64_t* ids, const int64
   c->idx.slot_signed = d_signed;
   c->idx.nslots = static_cast<uint32_t>(n);
   c->idx.windows = bi.windows;
+  c->idx.filter = bi.filter;
+  c->idx.filter_mask = bi.filter_mask;
   c->idx.win_off = bi.win_off;
   c->idx.nkeys = bi.nsolid + bi.nrep;
   c->idx.nrep = bi.nrep;
@@ -894,10 +912,10 @@ void build_index_entries(cuflye_ctx* c, int k, size_t n, const int64_t* tids, co
     release(c, t);
   c->idx.k = k;
   c->idx.transform = false;
-  release(c, "ix_windows");
-  release(c, "ix_winoff");
+  for (const char* t : {"ix_windows", "ix_winoff", "ix_filter"}) release(c, t);
   drop_run_tables(c);
   c->idx.windows = nullptr;
+  c->idx.filter = nullptr;
   c->idx.win_off = nullptr;
   c->idx.table = table;
   c->idx.cap = cap;

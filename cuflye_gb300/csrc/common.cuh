@@ -86,6 +86,14 @@ __device__ __forceinline__ uint64_t table_next(uint64_t slot, uint64_t cap) {
   return slot + 1 == cap ? 0 : slot + 1;
 }
 
+// A key's word of the filter and its two bits there.
+__device__ __forceinline__ uint64_t filter_word(uint64_t hash, uint64_t mask) {
+  return hash & mask;
+}
+__device__ __forceinline__ uint32_t filter_bits(uint64_t hash) {
+  return 1u << (hash >> 32 & 31) | 1u << (hash >> 37 & 31);
+}
+
 // The table keeps its load at 1/2 or below, so a probe always meets an
 // empty slot.
 __device__ __forceinline__ uint64_t table_probe(const TableEntry* __restrict__ table,

@@ -39,6 +39,20 @@ __device__ __forceinline__ uint32_t query_of_warp(const uint64_t* __restrict__ w
   return lo;
 }
 
+// The table word of a standard form, if the index has it.
+__device__ __forceinline__ uint64_t index_probe(const DeviceIndex& idx, uint64_t key,
+                                                bool* found) {
+  if (idx.filter) {
+    const uint64_t h = mix64(key);
+    const uint32_t bits = filter_bits(h);
+    if ((__ldg(idx.filter + filter_word(h, idx.filter_mask)) & bits) != bits) {
+      *found = false;
+      return 0;
+    }
+  }
+  return table_probe(idx.table, idx.cap, key, found);
+}
+
 struct WindowKmer {
   uint64_t x;    // forward k-mer (Kmer::numRepr)
   uint64_t key;  // standard form
@@ -127,7 +141,7 @@ __device__ __forceinline__ WindowProbe probe_window(const DeviceIndex& idx, cons
   const bool recorded = own_window(idx, q.qdi[qi], p, km.x, rec) && idx.windows;
   bool found = rec.w & kWindowFound;
   const uint64_t meta = recorded ? static_cast<uint64_t>(rec.y) << 32 | rec.x
-                                 : table_probe(idx.table, idx.cap, km.key, &found);
+                                 : index_probe(idx, km.key, &found);
   uint32_t c = 0, self = 0;
   uint8_t fl = km.rev ? kWinRev : 0;
   if (found && (meta & kRepetitiveBit)) {

@@ -215,8 +215,10 @@ __global__ void copy_positions_kernel(const uint64_t* __restrict__ vals,
   if (place) place[i] = static_cast<uint32_t>(at);
 }
 
-// The record of every window (DeviceIndex::windows).  Bound by its
-// scattered 16-byte stores, one a window, in bucket order.
+// The record of every window (DeviceIndex::windows).  Bound by its scattered
+// accesses, a target's offset and a 16-byte store for each window in bucket
+// order (40e6 windows: 1.55 ms; taking the windows in stretches that fit L2 costs
+// more in repeated lookups than it saves in stores, 4.5 ms in ten).
 __global__ void window_records_kernel(const uint64_t* __restrict__ vals,
                                       const uint64_t* __restrict__ flags_scan,
                                       const uint64_t* __restrict__ run_start,
@@ -230,9 +232,15 @@ __global__ void window_records_kernel(const uint64_t* __restrict__ vals,
                                       uint4* __restrict__ windows) {
   const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const uint64_t r = run_of(flags_scan, run_start, i);
-  const uint64_t m = meta[r], v = vals[i];
+  // the window this entry came from: its forward position in its target
+  const uint64_t v = vals[i];
   const uint32_t sid = static_cast<uint32_t>(v >> 32);
+  const uint32_t slot = sid >> 1;
+  const uint32_t sp = static_cast<uint32_t>(v);
+  const uint64_t p = (sid & 1u) ? static_cast<uint32_t>(slot_len[slot] - k) - sp : sp;
+  const uint64_t w = win_off[slot] + p;
+  const uint64_t r = run_of(flags_scan, run_start, i);
+  const uint64_t m = meta[r];
   uint4 rec = make_uint4(0, 0, 0, 0);
   if (m != kNoMeta) {
     rec.x = static_cast<uint32_t>(m);
@@ -249,12 +257,7 @@ __global__ void window_records_kernel(const uint64_t* __restrict__ vals,
     }
   }
   if (sid & 1u) rec.w |= kWindowRev;
-  // the window this entry came from: its forward position in its target
-  const uint32_t slot = sid >> 1;
-  const int64_t sp = static_cast<int64_t>(v & 0xffffffffu);
-  const int64_t p = (sid & 1u) ? static_cast<int64_t>(slot_len[slot]) - sp - k : sp;
-  const uint64_t w = win_off[slot] + static_cast<uint64_t>(p);
-  if (p >= 0 && w < win_off[slot + 1]) windows[w] = rec;
+  windows[w] = rec;
 }
 
 __device__ bool table_insert(TableEntry* table, uint64_t cap, uint64_t key, uint64_t meta,
@@ -335,8 +338,8 @@ __global__ void insert_kernel(const uint64_t* __restrict__ keys,
                               const uint64_t* __restrict__ run_start, uint8_t* cls,
                               uint64_t* kept_off, uint64_t nruns, uint64_t pos_base,
                               bool sorted_ids, TableEntry* table, uint64_t cap, DeviceStatus* st,
-                              uint32_t* __restrict__ records,
-                              const uint8_t* __restrict__ nbr) {
+                              uint32_t* __restrict__ records, const uint8_t* __restrict__ nbr,
+                              uint32_t* filter, uint64_t filter_mask) {
   const uint64_t r = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (r >= nruns) return;
   const uint8_t cl = cls[r];
@@ -352,7 +355,12 @@ __global__ void insert_kernel(const uint64_t* __restrict__ keys,
     cls[r] = nbr && cl == 1 ? bucket_sides(nbr + off, n, others) : static_cast<uint8_t>(63);
     records[r] = others;
   }
-  if (!table_insert(table, cap, keys[r0], meta, false)) raise_status(st, kDevTableFull, 0, r);
+  const uint64_t key = keys[r0];
+  if (filter) {
+    const uint64_t h = mix64(key);
+    atomicOr(filter + filter_word(h, filter_mask), filter_bits(h));
+  }
+  if (!table_insert(table, cap, key, meta, false)) raise_status(st, kDevTableFull, 0, r);
 }
 
 // Per key prefix (key >> shift): solid positions and table entries (solid
@@ -487,12 +495,13 @@ cudaError_t index_copy_positions(const uint64_t* vals, const uint64_t* run_id,
 cudaError_t index_insert(const uint64_t* keys, const uint64_t* pos, const uint64_t* run_start,
                          uint8_t* cls, uint64_t* kept_off, uint64_t nruns, uint64_t pos_base,
                          bool sorted_ids, TableEntry* table, uint64_t cap, DeviceStatus* st,
-                         cudaStream_t s, uint32_t* records, const uint8_t* nbr) {
+                         cudaStream_t s, uint32_t* records, const uint8_t* nbr, uint32_t* filter,
+                         uint64_t filter_mask) {
   if (nruns == 0) return cudaSuccess;
   count_launch();
   insert_kernel<<<grid(nruns, 256), 256, 0, s>>>(keys, pos, run_start, cls, kept_off, nruns,
                                                  pos_base, sorted_ids, table, cap, st, records,
-                                                 nbr);
+                                                 nbr, filter, filter_mask);
   return cudaGetLastError();
 }
 

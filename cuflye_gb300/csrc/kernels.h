@@ -120,6 +120,12 @@ struct DeviceIndex {
   // where a table probe is a scattered load, and most of their neighbours too
   uint4* windows = nullptr;
   uint64_t* win_off = nullptr;
+  // optional (one-range builds of up to kFilterKeys keys): two bits a key in one
+  // of filter_mask + 1 words.  It stays in L2 where the table does not: a lookup
+  // of a k-mer that the index lacks (two of three windows of a read with 8 %
+  // errors) ends there, without the table's line from memory
+  uint32_t* filter = nullptr;
+  uint64_t filter_mask = 0;
   // optional (built indexes of an odd k, when memory allows): the bases around
   // each stored entry's k-mer, one byte an entry in bucket order, and the
   // packed targets with each slot's first base (the run path, runs.cu)
@@ -127,6 +133,9 @@ struct DeviceIndex {
   uint64_t* twords = nullptr;
   uint64_t* tbase = nullptr;
 };
+
+constexpr uint64_t kFilterWords = 1ull << 23;  // 32 MiB, a quarter of L2, at most
+constexpr uint64_t kFilterKeys = kFilterWords * 8;
 
 // Window enumeration over packed targets: keys = standard forms, vals =
 // (stored dense id << 32) | stored position.
@@ -171,7 +180,8 @@ cudaError_t index_insert(const uint64_t* keys, const uint64_t* pos, const uint64
                          uint8_t* cls, uint64_t* kept_off, uint64_t nruns, uint64_t pos_base,
                          bool sorted_ids, TableEntry* table, uint64_t cap, DeviceStatus* st,
                          cudaStream_t s, uint32_t* records = nullptr,
-                         const uint8_t* nbr = nullptr);
+                         const uint8_t* nbr = nullptr, uint32_t* filter = nullptr,
+                         uint64_t filter_mask = 0);
 // Window records (DeviceIndex::windows) from index_insert's (records, a word a
 // run: it takes the counts of others, and kept_off and cls then hold the run's
 // table word, kNoMeta for none, and sides).

@@ -162,7 +162,7 @@ __device__ __forceinline__ uint8_t probe_run_window(const DeviceIndex& idx, cons
   const bool own = own_window(idx, qdi, p, km.x, rec), recorded = own && idx.windows;
   bool found = rec.w & kWindowFound;
   meta = recorded ? static_cast<uint64_t>(rec.y) << 32 | rec.x
-                  : table_probe(idx.table, idx.cap, km.key, &found);
+                  : index_probe(idx, km.key, &found);
   uint8_t fl = km.rev ? kWinRev : 0;
   self = kNoSelf;
   side = BucketSide{7, 0};

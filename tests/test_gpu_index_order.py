@@ -105,3 +105,23 @@ def test_rebuilds_reuse_released_buffers(built_lib, room):
         assert be.memory_stats()[1] <= budget
         be.trim()
         assert be.overlaps(cases[0].reads, OverlapParams.make(**cases[0].params)).tobytes() == fresh[0][1]
+
+
+@pytest.mark.parametrize("n", [16, 19, 20, 40, 300, 5_000, 70_000])
+def test_lookups_of_absent_kmers(gpu, oracle_mod, n):
+    """Queries under ids the index does not have, at indexes of one key up: half
+    their k-mers indexed, half not."""
+    from cuflye_gb300 import synth
+    rng = np.random.default_rng(n)
+    genome = synth.random_genome(rng, n)
+    t = synth.ReadSet.from_strings(np.array([1]), [genome.tobytes()])
+    queries = [genome, synth.revcomp(genome), synth.mutate(rng, genome, 0.1, 0.0, 0.0),
+               synth.random_genome(rng, 2 * n)]
+    q = synth.ReadSet.from_strings(np.arange(10, 14), [x.tobytes() for x in queries])
+    idx, _ = oracle_index(oracle_mod, t, 15, 1, 100)
+    gpu.build_index(t, 15, 1, 100)
+    b = oracle_mod.SeqBatch(q.ids, q.offsets, q.bases.tobytes())
+    cand, _ = gpu.candidates(q)
+    exp = oracle_mod.candidates(idx, b)
+    assert len(cand) >= 2 * (n - 14)
+    assert cand_tuples_gpu(cand) == cand_tuples_oracle(exp)
