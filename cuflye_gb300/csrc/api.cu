@@ -109,7 +109,7 @@ struct cuflye_ctx {
   // a pass body's buffers beyond the per-hit ones, per hit ([1]: beyond the
   // per-run ones, per run, on the run path)
   double other_per_hit[2] = {0, 0};
-  uint64_t runs_chained = 0, hits_in_runs = 0;  // of the last call, on the run path
+  uint64_t runs_chained = 0;  // of the last call, on the run path
   std::map<std::string, uint64_t> pass_need;  // bytes each buffer was asked for in this pass
   uint64_t pass_retries = 0;   // passes of the last call run again on half their queries
   uint64_t pass_hit_cap = 0;   // hits a pass may take after a retry in this call (0: no cap)
@@ -964,7 +964,7 @@ struct PassState {
   // run path: the pass's runs instead of hits; nhits counts those of its hits
   // that the hit path chains
   bool runs = false;
-  uint64_t run_hits = 0, longest = 0;  // hits in runs; runs of the longest query
+  uint64_t longest = 0;                // runs of the longest query
   uint32_t on_chip = 0;                // runs up to which a query is sorted on chip
   uint32_t* long_list = nullptr;       // queries that the sort's large form takes
   const unsigned long long* long_count = nullptr;
@@ -1247,31 +1247,28 @@ void run_runs(cuflye_ctx* c, PassState& ps) {
   uint32_t* tstart = buf<uint32_t>(c, "n_tstart", nt);
   uint64_t* tile_off = buf<uint64_t>(c, "n_toff", nt + 1);
   uint64_t* ftile_off = buf<uint64_t>(c, "n_ftoff", nt + 1);
-  // 64 partial sums of hits, the totals of runs_query_offsets
-  unsigned long long* total = buf<unsigned long long>(c, "n_total", 68);
-  CUFLYE_CHECK(cudaMemsetAsync(total, 0, 68 * sizeof(unsigned long long), st));
-  CUFLYE_CHECK(runs_count(c->idx, ps.qb, recs, nstart, cbits, fbits, tfilt, tstart, total,
-                          c->num_sms, st));
+  unsigned long long* total = buf<unsigned long long>(c, "n_total", 4);
+  CUFLYE_CHECK(cudaMemsetAsync(total, 0, 4 * sizeof(unsigned long long), st));
+  CUFLYE_CHECK(runs_count(c->idx, ps.qb, recs, nstart, cbits, fbits, tfilt, tstart, c->num_sms,
+                          st));
   CUFLYE_CHECK(exclusive_scan_pair(tstart, tile_off, tfilt, ftile_off, nt,
                                    buf<uint64_t>(c, "n_scan", scan_temp_words(nt)), st));
   ps.q_off = buf<uint64_t>(c, "n_qoff", nq + 1);
   ps.long_list = buf<uint32_t>(c, "n_qlong", nq);
-  ps.long_count = total + 67;
+  ps.long_count = total + 3;
   ps.f_off = buf<uint64_t>(c, "n_foff", nq + 1);
   CUFLYE_CHECK(runs_query_offsets(ps.qb, nstart, tile_off, fbits, ftile_off, ps.q_off, ps.f_off,
-                                  total + 64, ps.long_list, st));
+                                  total, ps.long_list, st));
   ReadBack rb{c};
-  const unsigned long long* nh = rb.add(total, 68);
+  const unsigned long long* nh = rb.add(total, 4);
   rb.read_all();
-  uint64_t hits = 0;
-  for (int i = 0; i < 64; ++i) hits += nh[i];
-  ps.longest = nh[64];
-  ps.units = nh[65];
-  ps.nfilt = nh[66];
+  ps.longest = nh[0];
+  ps.units = nh[1];
+  ps.nfilt = nh[2];
   // many queries for the sort's large form, and longer ones beside them: the
   // radix passes that these need take them all (59e6 runs in 3583 queries: 1.27
   // against 1.39 ms; 36e6 in 13301, none longer: 2.24 against 1.98)
-  const bool large = nh[67] <= 4ull * c->num_sms || ps.longest <= kRunSortLarge;
+  const bool large = nh[3] <= 4ull * c->num_sms || ps.longest <= kRunSortLarge;
   ps.on_chip = large ? kRunSortLarge : kRunSortCap;
   const uint64_t limit = effective_budget(c);
   const uint64_t used = c->in_use - reusable_bytes(c, true, false);
@@ -1295,8 +1292,6 @@ void run_runs(cuflye_ctx* c, PassState& ps) {
       ps.nq = 1;
       throw Error(CUFLYE_ERR_BUDGET, "device memory budget exceeded: a query's runs");
     }
-    hits = static_cast<uint64_t>(static_cast<double>(hits) * static_cast<double>(qoff[m]) /
-                                 static_cast<double>(ps.units));
     ps.nq = m;
     ps.units = qoff[m];
     ps.nwin = ps.win_off_h[m];
@@ -1304,7 +1299,6 @@ void run_runs(cuflye_ctx* c, PassState& ps) {
     ps.qb.nwin = ps.nwin;
     ps.nfilt = read_scalar(c, ps.f_off + m);
   }
-  ps.run_hits = hits;
   ps.keys = buf<uint64_t>(c, "n_keys", ps.units);
   ps.vals = buf<uint32_t>(c, "n_vals", ps.units);
   ps.fpos = buf<int32_t>(c, "n_fpos", ps.nfilt);
@@ -2085,7 +2079,6 @@ ChainRows chain_runs(cuflye_ctx* c, PassState& ps, const ChainParams& cp) {
   c->sort_stats[1] += exact;
   c->sort_stats[2] += ext;
   c->sort_stats[4] += chained;
-  c->hits_in_runs += ps.run_hits;
   c->runs_chained += NR;
   return out;
 }
@@ -2111,7 +2104,7 @@ void reset_timing(cuflye_ctx* c) {
   c->pass_retries = 0;
   c->pass_hit_cap = 0;
   c->alloc_ms = 0;
-  c->runs_chained = c->hits_in_runs = 0;
+  c->runs_chained = 0;
   c->emission_fallbacks = 0;
   c->sort_stats[7] = 0;
   c->hits_sorted_emission = c->hits_flagged = c->hits_prefiltered = c->hits_emit_sort = 0;
@@ -2138,20 +2131,21 @@ void accumulate_timing(cuflye_ctx* c, bool chained) {
     c->stage_ms[c->clock_stage[i]] += elapsed(c->clock[i - 1], c->clock[i]);
 }
 
-// Compulsory traffic per stage, for the hits the hit path took: the bases and one probe sector per window,
-// bucket entries read (8 B) and hit records written (12 B); a read and a
+// Compulsory traffic per stage: the bases and a 16-byte table entry (or window
+// record) per window; for the hits the hit path took, bucket
+// entries read (8 B) and hit records written (12 B); a read and a
 // write of every 12-byte record the KmerMatch sort moves (all hits on the
 // emit + sort path, the flagged queries' hits on the sorted emission); the
 // group stage reads the records of the groups it prefilters (12 B each, and
 // on the emit + sort path another 8 B for the group bounds and ext
 // positions); the DP reads (cur, ext) and writes (score, backtrack); the
-// backtrack reads its table once.  On the run path a hit costs the byte of
-// its bucket entry's neighbours; a run its entry (8) and record (12), the sort's
-// 24, its record read and its piece written (24), the piece read and its score
-// and link written (24), and the link table read (12).
+// backtrack reads its table once.  On the run path a hit inside a run costs
+// nothing; a run its entry (8) and record (12), the sort's 24, its record read
+// and its piece written (24), the piece read and its score and link written
+// (24), and the link table read (12).
 void set_stage_bytes(cuflye_ctx* c, uint64_t bases, uint64_t windows, uint64_t hits) {
   const uint64_t r = c->runs_chained;
-  c->stage_bytes[0] = bases / 4 + windows * 32 + hits * 20 + c->hits_in_runs + r * 20;
+  c->stage_bytes[0] = bases / 4 + windows * 16 + hits * 20 + r * 20;
   c->stage_bytes[1] = (c->hits_emit_sort + c->hits_flagged + r) * 24;
   c->stage_bytes[2] = c->hits_emit_sort * 20 + c->hits_prefiltered * 12 + r * 24;
   c->stage_bytes[3] = hits * 16 + r * 24;

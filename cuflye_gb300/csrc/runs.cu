@@ -14,13 +14,13 @@
 // its runs.  run_chain.cu chains them.
 //
 // Measured on all reads of a 5 Mb genome at 40x (HiFi, k = 17: 7.2e9 hits in
-// 36e6 runs, 64 GiB budget): hit generation 183 -> 16.7 ms, KmerMatch sort 54 ->
-// 4 ms, groups 51 -> 19 ms, DP 50 -> 4 ms, backtrack 27 -> 4 ms against writing,
-// sorting and chaining every hit (the hit path, which remains for what the run
-// path leaves open and for indexes without its tables).  At 6 % error (3 Mb
-// genome, 30x ONT reads: 4.7e8 hits in 59e6 runs) 50 -> 25 ms.  One read: 1.0 ->
-// 0.41 ms, its groups' serial scans being as many times shorter as its runs are
-// long.
+// 36e6 runs, 64 GiB budget): hit generation 183 -> 4.9 ms, KmerMatch sort 54 ->
+// 2.0 ms, groups 51 -> 3.9 ms, DP 50 -> 2.1 ms, backtrack 27 -> 3.3 ms against
+// writing, sorting and chaining every hit (the hit path, which remains for what
+// the run path leaves open and for indexes without its tables).  At 6 % error (3
+// Mb genome, 30x ONT reads: 4.7e8 hits in 59e6 runs) 50 -> 8.6 ms.  One read:
+// 1.0 -> 0.24 ms, its groups' serial scans being as many times shorter as its
+// runs are long.
 //
 // Needs an odd k: an even k has k-mers equal to their own reverse complement,
 // stored on one strand only, so that a run on the other strand has holes.
@@ -232,13 +232,14 @@ constexpr int kProbeBlock = 256;
 // windows a block: the table probe (or the index's record of the window), then
 // the run starts in the window's bucket.  Bound by latency: a chain of loads
 // (the block's query, its target, bases, then a table slot and neighbours, all
-// scattered, for a query that is no target of the index).
+// scattered, for a query that is no target of the index).  All HiFi reads (200
+// million windows of indexed queries): 8.4 ms with a table probe and neighbours
+// for each window, 2.2 with the records; 30 million windows of reads with 8 %
+// errors: 1.95 ms, 1.55 with the index's filter.
 __global__ void __launch_bounds__(kProbeBlock, 6) probe_kernel(
     DeviceIndex idx, QueryBatch q, int rounds, uint4* __restrict__ recs,
     uint32_t* __restrict__ nstart, uint32_t* __restrict__ cbits, uint32_t* __restrict__ fbits,
-    uint32_t* __restrict__ tile_filt, uint32_t* __restrict__ tile_start,
-    unsigned long long* __restrict__ hit_total) {
-  __shared__ uint32_t wsum[kProbeBlock / 32];
+    uint32_t* __restrict__ tile_filt, uint32_t* __restrict__ tile_start) {
   __shared__ uint32_t ends[2];             // queries of the block's first and last windows
   __shared__ bool solid[kProbeBlock + 1];  // of the windows before and in the block
   const uint64_t w0 = static_cast<uint64_t>(blockIdx.x) * kProbeBlock * rounds;
@@ -249,7 +250,7 @@ __global__ void __launch_bounds__(kProbeBlock, 6) probe_kernel(
     if (lane == 0) ends[threadIdx.x >> 5] = e;
   }
   __syncthreads();
-  uint32_t lo = ends[0], block_hits = 0;
+  uint32_t lo = ends[0];
   const bool indexed = ends[0] == ends[1] && indexed_windows(idx, q, lo, w0, w1);
   const uint4* row = nullptr;  // records of the query's target
   int64_t last = 0;            // the target's last window, for a query that is its reverse
@@ -315,16 +316,15 @@ __global__ void __launch_bounds__(kProbeBlock, 6) probe_kernel(
     solid[threadIdx.x + 1] = fl & kWinSolid;
     __syncthreads();
     const bool continues = solid[threadIdx.x];
-    uint32_t ns = 0, hits = 0;
+    uint32_t ns = 0;
     RunTest rt{7, (fl & kWinRev) ? 4 : 0};
     if (fl & kWinSolid) {
       if (left != 7 && continues) rt.expect = rt.shift ? 3u - left : left;
       const uint64_t off = meta & kOffsetMask;
       const uint32_t c = bucket_size(meta), own = self != kNoSelf ? 1u : 0u;
-      hits = c - own;
       if (side.most != 7 && side.most != rt.expect && side.others == 0) rt.expect = 7;
       if (rt.expect == 7) {
-        ns = hits;
+        ns = c - own;
       } else {
         ns = side.most == rt.expect ? side.others : count_starts(idx, off, c, rt);
         // the query's own position is no hit
@@ -334,7 +334,6 @@ __global__ void __launch_bounds__(kProbeBlock, 6) probe_kernel(
     const uint32_t cb = __ballot_sync(0xffffffffu, fl & kWinSolid);
     const uint32_t fb = __ballot_sync(0xffffffffu, fl & kWinFiltered);
     const uint32_t starts = __reduce_add_sync(0xffffffffu, ns);
-    block_hits += __reduce_add_sync(0xffffffffu, hits);
     if (w < w1) {
       nstart[w] = ns;
       if (ns || (fl & kWinFiltered))
@@ -350,13 +349,6 @@ __global__ void __launch_bounds__(kProbeBlock, 6) probe_kernel(
     }
     __syncthreads();  // solid is read
     if (threadIdx.x == kProbeBlock - 1) solid[0] = fl & kWinSolid;
-  }
-  if (lane == 0) wsum[threadIdx.x >> 5] = block_hits;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned long long s = 0;
-    for (int i = 0; i < kProbeBlock / 32; ++i) s += wsum[i];
-    if (s) atomicAdd(hit_total + (blockIdx.x & 63u), s);
   }
 }
 
@@ -658,7 +650,7 @@ __global__ void __launch_bounds__(BLOCK, BLOCK > 512 ? 1 : 2)
 
 // The groups of each query: runs of one ext id among its sorted runs.  Bound by
 // the latency of its steps, so a step takes eight runs a thread (59e6 runs in
-// 3583 queries: 450 us with one).
+// 3583 queries: 450 us with one, 255 with eight).
 constexpr int kBoundItems = 8;
 
 __global__ void __launch_bounds__(256) bounds_kernel(const uint64_t* __restrict__ q_off,
@@ -803,11 +795,10 @@ constexpr int kGroupWarps = 8;
 
 // A warp a group.  Warps take chunks of consecutive groups from a counter and
 // list a chunk's survivors with one counter update a list.  A warp's lanes
-// wait for its longest run, so the kernel is bound by the latency of that
-// chain and wants warps: four blocks an SM (64 registers).  1.0e6 groups of 36
-// runs of 200 hits: 7.2 ms (17.9 with a barrier between a block's warps for a
-// shared counter update, and 32 bases a step); 2.7e5 groups of 218 runs of 8
-// hits: 1.6 ms (3.0).
+// wait for its longest run, and the loads of a step are scattered: four blocks
+// an SM (64 registers; at five the spills cost more than the warps gain).  All
+// groups of all HiFi reads (36e6 runs of 200 hits): 3.3 ms, at 0.7 instructions
+// a cycle; 2.7e5 groups of 218 runs of 8 hits: 1.4 ms.
 __global__ void __launch_bounds__(kGroupWarps * 32, 4) run_groups_kernel(RunTables t, ChainParams p,
                                                                       uint32_t chunk,
                                                                       uint32_t* work) {
@@ -1065,15 +1056,14 @@ cudaError_t index_neighbours(const uint64_t* pos, uint64_t npos, const uint64_t*
 
 cudaError_t runs_count(const DeviceIndex& idx, const QueryBatch& q, uint4* recs, uint32_t* nstart,
                        uint32_t* cbits, uint32_t* fbits, uint32_t* tile_filt,
-                       uint32_t* tile_start, unsigned long long* hit_total, int num_sms,
-                       cudaStream_t s) {
+                       uint32_t* tile_start, int num_sms, cudaStream_t s) {
   if (q.nwin == 0) return cudaSuccess;
   // up to eight rounds a block, as long as the blocks fill the chip four times
   const int rounds = static_cast<int>(std::clamp<uint64_t>(
       q.nwin / (4ull * 6 * num_sms * kProbeBlock), 1, 8));
   count_launch();
   probe_kernel<<<grid(q.nwin, kProbeBlock * rounds), kProbeBlock, 0, s>>>(
-      idx, q, rounds, recs, nstart, cbits, fbits, tile_filt, tile_start, hit_total);
+      idx, q, rounds, recs, nstart, cbits, fbits, tile_filt, tile_start);
   return cudaGetLastError();
 }
 

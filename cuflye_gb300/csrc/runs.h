@@ -92,12 +92,10 @@ cudaError_t index_neighbours(const uint64_t* pos, uint64_t npos, const uint64_t*
 
 // Per window its run starts (nstart), and a record (recs) for runs_emit where
 // it has some or is filtered; per 32 windows the run starts, and the bits of
-// solid and of filtered windows; hit totals spread over 64 words of hit_total
-// (zeroed by the caller).
+// solid and of filtered windows.
 cudaError_t runs_count(const DeviceIndex& idx, const QueryBatch& q, uint4* recs, uint32_t* nstart,
                        uint32_t* cbits, uint32_t* fbits, uint32_t* tile_filt,
-                       uint32_t* tile_start, unsigned long long* hit_total, int num_sms,
-                       cudaStream_t s);
+                       uint32_t* tile_start, int num_sms, cudaStream_t s);
 // Each query's first run and first filtered position (nq + 1 entries each);
 // totals (zeroed by the caller): [0] the most runs of a query, [1] and [2] all
 // runs and filtered positions, [3] the queries in list (nq words): those of

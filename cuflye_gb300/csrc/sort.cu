@@ -4,7 +4,8 @@
 // Segments are classified by size and sorted by four kernels:
 //   * <= kTiny elements:      one thread runs the serial algorithm;
 //   * <= kWarpSeg elements:   one warp, segment staged in its own shared-memory
-//                             slice, partitions by warp ballots, leaves per lane;
+//     (kWarpSegFew for few    slice, partitions by warp ballots, leaves per lane;
+//     or short segments)
 //   * <= kCap elements:       one CTA, segment in shared memory; block-wide
 //                             partitions while tasks exceed kWarpMax, then all
 //                             16 warps partition different tasks concurrently
@@ -692,6 +693,7 @@ __global__ void __launch_bounds__(kBlock, 3) sort_cta(uint64_t* K, uint32_t* V,
 constexpr int kBigBlock = 512;
 constexpr int kBigPerSm = 2;
 constexpr int kCluster = 8;
+// below it a cluster's barriers cost what its seven more CTAs save
 constexpr uint32_t kWide = 16384;
 
 // A range of a round: its elements [f, f + n), depth budget d, segment seg,
@@ -788,7 +790,8 @@ __global__ void round_seed(const uint64_t* __restrict__ begin, const uint64_t* _
 // its slice's stoppers as round_partition does its tiles' (maps in the slice's
 // own index range), the slices' counts meet in shared memory, and the CTAs
 // share the swaps.  A range of n elements takes one CTA n / 4096 steps in a
-// row: for the first ranges of a long segment that chain was the whole round.
+// row: for the first ranges of a long segment that chain was the whole round
+// (2e6 elements in three segments: 6.1 -> 1.74 ms; 2e5 in one: 1.28 -> 0.71).
 struct ClusterScratch {
   uint32_t count[2];                     // this slice's stoppers
   uint32_t upto[2][kCluster + 1];        // stoppers before each slice

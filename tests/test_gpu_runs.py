@@ -116,9 +116,9 @@ def test_queries_around_the_sort_capacity(gpu, oracle_mod):
     from cuflye_gb300 import synth
     from cuflye_gb300.backend import OverlapParams
     rng = np.random.default_rng(4096)
-    genome = synth.random_genome(rng, 2000)
+    genome = synth.random_genome(rng, 4000)
     seqs = [synth.mutate(rng, genome[:n], 0.04, 0.01, 0.01)
-            for n in np.linspace(60, 2000, 160).astype(int)]
+            for n in np.linspace(60, 4000, 160).astype(int)]
     reads = synth.ReadSet.from_strings(np.arange(1, len(seqs) + 1), [x.tobytes() for x in seqs])
     params = dict(synth.OVERLAP_PARAMS, min_overlap=200)
     assert _check(gpu, oracle_mod, reads, reads, 11, 1, 1000, params, VARIANTS[:2]) > 0
@@ -126,7 +126,7 @@ def test_queries_around_the_sort_capacity(gpu, oracle_mod):
     for i in (0, reads.n - 1):
         one = synth.ReadSet.from_strings(np.array([i + 1]), [reads.seq(i)])
         gpu.overlaps(one, OverlapParams.make(**dict(params, kmer_size=11)))
-        runs.append(gpu.last_timing()[1][1] // 8)
+        runs.append(gpu.last_timing()[1][1] // 24)
     assert runs[0] < 4096 < runs[1]
 
 
@@ -183,9 +183,9 @@ def test_queries_around_the_large_sort(gpu, oracle_mod, passes):
     from cuflye_gb300 import synth
     from cuflye_gb300.backend import OverlapParams
     rng = np.random.default_rng(16384)
-    genome = synth.random_genome(rng, 6000)
+    genome = synth.random_genome(rng, 12_000)
     seqs = [synth.mutate(rng, genome[:n], 0.05, 0.01, 0.01)
-            for n in rng.permutation(np.linspace(60, 6000, 160).astype(int))]
+            for n in rng.permutation(np.linspace(60, 12_000, 160).astype(int))]
     reads = synth.ReadSet.from_strings(np.arange(1, len(seqs) + 1), [x.tobytes() for x in seqs])
     params = dict(synth.OVERLAP_PARAMS, min_overlap=200)
     gpu.set_batch_queries(passes)
@@ -194,9 +194,9 @@ def test_queries_around_the_large_sort(gpu, oracle_mod, passes):
     finally:
         gpu.set_batch_queries(0)
     runs = []
-    for n in (200, 700, 6000):
+    for n in (200, 2500, 12_000):
         i = int(np.argmin([abs(len(x) - n) for x in seqs]))
         one = synth.ReadSet.from_strings(np.array([i + 1]), [reads.seq(i)])
         gpu.overlaps(one, OverlapParams.make(**dict(params, kmer_size=11)))
-        runs.append(gpu.last_timing()[1][1] // 8)
+        runs.append(gpu.last_timing()[1][1] // 24)
     assert runs[0] < 4096 < runs[1] < 16384 < runs[2], runs
