@@ -24,6 +24,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <fstream>
 #include <map>
 #include <mutex>
@@ -1490,7 +1491,8 @@ GroupRows chain_groups(cuflye_ctx* c, uint64_t* keys, uint32_t* vals, uint64_t H
                        GroupInfo* groups, uint64_t G, const uint32_t* ext_list,
                        const uint32_t* dp_list, const uint32_t* gcounts, const ChainParams& cp,
                        const QueryInfo* qinfo, const uint64_t* f_off, const int32_t* fpos,
-                       uint64_t* sstats, bool tally_pending);
+                       uint64_t* sstats, bool tally_pending,
+                       const std::function<void()>& sorted = nullptr);
 
 // Sort + chaining of the pass's hits.
 ChainRows chain_hits(cuflye_ctx* c, PassState& ps, const ChainParams& cp) {
@@ -1656,7 +1658,8 @@ GroupRows chain_groups(cuflye_ctx* c, uint64_t* keys, uint32_t* vals, uint64_t H
                        GroupInfo* groups, uint64_t G, const uint32_t* ext_list,
                        const uint32_t* dp_list, const uint32_t* gcounts, const ChainParams& cp,
                        const QueryInfo* qinfo, const uint64_t* f_off, const int32_t* fpos,
-                       uint64_t* sstats, bool tally_pending) {
+                       uint64_t* sstats, bool tally_pending,
+                       const std::function<void()>& sorted) {
   cudaStream_t st = c->stream;
   uint32_t* lscr = buf<uint32_t>(c, "s_l", H + 1);
   uint32_t* rscr = buf<uint32_t>(c, "s_r", H + 1);
@@ -1681,6 +1684,7 @@ GroupRows chain_groups(cuflye_ctx* c, uint64_t* keys, uint32_t* vals, uint64_t H
   CUFLYE_CHECK(sort_stats_add(sstats, 2, 3, gcounts + 0, 0, ecount, st));
   CUFLYE_CHECK(segmented_std_sort(keys, vals, lscr, rscr, sb, se, G32, ecount, glists,
                                   scounts, c->num_sms, st, sort_tasks(c, "s", H, G32)));
+  if (sorted) sorted();  // may take groups out of dp_list
   // 4. DP over the sorted pairs
   int32_t* score = buf<int32_t>(c, "c_score", H);
   int32_t* bt = buf<int32_t>(c, "c_bt", H);
@@ -1840,7 +1844,9 @@ uint64_t chain_open_groups(cuflye_ctx* c, PassState& ps, const RunTables& t, uin
     std::vector<uint32_t> list, src;
     std::vector<uint64_t> off;
     uint64_t X = 0;
+    bool ask = false;
     auto take = [&](uint32_t q) {
+      ask |= (info[j].flags & kRunFirst) != 0;
       list.push_back(info[j].group);
       src.push_back(q);
       off.push_back(X);
@@ -1917,9 +1923,33 @@ uint64_t chain_open_groups(cuflye_ctx* c, PassState& ps, const RunTables& t, uin
     uint32_t* gcounts = buf<uint32_t>(c, "g_counts", 4);
     CUFLYE_CHECK(cudaMemsetAsync(gcounts, 0, 4 * sizeof(uint32_t), st));
     CUFLYE_CHECK(runs_expand(t, o, keys, vals, groups, ext_list, dp_list, gcounts, c->num_sms, st));
-    const GroupRows open = chain_groups(c, keys, vals, X, groups, o.n, ext_list, dp_list, gcounts,
-                                        cp, ps.qinfo, ps.f_off, ps.fpos, sstats, false);
-    CUFLYE_CHECK(runs_fold_rows(o.list, o.n, open.rows, group_rows, st));
+    // groups that only lacked their element 0 go on as pieces (a long group's DP
+    // over its hits is one warp's chain: up to 5 ms); what is open then stays here
+    const auto settle = [&]() {
+      RunTables f = t;
+      f.max_groups = o.n;
+      f.lists = buf<uint32_t>(c, "n_flists", static_cast<uint64_t>(kRunClasses) * o.n);
+      f.open_list = buf<uint32_t>(c, "n_fopen", o.n);
+      f.counts = buf<uint32_t>(c, "n_fcounts", kRcWords);
+      CUFLYE_CHECK(cudaMemsetAsync(f.counts, 0, kRcWords * 4, st));
+      auto pool_count = [&](uint32_t* to, const uint32_t* from) {
+        CUFLYE_CHECK(cudaMemcpyAsync(to + kRcPool, from + kRcPool, 4, cudaMemcpyDeviceToDevice, st));
+      };
+      pool_count(f.counts, t.counts);
+      CUFLYE_CHECK(runs_settle_first(t, o, keys, vals, groups, f.lists, f.counts, st));
+      CUFLYE_CHECK(runs_dp(f, cp, c->num_sms, c->shape.dp_blocks_per_sm, st));
+      CUFLYE_CHECK(runs_backtrack(f, cp, ps.f_off, ps.fpos, c->logt, pool, pool_cap, group_rows,
+                                  c->status, c->num_sms, c->shape.backtrack_blocks_per_sm, st));
+      pool_count(t.counts, f.counts);
+      CUFLYE_CHECK(chain_open_rows(pool, pool_cap, t.counts + kRcPool, c->logt, cp, group_rows,
+                                   c->num_sms, st));
+      CUFLYE_CHECK(cudaMemsetAsync(gcounts + 1, 0, 4, st));
+      CUFLYE_CHECK(runs_unsettled(t, o, dp_list, gcounts + 1, st));
+    };
+    const GroupRows open =
+        chain_groups(c, keys, vals, X, groups, o.n, ext_list, dp_list, gcounts, cp, ps.qinfo,
+                     ps.f_off, ps.fpos, sstats, false, ask ? settle : std::function<void()>());
+    CUFLYE_CHECK(runs_fold_rows(t, o.list, o.n, open.rows, group_rows, st));
     CUFLYE_CHECK(runs_append_rows(open.pool, open.pool_count, o.list, pool, pool_cap,
                                   t.counts + kRcPool, c->status, c->num_sms, st));
     mark(c, 4);

@@ -488,6 +488,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) run_dp_kernel(RunTables t
     int32_t big = kNoScore;          // greatest end of the pieces before that one
     bool open = false;
     uint32_t first_tied = 0;  // pieces in a tie cluster at the first position
+    bool ask_first = false;   // left open only for which of them is element 0
     if (lane < static_cast<int>(n)) {
       na = t.pa[base + lane];
       nb = t.pb[base + lane];
@@ -527,14 +528,15 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) run_dp_kernel(RunTables t
       uint32_t u = 0;
       if (i0 == 0) {
         // Element 0 of the group: score 0, no link.  In a tie cluster at the
-        // group's first position any piece may be it; they score k, and if one
-        // of them becomes a link (with score 0 it never would) the group stays
-        // open
+        // group's first position any piece may be it, unless the group says
+        // which; they score k, and if one of them becomes a link (with score 0
+        // it never would) the group stays open for that
         const int32_t at0 = __shfl_sync(0xffffffffu, ca, 0);
         const bool at_first = lane < static_cast<int>(len) && ca == at0;
         first_tied = __popc(__ballot_sync(0xffffffffu, at_first));
         if (first_tied == 1) first_tied = 0;
-        s_prev = first_tied ? p.k : 0;
+        if (g.first) first_tied = 0;
+        s_prev = first_tied || g.first > 1 ? p.k : 0;
         e_prev = s_prev;
         if (lane == 0) {
           cs = s_prev;
@@ -663,9 +665,9 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) run_dp_kernel(RunTables t
             }
           }
         }
-        const int32_t si = max(best, p.k);
+        const int32_t si = i + 1 == g.first ? 0 : max(best, p.k);
         if (ties) {
-          if (best > p.k && bestj < first_tied) open = true;
+          if (best > p.k && bestj < first_tied) ask_first = open = true;
           // the cluster so far: could the elements inside one of two pieces
           // link into the other (one axis position back, so on a lower second
           // position)?
@@ -676,7 +678,10 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) run_dp_kernel(RunTables t
           const bool close = jd <= p.max_gap && jd + 1 < p.max_jump;
           const bool unsafe = mate && li_ > 1 && close && !(d > 0 ? si > rs - gc : rs > si - gc);
           const unsigned mates = __ballot_sync(0xffffffffu, mate);
-          if (__any_sync(0xffffffffu, unsafe) || mates == 0xffffffffu) open = true;
+          if (__any_sync(0xffffffffu, unsafe) || mates == 0xffffffffu) {
+            open = true;
+            ask_first = false;
+          }
         }
         if (lane == static_cast<int>(u)) {
           cs = si;
@@ -706,7 +711,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) run_dp_kernel(RunTables t
       if (lane == 0) qmax = kNoScore;
     }
     if (open && lane == 0) {
-      t.groups[gidx].flags = g.flags | kRunOpen;
+      t.groups[gidx].flags = g.flags | kRunOpen | (ask_first ? kRunFirst : 0u);
       leave_open(t, gidx);
     }
   }
@@ -955,6 +960,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 4) run_backtrack_kernel(
     __syncwarp();
     if (lane != 0) continue;
     if (ambiguous) {
+      t.groups[gidx].flags = g.flags | kRunOpen;
       leave_open(t, gidx);
     } else if (overflow) {
       group_rows[gidx] = 0;

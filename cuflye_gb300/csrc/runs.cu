@@ -1024,11 +1024,51 @@ __global__ void append_rows_kernel(const OverlapRow* __restrict__ from,
   }
 }
 
-__global__ void fold_rows_kernel(const uint32_t* __restrict__ open_list, uint32_t nopen,
-                                 const uint32_t* __restrict__ rows,
+// A group that runs_settle_first listed and the run path then finished.
+__device__ __forceinline__ bool settled(const RunGroup& g) {
+  return g.first != 0 && !(g.flags & kRunOpen);
+}
+
+__global__ void settle_first_kernel(RunTables t, OpenBatch o, const uint64_t* __restrict__ keys,
+                                    const uint32_t* __restrict__ vals,
+                                    const GroupInfo* __restrict__ groups,
+                                    uint32_t* __restrict__ lists, uint32_t* __restrict__ counts) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= o.n) return;
+  RunGroup& g = t.groups[o.list[i]];
+  if (!(g.flags & kRunFirst)) return;
+  const GroupInfo gi = groups[i];
+  int32_t cur = static_cast<int32_t>(keys[gi.start] & 0xffffffffu);
+  int32_t ext = static_cast<int32_t>(vals[gi.start]);
+  if (gi.ext_sorted == 1) {  // re-sorted: key ext pos, value cur pos
+    const int32_t x = cur;
+    cur = ext;
+    ext = x;
+  }
+  const bool es = g.flags & kRunExt;
+  const int32_t a = es ? ext : cur, b = es ? cur : ext;
+  const uint32_t n = min(g.npieces, 32u);
+  for (uint32_t z = 0; z < n && t.pa[g.piece0 + z] == a; ++z) {
+    if (t.pb[g.piece0 + z] != b) continue;
+    if (t.pl[g.piece0 + z] != 1) return;  // element 0 is a piece of its own
+    g.first = z + 1;
+    g.flags &= ~static_cast<uint32_t>(kRunOpen | kRunFirst);
+    lists[atomicAdd(counts + kRcList, 1u)] = o.list[i];  // one class: all in the first list
+    return;
+  }
+}
+
+__global__ void unsettled_kernel(RunTables t, OpenBatch o, uint32_t* __restrict__ dp_list,
+                                 uint32_t* __restrict__ count) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < o.n && !settled(t.groups[o.list[i]])) dp_list[atomicAdd(count, 1u)] = i;
+}
+
+__global__ void fold_rows_kernel(RunTables t, const uint32_t* __restrict__ open_list,
+                                 uint32_t nopen, const uint32_t* __restrict__ rows,
                                  uint32_t* __restrict__ group_rows) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < nopen) group_rows[open_list[i]] = rows[i];
+  if (i < nopen && !settled(t.groups[open_list[i]])) group_rows[open_list[i]] = rows[i];
 }
 
 __global__ void scatter_rows_kernel(const OverlapRow* __restrict__ pool,
@@ -1174,11 +1214,28 @@ cudaError_t runs_append_rows(const OverlapRow* from, const uint32_t* nfrom, cons
   return cudaGetLastError();
 }
 
-cudaError_t runs_fold_rows(const uint32_t* open_list, uint32_t nopen, const uint32_t* rows,
-                           uint32_t* group_rows, cudaStream_t s) {
+cudaError_t runs_settle_first(const RunTables& t, const OpenBatch& o, const uint64_t* keys,
+                              const uint32_t* vals, const GroupInfo* groups, uint32_t* lists,
+                              uint32_t* counts, cudaStream_t s) {
+  if (o.n == 0) return cudaSuccess;
+  count_launch();
+  settle_first_kernel<<<grid(o.n, 128), 128, 0, s>>>(t, o, keys, vals, groups, lists, counts);
+  return cudaGetLastError();
+}
+
+cudaError_t runs_unsettled(const RunTables& t, const OpenBatch& o, uint32_t* dp_list,
+                           uint32_t* count, cudaStream_t s) {
+  if (o.n == 0) return cudaSuccess;
+  count_launch();
+  unsettled_kernel<<<grid(o.n, 128), 128, 0, s>>>(t, o, dp_list, count);
+  return cudaGetLastError();
+}
+
+cudaError_t runs_fold_rows(const RunTables& t, const uint32_t* open_list, uint32_t nopen,
+                           const uint32_t* rows, uint32_t* group_rows, cudaStream_t s) {
   if (nopen == 0) return cudaSuccess;
   count_launch();
-  fold_rows_kernel<<<grid(nopen, 256), 256, 0, s>>>(open_list, nopen, rows, group_rows);
+  fold_rows_kernel<<<grid(nopen, 256), 256, 0, s>>>(t, open_list, nopen, rows, group_rows);
   return cudaGetLastError();
 }
 

@@ -23,6 +23,7 @@ enum : uint32_t {
   kRunTies = 4,     // its pieces hold tie clusters
   kRunLarge = 16,   // more pieces than the smaller ordering kernel holds
   kRunOpen = 8,     // left to the hit path: its result may depend on an order of equal keys
+  kRunFirst = 32,   // left open only for which piece of its first position is element 0
 };
 
 struct RunGroup {
@@ -33,7 +34,9 @@ struct RunGroup {
   uint32_t query, ext_di;
   int32_t ext_len;
   uint32_t flags;
-  uint32_t pad;
+  // 1 + the piece that is element 0, of several at the group's first position
+  // (0: not known): found from the order of its hits, see runs_settle_first
+  uint32_t first;
 };
 
 // Length classes of the surviving groups, longest first; list c holds the
@@ -165,8 +168,19 @@ cudaError_t runs_append_rows(const OverlapRow* from, const uint32_t* nfrom, cons
                              OverlapRow* pool, uint64_t pool_cap, uint32_t* pool_count,
                              DeviceStatus* st, int num_sms, cudaStream_t s);
 // group_rows[list[i]] = rows[i].
-cudaError_t runs_fold_rows(const uint32_t* list, uint32_t n, const uint32_t* rows,
-                           uint32_t* group_rows, cudaStream_t s);
+// Open groups whose flags hold kRunFirst, once their hits are in Flye's order
+// (keys, vals, groups: a batch's hits as chain_groups sorts them): their element
+// 0 is set, their flags are cleared, and they are listed for runs_dp and
+// runs_backtrack in lists / counts of a RunTables of their own.
+cudaError_t runs_settle_first(const RunTables& t, const OpenBatch& o, const uint64_t* keys,
+                              const uint32_t* vals, const GroupInfo* groups, uint32_t* lists,
+                              uint32_t* counts, cudaStream_t s);
+// The batch's groups that are still the hit path's (not settled) into dp_list,
+// their number into *count (zeroed by the caller).
+cudaError_t runs_unsettled(const RunTables& t, const OpenBatch& o, uint32_t* dp_list,
+                           uint32_t* count, cudaStream_t s);
+cudaError_t runs_fold_rows(const RunTables& t, const uint32_t* open_list, uint32_t nopen,
+                           const uint32_t* rows, uint32_t* group_rows, cudaStream_t s);
 // Pool rows to their places.
 cudaError_t runs_scatter_rows(const OverlapRow* pool, const uint32_t* npool, uint64_t max_pool,
                               const uint32_t* kept, const uint64_t* kept_off, OverlapRow* rows,

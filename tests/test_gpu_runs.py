@@ -200,3 +200,33 @@ def test_queries_around_the_large_sort(gpu, oracle_mod, passes):
         gpu.overlaps(one, OverlapParams.make(**dict(params, kmer_size=11)))
         runs.append(gpu.last_timing()[1][1] // 24)
     assert runs[0] < 4096 < runs[1] < 16384 < runs[2], runs
+
+
+@pytest.mark.parametrize("copies", [2, 3, 6])
+@pytest.mark.parametrize("longer_query", [False, True])
+def test_ties_at_the_first_position(gpu, oracle_mod, copies, longer_query):
+    """Several hits at a group's first position, one of them the chain's start:
+    which of them is element 0 decides the chain's score."""
+    from cuflye_gb300 import synth
+    rng = np.random.default_rng(10 * copies + longer_query)
+    targets, queries = [], []
+    for i in range(24):
+        base = synth.random_genome(rng, 900)
+        parts = [base]
+        for c in range(copies - 1):  # copies of its start, before or after it
+            copy = base[:int(rng.integers(20, 120))]
+            gap = synth.random_genome(rng, int(rng.integers(10, 200)))
+            parts = [copy, gap] + parts if rng.random() < 0.5 else parts + [gap, copy]
+        t = np.concatenate(parts)
+        q = synth.mutate(rng, base, 0.01, 0.003, 0.003) if i % 3 else base
+        q = np.concatenate([q, synth.random_genome(rng, 4000 if longer_query else 10)])
+        if i % 2:
+            t = synth.revcomp(t)
+        if i % 4 > 1:
+            q = synth.revcomp(q)
+        targets.append(t.tobytes())
+        queries.append(q.tobytes())
+    ts = synth.ReadSet.from_strings(np.arange(1, 25), targets)
+    qs = synth.ReadSet.from_strings(np.arange(100, 124), queries)
+    params = dict(synth.OVERLAP_PARAMS, min_overlap=100)
+    assert _check(gpu, oracle_mod, ts, qs, 15, 1, 100, params, VARIANTS[1:3]) > 0
