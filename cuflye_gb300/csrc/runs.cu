@@ -934,26 +934,48 @@ __global__ void open_info_kernel(RunTables t, uint32_t nopen, OpenInfo* __restri
 __global__ void tie_keys_kernel(RunTables t, OpenBatch o, uint64_t* __restrict__ tie_q,
                                 uint64_t* __restrict__ tie_key, uint32_t* __restrict__ count,
                                 uint32_t cap) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
   if (i >= o.n || o.src_q[i] == kNoLink) return;
   const RunGroup rg = t.groups[o.list[i]];
-  uint32_t end = 0;
-  for (uint32_t r = 0; r < rg.nruns; ++r) {
-    const uint64_t key = t.keys[rg.run0 + r];
-    const uint32_t c = static_cast<uint32_t>(key), e = c + t.rlen[rg.run0 + r];
-    for (uint32_t x = c; x < min(e, end); ++x) {
-      const uint32_t s = atomicAdd(count, 1u);
-      if (s < cap) {
-        tie_q[s] = o.src_q[i];
-        tie_key[s] = key + (x - c);
-      }
+  uint32_t end = 0;  // greatest end of the runs so far
+  for (uint32_t r0 = 0; r0 < rg.nruns; r0 += 32) {
+    const uint32_t r = r0 + lane;
+    const bool in = r < rg.nruns;
+    const uint64_t key = in ? t.keys[rg.run0 + r] : 0;
+    const uint32_t c = static_cast<uint32_t>(key), e = in ? c + t.rlen[rg.run0 + r] : 0u;
+    uint32_t most = e;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, most, d);
+      if (lane >= d) most = max(most, y);
     }
-    end = max(end, e);
+    uint32_t before = __shfl_up_sync(0xffffffffu, most, 1);
+    before = lane == 0 ? end : max(before, end);
+    const uint32_t n = in && min(e, before) > c ? min(e, before) - c : 0u;
+    uint32_t upto = n;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, upto, d);
+      if (lane >= d) upto += y;
+    }
+    const uint32_t total = __shfl_sync(0xffffffffu, upto, 31);
+    uint32_t at = 0;
+    if (lane == 0 && total) at = atomicAdd(count, total);
+    at = __shfl_sync(0xffffffffu, at, 0) + upto - n;
+    for (uint32_t x = 0; x < n && at + x < cap; ++x) {
+      tie_q[at + x] = o.src_q[i];
+      tie_key[at + x] = key + x;
+    }
+    end = max(end, __shfl_sync(0xffffffffu, most, 31));
   }
 }
 
 // The open groups' hits in KmerMatch order: from their runs, or (groups that
-// repeat a cur position) from their query's sorted hits.
+// repeat a cur position) from their query's sorted hits.  kExpandSlices warps
+// share a group: few groups are open, some of them long.
+constexpr uint32_t kExpandSlices = 16;
+
 __global__ void expand_kernel(RunTables t, OpenBatch o, uint64_t* __restrict__ keys,
                               uint32_t* __restrict__ vals, GroupInfo* __restrict__ groups,
                               uint32_t* __restrict__ ext_list, uint32_t* __restrict__ dp_list,
@@ -962,8 +984,9 @@ __global__ void expand_kernel(RunTables t, OpenBatch o, uint64_t* __restrict__ k
   const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
   for (uint32_t li = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; li < o.n; li += nwarps) {
     const RunGroup rg = t.groups[o.list[li]];
+    const uint32_t slice = blockIdx.y;
     uint64_t d = o.off[li];
-    if (lane == 0) {
+    if (lane == 0 && slice == 0) {
       GroupInfo gi{};
       gi.start = d;
       gi.n = rg.nhits;
@@ -987,20 +1010,31 @@ __global__ void expand_kernel(RunTables t, OpenBatch o, uint64_t* __restrict__ k
         else
           hi = mid;
       }
-      for (uint32_t j = lane; j < rg.nhits && lo + j < end; j += 32) {
+      for (uint32_t j = slice * 32 + lane; j < rg.nhits && lo + j < end;
+           j += 32 * kExpandSlices) {
         keys[d + j] = o.sorted_keys[lo + j];
         vals[d + j] = o.sorted_vals[lo + j];
       }
       continue;
     }
-    for (uint32_t i = 0; i < rg.nruns; ++i) {
-      const uint64_t key = t.keys[rg.run0 + i];
-      const uint32_t e = t.vals[rg.run0 + i], l = t.rlen[rg.run0 + i];
-      for (uint32_t j = lane; j < l; j += 32) {
-        keys[d + j] = key + j;
-        vals[d + j] = e + j;
+    for (uint32_t i0 = 0; i0 < rg.nruns; i0 += 32) {
+      const uint32_t i = i0 + lane, n = min(32u, rg.nruns - i0);
+      const uint32_t len = lane < static_cast<int>(n) ? t.rlen[rg.run0 + i] : 0u;
+      if (i0 / 32 % kExpandSlices != slice) {
+        d += __reduce_add_sync(0xffffffffu, len);
+        continue;
       }
-      d += l;
+      const uint64_t first = lane < static_cast<int>(n) ? t.keys[rg.run0 + i] : 0;
+      const uint32_t ext = lane < static_cast<int>(n) ? t.vals[rg.run0 + i] : 0u;
+      for (uint32_t r = 0; r < n; ++r) {
+        const uint64_t key = __shfl_sync(0xffffffffu, first, r);
+        const uint32_t e = __shfl_sync(0xffffffffu, ext, r), l = __shfl_sync(0xffffffffu, len, r);
+        for (uint32_t j = lane; j < l; j += 32) {
+          keys[d + j] = key + j;
+          vals[d + j] = e + j;
+        }
+        d += l;
+      }
     }
   }
 }
@@ -1191,7 +1225,7 @@ cudaError_t runs_tie_keys(const RunTables& t, const OpenBatch& o, uint64_t* tie_
                           uint64_t* tie_key, uint32_t* count, uint32_t cap, cudaStream_t s) {
   if (o.n == 0) return cudaSuccess;
   count_launch();
-  tie_keys_kernel<<<grid(o.n, 64), 64, 0, s>>>(t, o, tie_q, tie_key, count, cap);
+  tie_keys_kernel<<<grid(o.n * 32ull, 64), 64, 0, s>>>(t, o, tie_q, tie_key, count, cap);
   return cudaGetLastError();
 }
 
@@ -1200,9 +1234,10 @@ cudaError_t runs_expand(const RunTables& t, const OpenBatch& o, uint64_t* keys, 
                         uint32_t* counts, int num_sms, cudaStream_t s) {
   if (o.n == 0) return cudaSuccess;
   count_launch();
-  expand_kernel<<<static_cast<unsigned>(std::min<uint64_t>(grid(o.n * 32ull, 256),
-                                                           16ull * num_sms)),
-                  256, 0, s>>>(t, o, keys, vals, groups, ext_list, dp_list, counts);
+  const dim3 blocks(static_cast<unsigned>(std::min<uint64_t>(grid(o.n * 32ull, 256),
+                                                             16ull * num_sms)),
+                    kExpandSlices);
+  expand_kernel<<<blocks, 256, 0, s>>>(t, o, keys, vals, groups, ext_list, dp_list, counts);
   return cudaGetLastError();
 }
 
