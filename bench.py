@@ -621,9 +621,8 @@ def run_ours(args, world, rank, local) -> None:
     if tfile.exists():
         tj = json.loads(tfile.read_text())
         per = tj.get("stages", {}).get(names[dom])
-        if per and per.get("dram_bytes_per_hit"):
-            traffic = per["dram_bytes_per_hit"] * (bytes_tot[dom] / args.steps) / max(
-                1.0, per.get("alg_bytes_per_hit", 1.0))
+        if per and per.get("dram_over_alg"):
+            traffic = per["dram_over_alg"] * bytes_tot[dom] / args.steps
     # plain path: one read per launch, sample
     plain = None
     lat = []
@@ -693,8 +692,9 @@ def run_ours(args, world, rank, local) -> None:
         "roofline": {"bound": "hbm", "stage": names[dom], "achieved": achieved, "peak": peak,
                      "unit": "GB/s", "frac": (achieved / peak) if peak else None,
                      "traffic": traffic,
-                     "traffic_unit": "DRAM bytes per step of the stage's kernels (ncu bytes per "
-                                     "hit from profiles/ncu_traffic.json x hits per step)",
+                     "traffic_unit": "DRAM bytes per step of the stage's kernels (ncu bytes over "
+                                     "algorithmic bytes in profiles/ncu_traffic.json x the "
+                                     "step's algorithmic bytes)",
                      "peak_source": "MEASURED_PEAKS.json hbm_gbs (measured)"
                      if peak else "missing"},
         "clocks": clocks,
