@@ -693,7 +693,8 @@ __global__ void __launch_bounds__(kBlock, 3) sort_cta(uint64_t* K, uint32_t* V,
 constexpr int kBigBlock = 512;
 constexpr int kBigPerSm = 2;
 constexpr int kCluster = 8;
-// below it a cluster's barriers cost what its seven more CTAs save
+// 8,192 gains 2 % on one segment of 2e5 and loses 2 % on 611 segments of 3273;
+// 32,768 loses 2 to 5 % on one to forty long segments
 constexpr uint32_t kWide = 16384;
 
 // A range of a round: its elements [f, f + n), depth budget d, segment seg,

@@ -125,3 +125,26 @@ def test_lookups_of_absent_kmers(gpu, oracle_mod, n):
     exp = oracle_mod.candidates(idx, b)
     assert len(cand) >= 2 * (n - 14)
     assert cand_tuples_gpu(cand) == cand_tuples_oracle(exp)
+
+
+@pytest.mark.parametrize("n", [15, 31, 32, 33, 63, 64, 200, 1000])
+def test_letters_and_other_characters(gpu, oracle_mod, n):
+    """Packing: both cases of the four letters, and every other byte as A."""
+    from cuflye_gb300 import synth
+    rng = np.random.default_rng(n)
+    genome = synth.random_genome(rng, n)
+    lower = np.frombuffer(genome.tobytes().lower(), dtype=np.uint8).copy()
+    odd = genome.copy()
+    at = rng.integers(0, n, size=max(1, n // 20))
+    odd[at] = rng.integers(1, 256, size=len(at))
+    plain = np.array([x if x in b"CGTcgt" else ord("A") for x in odd], dtype=np.uint8)
+    t = synth.ReadSet.from_strings(np.array([1, 2]), [genome.tobytes(), odd.tobytes()])
+    gpu.build_index(t, 15, 1, 100)
+    got = []
+    for a, b in ((genome, odd), (lower, plain)):
+        q = synth.ReadSet.from_strings(np.array([5, 6]), [a.tobytes(), b.tobytes()])
+        got.append(gpu.candidates(q)[0].tobytes())
+    assert got[0] == got[1] and len(got[0]) > 0
+    t2 = synth.ReadSet.from_strings(np.array([1, 2]), [lower.tobytes(), plain.tobytes()])
+    gpu.build_index(t2, 15, 1, 100)
+    assert gpu.candidates(q)[0].tobytes() == got[0]
