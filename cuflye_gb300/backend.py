@@ -88,6 +88,9 @@ class LaunchShape(ctypes.Structure):
         return {f: int(getattr(self, f)) for f, _ in self._fields_}
 
 
+# cuflye_set_run_limit's tables, by their number.
+RUN_LIMITS = ("spare_pieces",)
+
 _vp = ctypes.c_void_p
 _i64p = ctypes.POINTER(ctypes.c_int64)
 _i32p = ctypes.POINTER(ctypes.c_int32)
@@ -169,6 +172,8 @@ def load_library(path: Path | None = None) -> ctypes.CDLL:
     L.cuflye_last_passes.argtypes = [_vp, _u64p]
     L.cuflye_set_sorted_emission.restype = S
     L.cuflye_set_sorted_emission.argtypes = [_vp, ctypes.c_int]
+    L.cuflye_set_run_limit.restype = S
+    L.cuflye_set_run_limit.argtypes = [_vp, ctypes.c_int, ctypes.c_uint64]
     L.cuflye_set_launch_shape.restype = S
     L.cuflye_set_launch_shape.argtypes = [_vp, ctypes.POINTER(LaunchShape)]
     L.cuflye_get_launch_shape.restype = S
@@ -355,6 +360,11 @@ class CudaBackend:
                                             ctypes.byref(params), ctypes.byref(shape),
                                             ctypes.byref(a), ctypes.byref(b)))
         return {"shape": shape.as_dict(), "ms_start": a.value, "ms_chosen": b.value}
+
+    def set_run_limit(self, which: str, most: int | None) -> None:
+        """Bounds a side table of the run path (None: no bound of its own)."""
+        self._check(self._L.cuflye_set_run_limit(
+            self._h, RUN_LIMITS.index(which), (1 << 64) - 1 if most is None else int(most)))
 
     def set_index_build_windows(self, max_windows: int) -> None:
         """Caps the windows of one key range of the index build (0: budget decides)."""

@@ -26,6 +26,7 @@
 #include <cstring>
 #include <functional>
 #include <fstream>
+#include <iterator>
 #include <map>
 #include <mutex>
 #include <stdexcept>
@@ -102,6 +103,7 @@ struct cuflye_ctx {
   unsigned long long emit_tally[2]{};  // a pass's flagged and prefiltered hits, read back
   uint64_t passes = 0;       // see cuflye_last_passes
   uint64_t build_window_cap = 0;  // see cuflye_set_index_build_windows
+  uint64_t run_limit[1] = {~0ull};  // see cuflye_set_run_limit
   cuflye_launch_shape shape{0, 0, 0, 0};  // see cuflye_set_launch_shape (0: defaults)
   uint64_t build_ranges = 0;      // key ranges of the last index build
   int servers = 0;           // open serving loops and shared contexts borrowing this index
@@ -2024,7 +2026,7 @@ ChainRows chain_runs(cuflye_ctx* c, PassState& ps, const ChainParams& cp) {
   t.rlen = buf<uint32_t>(c, "n_rlen", NR);
   t.groups = buf<RunGroup>(c, "n_groups", G);
   t.spare0 = NR + G;
-  t.spare_cap = NR / 2 + 8192;
+  t.spare_cap = std::min<uint64_t>(NR / 2 + 8192, c->run_limit[CUFLYE_RUN_SPARE_PIECES]);
   const uint64_t P = t.spare0 + t.spare_cap;
   t.pa = buf<int32_t>(c, "n_pa", P);
   t.pb = buf<int32_t>(c, "n_pb", P);
@@ -3224,6 +3226,13 @@ cuflye_status cuflye_last_pass_stats(const cuflye_ctx* c, uint64_t* passes, uint
 cuflye_status cuflye_set_index_build_windows(cuflye_ctx* c, uint64_t max_windows) {
   if (!c) return CUFLYE_ERR_INVALID;
   c->build_window_cap = max_windows;
+  return CUFLYE_OK;
+}
+
+cuflye_status cuflye_set_run_limit(cuflye_ctx* c, int which, uint64_t most) {
+  if (!c || which < 0 || which >= static_cast<int>(std::size(c->run_limit)))
+    return CUFLYE_ERR_INVALID;
+  c->run_limit[which] = most;
   return CUFLYE_OK;
 }
 

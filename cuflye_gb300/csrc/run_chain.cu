@@ -167,8 +167,24 @@ struct OrderSmem {
   uint64_t pk[PCAP];      // pieces: axis << 32 | slot in pb / pl
   int32_t pb[PCAP], pl[PCAP];
   int32_t wmax[32];
-  uint32_t item, np, base, over;
+  uint32_t item, np, base;
+  bool over, room;  // more pieces than pk holds; spare slots found
 };
+
+// np consecutive spare slots, or false when fewer are left (the cursor stays
+// then: smaller groups may still find room).
+__device__ __forceinline__ bool claim_spares(const RunTables& t, uint32_t np, uint32_t& base) {
+  unsigned long long at = *reinterpret_cast<volatile unsigned long long*>(t.spare_cursor);
+  while (at + np <= t.spare_cap) {
+    const unsigned long long was = atomicCAS(t.spare_cursor, at, at + np);
+    if (was == at) {
+      base = static_cast<uint32_t>(at);
+      return true;
+    }
+    at = was;
+  }
+  return false;
+}
 
 // Bitonic sort of key[0, n) (room up to a power of two).
 template <int BLOCK, class K>
@@ -278,7 +294,7 @@ __global__ void __launch_bounds__(BLOCK) order_block_kernel(RunTables t, uint32_
       over |= static_cast<int32_t>(sm.rk[i] >> 32) < max(sm.ms[i], before);
     if (tid == 0) {
       sm.np = 0;
-      sm.over = 0;
+      sm.over = false;
     }
     if (!__syncthreads_or(over)) {  // only out of order: one piece a run
       const uint64_t slot = rg.run0 + g;
@@ -311,7 +327,7 @@ __global__ void __launch_bounds__(BLOCK) order_block_kernel(RunTables t, uint32_
       cut_run(sm.cuts, 2 * n, a, a + l, a0, [&](int32_t, int32_t) { ++m; });
       uint32_t d = m <= PCAP ? atomicAdd(&sm.np, m) : PCAP;
       if (d + m > PCAP) {
-        sm.over = 1;
+        sm.over = true;
         continue;
       }
       cut_run(sm.cuts, 2 * n, a, a + l, a0, [&](int32_t x, int32_t len) {
@@ -323,20 +339,13 @@ __global__ void __launch_bounds__(BLOCK) order_block_kernel(RunTables t, uint32_
     }
     __syncthreads();
     const uint32_t np = sm.np;
-    if (sm.over && !LAST) {  // (uniform) for the last kernel
+    if (sm.over && !LAST) {  // for the last kernel (over does not change until the next group)
       if (tid == 0) t.groups[g].flags = rg.flags | kRunLarge;
       continue;
     }
-    if (tid == 0 && !sm.over) {
-      const unsigned long long s =
-          atomicAdd(t.spare_cursor, static_cast<unsigned long long>(np));
-      if (s + np > t.spare_cap)
-        sm.over = 1;
-      else
-        sm.base = static_cast<uint32_t>(s);
-    }
+    if (tid == 0) sm.room = !sm.over && claim_spares(t, np, sm.base);
     __syncthreads();
-    if (sm.over) {
+    if (!sm.room) {
       if (tid == 0) leave_open(t, g);
       continue;
     }

@@ -225,6 +225,13 @@ cuflye_status cuflye_set_batch_queries(cuflye_ctx* ctx, size_t queries_per_pass)
  * + sort path by itself (counted in cuflye_last_sort_stats, entry 7). */
 cuflye_status cuflye_set_sorted_emission(cuflye_ctx* ctx, int enable);
 
+/* Bounds of the run path's side tables, which it sizes by the pass (~0, the
+ * default: no other bound).  What does not fit takes the hit path, so the rows are
+ * the same under any bound.  CUFLYE_RUN_SPARE_PIECES: pieces of groups whose
+ * runs overlap and are cut, in one pass. */
+enum { CUFLYE_RUN_SPARE_PIECES = 0 };
+cuflye_status cuflye_set_run_limit(cuflye_ctx* ctx, int which, uint64_t most);
+
 /* --------------------------------------------------------------------------
  * Launch shapes and the autotuner (no counterpart in the reference).
  * Blocks per SM of the four kernels that take their work from a counter or
