@@ -89,7 +89,7 @@ class LaunchShape(ctypes.Structure):
 
 
 # cuflye_set_run_limit's tables, by their number.
-RUN_LIMITS = ("spare_pieces",)
+RUN_LIMITS = ("spare_pieces", "tie_keys")
 
 _vp = ctypes.c_void_p
 _i64p = ctypes.POINTER(ctypes.c_int64)

@@ -103,7 +103,7 @@ struct cuflye_ctx {
   unsigned long long emit_tally[2]{};  // a pass's flagged and prefiltered hits, read back
   uint64_t passes = 0;       // see cuflye_last_passes
   uint64_t build_window_cap = 0;  // see cuflye_set_index_build_windows
-  uint64_t run_limit[1] = {~0ull};  // see cuflye_set_run_limit
+  uint64_t run_limit[2] = {~0ull, ~0ull};  // see cuflye_set_run_limit
   cuflye_launch_shape shape{0, 0, 0, 0};  // see cuflye_set_launch_shape (0: defaults)
   uint64_t build_ranges = 0;      // key ranges of the last index build
   int servers = 0;           // open serving loops and shared contexts borrowing this index
@@ -1760,8 +1760,10 @@ constexpr uint64_t kChainBytesPerHit = 8 + 4 + 4 + 4 + 8 + 4 + 4 + 4 + 2;
 // among the equal keys listed as (query of sp, key): a stable radix sort by ext
 // id, and libstdc++'s introsort emulated on a copy over the ranges that may
 // hold listed keys, which replace the radix sort's (see flagged_sort).  Hits
-// with other equal keys may come out wrong: nothing reads them.
-void sort_listed_ties(cuflye_ctx* c, PassState& sp, std::vector<std::pair<uint32_t, uint64_t>> ties) {
+// with other equal keys may come out wrong: nothing reads them.  Without a list
+// the whole introsort is emulated.
+void sort_ties(cuflye_ctx* c, PassState& sp,
+               std::vector<std::pair<uint32_t, uint64_t>>* listed) {
   cudaStream_t st = c->stream;
   const uint64_t H = sp.nhits;
   const uint32_t nq = sp.nq;
@@ -1770,12 +1772,12 @@ void sort_listed_ties(cuflye_ctx* c, PassState& sp, std::vector<std::pair<uint32
   uint32_t* lists = buf<uint32_t>(c, "s_lists", 4ull * std::max<uint64_t>(nq, 1));
   uint32_t* scounts = buf<uint32_t>(c, "s_counts", 16);
   const uint64_t* qb = sp.q_off;
-  if (ties.size() * 64u > H) {
-    // equal keys everywhere: the pruning would keep most ranges
+  if (!listed) {
     CUFLYE_CHECK(segmented_std_sort(sp.keys, sp.vals, lscr, rscr, qb, qb + 1, nq, nullptr, lists,
                                     scounts, c->num_sms, st, sort_tasks(c, "s", H, nq)));
     return;
   }
+  std::vector<std::pair<uint32_t, uint64_t>>& ties = *listed;
   std::sort(ties.begin(), ties.end());
   ties.erase(std::unique(ties.begin(), ties.end()), ties.end());
   std::vector<uint32_t> poff(nq + 1, 0);
@@ -1893,22 +1895,25 @@ uint64_t chain_open_groups(cuflye_ctx* c, PassState& ps, const RunTables& t, uin
     uint64_t* keys;
     uint32_t* vals;
     if (sp.nq) {
-      const uint32_t cap = static_cast<uint32_t>(std::min<uint64_t>(sp.nhits / 16 + 1024, 1u << 22));
+      const uint64_t cap = std::min(std::min<uint64_t>(sp.nhits / 16 + 1024, 1u << 22),
+                                    c->run_limit[CUFLYE_RUN_TIE_KEYS]);
       uint64_t* tq = buf<uint64_t>(c, "f_tieh0", cap);
       uint64_t* tk = buf<uint64_t>(c, "f_tiekey", cap);
-      uint32_t* count = buf<uint32_t>(c, "s_ecount", 1);
-      CUFLYE_CHECK(cudaMemsetAsync(count, 0, 4, st));
+      unsigned long long* count = buf<unsigned long long>(c, "f_tiecount", 1);
+      CUFLYE_CHECK(cudaMemsetAsync(count, 0, sizeof(*count), st));
       CUFLYE_CHECK(runs_tie_keys(t, o, tq, tk, count, cap, st));
-      const uint32_t T = read_scalar(c, count);
-      std::vector<std::pair<uint32_t, uint64_t>> ties(T);
-      if (T <= cap) {
+      const uint64_t T = read_scalar(c, count);
+      std::vector<std::pair<uint32_t, uint64_t>> ties;
+      // equal keys everywhere: the pruning would keep most ranges
+      const bool listed = T <= cap && T * 64 <= sp.nhits;
+      if (listed) {
         std::vector<uint64_t> hq(T), hk(T);
-        CUFLYE_CHECK(cudaMemcpyAsync(hq.data(), tq, T * 8ull, cudaMemcpyDeviceToHost, st));
-        CUFLYE_CHECK(cudaMemcpyAsync(hk.data(), tk, T * 8ull, cudaMemcpyDeviceToHost, st));
+        CUFLYE_CHECK(cudaMemcpyAsync(hq.data(), tq, T * 8, cudaMemcpyDeviceToHost, st));
+        CUFLYE_CHECK(cudaMemcpyAsync(hk.data(), tk, T * 8, cudaMemcpyDeviceToHost, st));
         sync(c);
-        for (uint32_t a = 0; a < T; ++a) ties[a] = {static_cast<uint32_t>(hq[a]), hk[a]};
-      }  // else: more than one tie per 64 hits
-      sort_listed_ties(c, sp, std::move(ties));
+        for (uint64_t a = 0; a < T; ++a) ties.emplace_back(static_cast<uint32_t>(hq[a]), hk[a]);
+      }
+      sort_ties(c, sp, listed ? &ties : nullptr);
       o.sorted_off = sp.q_off;
       o.sorted_keys = sp.keys;
       o.sorted_vals = sp.vals;

@@ -932,8 +932,8 @@ __global__ void open_info_kernel(RunTables t, uint32_t nopen, OpenInfo* __restri
 // Cur positions that hits of an open group share, as (sub-batch query, key):
 // where a run (in cur order) starts before the greatest end of the ones before.
 __global__ void tie_keys_kernel(RunTables t, OpenBatch o, uint64_t* __restrict__ tie_q,
-                                uint64_t* __restrict__ tie_key, uint32_t* __restrict__ count,
-                                uint32_t cap) {
+                                uint64_t* __restrict__ tie_key,
+                                unsigned long long* __restrict__ count, uint64_t cap) {
   const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (i >= o.n || o.src_q[i] == kNoLink) return;
@@ -960,8 +960,8 @@ __global__ void tie_keys_kernel(RunTables t, OpenBatch o, uint64_t* __restrict__
       if (lane >= d) upto += y;
     }
     const uint32_t total = __shfl_sync(0xffffffffu, upto, 31);
-    uint32_t at = 0;
-    if (lane == 0 && total) at = atomicAdd(count, total);
+    unsigned long long at = 0;
+    if (lane == 0 && total) at = atomicAdd(count, static_cast<unsigned long long>(total));
     at = __shfl_sync(0xffffffffu, at, 0) + upto - n;
     for (uint32_t x = 0; x < n && at + x < cap; ++x) {
       tie_q[at + x] = o.src_q[i];
@@ -1222,7 +1222,8 @@ cudaError_t runs_open_info(const RunTables& t, uint32_t nopen, OpenInfo* out, cu
 }
 
 cudaError_t runs_tie_keys(const RunTables& t, const OpenBatch& o, uint64_t* tie_q,
-                          uint64_t* tie_key, uint32_t* count, uint32_t cap, cudaStream_t s) {
+                          uint64_t* tie_key, unsigned long long* count, uint64_t cap,
+                          cudaStream_t s) {
   if (o.n == 0) return cudaSuccess;
   count_launch();
   tie_keys_kernel<<<grid(o.n * 32ull, 64), 64, 0, s>>>(t, o, tie_q, tie_key, count, cap);

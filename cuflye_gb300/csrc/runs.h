@@ -159,7 +159,8 @@ cudaError_t runs_open_info(const RunTables& t, uint32_t nopen, OpenInfo* out, cu
 // KmerMatch keys that two hits of such a group share, as (src_q, key), in
 // any order and possibly repeated; *count counts them all, cap are stored.
 cudaError_t runs_tie_keys(const RunTables& t, const OpenBatch& o, uint64_t* tie_q,
-                          uint64_t* tie_key, uint32_t* count, uint32_t cap, cudaStream_t s);
+                          uint64_t* tie_key, unsigned long long* count, uint64_t cap,
+                          cudaStream_t s);
 // Hits and a GroupInfo per group; counts[0] / [1]: ext_list and dp_list.
 cudaError_t runs_expand(const RunTables& t, const OpenBatch& o, uint64_t* keys, uint32_t* vals,
                         GroupInfo* groups, uint32_t* ext_list, uint32_t* dp_list,

@@ -228,8 +228,9 @@ cuflye_status cuflye_set_sorted_emission(cuflye_ctx* ctx, int enable);
 /* Bounds of the run path's side tables, which it sizes by the pass (~0, the
  * default: no other bound).  What does not fit takes the hit path, so the rows are
  * the same under any bound.  CUFLYE_RUN_SPARE_PIECES: pieces of groups whose
- * runs overlap and are cut, in one pass. */
-enum { CUFLYE_RUN_SPARE_PIECES = 0 };
+ * runs overlap and are cut, in one pass.  CUFLYE_RUN_TIE_KEYS: hits of such
+ * groups that share a position, in one sort of their queries' hits. */
+enum { CUFLYE_RUN_SPARE_PIECES = 0, CUFLYE_RUN_TIE_KEYS = 1 };
 cuflye_status cuflye_set_run_limit(cuflye_ctx* ctx, int which, uint64_t most);
 
 /* --------------------------------------------------------------------------

@@ -47,3 +47,44 @@ def test_spare_pieces_run_out(gpu, oracle_mod, copy_div):
         gpu.set_run_limit("spare_pieces", None)
     # without room every such group takes its query's sorted hits
     assert chained[0] == max(chained) > 0
+
+
+@pytest.mark.parametrize("copies", [2, 4])
+def test_tie_list_runs_out(gpu, oracle_mod, copies):
+    """More hits at shared positions than the list holds, few beside their
+    queries' hits: Flye's order among them decides which one a chain starts at."""
+    import numpy as np
+    from cuflye_gb300 import synth
+    from cuflye_gb300.backend import OverlapParams
+    rng = np.random.default_rng(copies)
+    targets, queries = [], []
+    for i in range(32):
+        base = synth.random_genome(rng, int(rng.integers(12_000, 30_000)))
+        parts = [base]
+        for _ in range(copies - 1):  # copies of its start, before or after it
+            copy = base[:int(rng.integers(20, 80))]
+            gap = synth.random_genome(rng, int(rng.integers(10, 200)))
+            parts = [copy, gap] + parts if rng.random() < 0.5 else parts + [gap, copy]
+        targets.append(np.concatenate(parts))
+        q = synth.mutate(rng, base, 0.01, 0.003, 0.003) if i % 3 else base
+        queries.append(np.concatenate([q, synth.random_genome(rng, 40_000)]))  # the longer one
+    ts = synth.ReadSet.from_strings(np.arange(1, 33), [x.tobytes() for x in targets])
+    qs = synth.ReadSet.from_strings(np.arange(100, 132), [x.tobytes() for x in queries])
+    params = dict(synth.OVERLAP_PARAMS, kmer_size=15, only_max_ext=0, check_overhang=0)
+    p = OverlapParams.make(**params)
+    idx, _ = oracle_index(oracle_mod, ts, 15, 1, 100)
+    b = oracle_mod.SeqBatch(qs.ids, qs.offsets, qs.bases.tobytes())
+    exp = {}
+    for stable in (True, False):
+        oracle_mod.set_stable(stable)
+        rows = oracle_mod.overlaps(idx, b, oracle_mod.default_params(**params))
+        exp[stable] = overlap_tuples_oracle(rows)
+    assert exp[True] != exp[False]  # the order among equal keys shows in the rows
+    gpu.build_index(ts, 15, 1, 100)
+    try:
+        for most in (0, 1, 16, 200, None):
+            gpu.set_run_limit("tie_keys", most)
+            assert overlap_tuples_gpu(gpu.overlaps(qs, p)) == exp[False], most
+            assert gpu.last_sort_stats()["match_libstdcxx"] > 0
+    finally:
+        gpu.set_run_limit("tie_keys", None)
