@@ -290,6 +290,10 @@ void raise_device_status(cuflye_ctx* c, const DeviceStatus& st) {
   CUFLYE_CHECK(cudaMemsetAsync(c->status, 0, sizeof(DeviceStatus), c->stream));
   switch (st.code) {
     case kDevProposalOverflow:
+      if (st.where == 1)
+        throw Error(CUFLYE_ERR_UNSUPPORTED,
+                    "unsupported shape: a pass's overlap rows exceed their pool (nine a target "
+                    "group on average; group " + std::to_string(st.detail) + ")");
       throw Error(CUFLYE_ERR_UNSUPPORTED,
                   "unsupported shape: a target group produced more than 64 overlap proposals "
                   "(group " + std::to_string(st.detail) + ")");
@@ -2053,12 +2057,12 @@ ChainRows chain_runs(cuflye_ctx* c, PassState& ps, const ChainParams& cp) {
   mark(c, 2);
   // 3. DP, backtrack
   uint64_t survivors = G;
-  if (!small) {
+  if (!small) {  // those that are listed, and those that are left open already
     ReadBack rb{c};
-    const uint32_t* n = rb.add(t.counts, kRunClasses);
+    const uint32_t* n = rb.add(t.counts, kRcOpen + 1);
     rb.read_all();
-    survivors = 0;
-    for (int i = 0; i < kRunClasses; ++i) survivors += n[i];
+    survivors = n[kRcOpen];
+    for (int i = 0; i < kRunClasses; ++i) survivors += n[kRcList + i];
   }
   CUFLYE_CHECK(runs_dp(t, cp, c->num_sms, c->shape.dp_blocks_per_sm, st));
   mark(c, 3);

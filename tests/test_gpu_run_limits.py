@@ -88,3 +88,34 @@ def test_tie_list_runs_out(gpu, oracle_mod, copies):
             assert gpu.last_sort_stats()["match_libstdcxx"] > 0
     finally:
         gpu.set_run_limit("tie_keys", None)
+
+
+@pytest.mark.parametrize("most", [None, 0])
+def test_open_groups_rows_find_room(gpu, oracle_mod, most):
+    """A large pass (above 32,768 runs) whose groups nearly all repeat positions,
+    with room for the pieces of some and of none: every group's rows are kept."""
+    import numpy as np
+    from cuflye_gb300 import synth
+    from cuflye_gb300.backend import OverlapParams
+    rng = np.random.default_rng(8)
+    unit = synth.random_genome(rng, 200)
+    read = np.concatenate([synth.random_genome(rng, 300), unit, unit, synth.random_genome(rng, 300)])
+    n = 120
+    reads = synth.ReadSet.from_strings(
+        np.arange(1, n + 1), [(synth.revcomp(read) if i % 3 == 1 else read).tobytes()
+                              for i in range(n)])
+    params = dict(synth.OVERLAP_PARAMS, kmer_size=15, min_overlap=400)
+    p = OverlapParams.make(**params)
+    oracle_mod.set_stable(False)
+    idx, batch = oracle_index(oracle_mod, reads, 15, 1, 1000)
+    exp = overlap_tuples_oracle(
+        oracle_mod.overlaps(idx, batch, oracle_mod.default_params(**params)))
+    assert len(exp) >= n * (n - 1)
+    gpu.build_index(reads, 15, 1, 1000)
+    gpu.set_run_limit("spare_pieces", most)
+    try:
+        rows = gpu.overlaps(reads, p)
+        assert gpu.last_timing()[1][1] // 24 > 32_768  # runs (and no other hits) sorted
+    finally:
+        gpu.set_run_limit("spare_pieces", None)
+    assert overlap_tuples_gpu(rows) == exp
