@@ -20,6 +20,7 @@
 #include <chrono>
 #include <condition_variable>
 #include <deque>
+#include <exception>
 #include <thread>
 #include <cstdio>
 #include <cstdlib>
@@ -979,6 +980,19 @@ struct PassState {
   std::vector<uint64_t> base_off_h, win_off_h;  // nq + 1
   std::vector<int32_t> qdi_h;
   std::vector<QueryInfo> qinfo_h;
+  std::vector<unsigned char> batch_h;  // what upload_batch's copy reads, until the pass first waits
+};
+
+// Work that ends in an exception waits for what it queued: the copies read host
+// memory that goes with it (a copy from pageable memory need not have been
+// staged when the call returns: the device can read host pages itself).
+struct WaitOnUnwind {
+  cuflye_ctx* c;
+  int pending = std::uncaught_exceptions();
+  explicit WaitOnUnwind(cuflye_ctx* ctx) : c(ctx) {}
+  ~WaitOnUnwind() {
+    if (std::uncaught_exceptions() > pending) cudaStreamSynchronize(c->stream);
+  }
 };
 
 // Buffers sized by the hit count of a pass (reused by the next pass).
@@ -1055,13 +1069,14 @@ size_t run_end(cuflye_ctx* c, const Queries& Q, size_t q0, size_t q1, uint64_t b
   return q;
 }
 
-// ps's queries (host vectors) as a device batch in one copy; ps.qb (but its
-// words) and ps.qinfo point into it.
+// ps's queries (host vectors) as a device batch in one copy, from ps.batch_h;
+// ps.qb (but its words) and ps.qinfo point into it.
 void upload_batch(cuflye_ctx* c, const char* name, PassState& ps) {
   const size_t nq = ps.nq;
   const size_t o_win = (nq + 1) * 8, o_info = o_win + (nq + 1) * 8,
                o_qdi = o_info + nq * sizeof(QueryInfo), bytes = o_qdi + nq * 4;
-  std::vector<unsigned char> h(bytes);
+  std::vector<unsigned char>& h = ps.batch_h;
+  h.resize(bytes);
   std::memcpy(h.data(), ps.base_off_h.data(), (nq + 1) * 8);
   std::memcpy(h.data() + o_win, ps.win_off_h.data(), (nq + 1) * 8);
   if (nq) {
@@ -1786,6 +1801,7 @@ void sort_ties(cuflye_ctx* c, PassState& sp,
   ties.erase(std::unique(ties.begin(), ties.end()), ties.end());
   std::vector<uint32_t> poff(nq + 1, 0);
   std::vector<uint64_t> pkeys;
+  const WaitOnUnwind wait(c);
   for (const auto& t : ties) {
     ++poff[t.first + 1];
     pkeys.push_back(t.second);
@@ -1862,6 +1878,7 @@ uint64_t chain_open_groups(cuflye_ctx* c, PassState& ps, const RunTables& t, uin
       ++j;
     };
     PassState sp;
+    const WaitOnUnwind wait(c);
     if (!(info[i].flags & kRunCurTies)) {
       while (j < info.size() && !(info[j].flags & kRunCurTies)) take(kNoLink);
     } else {
@@ -2243,6 +2260,7 @@ void for_each_pass(cuflye_ctx* c, const Queries& Q, bool kmers, uint64_t bytes_p
     size_t q1 = run_end(c, Q, q0, std::min(Q.n, q0 + step), by_runs ? kRunBytes : bytes_per_hit,
                         upw, by_runs);
     PassState ps;
+    const WaitOnUnwind wait(c);
     c->pass_need.clear();
     clock_start(c);
     upload_queries(c, Q, q0, q1, ps);
@@ -3298,6 +3316,7 @@ void overlaps_collect(cuflye_ctx* c, const Queries& Q, const ChainParams& cp,
     const ChainRows cr = run_chain(c, ps, cp);
     const uint64_t R = cr.n;
     std::vector<uint64_t> first(ps.nq + 1ull);
+    const WaitOnUnwind wait(c);
     CUFLYE_CHECK(cudaMemcpyAsync(first.data(), cr.q_row, first.size() * 8, cudaMemcpyDeviceToHost,
                                  c->stream));
     cuflye_overlap_range* d_out = buf<cuflye_overlap_range>(c, "a_ovl", R);
