@@ -171,19 +171,17 @@ struct OrderSmem {
   bool over, room;  // more pieces than pk holds; spare slots found
 };
 
-// np consecutive spare slots, or false when fewer are left (the cursor stays
-// then: smaller groups may still find room).
+// np consecutive spare slots, or false when fewer are left.  A group that sees
+// that it does not fit leaves the cursor where it is: smaller ones may still find
+// room.  (One addition a claim: a compare-and-swap loop, which would also keep what
+// a lost race for the last slots spends, waits a round trip for each claim of
+// another block; all reads of a 1 Mb genome at 20x: 4.36 -> 4.70 ms.)
 __device__ __forceinline__ bool claim_spares(const RunTables& t, uint32_t np, uint32_t& base) {
-  unsigned long long at = *reinterpret_cast<volatile unsigned long long*>(t.spare_cursor);
-  while (at + np <= t.spare_cap) {
-    const unsigned long long was = atomicCAS(t.spare_cursor, at, at + np);
-    if (was == at) {
-      base = static_cast<uint32_t>(at);
-      return true;
-    }
-    at = was;
-  }
-  return false;
+  if (*reinterpret_cast<volatile unsigned long long*>(t.spare_cursor) + np > t.spare_cap)
+    return false;
+  const unsigned long long at = atomicAdd(t.spare_cursor, static_cast<unsigned long long>(np));
+  base = static_cast<uint32_t>(at);
+  return at + np <= t.spare_cap;
 }
 
 // Bitonic sort of key[0, n) (room up to a power of two).
