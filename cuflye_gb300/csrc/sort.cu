@@ -3,9 +3,9 @@
 //
 // Segments are classified by size and sorted by four kernels:
 //   * <= kTiny elements:      one thread runs the serial algorithm;
-//   * <= kWarpSeg elements:   one warp, segment staged in its own shared-memory
-//     (kWarpSegFew for few    slice, partitions by warp ballots, leaves per lane;
-//     or short segments)
+//   * <= kWarpSegFew elements: one warp, segment staged in its own shared-memory
+//     (kWarpSeg for many and  slice, partitions by warp ballots, leaves per lane;
+//     long segments)
 //   * <= kCap elements:       one CTA, segment in shared memory; block-wide
 //                             partitions while tasks exceed kWarpMax, then all
 //                             16 warps partition different tasks concurrently
@@ -43,7 +43,11 @@ constexpr uint32_t kWarpSeg = 2048;   // segments up to this size: warp kernel
 // kernel idle while the warps' longest is the call: CTAs take them from
 // kWarpSegFew on.  30 segments of 1000: .44 -> .20 ms; 2000 of 500: .75 -> .50;
 // 611 of 3273, whose CTAs are busy, stay as they are (.84; .89 with kWarpSegFew).
+// The segments' own number and lengths decide, which a call with its list on the
+// device does not know: between the two bounds they form a class of their own, and
+// both kernels look at the counts (few_segments).
 constexpr uint32_t kFewPerSm = 2, kFewMean = 1024, kWarpSegFew = 512;
+constexpr int kMiddleCount = 10, kElemCount = 12;  // words of counts: middle class; elements (64 bits)
 constexpr int kWarpSegWarps = 6;      // warps per CTA in the warp kernel
 constexpr int kMaxWarpTasks = 256;    // warp subtrees per CTA task (<= 2 per partition)
 
@@ -593,24 +597,36 @@ __device__ void cta_load_sort_store(uint64_t* K, uint32_t* V, uint64_t begin, ui
 
 // ---------------------------------------------------------------- kernels
 
+// Lists by class: [c * nseg ..) of class c, the middle class (between the warp
+// kernel's two bounds) from the top of class 1's.
 __global__ void classify_segments(const uint64_t* __restrict__ begin,
                                   const uint64_t* __restrict__ end, uint32_t nseg,
-                                  const uint32_t* __restrict__ nseg_dev, uint32_t warp_max,
-                                  uint32_t* lists, uint32_t* counts) {
+                                  const uint32_t* __restrict__ nseg_dev, uint32_t* lists,
+                                  uint32_t* counts) {
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nseg || (nseg_dev && s >= *nseg_dev)) return;
-  const uint64_t n = end[s] - begin[s];
+  uint64_t n = 0;
+  if (s < nseg && !(nseg_dev && s >= *nseg_dev)) n = end[s] - begin[s];
+  uint64_t sum = n;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
+  if ((threadIdx.x & 31) == 0 && sum)
+    atomicAdd(reinterpret_cast<unsigned long long*>(counts + kElemCount),
+              static_cast<unsigned long long>(sum));
   if (n <= 1) return;
-  int c;
-  if (n <= kTiny)
-    c = 0;
-  else if (n <= warp_max)
-    c = 1;
-  else if (n <= kCap)
-    c = 2;
-  else
-    c = 3;
+  if (n > kWarpSegFew && n <= kWarpSeg) {
+    lists[2 * static_cast<size_t>(nseg) - 1 - atomicAdd(&counts[kMiddleCount], 1u)] = s;
+    return;
+  }
+  const int c = n <= kTiny ? 0 : n <= kWarpSegFew ? 1 : n <= kCap ? 2 : 3;
   lists[static_cast<size_t>(c) * nseg + atomicAdd(&counts[c], 1u)] = s;
+}
+
+// Whether CTAs take the middle class: few segments, or short ones.
+__device__ __forceinline__ bool few_segments(const uint32_t* counts, uint32_t nseg,
+                                             const uint32_t* nseg_dev, uint32_t few) {
+  const uint32_t n = nseg_dev ? min(nseg, *nseg_dev) : nseg;
+  return n <= few || *reinterpret_cast<const uint64_t*>(counts + kElemCount) <=
+                         static_cast<uint64_t>(kFewMean) * n;
 }
 
 __global__ void sort_tiny(uint64_t* K, uint32_t* V, const uint64_t* __restrict__ begin,
@@ -637,15 +653,17 @@ struct WarpSlice {
 // One warp per segment of up to kWarpSeg elements.
 __global__ void __launch_bounds__(kWarpSegWarps * 32) sort_warp(
     uint64_t* K, uint32_t* V, const uint64_t* __restrict__ begin,
-    const uint64_t* __restrict__ end, const uint32_t* __restrict__ list,
-    const uint32_t* __restrict__ counts) {
+    const uint64_t* __restrict__ end, uint32_t nseg, const uint32_t* __restrict__ nseg_dev,
+    uint32_t few, const uint32_t* __restrict__ list, const uint32_t* __restrict__ counts) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   WarpSlice& ws = reinterpret_cast<WarpSlice*>(smem_raw)[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
-  const uint32_t cnt = counts[1];
+  const uint32_t low = counts[1];
+  const uint32_t cnt =
+      low + (few_segments(counts, nseg, nseg_dev, few) ? 0u : counts[kMiddleCount]);
   const uint32_t nwarps = gridDim.x * kWarpSegWarps;
   for (uint32_t li = blockIdx.x * kWarpSegWarps + (threadIdx.x >> 5); li < cnt; li += nwarps) {
-    const uint32_t s = list[li];
+    const uint32_t s = list[li < low ? li : nseg - 1 - (li - low)];
     const uint64_t b = begin[s];
     const uint32_t n = static_cast<uint32_t>(end[s] - b);
     for (uint32_t i = lane; i < n; i += 32) {
@@ -665,13 +683,19 @@ __global__ void __launch_bounds__(kWarpSegWarps * 32) sort_warp(
 __global__ void __launch_bounds__(kBlock, 3) sort_cta(uint64_t* K, uint32_t* V,
                                                    const uint64_t* __restrict__ begin,
                                                    const uint64_t* __restrict__ end,
-                                                   const uint32_t* __restrict__ list,
+                                                   uint32_t nseg,
+                                                   const uint32_t* __restrict__ nseg_dev,
+                                                   uint32_t few,
+                                                   const uint32_t* __restrict__ lists,
                                                    const uint32_t* __restrict__ counts) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   CtaSmem& sm = *reinterpret_cast<CtaSmem*>(smem_raw);
-  const uint32_t cnt = counts[2];
+  const uint32_t high = counts[2];
+  const uint32_t cnt =
+      high + (few_segments(counts, nseg, nseg_dev, few) ? counts[kMiddleCount] : 0u);
   for (uint32_t i = blockIdx.x; i < cnt; i += gridDim.x) {
-    const uint32_t s = list[i];
+    const uint32_t s = i < high ? lists[2 * static_cast<size_t>(nseg) + i]
+                                : lists[2 * static_cast<size_t>(nseg) - 1 - (i - high)];
     const uint64_t b = begin[s];
     const uint32_t n = static_cast<uint32_t>(end[s] - b);
     cta_load_sort_store(K, V, b, n, isort::depth_limit(n), sm);
@@ -1658,12 +1682,11 @@ cudaError_t segmented_std_sort(uint64_t* keys, uint32_t* vals, uint32_t* lscratc
                      tasks.join2;
   cudaStream_t side = split ? tasks.side : stream;
   cudaStream_t side2 = split ? tasks.side2 : stream;
-  cudaMemsetAsync(counts, 0, 10 * sizeof(uint32_t), stream);
+  cudaMemsetAsync(counts, 0, 16 * sizeof(uint32_t), stream);
   count_launch();
-  const bool few = nseg <= kFewPerSm * static_cast<uint32_t>(num_sms) ||
-                   tasks.nelems <= static_cast<uint64_t>(kFewMean) * nseg;
-  classify_segments<<<(nseg + 255) / 256, 256, 0, stream>>>(
-      begin, end, nseg, nseg_dev, few ? kWarpSegFew : kWarpSeg, lists, counts);
+  const uint32_t few = kFewPerSm * static_cast<uint32_t>(num_sms);
+  classify_segments<<<(nseg + 255) / 256, 256, 0, stream>>>(begin, end, nseg, nseg_dev, lists,
+                                                            counts);
   if (split) {
     cudaError_t e = cudaEventRecord(tasks.fork, stream);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(side, tasks.fork, 0);
@@ -1674,11 +1697,10 @@ cudaError_t segmented_std_sort(uint64_t* keys, uint32_t* vals, uint32_t* lscratc
   sort_tiny<<<num_sms * 4, 128, 0, side>>>(keys, vals, begin, end, lists, counts);
   count_launch();
   sort_warp<<<num_sms, kWarpSegWarps * 32, sizeof(WarpSlice) * kWarpSegWarps, side>>>(
-      keys, vals, begin, end, lists + nseg, counts);
+      keys, vals, begin, end, nseg, nseg_dev, few, lists + nseg, counts);
   count_launch();
-  sort_cta<<<num_sms * 3, kBlock, sizeof(CtaSmem), side2>>>(keys, vals, begin, end,
-                                                       lists + 2 * static_cast<size_t>(nseg),
-                                                       counts);
+  sort_cta<<<num_sms * 3, kBlock, sizeof(CtaSmem), side2>>>(keys, vals, begin, end, nseg, nseg_dev,
+                                                            few, lists, counts);
   if (tasks.nelems > kCap) {
     // global phase in rounds; the host looks at the next round's list after
     // rounds 0, 1, 3, 7, ... and stops when it is empty (every range's budget
