@@ -116,7 +116,10 @@ struct cuflye_ctx {
   uint64_t runs_chained = 0;  // of the last call, on the run path
   std::map<std::string, uint64_t> pass_need;  // bytes each buffer was asked for in this pass
   uint64_t pass_retries = 0;   // passes of the last call run again on half their queries
-  uint64_t pass_hit_cap = 0;   // hits a pass may take after a retry in this call (0: no cap)
+  // hits ([1]: runs) a pass may take after a retry in this call (0: no cap); the
+  // hits also bound a batch of open groups' queries
+  uint64_t pass_cap[2] = {0, 0};
+  uint64_t open_hits = 0;      // of the batch of open groups' queries in work
   double alloc_ms = 0;         // host time of the last call in cudaMalloc / cudaFree
   uint64_t emission_fallbacks = 0;  // passes of the last call that fell back to emit + sort
 };
@@ -1185,7 +1188,7 @@ void run_hits(cuflye_ctx* c, PassState& ps, bool want_kmers, uint64_t bytes_per_
       static_cast<double>(avail) / (static_cast<double>(bytes_per_hit) + c->other_per_hit[0]));
   uint64_t hit_limit = fits;
   ps.fit_units = fits;
-  if (c->pass_hit_cap) hit_limit = std::min(hit_limit, c->pass_hit_cap);
+  if (c->pass_cap[0]) hit_limit = std::min(hit_limit, c->pass_cap[0]);
   // Under a caller's budget a pass keeps to the per-hit buffers an earlier
   // pass grew when they hold at least 90 % of what fits: growing them frees
   // and reallocates them, and that synchronizes the device.
@@ -1301,7 +1304,7 @@ void run_runs(cuflye_ctx* c, PassState& ps) {
   fits = std::min<uint64_t>(fits, 0xf0000000ull);  // group numbers are 32 bits
   ps.fit_units = fits;
   uint64_t run_limit = fits;
-  if (c->pass_hit_cap) run_limit = std::min(run_limit, c->pass_hit_cap);
+  if (c->pass_cap[1]) run_limit = std::min(run_limit, c->pass_cap[1]);
   if (ps.units > run_limit) {
     std::vector<uint64_t> qoff(nq + 1);
     CUFLYE_CHECK(cudaMemcpyAsync(qoff.data(), ps.q_off, (nq + 1) * 8ull, cudaMemcpyDeviceToHost,
@@ -1774,6 +1777,9 @@ uint64_t* upload(cuflye_ctx* c, const char* name, const std::vector<uint64_t>& v
 // radix sort's second key / value buffer, score and backtrack, plus about 2
 // bytes for the per-group tables, tiles, bitmaps and the sort's task list.
 constexpr uint64_t kChainBytesPerHit = 8 + 4 + 4 + 4 + 8 + 4 + 4 + 4 + 2;
+// And of a batch of open groups' queries: beside them the introsort's copy and
+// the groups' own hits.
+constexpr uint64_t kOpenBytesPerHit = kChainBytesPerHit + 12 + 12;
 
 // Hits of sp (generation order, sp.keys / sp.vals) in KmerMatch order, exact
 // among the equal keys listed as (query of sp, key): a stable radix sort by ext
@@ -1896,7 +1902,8 @@ uint64_t chain_open_groups(cuflye_ctx* c, PassState& ps, const RunTables& t, uin
       sp.nwin = sp.win_off_h.back();
       upload_batch(c, "x_batch", sp);
       sp.qb.words = ps.qb.words;
-      run_hits(c, sp, false, kChainBytesPerHit, true);  // a prefix of them, as many as fit
+      run_hits(c, sp, false, kOpenBytesPerHit, true);  // a prefix of them, as many as fit
+      c->open_hits = sp.nhits;
       uint32_t sq = 0;
       for (;;) {
         take(sq);
@@ -1982,6 +1989,7 @@ uint64_t chain_open_groups(cuflye_ctx* c, PassState& ps, const RunTables& t, uin
                                   t.counts + kRcPool, c->status, c->num_sms, st));
     mark(c, 4);
     ps.nhits += X;
+    c->open_hits = 0;
     i = j;
   }
   return exact;
@@ -2160,7 +2168,7 @@ float elapsed(cudaEvent_t a, cudaEvent_t b) {
 void reset_timing(cuflye_ctx* c) {
   c->passes = 0;
   c->pass_retries = 0;
-  c->pass_hit_cap = 0;
+  c->pass_cap[0] = c->pass_cap[1] = 0;
   c->alloc_ms = 0;
   c->runs_chained = 0;
   c->emission_fallbacks = 0;
@@ -2262,6 +2270,7 @@ void for_each_pass(cuflye_ctx* c, const Queries& Q, bool kmers, uint64_t bytes_p
     PassState ps;
     const WaitOnUnwind wait(c);
     c->pass_need.clear();
+    c->open_hits = 0;
     clock_start(c);
     upload_queries(c, Q, q0, q1, ps);
     if (!by_runs) run_hits(c, ps, kmers, bytes_per_hit);
@@ -2282,8 +2291,10 @@ void for_each_pass(cuflye_ctx* c, const Queries& Q, bool kmers, uint64_t bytes_p
         upw = 0;
         continue;
       }
-      // later passes of the call stay at the size that is tried next
-      c->pass_hit_cap = std::max<uint64_t>(1, ps.units / 2);
+      // later passes of the call stay at the size that is tried next (units are
+      // not known yet when the counting itself found no room)
+      if (ps.units) c->pass_cap[by_runs ? 1 : 0] = std::max<uint64_t>(1, ps.units / 2);
+      if (c->open_hits) c->pass_cap[0] = std::max<uint64_t>(1, c->open_hits / 2);
       step = std::max<size_t>(ps.nq / 2, 1);
       continue;
     }

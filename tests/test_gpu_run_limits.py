@@ -1,6 +1,8 @@
 """GPU: the run path where its side tables run out.  What does not fit takes the
 hit path; the rows stay those of the hit path and of the oracle."""
 
+import ctypes
+
 import pytest
 
 from test_gpu_parity import oracle_index, overlap_tuples_gpu, overlap_tuples_oracle
@@ -15,6 +17,12 @@ def _rows(gpu, reads, params):
         return gpu.overlaps(reads, params).tobytes()
     finally:
         gpu.set_sorted_emission(1)
+
+
+def _launches(be):
+    n = ctypes.c_uint64()
+    be._L.cuflye_kernel_launches(ctypes.byref(n))
+    return n.value
 
 
 def _tandem(copy_div, seed=21, **kw):
@@ -119,3 +127,42 @@ def test_open_groups_rows_find_room(gpu, oracle_mod, most):
     finally:
         gpu.set_run_limit("spare_pieces", None)
     assert overlap_tuples_gpu(rows) == exp
+
+
+def test_open_groups_share_batches_under_a_budget(built_lib):
+    """Queries of open groups whose hits take about four times the memory there is
+    go through in batches of many queries, not one by one: the launches stay
+    within a multiple of an unbounded call's, which takes them in one batch."""
+    import numpy as np
+    from cuflye_gb300 import synth
+    from cuflye_gb300.backend import CudaBackend, OverlapParams
+    rng = np.random.default_rng(12)
+    unit = synth.random_genome(rng, 250)
+    genome = np.concatenate([synth.random_genome(rng, 2500), unit, unit, unit,
+                             synth.random_genome(rng, 2500)])
+    n = 100
+    seqs = []
+    for _ in range(n):
+        a, b = int(rng.integers(0, 2000)), int(rng.integers(3800, len(genome)))
+        s = synth.mutate(rng, genome[a:b], 0.002, 0.0005, 0.0005)
+        seqs.append((synth.revcomp(s) if rng.random() < 0.5 else s).tobytes())
+    reads = synth.ReadSet.from_strings(np.arange(1, n + 1), seqs)
+    p = OverlapParams.make(**dict(synth.OVERLAP_PARAMS, kmer_size=15))
+    got, launches, held = [], [], 0
+    for budget in (0, 1):
+        with CudaBackend(device=0, memory_budget_bytes=budget and held) as be:
+            be.build_index(reads, 15, 1, 2000)
+            index_bytes = be.memory_stats()[0]
+            be.set_run_limit("spare_pieces", 0)  # every group with a repeated position is open
+            before = _launches(be)
+            got.append(be.overlaps(reads, p).tobytes())
+            launches.append(_launches(be) - before)
+            assert be.last_sort_stats()["match_libstdcxx"] == n
+            if not budget:
+                be.set_sorted_emission(0)
+                assert be.overlaps(reads, p).tobytes() == got[0]
+                hits = be.last_timing()[1][1] // 24
+                held = index_bytes + 66 * hits // 4
+    assert got[0] == got[1]
+    # eight batches (half the memory each, at worst) and as many passes
+    assert launches[1] <= 16 * launches[0], launches
