@@ -421,6 +421,7 @@ struct KeyRuns {
   uint64_t* kept_off;
   uint32_t* free_words;      // nw words that nothing needs any more
   uint32_t* free_run_words;  // nruns words
+  uint64_t* free_hist;       // the radix sort's scratch: nw / 32 + 1 words and more
   uint64_t nw, nruns, npos, nsolid, nrep;
 };
 
@@ -460,6 +461,7 @@ KeyRuns sort_and_classify(cuflye_ctx* c, uint64_t nw, const std::vector<int>& di
   CUFLYE_CHECK(cudaMemcpyAsync(t, tally, sizeof(t), cudaMemcpyDeviceToHost, st));
   sync(c);
   return KeyRuns{keys, vals, run_id, run_start, cls,   kept_off, flags, kept,
+                 reinterpret_cast<uint64_t*>(hist),
                  nw,   nruns, npos,  t[0],      t[1]};
 }
 
@@ -539,7 +541,7 @@ BuiltIndex build_one_range(cuflye_ctx* c, const WindowSet& w, const std::vector<
   }
   CUFLYE_CHECK(cudaMemsetAsync(bi.table, 0xff, bi.cap * sizeof(TableEntry), st));
   CUFLYE_CHECK(index_copy_positions(r.vals, r.run_id, r.run_start, r.cls, r.kept_off, w.nwin,
-                                    bi.pos, true, st, place));
+                                    bi.pos, true, st, place, r.free_hist));
   if (bi.nbr)
     CUFLYE_CHECK(index_neighbours(bi.pos, r.npos, w.words, w.base_off, w.slot_len, w.k, bi.nbr, st));
   CUFLYE_CHECK(index_insert(r.keys, bi.pos, r.run_start, r.cls, r.kept_off, r.nruns, 0, true,

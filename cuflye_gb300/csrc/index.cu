@@ -25,6 +25,7 @@
 // position array is then the same as one range's.
 // A standard form never equals ~0 (the all-T k-mer's standard form is the
 // all-A k-mer, 0), so ~0 marks an empty slot.
+#include <algorithm>
 #include <cstdint>
 
 #include "common.cuh"
@@ -183,15 +184,22 @@ __device__ __forceinline__ uint64_t run_of(const uint64_t* __restrict__ flags_sc
   return r;
 }
 
+// Entries of one target in a run up to which each finds its place by walking them.
+constexpr uint32_t kNear = 32;
+
 // window_order: the runs are in (target, window) order, not in bucket order.
-// place (optional): each solid element's place in its bucket.
+// place (optional): each solid element's place in its bucket.  A k-mer that one
+// target holds more than kNear times is left to far_positions_kernel: the walk
+// is quadratic (a build of one target of 2e6 equal k-mers: 2,474 ms, 1.4 so; of
+// 2e4: 2.0, 0.28).  far: the number of those
+// (zeroed by the caller), then where each starts.
 __global__ void copy_positions_kernel(const uint64_t* __restrict__ vals,
                                       const uint64_t* __restrict__ flags_scan,
                                       const uint64_t* __restrict__ run_start,
                                       const uint8_t* __restrict__ cls,
                                       const uint64_t* __restrict__ kept_off, uint64_t n,
                                       uint64_t* __restrict__ pos, bool window_order,
-                                      uint32_t* __restrict__ place) {
+                                      uint32_t* __restrict__ place, uint64_t* __restrict__ far) {
   const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const uint64_t r = run_of(flags_scan, run_start, i);
@@ -207,12 +215,81 @@ __global__ void copy_positions_kernel(const uint64_t* __restrict__ vals,
     const bool rev = (v >> 32) & 1u;
     uint64_t ahead = 0, later = 0;  // entries that go before this one, either side of it
     uint64_t lo = i, hi = i + 1;
-    for (; lo > r0 && (vals[lo - 1] >> 33) == t; --lo) ahead += !((vals[lo - 1] >> 32) & 1u);
-    for (; hi < r1 && (vals[hi] >> 33) == t; ++hi) later += rev || !((vals[hi] >> 32) & 1u);
+    for (; lo > r0 && i - lo <= kNear && (vals[lo - 1] >> 33) == t; --lo)
+      ahead += !((vals[lo - 1] >> 32) & 1u);
+    for (; hi < r1 && hi - lo <= kNear && (vals[hi] >> 33) == t; ++hi) later += 1;
+    if (hi - lo > kNear) {
+      if (lo == i)
+        far[1 + atomicAdd(reinterpret_cast<unsigned long long*>(far), 1ull)] = i;
+      return;
+    }
     at = (lo - r0) + ahead + (rev ? later : 0u);
   }
   pos[kept_off[r] + at] = v;
   if (place) place[i] = static_cast<uint32_t>(at);
+}
+
+constexpr int kFarBlock = 512;
+constexpr int kFarItems = 8;  // entries a thread and step: a step waits for its loads
+
+// The places of the entries that copy_positions_kernel left, in the same order: a
+// block a (k-mer, target), the forward entries before each by a scan.  Bound by
+// the latency of its steps of 4,096 entries.
+__global__ void __launch_bounds__(kFarBlock) far_positions_kernel(
+    const uint64_t* __restrict__ vals, const uint64_t* __restrict__ flags_scan,
+    const uint64_t* __restrict__ run_start, const uint64_t* __restrict__ kept_off,
+    const uint64_t* __restrict__ far, uint64_t* __restrict__ pos, uint32_t* __restrict__ place) {
+  __shared__ uint32_t ws[2][kFarBlock / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint64_t n = far[0];
+  for (uint64_t g = blockIdx.x; g < n; g += gridDim.x) {
+    const uint64_t first = far[1 + g];
+    const uint64_t r = run_of(flags_scan, run_start, first), r0 = run_start[r];
+    const uint64_t t = vals[first] >> 33, off = kept_off[r];
+    uint64_t end = first + 1, hi = run_start[r + 1];  // past the target's last entry
+    while (end < hi) {
+      const uint64_t mid = (end + hi) >> 1;
+      if ((vals[mid] >> 33) == t)
+        end = mid + 1;
+      else
+        hi = mid;
+    }
+    uint64_t forward = 0;  // of the entries before this step
+    int side = 0;
+    for (uint64_t i0 = first; i0 < end; i0 += kFarBlock * kFarItems, side ^= 1) {
+      const uint64_t w0 = i0 + warp * (32 * kFarItems) + lane;  // a warp's are consecutive
+      uint64_t v[kFarItems];
+      unsigned b[kFarItems];
+#pragma unroll
+      for (int u = 0; u < kFarItems; ++u) v[u] = w0 + 32 * u < end ? vals[w0 + 32 * u] : 0;
+      uint32_t mine = 0;
+#pragma unroll
+      for (int u = 0; u < kFarItems; ++u) {
+        b[u] = __ballot_sync(0xffffffffu, w0 + 32 * u < end && !((v[u] >> 32) & 1u));
+        mine += __popc(b[u]);
+      }
+      if (lane == 0) ws[side][warp] = mine;
+      __syncthreads();
+      uint64_t ahead = forward;
+      for (int w = 0; w < kFarBlock / 32; ++w) {
+        ahead += w < warp ? ws[side][w] : 0u;
+        forward += ws[side][w];
+      }
+#pragma unroll
+      for (int u = 0; u < kFarItems; ++u) {
+        const uint64_t i = w0 + 32 * u;
+        if (i < end) {
+          const bool rev = (v[u] >> 32) & 1u;
+          const uint64_t at = (first - r0) + ahead + __popc(b[u] & ((1u << lane) - 1u)) +
+                              (rev ? end - i - 1 : 0u);
+          pos[off + at] = v[u];
+          if (place) place[i] = static_cast<uint32_t>(at);
+        }
+        ahead += __popc(b[u]);
+      }
+    }
+    __syncthreads();  // ws is free for the next one
+  }
 }
 
 // The record of every window (DeviceIndex::windows).  Bound by its scattered
@@ -484,11 +561,21 @@ cudaError_t index_classify_runs(const uint64_t* run_start, uint64_t nruns, uint3
 cudaError_t index_copy_positions(const uint64_t* vals, const uint64_t* run_id,
                                  const uint64_t* run_start, const uint8_t* cls,
                                  const uint64_t* kept_off, uint64_t n, uint64_t* pos,
-                                 bool window_order, cudaStream_t s, uint32_t* place) {
+                                 bool window_order, cudaStream_t s, uint32_t* place,
+                                 uint64_t* far) {
   if (n == 0) return cudaSuccess;
+  if (window_order) {
+    const cudaError_t e = cudaMemsetAsync(far, 0, sizeof(uint64_t), s);
+    if (e != cudaSuccess) return e;
+  }
   count_launch();
   copy_positions_kernel<<<grid(n, 256), 256, 0, s>>>(vals, run_id, run_start, cls, kept_off, n,
-                                                     pos, window_order, place);
+                                                     pos, window_order, place, far);
+  if (window_order && n > kNear) {
+    count_launch();
+    far_positions_kernel<<<static_cast<unsigned>(std::min<uint64_t>(n / kNear, 1024)), kFarBlock, 0,
+                           s>>>(vals, run_id, run_start, kept_off, far, pos, place);
+  }
   return cudaGetLastError();
 }
 

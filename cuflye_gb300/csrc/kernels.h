@@ -166,12 +166,14 @@ cudaError_t index_classify_runs(const uint64_t* run_start, uint64_t nruns, uint3
                                 uint32_t max_freq, uint32_t* kept, uint8_t* cls,
                                 unsigned long long* tally, cudaStream_t s);
 // Solid runs' entries into pos, in (stored id, stored position) order.
-// window_order: the runs hold them in (target, window) order instead.
-// place (optional): each solid element's place in its bucket.
+// window_order: the runs hold them in (target, window) order instead; far is
+// then scratch of n / 32 + 1 words.  place (optional): each solid element's
+// place in its bucket.
 cudaError_t index_copy_positions(const uint64_t* vals, const uint64_t* run_id,
                                  const uint64_t* run_start, const uint8_t* cls,
                                  const uint64_t* kept_off, uint64_t n, uint64_t* pos,
-                                 bool window_order, cudaStream_t s, uint32_t* place = nullptr);
+                                 bool window_order, cudaStream_t s, uint32_t* place = nullptr,
+                                 uint64_t* far = nullptr);
 // Table insert of every solid and repetitive run, a solid run's positions
 // at pos + kept_off (pos_base + kept_off of the position array).  Solid buckets that list
 // one stored id twice get kDupIdsBit (sorted_ids: runs are in (id, position)
