@@ -30,6 +30,7 @@
 #include <iterator>
 #include <map>
 #include <mutex>
+#include <shared_mutex>
 #include <stdexcept>
 #include <string>
 #include <unordered_map>
@@ -109,6 +110,15 @@ struct cuflye_ctx {
   uint64_t build_ranges = 0;      // key ranges of the last index build
   int servers = 0;           // open serving loops and shared contexts borrowing this index
   cuflye_ctx* lender = nullptr;  // the context whose index this one borrows (cuflye_open_shared)
+  // the context whose index this one reads, if not its own (also of a serving
+  // worker); such a context's passes hold that one's index_mu shared, and taking
+  // tables out of the index holds it exclusively (after that context's mu)
+  cuflye_ctx* index_of = nullptr;
+  std::shared_mutex index_mu;
+  // bytes of the index's tables given back; a serving worker's budget is its share
+  // of what the owner has left, and of what is given back from then on
+  uint64_t given_back = 0;
+  uint64_t base_budget = 0, base_given = 0, workers = 0;
   int sorted_emission = 1;  // see cuflye_set_sorted_emission
   // a pass body's buffers beyond the per-hit ones, per hit ([1]: beyond the
   // per-run ones, per run, on the run path)
@@ -703,6 +713,22 @@ void drop_run_tables(cuflye_ctx* c) {
   c->idx.tbase = nullptr;
 }
 
+// Whether the index has tables that only make calls faster: the run path's, the
+// windows' records and the filter.
+bool has_extras(const DeviceIndex& idx) { return idx.nbr || idx.windows || idx.filter; }
+
+// Gives them back (the caller holds c's mu and index_mu).
+void drop_extras(cuflye_ctx* c) {
+  const uint64_t before = c->in_use;
+  drop_run_tables(c);
+  for (const char* t : {"ix_windows", "ix_winoff", "ix_filter"}) release(c, t);
+  c->idx.windows = nullptr;
+  c->idx.filter = nullptr;
+  c->idx.win_off = nullptr;
+  c->given_back += before - c->in_use;
+  drop_spares(c, 0);
+}
+
 // A build in one range has the bytes already (its records need them).
 void keep_run_tables(cuflye_ctx* c, const BuiltIndex& bi, int k, const int32_t* d_len) {
   uint8_t* nbr = bi.nbr ? bi.nbr : neighbour_bytes(c, k, bi.npos);
@@ -848,6 +874,11 @@ void build_index_entries(cuflye_ctx* c, int k, size_t n, const int64_t* tids, co
                          const uint64_t* keys_h, size_t nrep, const uint64_t* rep_h) {
   if (k < 1 || k > 31) throw Error(CUFLYE_ERR_UNSUPPORTED, "k must be in [1, 31]");
   c->has_index = false;
+  for (const char* x : {"ix_windows", "ix_winoff", "ix_filter"}) release(c, x);
+  drop_run_tables(c);
+  c->idx.windows = nullptr;
+  c->idx.filter = nullptr;
+  c->idx.win_off = nullptr;
   std::vector<int64_t> absids;
   for (size_t i = 0; i < n; ++i) {
     if (tids[i] == 0) throw Error(CUFLYE_ERR_INVALID, "target id must not be zero");
@@ -925,11 +956,6 @@ void build_index_entries(cuflye_ctx* c, int k, size_t n, const int64_t* tids, co
     release(c, t);
   c->idx.k = k;
   c->idx.transform = false;
-  for (const char* t : {"ix_windows", "ix_winoff", "ix_filter"}) release(c, t);
-  drop_run_tables(c);
-  c->idx.windows = nullptr;
-  c->idx.filter = nullptr;
-  c->idx.win_off = nullptr;
   c->idx.table = table;
   c->idx.cap = cap;
   c->idx.pos = pos;
@@ -2249,17 +2275,72 @@ void release_pass_buffers(cuflye_ctx* c) {
   for (const std::string& n : names) release(c, n);
 }
 
+// Frees every buffer but the index, the graph, the logf table and the status word.
+void release_scratch(cuflye_ctx* c) {
+  std::vector<std::string> names;
+  for (const auto& kv : c->bufs) {
+    const std::string& n = kv.first;
+    const bool keep = n.compare(0, 3, "ix_") == 0 || n.compare(0, 3, "gr_") == 0 ||
+                      n.compare(0, 5, "logf_") == 0 || n == "status";
+    if (!keep) names.push_back(n);
+  }
+  for (const std::string& n : names) release(c, n);
+  drop_spares(c, 0);
+}
+
+// The index as a call reads it: a context that borrows it holds it against
+// give_back and takes up what that has changed.
+using IndexHold = std::shared_lock<std::shared_mutex>;
+void hold_index(cuflye_ctx* c, IndexHold& hold) {
+  if (!c->index_of) return;
+  hold = IndexHold(c->index_of->index_mu);
+  const DeviceIndex& o = c->index_of->idx;
+  c->idx.nbr = o.nbr;
+  c->idx.twords = o.twords;
+  c->idx.tbase = o.tbase;
+  c->idx.windows = o.windows;
+  c->idx.win_off = o.win_off;
+  c->idx.filter = o.filter;
+  if (c->workers)
+    c->budget = c->base_budget + (c->index_of->given_back - c->base_given) / c->workers;
+}
+
+// Makes room for a query that does not fit: this context's scratch and the
+// index's extra tables go (from all contexts that read it; later calls do without
+// until the next build).  False when there were none.
+bool give_back(cuflye_ctx* c, IndexHold& hold) {
+  if (!has_extras(c->idx)) return false;
+  release_scratch(c);
+  if (!c->index_of) {
+    std::unique_lock<std::shared_mutex> alone(c->index_mu);
+    drop_extras(c);
+    return true;
+  }
+  if (hold.owns_lock()) hold.unlock();
+  {
+    std::lock_guard<std::mutex> lock(c->index_of->mu);
+    std::unique_lock<std::shared_mutex> alone(c->index_of->index_mu);
+    if (has_extras(c->index_of->idx)) drop_extras(c->index_of);
+  }
+  hold_index(c, hold);
+  return true;
+}
+
 // Runs passes over [0, n): `body(q0, q1, ps)` consumes each pass.  A body
 // whose later buffers (per-group tables, the row pool) do not fit the budget
 // runs again on the first half of the pass's queries; bodies make their
 // results visible only after their last allocation, so the retry repeats no
 // output.
 //
-// runs: passes take the run path.  A single query whose run path does not fit
-// takes the hit path.
+// chains: what the passes chain with, if they do; they take the run path where
+// run_path says so.  A single query whose run path does not fit takes the hit path,
+// and one that does not fit there takes it without the index's extra tables.
 template <typename Body>
-void for_each_pass(cuflye_ctx* c, const Queries& Q, bool kmers, uint64_t bytes_per_hit, bool runs,
-                   Body body) {
+void for_each_pass(cuflye_ctx* c, const Queries& Q, bool kmers, uint64_t bytes_per_hit,
+                   const ChainParams* chains, Body body) {
+  IndexHold hold;
+  hold_index(c, hold);
+  bool runs = chains && run_path(c, *chains);
   size_t q0 = 0;
   const size_t full = std::max<size_t>(pass_size(c, Q.n), 1);
   size_t step = full;
@@ -2274,16 +2355,27 @@ void for_each_pass(cuflye_ctx* c, const Queries& Q, bool kmers, uint64_t bytes_p
     c->pass_need.clear();
     c->open_hits = 0;
     clock_start(c);
-    upload_queries(c, Q, q0, q1, ps);
-    if (!by_runs) run_hits(c, ps, kmers, bytes_per_hit);
+    bool counted = false;
     try {
-      if (by_runs) run_runs(c, ps);
+      upload_queries(c, Q, q0, q1, ps);
+      if (by_runs)
+        run_runs(c, ps);
+      else
+        run_hits(c, ps, kmers, bytes_per_hit);
+      counted = true;
       q1 = q0 + ps.nq;
       body(q0, q1, ps);
     } catch (const Error& e) {
-      if (e.code != CUFLYE_ERR_BUDGET || (ps.nq <= 1 && !by_runs)) throw;
-      // the failed body's buffers go, so that half the queries find room
+      if (e.code != CUFLYE_ERR_BUDGET) throw;
       sync(c);
+      if (!by_runs && (ps.nq <= 1 || !counted)) {
+        // one query does not fit (the counting takes as many as do)
+        if (!give_back(c, hold)) throw;
+        ++c->pass_retries;
+        runs = false;
+        continue;
+      }
+      // the failed body's buffers go, so that half the queries find room
       release_pass_buffers(c);
       ++c->pass_retries;
       if (ps.nq <= 1) {
@@ -2375,6 +2467,19 @@ thread_local std::string t_open_error;
   if (!(ctx)) return CUFLYE_ERR_INVALID;        \
   std::lock_guard<std::mutex> lock_((ctx)->mu); \
   try {
+// A call that does not read the index's extra tables, as a whole: it runs once more
+// without them when the memory they take is what it lacks.
+#define CUFLYE_ROOM_BEGIN           \
+  for (IndexHold hold_;;) {         \
+    try {
+#define CUFLYE_ROOM_END(ctx)                        \
+      break;                                        \
+    } catch (const Error& e) {                      \
+      if (e.code != CUFLYE_ERR_BUDGET) throw;       \
+      sync(ctx);                                    \
+      if (!give_back(ctx, hold_)) throw;            \
+    }                                               \
+  }
 #define CUFLYE_API_END(ctx)           \
   }                                   \
   catch (const Error& e) {            \
@@ -2496,7 +2601,7 @@ cuflye_status cuflye_open_shared(cuflye_ctx* owner, uint64_t memory_budget_bytes
   c->slot_of = owner->slot_of;
   c->slot_signed_h = owner->slot_signed_h;
   c->has_index = true;
-  c->lender = owner;
+  c->lender = c->index_of = owner;  // (an owner's index is its own)
   ++owner->servers;
   *out = c;
   return CUFLYE_OK;
@@ -2612,7 +2717,7 @@ namespace {
 // device.
 double overlaps_device_ms(cuflye_ctx* c, const Queries& Q, const ChainParams& cp) {
   reset_timing(c);
-  for_each_pass(c, Q, false, kChainBytesPerHit, run_path(c, cp),
+  for_each_pass(c, Q, false, kChainBytesPerHit, &cp,
                 [&](size_t, size_t, PassState& ps) {
     run_chain(c, ps, cp);
     mark(c, 5);
@@ -2688,7 +2793,7 @@ cuflye_status cuflye_candidates(cuflye_ctx* c, size_t n, const int64_t* ids,
   Queries Q{n, ids, offsets, bases};
   size_t total = 0, ftotal = 0;
   bool overflow = false;
-  for_each_pass(c, Q, true, 8 + 4 + 8 + 32, false, [&](size_t, size_t, PassState& ps) {
+  for_each_pass(c, Q, true, 8 + 4 + 8 + 32, nullptr, [&](size_t, size_t, PassState& ps) {
     mark(c, 0);
     if (!overflow && total + ps.nhits <= out_cap && ftotal + ps.nfilt <= filtered_cap) {
       cuflye_candidate* d_out = buf<cuflye_candidate>(c, "a_cand", ps.nhits);
@@ -2734,7 +2839,7 @@ cuflye_status cuflye_overlaps(cuflye_ctx* c, size_t n, const int64_t* ids, const
   size_t total = 0;
   bool overflow = false;
   uint64_t hits_total = 0, windows_total = 0, bases_total = 0;
-  for_each_pass(c, Q, false, kChainBytesPerHit, run_path(c, cp),
+  for_each_pass(c, Q, false, kChainBytesPerHit, &cp,
                 [&](size_t q0, size_t q1, PassState& ps) {
     const ChainRows rows = run_chain(c, ps, cp);
     const uint64_t R = rows.n;
@@ -2788,12 +2893,14 @@ cuflye_status cuflye_graph_set(cuflye_ctx* c, size_t ne, const int64_t* edge_ids
     if (eos[s] == 0)
       throw Error(CUFLYE_ERR_INVALID, "indexed sequence " + std::to_string(c->slot_signed_h[s]) +
                                           " has no graph edge");
+  CUFLYE_ROOM_BEGIN
   int64_t* de = buf<int64_t>(c, "gr_edge", ns);
   int32_t* dl = buf<int32_t>(c, "gr_left", ns);
   int32_t* dr = buf<int32_t>(c, "gr_right", ns);
   CUFLYE_CHECK(cudaMemcpy(de, eos.data(), ns * 8ull, cudaMemcpyHostToDevice));
   CUFLYE_CHECK(cudaMemcpy(dl, l.data(), ns * 4ull, cudaMemcpyHostToDevice));
   CUFLYE_CHECK(cudaMemcpy(dr, r.data(), ns * 4ull, cudaMemcpyHostToDevice));
+  CUFLYE_ROOM_END(c)
   c->has_graph = true;
   CUFLYE_API_END(c)
 }
@@ -2964,7 +3071,7 @@ cuflye_status cuflye_read_to_graph(cuflye_ctx* c, size_t n, const int64_t* ids,
   size_t total = 0;
   uint64_t chain_base = 0;
   bool overflow = false;
-  for_each_pass(c, Q, false, kChainBytesPerHit, run_path(c, cp),
+  for_each_pass(c, Q, false, kChainBytesPerHit, &cp,
                 [&](size_t q0, size_t, PassState& ps) {
     R2GPass r = r2g_candidates(c, ps, cp, rp, ids + q0);
     const uint64_t nrows =
@@ -3006,7 +3113,7 @@ cuflye_status cuflye_read_to_graph_chains(cuflye_ctx* c, size_t n, const int64_t
   Queries Q{n, ids, offsets, bases};
   size_t total = 0;
   bool overflow = false;
-  for_each_pass(c, Q, false, kChainBytesPerHit, run_path(c, cp),
+  for_each_pass(c, Q, false, kChainBytesPerHit, &cp,
                 [&](size_t q0, size_t, PassState& ps) {
     R2GPass r = r2g_candidates(c, ps, cp, rp, ids + q0);
     const uint64_t nrec = r2g_chain_records(c, r, rp, r.read_ids);
@@ -3058,6 +3165,7 @@ cuflye_status cuflye_chain_read_alignments(
   }
   if (fixture_offsets && n_fixtures && fixture_offsets[0] != 0)
     throw Error(CUFLYE_ERR_INVALID, "fixture offsets must start at 0");
+  CUFLYE_ROOM_BEGIN
   reset_timing(c);
   const R2GParams rp = to_r2g_params(r2g);
   cudaStream_t st = c->stream;
@@ -3147,6 +3255,7 @@ cuflye_status cuflye_chain_read_alignments(
     throw Error(CUFLYE_ERR_CAPACITY, "output capacity too small: need " + std::to_string(nrec) +
                                          " chain records, " + std::to_string(nchains) +
                                          " chains, " + std::to_string(nrows) + " rows");
+  CUFLYE_ROOM_END(c)
   CUFLYE_API_END(c)
 }
 
@@ -3195,6 +3304,7 @@ cuflye_status cuflye_std_sort_segments(cuflye_ctx* c, uint64_t* keys, uint32_t* 
   cudaStream_t st = c->stream;
   const uint64_t base = seg_offsets[0];
   const uint64_t m = n - base;
+  CUFLYE_ROOM_BEGIN
   uint64_t* dk = buf<uint64_t>(c, "t_keys", m);
   uint32_t* dv = buf<uint32_t>(c, "t_vals", m);
   uint32_t* dl = buf<uint32_t>(c, "t_l", m + 1);
@@ -3214,6 +3324,7 @@ cuflye_status cuflye_std_sort_segments(cuflye_ctx* c, uint64_t* keys, uint32_t* 
   CUFLYE_CHECK(cudaMemcpyAsync(keys + base, dk, m * 8, cudaMemcpyDeviceToHost, st));
   CUFLYE_CHECK(cudaMemcpyAsync(values + base, dv, m * 4, cudaMemcpyDeviceToHost, st));
   sync(c);
+  CUFLYE_ROOM_END(c)
   CUFLYE_API_END(c)
 }
 
@@ -3242,15 +3353,7 @@ cuflye_status cuflye_last_passes(const cuflye_ctx* c, uint64_t* passes) {
 cuflye_status cuflye_trim(cuflye_ctx* c) {
   CUFLYE_API_BEGIN(c)
   sync(c);
-  std::vector<std::string> names;
-  for (const auto& kv : c->bufs) {
-    const std::string& n = kv.first;
-    const bool keep = n.compare(0, 3, "ix_") == 0 || n.compare(0, 3, "gr_") == 0 ||
-                      n.compare(0, 5, "logf_") == 0 || n == "status";
-    if (!keep) names.push_back(n);
-  }
-  for (const std::string& n : names) release(c, n);
-  drop_spares(c, 0);
+  release_scratch(c);
   CUFLYE_API_END(c)
 }
 
@@ -3324,7 +3427,7 @@ void overlaps_collect(cuflye_ctx* c, const Queries& Q, const ChainParams& cp,
   rows.clear();
   per_query.assign(Q.n, 0);
   reset_timing(c);
-  for_each_pass(c, Q, false, kChainBytesPerHit, run_path(c, cp),
+  for_each_pass(c, Q, false, kChainBytesPerHit, &cp,
                 [&](size_t q0, size_t, PassState& ps) {
     const ChainRows cr = run_chain(c, ps, cp);
     const uint64_t R = cr.n;
@@ -3448,17 +3551,26 @@ cuflye_status cuflye_server_open(cuflye_ctx* owner, int workers,
   CUFLYE_CHECK(cudaSetDevice(owner->device));
   drop_spares(owner, 0);
   // the workers share what is left of the budget (or of the free memory)
-  uint64_t avail = 0;
-  if (owner->budget) {
-    avail = owner->budget > owner->in_use ? owner->budget - owner->in_use : 0;
-  } else {
-    size_t free_b = 0, total_b = 0;
-    CUFLYE_CHECK(cudaMemGetInfo(&free_b, &total_b));
-    const uint64_t margin = 8ull << 30;
-    avail = free_b > margin ? free_b - margin : free_b / 2;
+  auto share = [&]() -> uint64_t {
+    uint64_t avail = 0;
+    if (owner->budget) {
+      avail = owner->budget > owner->in_use ? owner->budget - owner->in_use : 0;
+    } else {
+      size_t free_b = 0, total_b = 0;
+      CUFLYE_CHECK(cudaMemGetInfo(&free_b, &total_b));
+      const uint64_t margin = 8ull << 30;
+      avail = free_b > margin ? free_b - margin : free_b / 2;
+    }
+    return avail / static_cast<uint64_t>(workers);
+  };
+  constexpr uint64_t kLeastShare = 64ull << 20;
+  uint64_t per = share();
+  if (per < kLeastShare && !owner->index_of && has_extras(owner->idx)) {
+    std::unique_lock<std::shared_mutex> alone(owner->index_mu);
+    drop_extras(owner);
+    per = share();
   }
-  const uint64_t per = avail / static_cast<uint64_t>(workers);
-  if (per < (64ull << 20))
+  if (per < kLeastShare)
     throw Error(CUFLYE_ERR_BUDGET, "memory budget leaves under 64 MiB per serving worker");
   s = new cuflye_server();
   s->owner = owner;
@@ -3478,6 +3590,13 @@ cuflye_status cuflye_server_open(cuflye_ctx* owner, int workers,
     c->slot_of = owner->slot_of;
     c->slot_signed_h = owner->slot_signed_h;
     c->has_index = true;
+    // (an owner that borrows its index itself has a budget that the index is not in)
+    c->index_of = owner->index_of ? owner->index_of : owner;
+    if (!owner->index_of) {
+      c->base_budget = per;
+      c->base_given = owner->given_back;
+      c->workers = static_cast<uint64_t>(workers);
+    }
     s->workers.push_back(c);
   }
   for (cuflye_ctx* c : s->workers) s->threads.emplace_back(serve_worker, s, c);
