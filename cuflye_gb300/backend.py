@@ -122,6 +122,8 @@ def load_library(path: Path | None = None) -> ctypes.CDLL:
     L.cuflye_last_error.argtypes = [_vp]
     L.cuflye_memory_stats.restype = S
     L.cuflye_memory_stats.argtypes = [_vp, _u64p, _u64p]
+    L.cuflye_memory_spares.restype = S
+    L.cuflye_memory_spares.argtypes = [_vp, _u64p]
     L.cuflye_index_build.restype = S
     L.cuflye_index_build.argtypes = [_vp, ctypes.c_int, ctypes.c_size_t, _i64p, _i64p,
                                      ctypes.c_char_p, ctypes.c_uint32, ctypes.c_uint32]
@@ -295,6 +297,12 @@ class CudaBackend:
         a, b = ctypes.c_uint64(), ctypes.c_uint64()
         self._check(self._L.cuflye_memory_stats(self._h, ctypes.byref(a), ctypes.byref(b)))
         return a.value, b.value
+
+    def memory_spares(self) -> int:
+        """Bytes of released buffers kept for the next allocations."""
+        a = ctypes.c_uint64()
+        self._check(self._L.cuflye_memory_spares(self._h, ctypes.byref(a)))
+        return a.value
 
     def set_batch_queries(self, n: int) -> None:
         self._check(self._L.cuflye_set_batch_queries(self._h, int(n)))

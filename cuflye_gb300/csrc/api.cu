@@ -75,7 +75,8 @@ struct cuflye_ctx {
   uint64_t in_use = 0, peak = 0;
   // released buffers kept for the next allocation of about their size, oldest
   // first: at most 1/16 of the budget (or of the device), given back when
-  // memory runs short and by cuflye_trim
+  // memory runs short, this context's or another's, and by cuflye_trim (behind
+  // spares_mu)
   std::vector<DevBuf> spare;
   uint64_t spare_bytes = 0, spare_limit = 0;
   DeviceStatus* status = nullptr;
@@ -148,8 +149,13 @@ struct AllocTimer {
   }
 };
 
-// Gives the oldest spare buffers back until at most `most` bytes are kept.
-void drop_spares(cuflye_ctx* c, uint64_t most) {
+// The open contexts, and the lock on every context's spares: one that finds no
+// memory frees those of all contexts on its device.
+std::mutex spares_mu;
+std::vector<cuflye_ctx*> open_contexts;
+
+// Frees the oldest spares until at most `most` bytes are kept (spares_mu held).
+void free_spares(cuflye_ctx* c, uint64_t most) {
   size_t n = 0;
   while (n < c->spare.size() && c->spare_bytes > most) {
     cudaFree(c->spare[n].p);
@@ -158,19 +164,65 @@ void drop_spares(cuflye_ctx* c, uint64_t most) {
   c->spare.erase(c->spare.begin(), c->spare.begin() + static_cast<std::ptrdiff_t>(n));
 }
 
+void drop_spares(cuflye_ctx* c, uint64_t most) {
+  std::lock_guard<std::mutex> lock(spares_mu);
+  free_spares(c, most);
+}
+
+// Frees the spares of every context on the device; false when there were none.
+// Work that another context queued may still use one of its own.
+bool drop_all_spares(int device) {
+  std::lock_guard<std::mutex> lock(spares_mu);
+  bool any = false;
+  for (cuflye_ctx* c : open_contexts) {
+    if (c->device != device || c->spare.empty()) continue;
+    if (!any) cudaDeviceSynchronize();
+    any = true;
+    free_spares(c, 0);
+  }
+  return any;
+}
+
+uint64_t all_spare_bytes(int device) {
+  std::lock_guard<std::mutex> lock(spares_mu);
+  uint64_t bytes = 0;
+  for (const cuflye_ctx* c : open_contexts)
+    if (c->device == device) bytes += c->spare_bytes;
+  return bytes;
+}
+
 // A buffer out of use: kept as a spare, or freed when it is beyond the limit.
 // Whoever takes it next uses it on the context's stream (the side streams join
 // that one before a call's next step), so after what was launched on it here.
 void retire(cuflye_ctx* c, const DevBuf& b) {
   if (!b.p) return;
+  std::lock_guard<std::mutex> lock(spares_mu);
   c->in_use -= b.cap;
   if (b.cap > c->spare_limit) {
     cudaFree(b.p);
     return;
   }
-  drop_spares(c, c->spare_limit - b.cap);
+  free_spares(c, c->spare_limit - b.cap);
   c->spare.push_back(b);
   c->spare_bytes += b.cap;
+}
+
+// The smallest spare of at least `bytes` and at most a quarter more, if any.
+bool take_spare(cuflye_ctx* c, size_t bytes, DevBuf& b) {
+  std::lock_guard<std::mutex> lock(spares_mu);
+  auto best = c->spare.end();
+  for (auto it = c->spare.begin(); it != c->spare.end(); ++it)
+    if (it->cap >= bytes && it->cap - bytes <= bytes / 4 &&
+        (!c->budget || c->in_use + it->cap <= c->budget) &&
+        (best == c->spare.end() || it->cap < best->cap))
+      best = it;
+  if (best == c->spare.end()) return false;
+  b = *best;
+  c->spare.erase(best);
+  c->spare_bytes -= b.cap;
+  c->in_use += b.cap;
+  c->peak = std::max(c->peak, c->in_use);
+  return true;
 }
 
 template <typename T>
@@ -196,21 +248,7 @@ T* buf(cuflye_ctx* c, const std::string& name, uint64_t count) {
   retire(c, b);
   b.p = nullptr;
   b.cap = 0;
-  // the smallest spare that is large enough and at most a quarter too large
-  auto best = c->spare.end();
-  for (auto it = c->spare.begin(); it != c->spare.end(); ++it)
-    if (it->cap >= alloc && it->cap - alloc <= alloc / 4 &&
-        (!c->budget || c->in_use + it->cap <= c->budget) &&
-        (best == c->spare.end() || it->cap < best->cap))
-      best = it;
-  if (best != c->spare.end()) {
-    b = *best;
-    c->spare.erase(best);
-    c->spare_bytes -= b.cap;
-    c->in_use += b.cap;
-    c->peak = std::max(c->peak, c->in_use);
-    return static_cast<T*>(b.p);
-  }
+  if (take_spare(c, alloc, b)) return static_cast<T*>(b.p);
   // a build's scratch comes in steps of a sixteenth, so that the next build's
   // fits it
   if (name.compare(0, 3, "ib_") == 0 && alloc >= (1u << 20)) {
@@ -219,13 +257,11 @@ T* buf(cuflye_ctx* c, const std::string& name, uint64_t count) {
     const size_t up = (alloc + step - 1) / step * step;
     if (!c->budget || c->in_use + up <= c->budget) alloc = up;
   }
-  if (c->budget && c->in_use + c->spare_bytes + alloc > c->budget)
-    drop_spares(c, c->budget - c->in_use - alloc);
+  if (c->budget) drop_spares(c, c->budget - c->in_use - alloc);
   cudaError_t e = cudaMalloc(&b.p, alloc);
-  if (e == cudaErrorMemoryAllocation && !c->spare.empty()) {
+  if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
-    drop_spares(c, 0);
-    e = cudaMalloc(&b.p, alloc);
+    if (drop_all_spares(c->device)) e = cudaMalloc(&b.p, alloc);
   }
   if (e != cudaSuccess) {
     cudaGetLastError();
@@ -381,7 +417,7 @@ uint64_t effective_budget(cuflye_ctx* c) {
   if (c->budget) return c->budget;
   size_t free_b = 0, total_b = 0;
   CUFLYE_CHECK(cudaMemGetInfo(&free_b, &total_b));
-  const uint64_t cap = static_cast<uint64_t>(free_b) + c->in_use + c->spare_bytes;
+  const uint64_t cap = static_cast<uint64_t>(free_b) + c->in_use + all_spare_bytes(c->device);
   const uint64_t margin = 8ull << 30;
   return cap > margin ? cap - margin : cap / 2;
 }
@@ -2532,6 +2568,8 @@ cuflye_status cuflye_open(int device, uint64_t memory_budget_bytes, cuflye_ctx**
     c->status = buf<DeviceStatus>(c, "status", 1);
     CUFLYE_CHECK(cudaMemset(c->status, 0, sizeof(DeviceStatus)));
     load_logf_table(c);
+    std::lock_guard<std::mutex> lock(spares_mu);
+    open_contexts.push_back(c);
   } catch (const Error& e) {
     t_open_error = stub_fields(device, memory_budget_bytes) + e.what();
     cuflye_close(c);
@@ -2617,7 +2655,12 @@ void cuflye_close(cuflye_ctx* c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   for (auto& kv : c->bufs)
     if (kv.second.p) cudaFree(kv.second.p);
-  drop_spares(c, 0);
+  {
+    std::lock_guard<std::mutex> lock(spares_mu);
+    open_contexts.erase(std::remove(open_contexts.begin(), open_contexts.end(), c),
+                        open_contexts.end());
+    free_spares(c, 0);
+  }
   if (c->side) cudaStreamSynchronize(c->side);
   if (c->side2) cudaStreamSynchronize(c->side2);
   for (auto& e : c->clock) cudaEventDestroy(e);
@@ -2638,6 +2681,13 @@ cuflye_status cuflye_memory_stats(const cuflye_ctx* c, uint64_t* in_use, uint64_
   if (!c) return CUFLYE_ERR_INVALID;
   if (in_use) *in_use = c->in_use;
   if (peak) *peak = c->peak;
+  return CUFLYE_OK;
+}
+
+cuflye_status cuflye_memory_spares(const cuflye_ctx* c, uint64_t* bytes) {
+  if (!c || !bytes) return CUFLYE_ERR_INVALID;
+  std::lock_guard<std::mutex> lock(spares_mu);
+  *bytes = c->spare_bytes;
   return CUFLYE_OK;
 }
 
@@ -3549,7 +3599,11 @@ cuflye_status cuflye_server_open(cuflye_ctx* owner, int workers,
   check_params(owner, params);
   if (workers < 1 || workers > 8) throw Error(CUFLYE_ERR_INVALID, "workers must be in [1, 8]");
   CUFLYE_CHECK(cudaSetDevice(owner->device));
-  drop_spares(owner, 0);
+  // (without a budget the others' spares are memory to share, too)
+  if (owner->budget)
+    drop_spares(owner, 0);
+  else
+    drop_all_spares(owner->device);
   // the workers share what is left of the budget (or of the free memory)
   auto share = [&]() -> uint64_t {
     uint64_t avail = 0;

@@ -88,12 +88,15 @@ void cuflye_close(cuflye_ctx* ctx);
  * patches/flye/2.9.6/0003-cuflye-cuda-backend-stub.patch:37-46 throws them. */
 const char* cuflye_last_error(const cuflye_ctx* ctx);
 
-/* Device memory of the context's buffers now and at its peak, in bytes.
- * Neither counts the released buffers that it keeps for its next allocations:
- * at most 1/16 of its budget (or of the device's memory without one), within
- * the budget, given back when memory runs short, by cuflye_trim and when a
- * serving loop opens on the context. */
+/* Device memory of the context's buffers now and at its peak, in bytes.  Beside
+ * them it keeps released ones for its next allocations (cuflye_memory_spares;
+ * neither figure counts them): at most 1/16 of its budget (or of the device's
+ * memory without one), within the budget, given back when memory runs short, by
+ * cuflye_trim and when a serving loop opens on the context.  An allocation that
+ * fails frees those of every context of the process on the device and is tried
+ * again. */
 cuflye_status cuflye_memory_stats(const cuflye_ctx* ctx, uint64_t* in_use, uint64_t* peak);
+cuflye_status cuflye_memory_spares(const cuflye_ctx* ctx, uint64_t* bytes);
 
 /* --------------------------------------------------------------------------
  * Index (Flye VertexIndex equivalent, device resident).
