@@ -1574,12 +1574,13 @@ struct GroupRows {
 
 // Chains groups of hits: the surviving groups in dp_list (counts[1]), those
 // of them sorted by ext pos in ext_list (counts[0]), the hits of group g at
-// groups[g].start in KmerMatch order.
+// groups[g].start in KmerMatch order.  They are a pass's groups, or some of them:
+// pass_rows is then the rows that the pass has room for.
 GroupRows chain_groups(cuflye_ctx* c, uint64_t* keys, uint32_t* vals, uint64_t H,
                        GroupInfo* groups, uint64_t G, const uint32_t* ext_list,
                        const uint32_t* dp_list, const uint32_t* gcounts, const ChainParams& cp,
                        const QueryInfo* qinfo, const uint64_t* f_off, const int32_t* fpos,
-                       uint64_t* sstats, bool tally_pending,
+                       uint64_t* sstats, bool tally_pending, uint64_t pass_rows = 0,
                        const std::function<void()>& sorted = nullptr);
 
 // Sort + chaining of the pass's hits.
@@ -1746,7 +1747,7 @@ GroupRows chain_groups(cuflye_ctx* c, uint64_t* keys, uint32_t* vals, uint64_t H
                        GroupInfo* groups, uint64_t G, const uint32_t* ext_list,
                        const uint32_t* dp_list, const uint32_t* gcounts, const ChainParams& cp,
                        const QueryInfo* qinfo, const uint64_t* f_off, const int32_t* fpos,
-                       uint64_t* sstats, bool tally_pending,
+                       uint64_t* sstats, bool tally_pending, uint64_t pass_rows,
                        const std::function<void()>& sorted) {
   cudaStream_t st = c->stream;
   uint32_t* lscr = buf<uint32_t>(c, "s_l", H + 1);
@@ -1802,8 +1803,11 @@ GroupRows chain_groups(cuflye_ctx* c, uint64_t* keys, uint32_t* vals, uint64_t H
     c->hits_flagged += c->emit_tally[0];
     c->hits_prefiltered += c->emit_tally[1];
   }
-  // (a row a group beyond eight: one that max_divergence drops later)
-  const uint64_t pool_cap = 9ull * survivors + 1024;
+  // (a row a group beyond eight: one that max_divergence drops later; some of a
+  // pass's groups may have what the others leave)
+  const uint64_t pool_cap =
+      std::max(9ull * survivors + 1024,
+               std::min<unsigned long long>(1ull * kMaxGroupRows * survivors, pass_rows));
   OverlapRow* pool = buf<OverlapRow>(c, "o_pool", pool_cap);
   uint32_t* pool_count = buf<uint32_t>(c, "o_poolcount", 1);
   uint32_t* group_rows = buf<uint32_t>(c, "o_grows", G);
@@ -2047,7 +2051,8 @@ uint64_t chain_open_groups(cuflye_ctx* c, PassState& ps, const RunTables& t, uin
     };
     const GroupRows open =
         chain_groups(c, keys, vals, X, groups, o.n, ext_list, dp_list, gcounts, cp, ps.qinfo,
-                     ps.f_off, ps.fpos, sstats, false, ask ? settle : std::function<void()>());
+                     ps.f_off, ps.fpos, sstats, false, pool_cap,
+                     ask ? settle : std::function<void()>());
     CUFLYE_CHECK(runs_fold_rows(t, o.list, o.n, open.rows, group_rows, st));
     CUFLYE_CHECK(runs_append_rows(open.pool, open.pool_count, o.list, pool, pool_cap,
                                   t.counts + kRcPool, c->status, c->num_sms, st));

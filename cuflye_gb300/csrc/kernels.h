@@ -248,6 +248,9 @@ struct GroupInfo {
   int32_t ext_sorted;  // 0: cur-pos order; 1: re-sorted by ext pos; 2: ext order already
 };
 
+// Overlaps that a target group may propose, and so its rows at most.
+constexpr int kMaxGroupRows = 64;
+
 // Device-side overlap row before the final ABI conversion.
 struct OverlapRow {
   uint32_t query;

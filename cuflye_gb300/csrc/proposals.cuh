@@ -12,7 +12,7 @@
 
 namespace cuflye {
 
-constexpr int kMaxProposals = 64;
+constexpr int kMaxProposals = kMaxGroupRows;
 
 struct Prop {
   int32_t cb, ce, eb, ee, score, clen;

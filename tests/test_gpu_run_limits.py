@@ -166,3 +166,36 @@ def test_open_groups_share_batches_under_a_budget(built_lib):
     assert got[0] == got[1]
     # eight batches (half the memory each, at worst) and as many passes
     assert launches[1] <= 16 * launches[0], launches
+
+
+def test_open_groups_of_many_rows(gpu, oracle_mod):
+    """Open groups of about twenty rows each beside many groups of one: the open
+    ones have the room that the others leave."""
+    import numpy as np
+    from cuflye_gb300 import synth
+    from cuflye_gb300.backend import OverlapParams
+    rng = np.random.default_rng(6)
+    unit = synth.random_genome(rng, 150)
+    base = np.concatenate([synth.random_genome(rng, 500), unit, unit, synth.random_genome(rng, 500)])
+    other = synth.random_genome(rng, 1000)
+    seqs = [synth.mutate(rng, base, 0.006, 0, 0.0015) for _ in range(20)] + [other] * 60
+    reads = synth.ReadSet.from_strings(np.arange(1, len(seqs) + 1), [s.tobytes() for s in seqs])
+    params = dict(synth.OVERLAP_PARAMS, kmer_size=15, min_overlap=1, max_jump=16, max_gap=1,
+                  check_overhang=0, force_local=1, only_max_ext=0)
+    p = OverlapParams.make(**params)
+    oracle_mod.set_stable(False)
+    idx, batch = oracle_index(oracle_mod, reads, 15, 1, 1000)
+    exp = overlap_tuples_oracle(
+        oracle_mod.overlaps(idx, batch, oracle_mod.default_params(**params)))
+    of_open = sum(r[0] <= 20 for r in exp)
+    assert 9 * 400 + 1024 < of_open and len(exp) < 8 * (60 * 59 + 380) + 1024
+    gpu.build_index(reads, 15, 1, 1000)
+    hits = _rows(gpu, reads, p)
+    gpu.set_run_limit("spare_pieces", 0)
+    try:
+        rows = gpu.overlaps(reads, p)
+        assert gpu.last_sort_stats()["match_libstdcxx"] >= 20
+    finally:
+        gpu.set_run_limit("spare_pieces", None)
+    assert rows.tobytes() == hits
+    assert overlap_tuples_gpu(rows) == exp
