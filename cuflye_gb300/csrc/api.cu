@@ -514,6 +514,13 @@ KeyRuns sort_and_classify(cuflye_ctx* c, uint64_t nw, const std::vector<int>& di
 // Table slots for `entries` keys: twice as many (load 1/2), at least 16.
 uint64_t table_capacity(uint64_t entries) { return std::max<uint64_t>(16, 2 * entries); }
 
+// Least k of the run path.  Short k-mers match anywhere: most hits are runs of their
+// own, and most groups repeat positions and are left open, so that the hit path
+// chains them after all.  Calls of 20 to 100 reads, run path against hit path: k = 5
+// 39.8 / 13.8 ms, 7 39.4 / 23.0, 9 10.7 / 8.1 and 24.7 / 18.8, 11 8.0 / 8.5 and
+// 10.3 / 10.6, 13 3.7 / 5.0.
+constexpr int kRunLeastK = 11;
+
 // The run path's byte an entry (the bases around its k-mer), or null.  Kept for
 // an odd k (an even k has k-mers that equal their reverse complement) and while
 // it takes at most a quarter of the memory the index leaves (1 byte an entry
@@ -521,7 +528,7 @@ uint64_t table_capacity(uint64_t entries) { return std::max<uint64_t>(16, 2 * en
 uint8_t* neighbour_bytes(cuflye_ctx* c, int k, uint64_t npos) {
   const uint64_t limit = effective_budget(c);
   const uint64_t left = limit > c->in_use ? limit - c->in_use : 0;
-  if (k % 2 == 0 || npos + 16 > left / 4) return nullptr;
+  if (k % 2 == 0 || k < kRunLeastK || npos + 16 > left / 4) return nullptr;
   try {
     return buf<uint8_t>(c, "ix_nbr", npos + 32);
   } catch (const Error& e) {
@@ -1312,7 +1319,7 @@ void run_hits(cuflye_ctx* c, PassState& ps, bool want_kmers, uint64_t bytes_per_
 // follows it in Flye's DP.  cuflye_set_sorted_emission modes 0 and 2 ask for a
 // hit path.
 bool run_path(const cuflye_ctx* c, const ChainParams& cp) {
-  return c->idx.nbr && c->sorted_emission == 1 && cp.k >= 2 && cp.max_jump >= 2 &&
+  return c->idx.nbr && c->sorted_emission == 1 && cp.max_jump >= 2 &&
          cp.max_gap >= 0;
 }
 

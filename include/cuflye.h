@@ -216,11 +216,11 @@ cuflye_status cuflye_set_batch_queries(cuflye_ctx* ctx, size_t queries_per_pass)
  * hits (no counterpart in the reference).  The rows are the same either way.
  * 1 (the default): as runs of hits at consecutive positions, found, sorted and
  * chained without writing the hits, where the index holds the tables for it
- * (an odd k, and memory for a byte an entry and a quarter byte a base beside the
- * index; a build in one range also keeps 16 bytes a window, where there is room,
- * which make the lookups of indexed queries cheaper, and a filter of at most 32
- * MiB.  A call that lacks the memory these tables take gets it: they go, and calls
- * on the index do without them until the next build);
+ * (an odd k from 11 on, and memory for a byte an entry and a quarter byte a base
+ * beside the index; a build in one range also keeps 16 bytes a window, where there
+ * is room, which make the lookups of indexed queries cheaper, and a filter of at
+ * most 32 MiB.  A call that lacks the memory these tables take gets it: they go,
+ * and calls on the index do without them until the next build);
  * groups whose result depends on an order of equal keys take the hit path.
  * Without the tables, passes whose windows average at least 6 hits and that
  * hold at least two queries per SM take the sorted emission, others emit and

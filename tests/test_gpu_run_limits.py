@@ -199,3 +199,23 @@ def test_open_groups_of_many_rows(gpu, oracle_mod):
         gpu.set_run_limit("spare_pieces", None)
     assert rows.tobytes() == hits
     assert overlap_tuples_gpu(rows) == exp
+
+
+@pytest.mark.parametrize("k", [5, 7, 9, 11])
+def test_least_k(gpu, oracle_mod, k):
+    """k-mers shorter than 11 are chained hit by hit."""
+    from cuflye_gb300 import synth
+    from cuflye_gb300.backend import OverlapParams
+    wl = synth.small_overlap_case(6, genome_len=2_000, coverage=6.0, sub=0.01, ins=0.002,
+                                  dele=0.002)
+    params = dict(wl.params, kmer_size=k, min_overlap=1000)
+    p = OverlapParams.make(**params)
+    oracle_mod.set_stable(False)
+    idx, batch = oracle_index(oracle_mod, wl.reads, k, 1, 400)
+    exp = oracle_mod.overlaps(idx, batch, oracle_mod.default_params(**params))
+    gpu.build_index(wl.reads, k, 1, 400)
+    rows = gpu.overlaps(wl.reads, p)
+    sorted_bytes = gpu.last_timing()[1][1]
+    assert overlap_tuples_gpu(rows) == overlap_tuples_oracle(exp)
+    assert rows.tobytes() == _rows(gpu, wl.reads, p)
+    assert (sorted_bytes < gpu.last_timing()[1][1]) == (k >= 11)
