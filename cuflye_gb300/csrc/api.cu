@@ -1275,14 +1275,16 @@ void run_hits(cuflye_ctx* c, PassState& ps, bool want_kmers, uint64_t bytes_per_
     sync(c);
     uint32_t m = 0;
     while (m < nq && qoff[m + 1] <= hit_limit) ++m;
-    if (m == 0 && qoff[1] <= fits) m = 1;  // a first query beyond the held buffers
+    // a first query beyond the held buffers, or beyond what other passes left
+    // beside theirs: tried by itself
+    if (m == 0 && qoff[1] <= free_b / bytes_per_hit) m = 1;
     if (m == 0)
       throw Error(CUFLYE_ERR_BUDGET,
                   "device memory budget exceeded: query " +
                       std::to_string(ps.qinfo_h[0].signed_id) + " has " +
                       std::to_string(qoff[1]) + " hits needing " +
                       std::to_string(qoff[1] * bytes_per_hit) + " bytes; " +
-                      std::to_string(avail) + " available");
+                      std::to_string(free_b) + " available");
     ps.nq = m;
     ps.nhits = qoff[m];
     ps.nwin = win_off[m];
@@ -1383,7 +1385,7 @@ void run_runs(cuflye_ctx* c, PassState& ps) {
     sync(c);
     uint32_t m = 0;
     while (m < nq && qoff[m + 1] <= run_limit) ++m;
-    if (m == 0 && qoff[1] <= fits) m = 1;
+    if (m == 0 && qoff[1] <= free_b / kRunBytes) m = 1;
     if (m == 0) {
       ps.nq = 1;
       throw Error(CUFLYE_ERR_BUDGET, "device memory budget exceeded: a query's runs");
@@ -2394,6 +2396,7 @@ void for_each_pass(cuflye_ctx* c, const Queries& Q, bool kmers, uint64_t bytes_p
   size_t step = full;
   double upw = 0;  // units (hits or runs) per window of the previous pass
   bool hit_path = !runs;
+  size_t cleaned = Q.n;  // the query from which a pass has run without left buffers
   while (q0 < Q.n) {
     const bool by_runs = !hit_path;
     size_t q1 = run_end(c, Q, q0, std::min(Q.n, q0 + step), by_runs ? kRunBytes : bytes_per_hit,
@@ -2417,10 +2420,17 @@ void for_each_pass(cuflye_ctx* c, const Queries& Q, bool kmers, uint64_t bytes_p
       if (e.code != CUFLYE_ERR_BUDGET) throw;
       sync(c);
       if (!by_runs && (ps.nq <= 1 || !counted)) {
-        // one query does not fit (the counting takes as many as do)
-        if (!give_back(c, hold)) throw;
+        // one query does not fit (the counting takes as many as do): once more
+        // without what earlier passes left, then without the index's extra tables
+        if (cleaned != q0) {
+          cleaned = q0;
+          release_scratch(c);
+        } else if (give_back(c, hold)) {
+          runs = false;
+        } else {
+          throw;
+        }
         ++c->pass_retries;
-        runs = false;
         continue;
       }
       // the failed body's buffers go, so that half the queries find room

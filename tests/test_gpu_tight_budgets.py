@@ -140,3 +140,35 @@ def test_other_calls_get_the_tables_room(built_lib, mode):
             assert "BUDGET" in str(e), e
             assert not admitted, (admitted[0], mib)
     assert admitted
+
+
+def test_run_path_admits_what_the_hit_path_does(built_lib):
+    """Reads of a tandem array under every budget around what they need: where the
+    hit path gives the rows, so does the run path, twice in a row."""
+    from cuflye_gb300 import synth
+    from cuflye_gb300.backend import CudaBackend, CuflyeError, OverlapParams
+    rng = np.random.default_rng(217)
+    unit = synth.random_genome(rng, 200)
+    genome = np.concatenate([synth.random_genome(rng, 2000)] + [unit] * 4 +
+                            [synth.random_genome(rng, 2000)])
+    seqs = []
+    for i in range(7):
+        a, b = int(rng.integers(0, 1900)), int(rng.integers(2900, len(genome)))
+        s = synth.mutate(rng, genome[a:b], 0.01, 0.003, 0.003)
+        seqs.append((synth.revcomp(s) if i % 2 else s).tobytes())
+    reads = synth.ReadSet.from_strings(np.arange(1, 8), seqs)
+    p = OverlapParams.make(**dict(synth.OVERLAP_PARAMS, kmer_size=17, min_overlap=100))
+    got, rows = {}, set()
+    for kib in range(2500, 8000, 30):
+        for mode in (0, 1):
+            try:
+                with CudaBackend(device=0, memory_budget_bytes=kib << 10) as be:
+                    be.build_index(reads, 17, 1, 3000)
+                    be.set_sorted_emission(mode)
+                    rows |= {be.overlaps(reads, p).tobytes() for _ in range(2)}
+                got[kib, mode] = True
+            except CuflyeError as e:
+                assert "udget" in str(e), e
+                got[kib, mode] = False
+        assert got[kib, 1] or not got[kib, 0], kib
+    assert len(rows) == 1 and not all(got.values())
