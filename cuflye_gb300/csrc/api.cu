@@ -2074,8 +2074,7 @@ uint64_t chain_open_groups(cuflye_ctx* c, PassState& ps, const RunTables& t, uin
 }
 
 // Chaining of the pass's runs (run_runs): sort, groups, pieces, DP and
-// backtrack over runs.  Groups left open take the hit path with their own hits,
-// queries left to it run through it whole.
+// backtrack over runs.  Groups left open take the hit path with their own hits.
 ChainRows chain_runs(cuflye_ctx* c, PassState& ps, const ChainParams& cp) {
   cudaStream_t st = c->stream;
   const uint64_t NR = ps.units;

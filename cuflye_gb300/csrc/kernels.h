@@ -51,11 +51,12 @@ struct SortTasks {
   // final order: it is dropped (left as it is) and not listed as a task.
   const uint64_t* prune_keys = nullptr;
   const uint32_t* prune_off = nullptr;
-  // Side streams (optional): the whole-segment sorts (tiny, warp and CTA
-  // segments) run on `side` beside the global phase, and the heap ranges on
-  // `side2` beside the final tasks once the global phase is done.  They all
-  // sort disjoint element ranges, and each ends with the serial chain of its
-  // slowest range, so their tails overlap instead of adding up.  fork and
+  // Side streams (optional): the whole-segment sorts run beside the global
+  // phase, tiny and warp segments on `side`, CTA segments on `side2`, where the
+  // heap ranges follow them once the global phase is done, beside the final tasks
+  // (a heap takes a whole SM's shared memory, so it waits for the CTA segments on
+  // any stream).  They all sort disjoint element ranges, and each ends with the
+  // serial chain of its slowest range, so their tails overlap instead of adding up.  fork and
   // rounds_done order the side streams after the call's stream; the call
   // returns with its stream waiting for both (join, join2).  Null:
   // everything on the call's stream.

@@ -44,10 +44,6 @@ namespace {
 
 constexpr int kWarpsPerBlock = 8;
 
-__device__ __forceinline__ int run_class(uint32_t npieces) {
-  return npieces > 1024 ? 0 : npieces > 256 ? 1 : npieces > 64 ? 2 : npieces > 16 ? 3 : 4;
-}
-
 __device__ __forceinline__ void list_group(const RunTables& t, uint32_t g, uint32_t npieces) {
   const int c = run_class(npieces);
   t.lists[c * t.max_groups + atomicAdd(t.counts + kRcList + c, 1u)] = g;

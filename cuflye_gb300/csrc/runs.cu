@@ -18,12 +18,13 @@
 // 2.0 ms, groups 51 -> 3.9 ms, DP 50 -> 2.1 ms, backtrack 27 -> 3.3 ms against
 // writing, sorting and chaining every hit (the hit path, which remains for what
 // the run path leaves open and for indexes without its tables).  At 6 % error (3
-// Mb genome, 30x ONT reads: 4.7e8 hits in 59e6 runs) 50 -> 8.6 ms.  One read:
-// 1.0 -> 0.24 ms, its groups' serial scans being as many times shorter as its
-// runs are long.
+// Mb genome, 30x ONT reads: 4.7e8 hits in 59e6 runs) 50 -> 8.6 ms without open
+// groups, 11 to 20 with them.  One read: 1.0 -> 0.24 ms, its groups' serial scans
+// being as many times shorter as its runs are long.
 //
 // Needs an odd k: an even k has k-mers equal to their own reverse complement,
-// stored on one strand only, so that a run on the other strand has holes.
+// stored on one strand only, so that a run on the other strand has holes.  Short
+// k-mers (below kRunLeastK in api.cu) stay with the hit path, which is faster there.
 #include <algorithm>
 #include <climits>
 #include <cstdint>
@@ -764,10 +765,6 @@ __device__ __forceinline__ int32_t run_length(const RunTables& t, uint64_t qbase
     }
   }
   return min(m + 1, most);
-}
-
-__device__ __forceinline__ int run_class(uint32_t npieces) {
-  return npieces > 1024 ? 0 : npieces > 256 ? 1 : npieces > 64 ? 2 : npieces > 16 ? 3 : 4;
 }
 
 // Pieces of a group whose n runs (a, b, l by lane, from run i on) follow one

@@ -42,6 +42,11 @@ struct RunGroup {
 // Length classes of the surviving groups, longest first; list c holds the
 // groups of class c at lists[c * cap ..].
 constexpr int kRunClasses = 5;
+#ifdef __CUDACC__
+__device__ __forceinline__ int run_class(uint32_t npieces) {
+  return npieces > 1024 ? 0 : npieces > 256 ? 1 : npieces > 64 ? 2 : npieces > 16 ? 3 : 4;
+}
+#endif
 
 // Device counters of a pass (u32 words, zeroed by the caller).
 enum : int {
@@ -51,7 +56,7 @@ enum : int {
   kRcExt = kRcOpen + 1,               // surviving ext-axis groups
   kRcPool = kRcExt + 1,               // rows in the pool
   kRcWork = kRcPool + 1,              // 5: work counters
-  kRcWords = kRcWork + 6,             // (an even number)
+  kRcWords = kRcWork + 6,             // one more, for an even number
 };
 
 struct RunTables {
@@ -115,8 +120,8 @@ cudaError_t runs_emit(const DeviceIndex& idx, const QueryBatch& q, const uint4* 
                       cudaStream_t s);
 
 // The runs of every query of up to on_chip (kRunSortCap or kRunSortLarge) runs
-// sorted by ext id, in place and stable (longer ones come sorted, by match_radix), and the groups of each
-// query.  longest, list, list_count: from runs_query_offsets.  work: two
+// sorted by ext id, in place and stable (longer ones come sorted, by match_radix),
+// and the groups of each query.  longest, list, list_count: from runs_query_offsets.  work: two
 // counters, zeroed by the caller.
 constexpr uint32_t kRunSortCap = 4096, kRunSortLarge = 16384;
 cudaError_t runs_sort(const uint64_t* q_off, uint32_t nq, uint64_t longest, uint32_t on_chip,
@@ -168,7 +173,6 @@ cudaError_t runs_expand(const RunTables& t, const OpenBatch& o, uint64_t* keys, 
 cudaError_t runs_append_rows(const OverlapRow* from, const uint32_t* nfrom, const uint32_t* list,
                              OverlapRow* pool, uint64_t pool_cap, uint32_t* pool_count,
                              DeviceStatus* st, int num_sms, cudaStream_t s);
-// group_rows[list[i]] = rows[i].
 // Open groups whose flags hold kRunFirst, once their hits are in Flye's order
 // (keys, vals, groups: a batch's hits as chain_groups sorts them): their element
 // 0 is set, their flags are cleared, and they are listed for runs_dp and
@@ -180,6 +184,7 @@ cudaError_t runs_settle_first(const RunTables& t, const OpenBatch& o, const uint
 // their number into *count (zeroed by the caller).
 cudaError_t runs_unsettled(const RunTables& t, const OpenBatch& o, uint32_t* dp_list,
                            uint32_t* count, cudaStream_t s);
+// group_rows[open_list[i]] = rows[i], for the groups that are not settled.
 cudaError_t runs_fold_rows(const RunTables& t, const uint32_t* open_list, uint32_t nopen,
                            const uint32_t* rows, uint32_t* group_rows, cudaStream_t s);
 // Pool rows to their places.
