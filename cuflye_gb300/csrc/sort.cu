@@ -45,9 +45,16 @@ constexpr uint32_t kWarpSeg = 2048;   // segments up to this size: warp kernel
 // 611 of 3273, whose CTAs are busy, stay as they are (.84; .89 with kWarpSegFew).
 // The segments' own number and lengths decide, which a call with its list on the
 // device does not know: between the two bounds they form a class of their own, and
-// both kernels look at the counts (few_segments).
+// both kernels ask for the rule (few_segments), which the device then finds.
 constexpr uint32_t kFewPerSm = 2, kFewMean = 1024, kWarpSegFew = 512;
 constexpr int kMiddleCount = 10, kElemCount = 12;  // words of counts: middle class; elements (64 bits)
+
+// The rule, where the host knows it (nseg_dev null): few.
+struct FewRule {
+  uint32_t nseg, most;
+  const uint32_t* nseg_dev;
+  bool few;
+};
 constexpr int kWarpSegWarps = 6;      // warps per CTA in the warp kernel
 constexpr int kMaxWarpTasks = 256;    // warp subtrees per CTA task (<= 2 per partition)
 
@@ -606,12 +613,14 @@ __global__ void classify_segments(const uint64_t* __restrict__ begin,
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   uint64_t n = 0;
   if (s < nseg && !(nseg_dev && s >= *nseg_dev)) n = end[s] - begin[s];
-  uint64_t sum = n;
+  if (nseg_dev) {
+    uint64_t sum = n;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
-  if ((threadIdx.x & 31) == 0 && sum)
-    atomicAdd(reinterpret_cast<unsigned long long*>(counts + kElemCount),
-              static_cast<unsigned long long>(sum));
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
+    if ((threadIdx.x & 31) == 0 && sum)
+      atomicAdd(reinterpret_cast<unsigned long long*>(counts + kElemCount),
+                static_cast<unsigned long long>(sum));
+  }
   if (n <= 1) return;
   if (n > kWarpSegFew && n <= kWarpSeg) {
     lists[2 * static_cast<size_t>(nseg) - 1 - atomicAdd(&counts[kMiddleCount], 1u)] = s;
@@ -622,11 +631,11 @@ __global__ void classify_segments(const uint64_t* __restrict__ begin,
 }
 
 // Whether CTAs take the middle class: few segments, or short ones.
-__device__ __forceinline__ bool few_segments(const uint32_t* counts, uint32_t nseg,
-                                             const uint32_t* nseg_dev, uint32_t few) {
-  const uint32_t n = nseg_dev ? min(nseg, *nseg_dev) : nseg;
-  return n <= few || *reinterpret_cast<const uint64_t*>(counts + kElemCount) <=
-                         static_cast<uint64_t>(kFewMean) * n;
+__device__ __forceinline__ bool few_segments(const uint32_t* counts, const FewRule& r) {
+  if (!r.nseg_dev) return r.few;
+  const uint32_t n = min(r.nseg, *r.nseg_dev);
+  return n <= r.most || *reinterpret_cast<const uint64_t*>(counts + kElemCount) <=
+                            static_cast<uint64_t>(kFewMean) * n;
 }
 
 __global__ void sort_tiny(uint64_t* K, uint32_t* V, const uint64_t* __restrict__ begin,
@@ -653,17 +662,17 @@ struct WarpSlice {
 // One warp per segment of up to kWarpSeg elements.
 __global__ void __launch_bounds__(kWarpSegWarps * 32) sort_warp(
     uint64_t* K, uint32_t* V, const uint64_t* __restrict__ begin,
-    const uint64_t* __restrict__ end, uint32_t nseg, const uint32_t* __restrict__ nseg_dev,
-    uint32_t few, const uint32_t* __restrict__ list, const uint32_t* __restrict__ counts) {
+    const uint64_t* __restrict__ end, FewRule rule, const uint32_t* __restrict__ list,
+    const uint32_t* __restrict__ counts) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   WarpSlice& ws = reinterpret_cast<WarpSlice*>(smem_raw)[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const uint32_t low = counts[1];
   const uint32_t cnt =
-      low + (few_segments(counts, nseg, nseg_dev, few) ? 0u : counts[kMiddleCount]);
+      low + (few_segments(counts, rule) ? 0u : counts[kMiddleCount]);
   const uint32_t nwarps = gridDim.x * kWarpSegWarps;
   for (uint32_t li = blockIdx.x * kWarpSegWarps + (threadIdx.x >> 5); li < cnt; li += nwarps) {
-    const uint32_t s = list[li < low ? li : nseg - 1 - (li - low)];
+    const uint32_t s = list[li < low ? li : rule.nseg - 1 - (li - low)];
     const uint64_t b = begin[s];
     const uint32_t n = static_cast<uint32_t>(end[s] - b);
     for (uint32_t i = lane; i < n; i += 32) {
@@ -683,16 +692,13 @@ __global__ void __launch_bounds__(kWarpSegWarps * 32) sort_warp(
 __global__ void __launch_bounds__(kBlock, 3) sort_cta(uint64_t* K, uint32_t* V,
                                                    const uint64_t* __restrict__ begin,
                                                    const uint64_t* __restrict__ end,
-                                                   uint32_t nseg,
-                                                   const uint32_t* __restrict__ nseg_dev,
-                                                   uint32_t few,
+                                                   FewRule rule,
                                                    const uint32_t* __restrict__ lists,
                                                    const uint32_t* __restrict__ counts) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   CtaSmem& sm = *reinterpret_cast<CtaSmem*>(smem_raw);
-  const uint32_t high = counts[2];
-  const uint32_t cnt =
-      high + (few_segments(counts, nseg, nseg_dev, few) ? counts[kMiddleCount] : 0u);
+  const uint32_t high = counts[2], nseg = rule.nseg;
+  const uint32_t cnt = high + (few_segments(counts, rule) ? counts[kMiddleCount] : 0u);
   for (uint32_t i = blockIdx.x; i < cnt; i += gridDim.x) {
     const uint32_t s = i < high ? lists[2 * static_cast<size_t>(nseg) + i]
                                 : lists[2 * static_cast<size_t>(nseg) - 1 - (i - high)];
@@ -1684,7 +1690,9 @@ cudaError_t segmented_std_sort(uint64_t* keys, uint32_t* vals, uint32_t* lscratc
   cudaStream_t side2 = split ? tasks.side2 : stream;
   cudaMemsetAsync(counts, 0, 16 * sizeof(uint32_t), stream);
   count_launch();
-  const uint32_t few = kFewPerSm * static_cast<uint32_t>(num_sms);
+  const uint32_t most = kFewPerSm * static_cast<uint32_t>(num_sms);
+  const FewRule rule{nseg, most, nseg_dev,
+                     nseg <= most || tasks.nelems <= static_cast<uint64_t>(kFewMean) * nseg};
   classify_segments<<<(nseg + 255) / 256, 256, 0, stream>>>(begin, end, nseg, nseg_dev, lists,
                                                             counts);
   if (split) {
@@ -1697,10 +1705,10 @@ cudaError_t segmented_std_sort(uint64_t* keys, uint32_t* vals, uint32_t* lscratc
   sort_tiny<<<num_sms * 4, 128, 0, side>>>(keys, vals, begin, end, lists, counts);
   count_launch();
   sort_warp<<<num_sms, kWarpSegWarps * 32, sizeof(WarpSlice) * kWarpSegWarps, side>>>(
-      keys, vals, begin, end, nseg, nseg_dev, few, lists + nseg, counts);
+      keys, vals, begin, end, rule, lists + nseg, counts);
   count_launch();
-  sort_cta<<<num_sms * 3, kBlock, sizeof(CtaSmem), side2>>>(keys, vals, begin, end, nseg, nseg_dev,
-                                                            few, lists, counts);
+  sort_cta<<<num_sms * 3, kBlock, sizeof(CtaSmem), side2>>>(keys, vals, begin, end, rule, lists,
+                                                            counts);
   if (tasks.nelems > kCap) {
     // global phase in rounds; the host looks at the next round's list after
     // rounds 0, 1, 3, 7, ... and stops when it is empty (every range's budget
