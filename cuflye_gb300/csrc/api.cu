@@ -516,9 +516,10 @@ uint64_t table_capacity(uint64_t entries) { return std::max<uint64_t>(16, 2 * en
 
 // Least k of the run path.  Short k-mers match anywhere: most hits are runs of their
 // own, and most groups repeat positions and are left open, so that the hit path
-// chains them after all.  Calls of 20 to 100 reads, run path against hit path: k = 5
-// 39.8 / 13.8 ms, 7 39.4 / 23.0, 9 10.7 / 8.1 and 24.7 / 18.8, 11 8.0 / 8.5 and
-// 10.3 / 10.6, 13 3.7 / 5.0.
+// chains them after all.  Run path against hits emitted and sorted: k = 5 39.8 / 13.8
+// ms (20 reads) and 1,959 / 1,139 (400), 7 39.4 / 23.0 and 512 / 301, 9 10.7 / 8.1,
+// 24.7 / 18.8 and 172 / 140 (800), 11 8.0 / 8.5, 10.3 / 10.6 and 4.2 / 6.6 (400), 13
+// 3.7 / 5.0.
 constexpr int kRunLeastK = 11;
 
 // The run path's byte an entry (the bases around its k-mer), or null.  Kept for
@@ -1308,9 +1309,12 @@ void run_hits(cuflye_ctx* c, PassState& ps, bool want_kmers, uint64_t bytes_per_
   // sparse hits (reads against a genome or a graph) or of a few queries (the
   // one-read path) is cheaper to emit and sort.
   // A call whose passes overflowed the dictionary twice (queries hitting
-  // more targets than it holds) emits the rest in generation order.
+  // more targets than it holds) emits the rest in generation order, and so do short
+  // k-mers: nearly every query lists a target twice in some bucket there, and is
+  // sorted all the same (k = 9, 250 to 800 reads: 36 to 255 ms, 20 to 140 so).
   ps.emitted = !(fused && (c->sorted_emission == 2 ||
-                           (ps.nhits >= kSortedEmissionMinHitsPerWindow * ps.nwin &&
+                           (c->idx.k >= kRunLeastK &&
+                            ps.nhits >= kSortedEmissionMinHitsPerWindow * ps.nwin &&
                             ps.nq >= 2ull * static_cast<uint64_t>(c->num_sms) &&
                             c->emission_fallbacks < 2)));
   if (ps.emitted) emit_generation_order(c, ps);

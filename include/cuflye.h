@@ -222,8 +222,8 @@ cuflye_status cuflye_set_batch_queries(cuflye_ctx* ctx, size_t queries_per_pass)
  * most 32 MiB.  A call that lacks the memory these tables take gets it: they go,
  * and calls on the index do without them until the next build);
  * groups whose result depends on an order of equal keys take the hit path.
- * Without the tables, passes whose windows average at least 6 hits and that
- * hold at least two queries per SM take the sorted emission, others emit and
+ * Without the tables, passes of k >= 11 whose windows average at least 6 hits and
+ * that hold at least two queries per SM take the sorted emission, others emit and
  * sort.  2: the sorted emission for every pass (each query's hits written
  * straight into the order of Flye's KmerMatch sort, one block per query, with
  * most target groups' prefilter decided on the way).  0: hits written in
