@@ -159,7 +159,7 @@ def test_run_path_admits_what_the_hit_path_does(built_lib):
     reads = synth.ReadSet.from_strings(np.arange(1, 8), seqs)
     p = OverlapParams.make(**dict(synth.OVERLAP_PARAMS, kmer_size=17, min_overlap=100))
     got, rows = {}, set()
-    for kib in range(2500, 8000, 30):
+    for kib in range(2500, 8000, 90):
         for mode in (0, 1):
             try:
                 with CudaBackend(device=0, memory_budget_bytes=kib << 10) as be:
@@ -172,3 +172,60 @@ def test_run_path_admits_what_the_hit_path_does(built_lib):
                 got[kib, mode] = False
         assert got[kib, 1] or not got[kib, 0], kib
     assert len(rows) == 1 and not all(got.values())
+
+
+def test_tables_go_while_others_read_the_index(built_lib):
+    """Two borrowing contexts and a server in full use while the owner's query takes
+    the tables: every call's rows stay the same."""
+    import threading
+
+    from cuflye_gb300 import synth
+    from cuflye_gb300.backend import CudaBackend, CudaServer, CuflyeError, OverlapParams
+    wl = synth.small_overlap_case(7, genome_len=60_000, sub=0.002, ins=0.001, dele=0.001)
+    unit = synth.random_genome(np.random.default_rng(1), 3000)
+    seqs = [wl.reads.seq(i) for i in range(wl.reads.n)] + [unit.tobytes()] * 300
+    targets = synth.ReadSet.from_strings(np.arange(1, len(seqs) + 1), seqs)
+    big = synth.ReadSet.from_strings(np.array([9000]), [np.resize(unit, 9000).tobytes()])
+    p = OverlapParams.make(**dict(wl.params, kmer_size=15))
+    parts = [wl.reads.subset(np.arange(i, min(i + 9, wl.reads.n)))
+             for i in range(0, wl.reads.n, 9)]
+    with CudaBackend(device=0, memory_budget_bytes=0) as be:
+        be.build_index(targets, 15, 1, 2000)
+        want = [be.overlaps(q, p).tobytes() for q in parts]
+        want_big = be.candidates(big)[0].tobytes()
+    gone = 0
+    for mib in range(140, 260, 8):
+        with CudaBackend(device=0, memory_budget_bytes=mib << 20) as be:
+            be.build_index(targets, 15, 1, 2000)
+            be.trim()
+            held = be.memory_stats()[0]
+            with _shared(be, 128 << 20) as a, _shared(be, 128 << 20) as b, \
+                    CudaServer(be, p, workers=1) as srv:
+                wrong, started = [], threading.Barrier(4)
+
+                def work(call):
+                    started.wait()
+                    for _ in range(6):
+                        for q, w in zip(parts, want):
+                            try:
+                                if call(q).tobytes() != w:
+                                    wrong.append("rows")
+                            except CuflyeError as e:
+                                wrong.append(str(e))
+
+                calls = [lambda q: a.overlaps(q, p), lambda q: b.overlaps(q, p),
+                         lambda q: srv.poll(srv.submit(q), -1)]
+                threads = [threading.Thread(target=work, args=(c,)) for c in calls]
+                for t in threads:
+                    t.start()
+                started.wait()
+                try:
+                    assert be.candidates(big)[0].tobytes() == want_big
+                except CuflyeError as e:
+                    assert "udget" in str(e), e  # too small a budget for the query
+                for t in threads:
+                    t.join()
+                assert not wrong, wrong[:3]
+                be.trim()
+                gone += be.memory_stats()[0] < held
+    assert gone
